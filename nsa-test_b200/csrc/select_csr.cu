@@ -12,14 +12,27 @@
 
 namespace nsa {
 
-constexpr int kChunk = 128;  // queries per histogram chunk (one warp orders the entries of a chunk)
+constexpr int kChunk = 128;      // queries per histogram chunk
+constexpr int kFillWarps = 8;    // warps ordering the entries of a chunk (one when the counters of eight do not fit)
 
 struct CsrArgs {
   const int* indices;
   int64_t sidx[4];
-  int B, G, Tq, Tkv, nslots, lprime, nblk, nchunks, causal, q0;
-  int *hist, *off, *csr_t;
+  int B, G, Tq, Tkv, nslots, lprime, nblk, nchunks, causal, q0, slots_pad;
+  int *hist, *off, *csr_t;       // hist: [BG][nchunks + 1][nblk], the last row holds the totals
 };
+
+// Block id of the (query, slot) pair a lane covers: lanes hold `slots_pad` slots of 32 / slots_pad consecutive queries.
+// -1 when the slot contributes nothing (the rules of slot_block); a repeated id is found by matching the lanes of one query.
+__device__ __forceinline__ int lane_block(const CsrArgs& a, int b, int g, int t, int t1, int lane) {
+  const int s = lane & (a.slots_pad - 1);
+  int id = -1;
+  if (t < t1 && s < a.nslots) id = a.indices[b * a.sidx[0] + g * a.sidx[1] + (int64_t)t * a.sidx[2] + s * a.sidx[3]];
+  const bool in = id >= 0 && (int64_t)id * a.lprime < a.Tkv && !(a.causal && (int64_t)id * a.lprime > a.q0 + t);
+  const int key = in ? id * 32 + (lane & ~(a.slots_pad - 1)) : -1 - lane;   // id < 2^26: checked by the host
+  const unsigned same = __match_any_sync(0xffffffffu, key);
+  return in && (same & ((1u << lane) - 1u)) == 0 ? id : -1;
+}
 
 __global__ void csr_count(const CsrArgs a) {
   extern __shared__ int sh[];
@@ -27,80 +40,104 @@ __global__ void csr_count(const CsrArgs a) {
   for (int i = threadIdx.x; i < a.nblk; i += blockDim.x) sh[i] = 0;
   __syncthreads();
   const int t0 = c * kChunk, t1 = min(a.Tq, t0 + kChunk);
-  for (int e = threadIdx.x; e < (t1 - t0) * a.nslots; e += blockDim.x) {
-    const int t = t0 + e / a.nslots, s = e % a.nslots;
-    const int* row = a.indices + b * a.sidx[0] + g * a.sidx[1] + (int64_t)t * a.sidx[2];
-    const int id = slot_block(row, a.sidx[3], s, a.q0 + t, a.Tkv, a.lprime, a.causal);
+  const int lane = threadIdx.x & 31, qpw = 32 / a.slots_pad;
+  for (int tb = t0 + (threadIdx.x >> 5) * qpw; tb < t1; tb += (blockDim.x >> 5) * qpw) {
+    const int id = lane_block(a, b, g, tb + lane / a.slots_pad, t1, lane);
     if (id >= 0) atomicAdd(&sh[id], 1);
   }
   __syncthreads();
-  int* h = a.hist + ((int64_t)bg * a.nchunks + c) * a.nblk;
+  int* h = a.hist + ((int64_t)bg * (a.nchunks + 1) + c) * a.nblk;
   for (int i = threadIdx.x; i < a.nblk; i += blockDim.x) h[i] = sh[i];
 }
 
-// hist[bg][c][blk] becomes the count of entries of blk in chunks < c; off[bg][blk] the block's start.
+// hist[bg][c][blk] becomes the count of entries of blk in chunks < c; row nchunks the block's total.  32 columns per
+// thread block, 32 threads per column, each owning a run of chunks.
 __global__ void csr_scan(const CsrArgs a) {
-  __shared__ int part[1024];
-  const int bg = blockIdx.x, tid = threadIdx.x;
-  int* h = a.hist + (int64_t)bg * a.nchunks * a.nblk;
-  int* off = a.off + (int64_t)bg * (a.nblk + 1);
-  const int per = (a.nblk + 1023) / 1024;
-  const int lo = min(a.nblk, tid * per), hi = min(a.nblk, lo + per);
-  int mine = 0;
-  for (int blk = lo; blk < hi; ++blk) {
-    int run = 0;
-    for (int c = 0; c < a.nchunks; ++c) {
-      const int v = h[(int64_t)c * a.nblk + blk];
-      h[(int64_t)c * a.nblk + blk] = run;
-      run += v;
-    }
-    off[blk + 1] = run;  // totals for now
-    mine += run;
-  }
-  part[tid] = mine;
+  __shared__ int part[32][33];
+  const int bg = blockIdx.y, x = threadIdx.x, y = threadIdx.y, blk = blockIdx.x * 32 + x;
+  int* h = a.hist + (int64_t)bg * (a.nchunks + 1) * a.nblk + blk;
+  const int per = (a.nchunks + 31) / 32, lo = min(a.nchunks, y * per), hi = min(a.nchunks, lo + per);
+  int sum = 0;
+  if (blk < a.nblk)
+#pragma unroll 4
+    for (int c = lo; c < hi; ++c) sum += h[(int64_t)c * a.nblk];
+  part[y][x] = sum;
   __syncthreads();
-  if (tid == 0) {
-    int run = 0;
-    for (int i = 0; i < 1024; ++i) {
-      const int v = part[i];
-      part[i] = run;
-      run += v;
-    }
-    off[0] = 0;
-  }
-  __syncthreads();
-  int run = part[tid];
-  for (int blk = lo; blk < hi; ++blk) {
-    const int v = off[blk + 1];
+  int run = 0;
+  for (int i = 0; i < y; ++i) run += part[i][x];
+  if (blk >= a.nblk) return;
+  if (y == 31) h[(int64_t)a.nchunks * a.nblk] = run + sum;
+#pragma unroll 4
+  for (int c = lo; c < hi; ++c) {
+    const int v = h[(int64_t)c * a.nblk];
+    h[(int64_t)c * a.nblk] = run;
     run += v;
-    off[blk + 1] = run;  // inclusive end = next block's start
   }
 }
 
-// One warp per chunk walks its queries in order; lanes cover (query, slot) pairs so that a lower lane
-// is always an earlier query, and equal block ids inside a step are ranked by lane.
-__global__ void csr_fill(const CsrArgs a, int slots_pad) {
-  extern __shared__ int cur[];
-  const int c = blockIdx.x, bg = blockIdx.y, b = bg / a.G, g = bg % a.G, lane = threadIdx.x;
-  const int* h = a.hist + ((int64_t)bg * a.nchunks + c) * a.nblk;
-  const int* off = a.off + (int64_t)bg * (a.nblk + 1);
-  for (int i = lane; i < a.nblk; i += 32) cur[i] = off[i] + h[i];
-  __syncwarp();
-  int* out = a.csr_t + (int64_t)bg * a.Tq * a.nslots;
-  const int qpw = 32 / slots_pad;  // queries per warp step
-  const int t0 = c * kChunk, t1 = min(a.Tq, t0 + kChunk);
+// Ordered fill of one chunk.  Latency-bound (the chunk's 128 x nslots ids are 8 KB): one warp walking the whole chunk
+// needed 64 dependent steps of a few hundred cycles each, 47 us per launch at every size.  Each of W warps now orders its
+// own kChunk / W queries with byte counters of its own (an id occurs at most once per query, so a chunk holds at most
+// 128 of it), the counters are prefixed over the warps, and a second walk writes the entries.
+// Lanes cover (query, slot) pairs so that a lower lane is always an earlier query; equal ids of a step are ranked by lane.
+__global__ void csr_fill(const CsrArgs a) {
+  extern __shared__ int base[];                                    // [nblk] start of each block's entries of this chunk
+  const int W = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint8_t* cnt = reinterpret_cast<uint8_t*>(base + a.nblk);        // [W][nblk]
+  __shared__ int wsum[32];
+  const int c = blockIdx.x, bg = blockIdx.y, b = bg / a.G, g = bg % a.G;
+  const int* h = a.hist + ((int64_t)bg * (a.nchunks + 1) + c) * a.nblk;
+  const int* tot = a.hist + ((int64_t)bg * (a.nchunks + 1) + a.nchunks) * a.nblk;
+  // block starts: exclusive prefix of the totals, every thread owning a run of blocks
+  const int per = (a.nblk + blockDim.x - 1) / blockDim.x, lo = min(a.nblk, (int)threadIdx.x * per), hi = min(a.nblk, lo + per);
+  int mine = 0;
+  for (int i = lo; i < hi; ++i) mine += tot[i];
+  int run = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, run, o);
+    if (lane >= o) run += v;
+  }
+  if (lane == 31) wsum[warp] = run;
+  for (int i = threadIdx.x; i < W * a.nblk; i += blockDim.x) cnt[i] = 0;
+  __syncthreads();
+  run -= mine;
+  for (int w = 0; w < warp; ++w) run += wsum[w];
+  int* off = a.off + (int64_t)bg * (a.nblk + 1);
+  if (c == 0 && threadIdx.x == 0) off[0] = 0;
+  for (int i = lo; i < hi; ++i) {
+    base[i] = run + h[i];
+    run += tot[i];
+    if (c == 0) off[i + 1] = run;
+  }
+  const int qpw = 32 / a.slots_pad, per_warp = kChunk / W;
+  const int t0 = c * kChunk + warp * per_warp, t1 = min(a.Tq, t0 + per_warp);
+  uint8_t* my = cnt + warp * a.nblk;
   for (int tb = t0; tb < t1; tb += qpw) {
-    const int t = tb + lane / slots_pad, s = lane % slots_pad;
-    int id = -1;
-    if (t < t1 && s < a.nslots) {
-      const int* row = a.indices + b * a.sidx[0] + g * a.sidx[1] + (int64_t)t * a.sidx[2];
-      id = slot_block(row, a.sidx[3], s, a.q0 + t, a.Tkv, a.lprime, a.causal);
+    const int id = lane_block(a, b, g, tb + lane / a.slots_pad, t1, lane);
+    const unsigned peers = __match_any_sync(0xffffffffu, id >= 0 ? id : -1 - lane);
+    if (id >= 0 && (peers & ((1u << lane) - 1u)) == 0) my[id] += __popc(peers);
+    __syncwarp();
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < a.nblk; i += blockDim.x) {
+    int before = 0;
+    for (int w = 0; w < W; ++w) {
+      const int v = cnt[w * a.nblk + i];
+      cnt[w * a.nblk + i] = (uint8_t)before;
+      before += v;
     }
+  }
+  __syncthreads();
+  int* out = a.csr_t + (int64_t)bg * a.Tq * a.nslots;
+  for (int tb = t0; tb < t1; tb += qpw) {
+    const int t = tb + lane / a.slots_pad, s = lane & (a.slots_pad - 1);
+    const int id = lane_block(a, b, g, t, t1, lane);
     const unsigned peers = __match_any_sync(0xffffffffu, id >= 0 ? id : -1 - lane);
     const int rank = __popc(peers & ((1u << lane) - 1u));
-    if (id >= 0) out[cur[id] + rank] = t | (s << 24);  // query position and its slot
+    if (id >= 0) out[base[id] + my[id] + rank] = t | (s << 24);  // query position and its slot
     __syncwarp();
-    if (id >= 0 && rank == 0) cur[id] += __popc(peers);
+    if (id >= 0 && rank == 0) my[id] += __popc(peers);
     __syncwarp();
   }
 }
@@ -113,7 +150,7 @@ static void csr_layout(int B, int G, int Tq, int Tkv, int nslots, int lprime, in
   *nchunks = (Tq + kChunk - 1) / kChunk;
   const size_t BG = (size_t)B * G;
   *o_hist = 0;
-  *o_off = align_up(*o_hist + BG * *nchunks * *nblk * sizeof(int));
+  *o_off = align_up(*o_hist + BG * (*nchunks + 1) * *nblk * sizeof(int));
   *o_t = align_up(*o_off + BG * (*nblk + 1) * sizeof(int));
   *total = align_up(*o_t + BG * (size_t)Tq * nslots * sizeof(int));
 }
@@ -143,20 +180,20 @@ int build_slc_csr(const int* indices, const int64_t* sidx, int B, int G, int Tq,
   a.hist = (int*)(w + o_hist);
   a.off = (int*)(w + o_off);
   a.csr_t = (int*)(w + o_t);
+  a.slots_pad = 1;
+  while (a.slots_pad < nslots) a.slots_pad *= 2;
   const size_t sm = (size_t)a.nblk * sizeof(int);
-  if (sm > 48 * 1024) {
-    cudaFuncSetAttribute(csr_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    cudaFuncSetAttribute(csr_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  }
+  const int W = (size_t)a.nblk * (sizeof(int) + kFillWarps) <= 200 * 1024 ? kFillWarps : 1;
+  const size_t sm_fill = (size_t)a.nblk * (sizeof(int) + W);
+  if (sm > 48 * 1024) cudaFuncSetAttribute(csr_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (sm_fill > 48 * 1024) cudaFuncSetAttribute(csr_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_fill);
   KernelTimer kt("slc_inverse_index", st);
   dim3 grid(a.nchunks, B * G);
   csr_count<<<grid, 256, sm, st>>>(a);
   if (int rc = check_launch("csr_count")) return rc;
-  csr_scan<<<B * G, 1024, 0, st>>>(a);
+  csr_scan<<<dim3((a.nblk + 31) / 32, B * G), dim3(32, 32), 0, st>>>(a);
   if (int rc = check_launch("csr_scan")) return rc;
-  int slots_pad = 1;
-  while (slots_pad < nslots) slots_pad *= 2;
-  csr_fill<<<grid, 32, sm, st>>>(a, slots_pad);
+  csr_fill<<<grid, 32 * W, sm_fill, st>>>(a);
   if (int rc = check_launch("csr_fill")) return rc;
   *csr_off = a.off;
   *csr_t = a.csr_t;
