@@ -26,7 +26,23 @@ namespace nsa {
 
 using namespace ptx;
 
-constexpr int kEntriesPerCta = 1024;  // inverse-index entries handled by one CTA
+// Each (batch, group)'s inverse index is cut into `nparts` equal ranges, one CTA each.  The grid (nparts x batch x group) is
+// a whole number of waves of the 148 SMs (one resident CTA per SM) with ranges of 1024 to 2048 entries, as long as there
+// is that much work: ranges of a fixed 1024 entries left a last wave of 108 of 256 CTAs at T = 4096 and ran 32 CTAs, 179 us,
+// on a chunk of 512 queries.  Longer ranges at large T save nothing: a block's K/V is 40 KB against 10 KB per entry.
+constexpr int kEntriesPerCta = 1024;
+constexpr int kSlcSms = 148;
+static int slc_nparts(int B, int G, int Tq, int nslots) {
+  const int64_t units = (int64_t)B * G * Tq * nslots;
+  const int64_t waves = units / ((int64_t)kSlcSms * kEntriesPerCta);
+  const int64_t n = (waves > 0 ? waves : 1) * kSlcSms / ((int64_t)B * G);
+  return (int)(n > 0 ? n : 1);
+}
+// entries per range: the same for the two product kernels and the reduction, from the index's own total (early queries
+// have fewer blocks than slots); a multiple of the `qpc` queries of an MMA tile
+__device__ __forceinline__ int slc_range(const int* off, int nblk, int nparts, int qpc) {
+  return ((off[nblk] + nparts - 1) / nparts + qpc - 1) / qpc * qpc;
+}
 constexpr float kLn2f = 0.6931471805599453f;
 constexpr float kLog2ef = 1.4426950408889634f;
 
@@ -138,8 +154,8 @@ slc_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
   const int bg = blockIdx.y, b = bg / p.G, g = bg % p.G;
   const int* off = p.csr_off + (int64_t)bg * (p.nblk + 1);
   const int* ent = p.csr_t + (int64_t)bg * p.Tq * p.nslots;
-  const int e0 = blockIdx.x * kEntriesPerCta;
   const int qpc = 128 / p.hpg;
+  const int per_cta = slc_range(off, p.nblk, gridDim.x, qpc), e0 = blockIdx.x * per_cta;
   // once any block has given up on a wait the device results are void: later blocks skip their work and end at once
   const bool has_work = e0 < off[p.nblk] && !(p.timeouts && *(volatile const int*)p.timeouts != 0);
 
@@ -168,7 +184,7 @@ slc_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
     // nothing to do for this CTA
   } else if (warp == 9) {
     // ------------------------------------------------------------ producer warp: K/V blocks and gathered Q rows, all by TMA
-    ChunkWalker w(off, p.nblk, e0, e0 + kEntriesPerCta, qpc);
+    ChunkWalker w(off, p.nblk, e0, e0 + per_cta, qpc);
     const int oob_row = p.B * p.H * p.Tq;
     const int oct0 = (b * p.H + g * p.hpg) >> 3;  // first head of the group, in units of 8 heads (rank-5 loads)
     bool ok = true;
@@ -222,7 +238,7 @@ slc_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
     constexpr uint32_t idS = idesc_bf16(128, 64, 0, 1);   // Q rows (K-major) x K block (MN-major: keys contiguous)
     constexpr uint32_t idO = idesc_bf16(128, DV, 0, 1);   // P (TMEM) x V block (MN-major: dv contiguous)
     const uint32_t sboQ = p.g5 ? (DK / 64) * 1024 : 1024, cbQ = p.g5 ? 1024 : 16384;  // Q tile: row-group / column-block strides
-    ChunkWalker w(off, p.nblk, e0, e0 + kEntriesPerCta, qpc);
+    ChunkWalker w(off, p.nblk, e0, e0 + per_cta, qpc);
     bool ok = true;
     int c = 0, kvidx = 0, ks_cur = 0, cur_blk = w.blk;
     auto issue_s = [&](int cc, int ks) -> bool {
@@ -290,7 +306,7 @@ slc_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
     uint8_t* stage = smem + SM::oStage + warp * 4096;
     const int boxrows = min(p.hpg, 32), nbox = 32 / boxrows;
     const int box_lane = (lane * boxrows) & 31;  // lane owning the first row of the box this lane would store
-    ChunkWalker w(off, p.nblk, e0, e0 + kEntriesPerCta, qpc);
+    ChunkWalker w(off, p.nblk, e0, e0 + per_cta, qpc);
     bool ok = true;
     if (grp == 1 && !w.done()) w.next();
     int entry_next = 0;
@@ -753,8 +769,8 @@ slc_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
   const int bg = blockIdx.y, b = bg / p.G, g = bg % p.G;
   const int* off = p.csr_off + (int64_t)bg * (p.nblk + 1);
   const int* ent = p.csr_t + (int64_t)bg * p.Tq * p.nslots;
-  const int e0 = blockIdx.x * kEntriesPerCta;
   const int qpc = 128 / p.hpg;
+  const int per_cta = slc_range(off, p.nblk, gridDim.x, qpc), e0 = blockIdx.x * per_cta;
   // once any block has given up on a wait the device results are void: later blocks skip their work and end at once
   const bool has_work = e0 < off[p.nblk] && !(p.timeouts && *(volatile const int*)p.timeouts != 0);
   const int nseg = gridDim.x + p.nblk;
@@ -798,7 +814,7 @@ slc_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
   } else if (!has_work) {
   } else if (warp == 9) {
     // producer warp: K/V block and gathered Q / dO rows by TMA (lane qi issues query qi)
-    ChunkWalker w(off, p.nblk, e0, e0 + kEntriesPerCta, qpc);
+    ChunkWalker w(off, p.nblk, e0, e0 + per_cta, qpc);
     const int oob_row = p.B * p.H * p.Tq;
     const int oct0 = (b * p.H + g * p.hpg) >> 3;  // first head of the group, in units of 8 heads (rank-5 loads)
     bool ok = true;
@@ -870,7 +886,7 @@ slc_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     const uint64_t dVk = smem_desc_sw128(smem_u32(sV), 16, 1024);
     const uint32_t sboQ = p.g5 ? (DK / 64) * 1024 : 1024, cbQ = p.g5 ? 1024 : 16384;  // Q tile: row-group / column-block strides
     const uint32_t sboO = p.g5 ? (DV / 64) * 1024 : 1024, cbO = p.g5 ? 1024 : 16384;  // dO tile
-    ChunkWalker w(off, p.nblk, e0, e0 + kEntriesPerCta, qpc);
+    ChunkWalker w(off, p.nblk, e0, e0 + per_cta, qpc);
     bool ok = true;
     int kvidx = 0;
     auto issue_s = [&](int cc) -> bool {  // S of chunk cc: its rows have landed, S / dP of the chunk before are in registers
@@ -943,7 +959,7 @@ slc_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     const uint64_t dSb = smem_desc_sw128(smem_u32(sdS), 16, 1024);
     const uint32_t sboQ = p.g5 ? (DK / 64) * 1024 : 1024, cbQ = p.g5 ? 1024 : 16384;
     const uint32_t sboO = p.g5 ? (DV / 64) * 1024 : 1024, cbO = p.g5 ? 1024 : 16384;
-    ChunkWalker w(off, p.nblk, e0, e0 + kEntriesPerCta, qpc);
+    ChunkWalker w(off, p.nblk, e0, e0 + per_cta, qpc);
     bool ok = true, fresh = true;      // fresh: the next accumulation starts a new segment
     int seg = 0, u = 0;
     for (int ch = 0; ok && !w.done(); ++ch) {
@@ -1000,7 +1016,7 @@ slc_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     const int r = warp4 * 32 + lane;
     const int half = warp4 >> 1, rr = r & 63;  // which 64-row half of the chunk this row is handed over in
     const uint32_t lane_base = (uint32_t)(warp4 * 32) << 16;
-    ChunkWalker w(off, p.nblk, e0, e0 + kEntriesPerCta, qpc);
+    ChunkWalker w(off, p.nblk, e0, e0 + per_cta, qpc);
     bool ok = true;
     int c = 0, last_blk = -1, seg = 0;
     auto flush = [&](int blk) -> bool {
@@ -1145,12 +1161,13 @@ slc_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
 // dK/dV of block `blk` += sum of its segment partials in segment order; a thread owns four consecutive columns of a row
 __global__ void slc_reduce_dkv_kernel(const float* __restrict__ dk_part, const float* __restrict__ dv_part,
                                       const int* __restrict__ csr_off, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
-                                      int G, int Tk, int nblk, int nparts, int DK, int DV, float scale) {
+                                      int G, int Tk, int nblk, int nparts, int qpc, int DK, int DV, float scale) {
   const int blk = blockIdx.x, bg = blockIdx.y;
   const int* off = csr_off + (int64_t)bg * (nblk + 1);
   const int lo = off[blk], hi = off[blk + 1];
   if (hi <= lo) return;
-  const int p_lo = lo / kEntriesPerCta, p_hi = (hi - 1) / kEntriesPerCta;
+  const int per_cta = slc_range(off, nblk, nparts, qpc);
+  const int p_lo = lo / per_cta, p_hi = (hi - 1) / per_cta;
   const int nseg = nparts + nblk;
   const int W4 = (DK + DV) / 4, DK4 = DK / 4;
   for (int i = threadIdx.x; i < 64 * W4; i += blockDim.x) {
@@ -1218,7 +1235,7 @@ static int launch_slc_fwd_t(const CUtensorMap& tk, const CUtensorMap& tv, const 
   auto kern = slc_fwd_kernel<DK, DV>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::kDynamic) != cudaSuccess)
     return fail(NSA_ERR_LAUNCH, "slc_fwd: cannot reserve shared memory");
-  const int nparts = (int)(((int64_t)p.Tq * p.nslots + kEntriesPerCta - 1) / kEntriesPerCta);
+  const int nparts = slc_nparts(p.B, p.G, p.Tq, p.nslots);
   {
     KernelTimer kt("slc_fwd", st);
     kern<<<dim3(nparts, p.B * p.G), 320, SM::kDynamic, st>>>(tk, tv, tqt, top, p);
@@ -1288,7 +1305,7 @@ void launch_bwd_prep(const void* o, const void* dout, const float* L, const floa
 static void slc_bwd_layout(int B, int H, int G, int Tq, int Tk, int dk, int dv, int nslots, int lprime, size_t* o_stat,
                            size_t* o_dq, size_t* o_dk, size_t* o_dv, size_t* o_qt, size_t* o_dot, size_t* total) {
   const size_t rows = (size_t)B * H * Tq;
-  const size_t nparts = ((size_t)Tq * nslots + kEntriesPerCta - 1) / kEntriesPerCta;
+  const size_t nparts = slc_nparts(B, G, Tq, nslots);
   const size_t nseg = nparts + (size_t)(Tk + 63) / 64;
   size_t o = al256(slc_csr_workspace_bytes(B, G, Tq, Tk, nslots, lprime));
   *o_stat = o; o += 2 * al256(rows * sizeof(float));
@@ -1310,7 +1327,7 @@ template <int DK, int DV>
 static int launch_slc_bwd_t(const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tqt, const CUtensorMap& tdot,
                             const SlcParams& p, const int* indices,
                             const int64_t* sidx, __nv_bfloat16* dq, const void* add0, const void* add1, cudaStream_t st) {
-  const int nparts = (int)(((int64_t)p.Tq * p.nslots + kEntriesPerCta - 1) / kEntriesPerCta);
+  const int nparts = slc_nparts(p.B, p.G, p.Tq, p.nslots);
   {
     auto kf = slc_bwd_fused_kernel<DK, DV>;
     if (cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, SlcBwdSmem<DK, DV>::kDynamic) != cudaSuccess)
@@ -1339,7 +1356,7 @@ static int launch_slc_bwd_t(const CUtensorMap& tk, const CUtensorMap& tv, const 
   if (int rc = check_launch("slc_combine_dq")) return rc;
   KernelTimer kt("slc_reduce_dkv", st);
   slc_reduce_dkv_kernel<<<dim3(p.nblk, p.B * p.G), 256, 0, st>>>(p.dk_part, p.dv_part, p.csr_off, p.dk_out, p.dv_out, p.G, p.Tk,
-                                                                 p.nblk, nparts, DK, DV, p.scale);
+                                                                 p.nblk, nparts, 128 / p.hpg, DK, DV, p.scale);
   return check_launch("slc_reduce_dkv");
 }
 
