@@ -227,6 +227,7 @@ class _BranchesAndMix(torch.autograd.Function):
         ctx.shared_win = (k_win.data_ptr() == k_slc.data_ptr() and v_win.data_ptr() == v_slc.data_ptr()
                           and k_win.shape == k_slc.shape and v_win.shape == v_slc.shape)
         ctx.mark_non_differentiable(gates, o_cmp, o_slc, o_win, indices)
+        ctx.set_materialize_grads(False)
         return out, gates, o_cmp, o_slc, o_win, indices
 
     @staticmethod
@@ -284,6 +285,7 @@ class _LayerC(torch.autograd.Function):
         ctx.desc, ctx.shared_kv = desc, shared_kv
         ctx.pdtypes = (gate_logits.dtype, pos_embed.dtype, w1.dtype, w2.dtype, b1 is not None, b2 is not None)
         ctx.mark_non_differentiable(saved)
+        ctx.set_materialize_grads(False)      # or every backward would be handed a zero-filled gradient of the whole context
         return out, saved
 
     @staticmethod
@@ -401,6 +403,7 @@ class _GateMix(torch.autograd.Function):
         ctx.save_for_backward(gates, o_cmp, o_slc, o_win)
         ctx.gate_mode, ctx.ldtype = gate_mode, logits.dtype
         ctx.mark_non_differentiable(gates)
+        ctx.set_materialize_grads(False)
         return out, gates
 
     @staticmethod
