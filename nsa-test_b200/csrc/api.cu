@@ -84,27 +84,30 @@ __global__ void add_dq_addends_kernel(T* __restrict__ dq, const T* __restrict__ 
   Elem<T>::st(dq + i, x);
 }
 
-// canonical contiguous layouts: q [B,H,T,dk], k [B,G,dk,Tk] (strides given as z,g,n,k), v [B,G,Tk,dv], o [B,H,T,dv]
-static bool canonical_fwd(const int64_t* s, int H, int G, int Tq, int Tk, int dk, int dv) {
+// canonical layouts: q [B,H,Tq,dk] and o [B,H,Tq,dv] contiguous; k [B,G,dk,Tk] (strides given as z,g,n,k) with gap-free rows
+// `k_ld` >= Tk elements apart, v [B,G,Tk,dv] with contiguous rows and groups `v_plane` apart: whole tensors, tensors padded
+// along time, and time slices of a longer key/value cache.  Strides of dimensions of extent 1 do not matter.
+static bool canonical_fwd(const int64_t* s, int B, int H, int G, int Tq, int Tk, int dk, int dv, KvLayout* kv) {
   const int64_t q[4] = {(int64_t)H * Tq * dk, (int64_t)Tq * dk, dk, 1};
-  const int64_t k[4] = {(int64_t)G * dk * Tk, (int64_t)dk * Tk, 1, Tk};
-  const int64_t v[4] = {(int64_t)G * Tk * dv, (int64_t)Tk * dv, dv, 1};
   const int64_t o[4] = {(int64_t)H * Tq * dv, (int64_t)Tq * dv, dv, 1};
   const int64_t lm[3] = {(int64_t)H * Tq, Tq, 1};
   for (int i = 0; i < 4; ++i)
-    if (s[i] != q[i] || s[4 + i] != k[i] || s[8 + i] != v[i] || s[12 + i] != o[i]) return false;
+    if (s[i] != q[i] || s[12 + i] != o[i]) return false;
   for (int i = 0; i < 3; ++i)
     if (s[16 + i] != lm[i] || s[19 + i] != lm[i]) return false;
-  return true;
+  kv->k_ld = s[7];
+  kv->v_plane = G > 1 ? s[9] : (B > 1 ? s[8] : (int64_t)Tk * dv);
+  if (s[6] != 1 || kv->k_ld < Tk || kv->k_ld % 8 != 0 || (G > 1 && s[5] != dk * kv->k_ld) || (B > 1 && s[4] != G * dk * kv->k_ld)) return false;
+  return s[11] == 1 && s[10] == dv && kv->v_plane >= (int64_t)Tk * dv && kv->v_plane % 8 == 0 && (B == 1 || s[8] == G * kv->v_plane);
 }
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // canonical contiguous gradients: dq like q, dk [B,G,Tk,dk], dv [B,G,Tk,dv]
 static bool tensor_core_bwd_ok(const int64_t* s, int dtype, int B, int H, int G, int Tq, int Tk, int dk, int dv,
                                const void* q, const void* k, const void* v, const void* o, const void* dout, const void* dq,
-                               const void* dkey, const void* dval) {
+                               const void* dkey, const void* dval, KvLayout* kv) {
   if (dtype != NSA_BF16 || !fa_fwd_sm100_supported(H, G, Tq, Tk, dk, dv)) return false;
-  if (!canonical_fwd(s, H, G, Tq, Tk, dk, dv) || (int64_t)B * H > 65535) return false;
+  if (!canonical_fwd(s, B, H, G, Tq, Tk, dk, dv, kv) || (int64_t)B * H > 65535) return false;
   const int64_t gq[4] = {(int64_t)H * Tq * dk, (int64_t)Tq * dk, dk, 1};
   const int64_t gk[4] = {(int64_t)G * Tk * dk, (int64_t)Tk * dk, dk, 1};
   const int64_t gv[4] = {(int64_t)G * Tk * dv, (int64_t)Tk * dv, dv, 1};
@@ -114,10 +117,10 @@ static bool tensor_core_bwd_ok(const int64_t* s, int dtype, int B, int H, int G,
          aligned16(dkey) && aligned16(dval);
 }
 
-static bool tensor_core_bwd_ok_slc(const int64_t* s, int dtype, int H, int G, int Tq, int Tk, int dk, int dv, const void* q,
+static bool tensor_core_bwd_ok_slc(const int64_t* s, int dtype, int B, int H, int G, int Tq, int Tk, int dk, int dv, const void* q,
                                    const void* k, const void* v, const void* o, const void* dout, const void* dq,
-                                   const void* dkey, const void* dval) {
-  if (dtype != NSA_BF16 || !canonical_fwd(s, H, G, Tq, Tk, dk, dv)) return false;
+                                   const void* dkey, const void* dval, KvLayout* kv) {
+  if (dtype != NSA_BF16 || !canonical_fwd(s, B, H, G, Tq, Tk, dk, dv, kv)) return false;
   const int64_t gq[4] = {(int64_t)H * Tq * dk, (int64_t)Tq * dk, dk, 1};
   const int64_t gk[4] = {(int64_t)G * Tk * dk, (int64_t)Tk * dk, dk, 1};
   const int64_t gv[4] = {(int64_t)G * Tk * dv, (int64_t)Tk * dv, dv, 1};
@@ -207,10 +210,11 @@ extern "C" NSA_API int nsa_sliding_fwd(const void* q, const void* k, const void*
   NSA_REQUIRE(q && k && v && out && strides, "sliding_fwd: null pointer");
   NSA_REQUIRE(window > 0, "sliding_fwd: window must be positive");
   NSA_REFUSE_AFTER_TIMEOUT("sliding_fwd");
+  KvLayout kv;
   if (want_tc(flags) && dtype == NSA_BF16 && L && M && fa_fwd_sm100_supported(H, G, T, T, dk, dv) &&
-      canonical_fwd(strides, H, G, T, T, dk, dv) && aligned16(q) && aligned16(k) && aligned16(v) && aligned16(out) &&
+      canonical_fwd(strides, B, H, G, T, T, dk, dv, &kv) && aligned16(q) && aligned16(k) && aligned16(v) && aligned16(out) &&
       (int64_t)B * (H / 2) <= 65535)
-    return fa_fwd_sm100(q, k, v, out, L, M, B, H, G, T, T, dk, dv, kWin, window, 0, 0, 0, scale, nullptr, nullptr, (cudaStream_t)stream);
+    return fa_fwd_sm100(q, k, v, out, L, M, B, H, G, T, T, dk, dv, kWin, window, 0, 0, 0, scale, nullptr, nullptr, kv, (cudaStream_t)stream);
   AttnArgs a = {};
   a.q = q; a.k = k; a.v = v; a.o = out; a.L = L; a.M = M;
   fill_fwd_strides(a, strides);
@@ -227,9 +231,10 @@ extern "C" NSA_API int nsa_sliding_bwd(const void* q, const void* k, const void*
   NSA_REQUIRE(q && k && v && out && dout && L && M && dq && dkey && dval && strides, "sliding_bwd: null pointer");
   NSA_REQUIRE(window > 0, "sliding_bwd: window must be positive");
   NSA_REFUSE_AFTER_TIMEOUT("sliding_bwd");
-  if (want_tc(flags) && tensor_core_bwd_ok(strides, dtype, B, H, G, T, T, dk, dv, q, k, v, out, dout, dq, dkey, dval))
+  KvLayout kv;
+  if (want_tc(flags) && tensor_core_bwd_ok(strides, dtype, B, H, G, T, T, dk, dv, q, k, v, out, dout, dq, dkey, dval, &kv))
     return fa_bwd_sm100(q, k, v, out, dout, L, M, dq, dkey, dval, B, H, G, T, T, dk, dv, kWin, window, 0, 0, 0, scale,
-                        row_delta, workspace, workspace_bytes, (cudaStream_t)stream);
+                        row_delta, kv, workspace, workspace_bytes, (cudaStream_t)stream);
   AttnArgs a = {};
   a.q = q; a.k = k; a.v = v; a.o_in = out; a.dout = dout; a.Lc = L; a.Mc = M; a.dq = dq; a.dk_out = dkey; a.dv_out = dval;
   fill_bwd_strides(a, strides);
@@ -248,12 +253,13 @@ extern "C" NSA_API int nsa_cmp_attn_fwd(const void* q, const void* k_cmp, const 
               "cmp_attn_fwd: bad block layout hint (l=%d, d=%d, n=%d)", blocks_l, blocks_d, blocks_n);
   NSA_REQUIRE(q_pos0 >= 0, "cmp_attn_fwd: negative query offset");
   NSA_REFUSE_AFTER_TIMEOUT("cmp_attn_fwd");
+  KvLayout kv;
   if (want_tc(flags) && blocks_d > 0 && dtype == NSA_BF16 && L && M && fa_fwd_sm100_supported(H, G, T, NB, dk, dv) &&
-      canonical_fwd(strides, H, G, T, NB, dk, dv) && aligned16(q) && aligned16(k_cmp) && aligned16(v_cmp) &&
+      canonical_fwd(strides, B, H, G, T, NB, dk, dv, &kv) && aligned16(q) && aligned16(k_cmp) && aligned16(v_cmp) &&
       aligned16(out) && (int64_t)B * (H / 2) <= 65535)
     // block i is visible to the query at position q0 + t iff i*d + l - 1 <= q0 + t: the same rule with l - q0 for row t
     return fa_fwd_sm100(q, k_cmp, v_cmp, out, L, M, B, H, G, T, NB, dk, dv, kCmp, 0, blocks_l - q_pos0, blocks_d, blocks_n,
-                        scale, k_cmp_lo, lse2_out, (cudaStream_t)stream);
+                        scale, k_cmp_lo, lse2_out, kv, (cudaStream_t)stream);
   if (k_cmp_lo)
     return fail(NSA_ERR_UNSUPPORTED, "cmp_attn_fwd: the hi + lo key form needs the bf16 tensor-core path (see nsa_cmp_attn_exact_supported)");
   NSA_NO_QUERY_OFFSET("cmp_attn_fwd");
@@ -281,10 +287,11 @@ extern "C" NSA_API int nsa_cmp_attn_bwd(const void* q, const void* k_cmp, const 
               "cmp_attn_bwd: bad block layout hint (l=%d, d=%d, n=%d)", blocks_l, blocks_d, blocks_n);
   NSA_REQUIRE(q_pos0 >= 0, "cmp_attn_bwd: negative query offset");
   NSA_REFUSE_AFTER_TIMEOUT("cmp_attn_bwd");
+  KvLayout kv;
   if (want_tc(flags) && blocks_d > 0 &&
-      tensor_core_bwd_ok(strides, dtype, B, H, G, T, NB, dk, dv, q, k_cmp, v_cmp, out, dout, dq, dk_cmp, dv_cmp))
+      tensor_core_bwd_ok(strides, dtype, B, H, G, T, NB, dk, dv, q, k_cmp, v_cmp, out, dout, dq, dk_cmp, dv_cmp, &kv))
     return fa_bwd_sm100(q, k_cmp, v_cmp, out, dout, L, M, dq, dk_cmp, dv_cmp, B, H, G, T, NB, dk, dv, kCmp, 0,
-                        blocks_l - q_pos0, blocks_d, blocks_n, scale, row_delta, workspace, workspace_bytes,
+                        blocks_l - q_pos0, blocks_d, blocks_n, scale, row_delta, kv, workspace, workspace_bytes,
                         (cudaStream_t)stream);
   NSA_NO_QUERY_OFFSET("cmp_attn_bwd");
   AttnArgs a = {};
@@ -306,11 +313,12 @@ static int slc_fwd_impl(const char* who, const void* q, const void* k, const voi
   if (timeout_flagged())
     return fail(NSA_ERR_LAUNCH, "%s: a tensor-core kernel gave up on a barrier wait earlier (device time-out); results since "
                 "then are invalid.  nsa_device_timeouts(1) reports and clears the condition", who);
+  KvLayout kv;
   if (want_tc(flags) && dtype == NSA_BF16 && L && M && B > 0 && slc_sm100_supported(H, G, Tq, Tkv, dk, dv, n_slots, l_prime) &&
-      canonical_fwd(strides, H, G, Tq, Tkv, dk, dv) && aligned16(q) && aligned16(k) && aligned16(v) && aligned16(out) &&
+      canonical_fwd(strides, B, H, G, Tq, Tkv, dk, dv, &kv) && aligned16(q) && aligned16(k) && aligned16(v) && aligned16(out) &&
       (!mix.out || (aligned16(mix.out) && aligned16(mix.o_cmp) && aligned16(mix.o_win))))
     return slc_fwd_sm100(q, k, v, indices, strides + 22, out, L, M, B, H, G, Tq, Tkv, dk, dv, n_slots, l_prime, scale,
-                         q_pos0, mix, workspace, workspace_bytes, (cudaStream_t)stream);
+                         q_pos0, mix, kv, workspace, workspace_bytes, (cudaStream_t)stream);
   NSA_REQUIRE(q_pos0 == 0, "%s: a query offset needs the bf16 tensor-core path of this call", who);
   AttnArgs a = {};
   a.q = q; a.k = k; a.v = v; a.o = out; a.L = L; a.M = M; a.indices = indices;
@@ -377,10 +385,11 @@ extern "C" NSA_API int nsa_slc_bwd(const void* q, const void* k, const void* v, 
   NSA_REQUIRE(q_pos0 >= 0, "slc_bwd: negative query offset");
   NSA_REFUSE_AFTER_TIMEOUT("slc_bwd");
   if (B == 0 || Tq == 0 || Tkv == 0) return NSA_OK;
+  KvLayout kv;
   if (want_tc(flags) && slc_sm100_supported(H, G, Tq, Tkv, dk, dv, n_slots, l_prime) &&
-      tensor_core_bwd_ok_slc(strides, dtype, H, G, Tq, Tkv, dk, dv, q, k, v, out, dout, dq, dkey, dval))
+      tensor_core_bwd_ok_slc(strides, dtype, B, H, G, Tq, Tkv, dk, dv, q, k, v, out, dout, dq, dkey, dval, &kv))
     return slc_bwd_sm100(q, k, v, indices, strides + 34, out, dout, L, M, dq, dkey, dval, B, H, G, Tq, Tkv, dk, dv, n_slots,
-                         l_prime, scale, q_pos0, row_delta, dq_add0, dq_add1, workspace, workspace_bytes,
+                         l_prime, scale, q_pos0, row_delta, dq_add0, dq_add1, kv, workspace, workspace_bytes,
                          (cudaStream_t)stream);
   NSA_NO_QUERY_OFFSET("slc_bwd");
   const void *add0 = dq_add0, *add1 = dq_add1;

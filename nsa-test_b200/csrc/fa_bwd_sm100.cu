@@ -56,7 +56,7 @@ struct FaBwdParams {
 };
 
 // Which 64-query sub-tiles meet key tile j (keys [128 j, 128 j + 128)).  The range is widened to whole 128-query tiles
-// (first sub-tile even, last odd; Tq is a multiple of 128), so that the dQ kernel, which works on 128-query tiles, finds
+// (first sub-tile even, last odd), so that the dQ kernel, which works on 128-query tiles, finds
 // either both halves of a tile written or neither.  Shared by the dK/dV kernel (writer of the dS^T tiles) and the dQ
 // kernel (reader): both must agree on the set of tiles.
 template <int MODE>
@@ -71,7 +71,7 @@ __host__ __device__ __forceinline__ void subtile_range(int j, int Tq, int window
     const int64_t tfirst = (int64_t)n0 * cmp_d + cmp_l - 1;
     if (n0 < cmp_nb && tfirst < Tq) {
       *qs_lo = (int)((tfirst > 0 ? tfirst : 0) / 64) & ~1;   // tfirst < 0: visible from the first row on
-      *qs_hi = (Tq - 1) / 64;
+      *qs_hi = ((Tq - 1) / 64) | 1;
     } else {
       *qs_lo = 1;
       *qs_hi = 0;
@@ -82,7 +82,7 @@ __host__ __device__ __forceinline__ void subtile_range(int j, int Tq, int window
 // diagonal (slot = distance from the first one), the compressed branch all of them
 template <int MODE>
 __host__ __device__ __forceinline__ int ds_slot(int j, int qs) { return MODE == kWin ? qs - 2 * j : qs; }
-static int ds_slots_per_key_tile(int mode, int Tq, int window) { return mode == kWin ? (((126 + window) / 64) | 1) + 1 : Tq / 64; }
+static int ds_slots_per_key_tile(int mode, int Tq, int window) { return mode == kWin ? (((126 + window) / 64) | 1) + 1 : ((Tq + 127) / 128) * 2; }
 
 
 // ------------------------------------------------------------------------------------------------
@@ -160,7 +160,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   // Work items: (query tile, batch, head), late (heavy) query tiles first, taken round robin by the CTAs of a persistent
   // grid; every role walks the same list on its own, so the loads and the first S/dP MMAs of an item overlap the dQ
   // epilogue of the one before.
-  const int per_qt = p.B * p.H, nqt = p.Tq / 128, nitems = nqt * per_qt;
+  const int per_qt = p.B * p.H, nqt = (p.Tq + 127) / 128, nitems = nqt * per_qt;
   // once any block has given up on a wait the device results are void: later blocks skip their work and end at once
   const bool poisoned = p.timeouts && *(volatile const int*)p.timeouts != 0;
   struct Item { int m0, b, h, g, jlo, ntiles; };
@@ -220,9 +220,9 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (!ok) break;
       if (elect_one()) {
         mbar_arrive_expect_tx(&bar->qdo_full, SM::kQ + SM::kdO);
-        const int qrow = (w.b * p.H + w.h) * p.Tq + w.m0;
-        for (int c = 0; c < DK / 64; ++c) tma_load_2d(&tmQ, &bar->qdo_full, sQ + c * 16384, c * 64, qrow);
-        for (int c = 0; c < DV / 64; ++c) tma_load_2d(&tmdO, &bar->qdo_full, sdO + c * 16384, c * 64, qrow);
+        const int plane = w.b * p.H + w.h;
+        for (int c = 0; c < DK / 64; ++c) tma_load_3d(&tmQ, &bar->qdo_full, sQ + c * 16384, c * 64, w.m0, plane);
+        for (int c = 0; c < DV / 64; ++c) tma_load_3d(&tmdO, &bar->qdo_full, sdO + c * 16384, c * 64, w.m0, plane);
       }
       __syncwarp();
       q_pending = true;
@@ -244,7 +244,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         if (elect_one()) {
           mbar_arrive_expect_tx(&bar->v_full, SM::kV);
           for (int c = 0; c < DV / 64; ++c)
-            tma_load_2d(&tmV, &bar->v_full, sV + c * 16384, c * 64, (w.b * p.G + w.g) * p.Tk + n0);
+            tma_load_3d(&tmV, &bar->v_full, sV + c * 16384, c * 64, n0, w.b * p.G + w.g);
         }
         __syncwarp();
       }
@@ -332,7 +332,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const Item w = item_at(it);
     const int jlo = w.jlo, ntiles = ok ? w.ntiles : 0, t = w.m0 + r;
     const int64_t row = ((int64_t)w.b * p.H + w.h) * p.Tq + t;
-    const float lse2 = p.lse2[row], Dr = p.D[row];
+    const float lse2 = t < p.Tq ? p.lse2[row] : CUDART_INF_F, Dr = t < p.Tq ? p.D[row] : 0.f;
     for (int j = 0; j < ntiles && ok; ++j) {
       const int n0 = (jlo + j) * 128 + gsel * 64;   // first key of this thread's columns
       ok = mbar_wait(&bar->sdp_full, (tc + j) & 1, abort);
@@ -401,6 +401,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
 #pragma unroll
       for (int c = 0; c < DK / 64; ++c) {
+        if (t >= p.Tq) break;
 #pragma unroll
         for (int e = 0; e < 32; e += 8) {
           uint4 pkt;
@@ -458,7 +459,7 @@ fa_bwd_dq_ds_kernel(const __grid_constant__ CUtensorMap tmDs, const __grid_const
   DqDsBarriers* bar = reinterpret_cast<DqDsBarriers*>(smem + SM::oBar);
   volatile int* abort = &bar->abort;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int per_qt = p.B * p.H, nqt = p.Tq / 128, nitems = nqt * per_qt, nkt = p.Tk / 128;
+  const int per_qt = p.B * p.H, nqt = (p.Tq + 127) / 128, nitems = nqt * per_qt, nkt = (p.Tk + 127) / 128;
   const bool poisoned = p.timeouts && *(volatile const int*)p.timeouts != 0;
   struct Item { int qt, b, h, g, jlo, ntiles; };
   // key tiles whose widened sub-tile range holds query tile qt: a contiguous run of j ending at jhi
@@ -584,7 +585,8 @@ fa_bwd_dq_ds_kernel(const __grid_constant__ CUtensorMap tmDs, const __grid_const
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
       const Item w = item_at(it);
       const int ntiles = ok ? w.ntiles : 0;
-      const int64_t row = ((int64_t)w.b * p.H + w.h) * p.Tq + w.qt * 128 + r;
+      const int t = w.qt * 128 + r;
+      const int64_t row = ((int64_t)w.b * p.H + w.h) * p.Tq + t;
       __nv_bfloat16* dst = p.dq + row * DK;
       const int a = ic & 1;
       if (ntiles > 0) {
@@ -606,6 +608,7 @@ fa_bwd_dq_ds_kernel(const __grid_constant__ CUtensorMap tmDs, const __grid_const
 #pragma unroll
           for (int e = 0; e < 32; ++e) ov[e] = 0;
         }
+        if (t >= p.Tq) continue;
 #pragma unroll
         for (int e = 0; e < 32; e += 8) {
           uint4 pkt;
@@ -705,7 +708,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       if (elect_one()) {
         mbar_arrive_expect_tx(&bar->kv_full, SM::kK + SM::kV);
         for (int hf = 0; hf < 2; ++hf) tma_load_2d(&tmK, &bar->kv_full, sK + hf * (DK * 128), n0 + hf * 64, (b * p.G + g) * DK);
-        for (int c = 0; c < DV / 64; ++c) tma_load_2d(&tmV, &bar->kv_full, sV + c * 16384, c * 64, (b * p.G + g) * p.Tk + n0);
+        for (int c = 0; c < DV / 64; ++c) tma_load_3d(&tmV, &bar->kv_full, sV + c * 16384, c * 64, n0, b * p.G + g);
       }
       __syncwarp();
       bool ok = true;
@@ -717,9 +720,8 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       int h_pf = hbeg, qs_pf = qs_lo, it_pf = 0;
       auto prefetch_next = [&]() {
         if (it_pf < n_it) {
-          const int row = (int)((((int64_t)b * p.H + h_pf) * p.Tq) + qs_pf * 64);
-          for (int c = 0; c < DK / 64; ++c) tma_prefetch_2d(&tmQ, c * 64, row);
-          for (int c = 0; c < DV / 64; ++c) tma_prefetch_2d(&tmdO, c * 64, row);
+          for (int c = 0; c < DK / 64; ++c) tma_prefetch_3d(&tmQ, c * 64, qs_pf * 64, b * p.H + h_pf);
+          for (int c = 0; c < DV / 64; ++c) tma_prefetch_3d(&tmdO, c * 64, qs_pf * 64, b * p.H + h_pf);
           ++it_pf;
           if (++qs_pf > qs_hi) { qs_pf = qs_lo; ++h_pf; }
         }
@@ -731,15 +733,17 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         const int tq0 = qs * 64;
         const int64_t qrow = ((int64_t)b * p.H + h) * p.Tq + tq0;
         // the statistics are fetched before the stage is free
-        const float s_l0 = p.lse2[qrow + lane], s_l1 = p.lse2[qrow + 32 + lane];
-        const float s_d0 = p.D[qrow + lane], s_d1 = p.D[qrow + 32 + lane];
+        // (rows past the last query: P = exp2(x - inf) = 0 and dS = 0)
+        const bool in0 = tq0 + lane < p.Tq, in1 = tq0 + 32 + lane < p.Tq;
+        const float s_l0 = in0 ? p.lse2[qrow + lane] : CUDART_INF_F, s_l1 = in1 ? p.lse2[qrow + 32 + lane] : CUDART_INF_F;
+        const float s_d0 = in0 ? p.D[qrow + lane] : 0.f, s_d1 = in1 ? p.D[qrow + 32 + lane] : 0.f;
         ok = mbar_wait_warp(&bar->empty[s], ph ^ 1, abort);
         if (!ok) break;
         uint8_t* st = sSt + s * SM::kStage;
         if (elect_one()) {
           mbar_arrive_expect_tx(&bar->full[s], SM::kQs + SM::kdOs);
-          for (int c = 0; c < DK / 64; ++c) tma_load_2d(&tmQ, &bar->full[s], st + c * 8192, c * 64, (int)qrow);
-          for (int c = 0; c < DV / 64; ++c) tma_load_2d(&tmdO, &bar->full[s], st + SM::kQs + c * 8192, c * 64, (int)qrow);
+          for (int c = 0; c < DK / 64; ++c) tma_load_3d(&tmQ, &bar->full[s], st + c * 8192, c * 64, tq0, b * p.H + h);
+          for (int c = 0; c < DV / 64; ++c) tma_load_3d(&tmdO, &bar->full[s], st + SM::kQs + c * 8192, c * 64, tq0, b * p.H + h);
           prefetch_next();
         }
         float* stat = reinterpret_cast<float*>(st + SM::kQs + SM::kdOs);
@@ -938,6 +942,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 #pragma unroll
             for (int e = 0; e < 32; ++e) ov[e] = 0;
           }
+          if (key >= p.Tk) continue;
           if (out_part) {
             float* dst = out_part + ((int64_t)hc * p.B * p.G * p.Tk + krow) * width + c * 32;
 #pragma unroll
@@ -991,7 +996,7 @@ static size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 static int pick_hsplit(int B, int G, int H, int Tk, int mode) {
   if (mode == kWin) return 1;
   const int hpg = H / G;
-  const long ctas = (long)B * G * (Tk / 128);
+  const long ctas = (long)B * G * ((Tk + 127) / 128);
   int hs = 1;
   while (hs < hpg && ctas * hs < 4 * 148 && hpg % (hs * 2) == 0) hs *= 2;
   return hs;
@@ -1007,7 +1012,7 @@ static size_t bwd_base_bytes(int B, int H, int G, int Tq, int Tk, int dk, int dv
 // recomputes S and dP) or its row count would not fit a tensor-map coordinate
 constexpr size_t kMaxDsBytes = (size_t)48 << 30;
 static size_t bwd_ds_bytes(int B, int H, int Tq, int Tk, int mode, int window) {
-  const size_t tiles = (size_t)B * H * (Tk / 128) * ds_slots_per_key_tile(mode, Tq, window);
+  const size_t tiles = (size_t)B * H * ((Tk + 127) / 128) * ds_slots_per_key_tile(mode, Tq, window);
   const size_t bytes = tiles * 16384;
   if (bytes > kMaxDsBytes || tiles * 128 >= ((size_t)1 << 31)) return 0;
   return bytes;
@@ -1029,8 +1034,8 @@ static int launch_bwd_t(const CUtensorMap& tq128, const CUtensorMap& tdo128, con
       cudaFuncSetAttribute(kqd, cudaFuncAttributeMaxDynamicSharedMemorySize, DqDsSmem<DK>::kDynamic) != cudaSuccess ||
       cudaFuncSetAttribute(kkv, cudaFuncAttributeMaxDynamicSharedMemorySize, DkvSmem<DK, DV>::kDynamic) != cudaSuccess)
     return fail(NSA_ERR_LAUNCH, "fa_bwd: cannot reserve shared memory");
-  const dim3 qgrid((unsigned)std::min((p.Tq / 128) * p.B * p.H, bwd_sm_count()));
-  const dim3 kvgrid(p.Tk / 128, p.hsplit, p.B * p.G);
+  const dim3 qgrid((unsigned)std::min(((p.Tq + 127) / 128) * p.B * p.H, bwd_sm_count()));
+  const dim3 kvgrid((p.Tk + 127) / 128, p.hsplit, p.B * p.G);
   if (p.ds) {
     // key-stationary kernel first: it leaves dS^T behind, from which the dQ kernel only has one product left to do
     {
@@ -1055,7 +1060,7 @@ static int launch_bwd_t(const CUtensorMap& tq128, const CUtensorMap& tdo128, con
 int fa_bwd_sm100(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* L,
                  const float* M, void* dq, void* dk_out, void* dv_out, int B, int H, int G, int Tq, int Tk, int dk, int dv,
                  int mode, int window, int cmp_l, int cmp_d, int cmp_nb, float scale, const float* row_delta,
-                 void* workspace, size_t workspace_bytes, cudaStream_t st) {
+                 const KvLayout& kv, void* workspace, size_t workspace_bytes, cudaStream_t st) {
   if (!fa_fwd_sm100_supported(H, G, Tq, Tk, dk, dv)) return fail(NSA_ERR_UNSUPPORTED, "fa_bwd_sm100: unsupported shape");
   if ((int64_t)B * H > 65535) return fail(NSA_ERR_UNSUPPORTED, "fa_bwd_sm100: B*H too large");
   const size_t need = bwd_base_bytes(B, H, G, Tq, Tk, dk, dv, mode);
@@ -1091,12 +1096,12 @@ int fa_bwd_sm100(const void* q, const void* k, const void* v, const void* o, con
   } else {
     tds = CUtensorMap{};
   }
-  if (int rc = make_tmap_bf16_2d(&tq128, q, (uint64_t)B * H * Tq, dk, 128)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tdo128, dout, (uint64_t)B * H * Tq, dv, 128)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tq64, q, (uint64_t)B * H * Tq, dk, 64)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tdo64, dout, (uint64_t)B * H * Tq, dv, 64)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tk, k, (uint64_t)B * G * dk, Tk, dk)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tv, v, (uint64_t)B * G * Tk, dv, 128)) return rc;
+  if (int rc = make_tmap_bf16_3d(&tq128, q, (uint64_t)B * H, Tq, dk, (uint64_t)Tq * dk, 128)) return rc;
+  if (int rc = make_tmap_bf16_3d(&tdo128, dout, (uint64_t)B * H, Tq, dv, (uint64_t)Tq * dv, 128)) return rc;
+  if (int rc = make_tmap_bf16_3d(&tq64, q, (uint64_t)B * H, Tq, dk, (uint64_t)Tq * dk, 64)) return rc;
+  if (int rc = make_tmap_bf16_3d(&tdo64, dout, (uint64_t)B * H, Tq, dv, (uint64_t)Tq * dv, 64)) return rc;
+  if (int rc = make_tmap_bf16_2d(&tk, k, (uint64_t)B * G * dk, Tk, dk, kv.k_ld)) return rc;
+  if (int rc = make_tmap_bf16_3d(&tv, v, (uint64_t)B * G, Tk, dv, kv.v_plane, 128)) return rc;
   int rc = NSA_ERR_UNSUPPORTED;
 #define NSA_BWD_CASE(DK_, DV_)                                                                               \
   if (dk == DK_ && dv == DV_)                                                                                \
@@ -1156,7 +1161,7 @@ extern "C" NSA_API int nsa_sliding_bwd_noalloc(const void* q, const void* k, con
   using namespace nsa;
   NSA_REQUIRE(q && k && v && out && dout && L && M && dq && dkey && dval, "sliding_bwd_noalloc: null pointer");
   NSA_REQUIRE(B > 0 && H > 0 && G > 0 && H % G == 0 && T > 0 && window > 0, "sliding_bwd_noalloc: bad sizes");
-  if (!fa_fwd_sm100_supported(H, G, T, T, dk, dv))
+  if (!fa_fwd_sm100_supported(H, G, T, T, dk, dv) || T % 128 != 0)
     return fail(NSA_ERR_UNSUPPORTED,
                 "sliding_bwd_noalloc covers bf16 tensors with head dims (192,128), (128,128) or (64,64), an even number of heads per "
                 "group and T a multiple of 128; other shapes run through nsa_sliding_bwd, whose stride-generic kernels need no scratch");
@@ -1170,6 +1175,7 @@ extern "C" NSA_API int nsa_sliding_bwd_noalloc(const void* q, const void* k, con
   float* scratch = nullptr;
   if (int rc = sliding_bwd_scratch_address(&scratch)) return rc;
   // Nothing in the scratch has to start at zero: the preparation kernel overwrites every row this call reads.
-  return fa_bwd_sm100(q, k, v, out, dout, L, M, dq, dkey, dval, B, H, G, T, T, dk, dv, kWin, window, 0, 0, 0, scale, nullptr, scratch,
+  return fa_bwd_sm100(q, k, v, out, dout, L, M, dq, dkey, dval, B, H, G, T, T, dk, dv, kWin, window, 0, 0, 0, scale, nullptr,
+                      KvLayout{T, (int64_t)T * dv}, scratch,
                       sizeof(float) * 2 * kNoAllocMaxRows, (cudaStream_t)stream);
 }

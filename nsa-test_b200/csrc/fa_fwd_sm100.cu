@@ -90,7 +90,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   // Work items: (query tile, batch, head pair), late (heavy) query tiles first; the CTAs of the persistent grid take
   // them round robin, and every role below walks the same item list on its own, so that the loads and the first
   // S MMAs of an item run while the softmax warps are still in the epilogue of the one before.
-  const int pairs = p.H / 2, per_qt = p.B * pairs, nqt = p.Tq / kBM;
+  const int pairs = p.H / 2, per_qt = p.B * pairs, nqt = (p.Tq + kBM - 1) / kBM;
   const int nitems = nqt * per_qt;
   // once any block has given up on a wait the device results are void: later blocks skip their work and end at once
   const bool poisoned = *(volatile const int*)&g_timeout_record.count != 0;
@@ -167,8 +167,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         mbar_arrive_expect_tx(&bar->q_full, 2 * SM::kQBytes);
         for (int i = 0; i < 2; ++i)
           for (int c = 0; c < DK / 64; ++c)
-            tma_load_2d(&tmQ, &bar->q_full, sQ + i * SM::kQBytes + c * (kBM * 128), c * 64,
-                        (w.b * p.H + w.h0 + i) * p.Tq + w.m0);
+            tma_load_3d(&tmQ, &bar->q_full, sQ + i * SM::kQBytes + c * (kBM * 128), c * 64, w.m0, w.b * p.H + w.h0 + i);
       }
       __syncwarp();
       q_pending = true;
@@ -193,7 +192,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         if (elect_one()) {
           mbar_arrive_expect_tx(&bar->v_full, SM::kVBytes);
           for (int c = 0; c < DV / 64; ++c)
-            tma_load_2d(&tmV, &bar->v_full, sV + c * (kBN * 128), c * 64, (w.b * p.G + w.g) * p.Tk + n0);
+            tma_load_3d(&tmV, &bar->v_full, sV + c * (kBN * 128), c * 64, n0, w.b * p.G + w.g);
         }
         __syncwarp();
       }
@@ -399,6 +398,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 #pragma unroll
           for (int e = 0; e < 32; ++e) ov[c][e] = 0;
       }
+      if (t < p.Tq) {
 #pragma unroll
       for (int c = 0; c < DV / 32; ++c) {
 #pragma unroll
@@ -418,6 +418,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       if (p.L) p.L[row] = l > 0.f ? logf(l) + (m_ref - m_true) * kLn2 : -CUDART_INF_F;
       if (p.M) p.M[row] = m_true * kLn2;  // back from log2 units to the natural-log scale of the logits
       if (p.lse2) p.lse2[row] = l > 0.f ? m_ref + log2f(l) : CUDART_INF_F;   // log-sum-exp in log2 units (+inf: the row saw nothing)
+      }
     }
     tc += ntiles;
     }  // items
@@ -453,17 +454,33 @@ static EncodeTiledFn encode_fn() {
 }
 
 // bf16 row-major [rows, cols] matrix, box [box_rows, 64 cols] (128 B inner extent), 128-byte swizzle
-int make_tmap_bf16_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+int make_tmap_bf16_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint64_t ld) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail(NSA_ERR_LAUNCH, "cuTensorMapEncodeTiled is not available from this driver");
   cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {cols * 2};
+  cuuint64_t strides[1] = {(ld ? ld : cols) * 2};
   cuuint32_t box[2] = {64, box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(NSA_ERR_LAUNCH, "cuTensorMapEncodeTiled failed with %d", (int)r);
+  return NSA_OK;
+}
+
+// bf16 [planes, rows, cols], box [1, box_rows, 64 cols], 128-byte swizzle
+int make_tmap_bf16_3d(CUtensorMap* map, const void* base, uint64_t planes, uint64_t rows, uint64_t cols, uint64_t plane,
+                      uint32_t box_rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(NSA_ERR_LAUNCH, "cuTensorMapEncodeTiled is not available from this driver");
+  cuuint64_t dims[3] = {cols, rows, planes};
+  cuuint64_t strides[2] = {cols * 2, plane * 2};
+  cuuint32_t box[3] = {64, box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(NSA_ERR_LAUNCH, "cuTensorMapEncodeTiled (planes) failed with %d", (int)r);
   return NSA_OK;
 }
 
@@ -506,7 +523,7 @@ static int launch_fa_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const C
   auto kern = fa_fwd_kernel<DK, DV, MODE, EXACT>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::kDynamic);
   if (e != cudaSuccess) return fail(NSA_ERR_LAUNCH, "fa_fwd: cannot reserve %d bytes of shared memory: %s", SM::kDynamic, cudaGetErrorString(e));
-  const int nitems = (p.Tq / kBM) * p.B * (p.H / 2);
+  const int nitems = ((p.Tq + kBM - 1) / kBM) * p.B * (p.H / 2);
   dim3 grid((unsigned)std::min(nitems, sm_count()));   // persistent: one CTA per SM walks the item list
   KernelTimer kt(MODE == kWin ? "fa_fwd_win" : (EXACT ? "fa_fwd_cmp_exact" : "fa_fwd_cmp"), st);
   kern<<<grid, kFaThreads, SM::kDynamic, st>>>(tq, tk, tv, tklo, p);
@@ -515,21 +532,21 @@ static int launch_fa_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const C
 
 bool fa_fwd_sm100_supported(int H, int G, int Tq, int Tk, int dk, int dv) {
   const bool dims = (dk == 192 && dv == 128) || (dk == 128 && dv == 128) || (dk == 64 && dv == 64);
-  return dims && G > 0 && H % G == 0 && (H / G) % 2 == 0 && Tq % kBM == 0 && Tk % kBN == 0 && Tq > 0 && Tk > 0;
+  return dims && G > 0 && H % G == 0 && (H / G) % 2 == 0 && Tq > 0 && Tk > 0;
 }
 
 int fa_fwd_sm100(const void* q, const void* k, const void* v, void* o, float* L, float* M, int B, int H, int G, int Tq,
                  int Tk, int dk, int dv, int mode, int window, int cmp_l, int cmp_d, int cmp_nb, float scale,
-                 const void* k_lo, float* lse2, cudaStream_t st) {
+                 const void* k_lo, float* lse2, const KvLayout& kv, cudaStream_t st) {
   if (!fa_fwd_sm100_supported(H, G, Tq, Tk, dk, dv)) return fail(NSA_ERR_UNSUPPORTED, "fa_fwd_sm100: unsupported shape");
   if (!fa_timeout_counter()) return fail(NSA_ERR_LAUNCH, "fa_fwd_sm100: cannot set up the time-out record of this device");
-  if ((int64_t)B * (H / 2) * (Tq / kBM) > 0x7fffffff) return fail(NSA_ERR_UNSUPPORTED, "fa_fwd_sm100: too many work items");
+  if ((int64_t)B * (H / 2) * ((Tq + kBM - 1) / kBM) > 0x7fffffff) return fail(NSA_ERR_UNSUPPORTED, "fa_fwd_sm100: too many work items");
   if (k_lo && mode != kCmp) return fail(NSA_ERR_ARG, "fa_fwd_sm100: a low-order key part belongs to the compressed branch");
   CUtensorMap tq, tk, tv, tklo;
-  if (int rc = make_tmap_bf16_2d(&tq, q, (uint64_t)B * H * Tq, dk, kBM)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tk, k, (uint64_t)B * G * dk, Tk, dk)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tklo, k_lo ? k_lo : k, (uint64_t)B * G * dk, Tk, dk)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tv, v, (uint64_t)B * G * Tk, dv, kBN)) return rc;
+  if (int rc = make_tmap_bf16_3d(&tq, q, (uint64_t)B * H, Tq, dk, (uint64_t)Tq * dk, kBM)) return rc;
+  if (int rc = make_tmap_bf16_2d(&tk, k, (uint64_t)B * G * dk, Tk, dk, kv.k_ld)) return rc;
+  if (int rc = make_tmap_bf16_2d(&tklo, k_lo ? k_lo : k, (uint64_t)B * G * dk, Tk, dk, kv.k_ld)) return rc;
+  if (int rc = make_tmap_bf16_3d(&tv, v, (uint64_t)B * G, Tk, dv, kv.v_plane, kBN)) return rc;
   FaFwdParams p;
   p.o = (__nv_bfloat16*)o; p.L = L; p.M = M;
   p.B = B; p.H = H; p.G = G; p.Tq = Tq; p.Tk = Tk;

@@ -21,12 +21,20 @@ struct FaFwdParams {
 // True when the tensor-core forward covers this shape (bf16, canonical contiguous layouts assumed).
 bool fa_fwd_sm100_supported(int H, int G, int Tq, int Tk, int dk, int dv);
 
-// q [B,H,Tq,dk], k [B,G,dk,Tk], v [B,G,Tk,dv], o [B,H,Tq,dv]: contiguous bf16.  mode = kWin or kCmp.
+// Memory layout of the keys and values of one call: k [B,G,dk,Tk] with rows `k_ld` elements apart (a multiple of 8, so that
+// every row starts on a TMA boundary; rows and groups follow one another without gaps), v [B,G,Tk,dv] with contiguous rows
+// and groups `v_plane` elements apart.
+struct KvLayout {
+  int64_t k_ld, v_plane;
+};
+
+// q [B,H,Tq,dk], o [B,H,Tq,dv]: contiguous bf16, any Tq and Tk (tiles reaching past them are filled with zeros by TMA and
+// their rows are not stored).  mode = kWin or kCmp.
 // k_lo (compressed branch, or null): low-order bf16 part of the keys, S = Q (k + k_lo)^T; lse2 (or null): receives the
 // log-sum-exp in log2 units.
 int fa_fwd_sm100(const void* q, const void* k, const void* v, void* o, float* L, float* M, int B, int H, int G, int Tq,
                  int Tk, int dk, int dv, int mode, int window, int cmp_l, int cmp_d, int cmp_nb, float scale,
-                 const void* k_lo, float* lse2, cudaStream_t st);
+                 const void* k_lo, float* lse2, const KvLayout& kv, cudaStream_t st);
 
 // Backward of the same two branches.  Adds into dk [B,G,Tk,dk] and dv [B,G,Tk,dv] (time-major, bf16),
 // overwrites dq [B,H,Tq,dk].  Three launches: delta/lse preparation, a query-stationary dQ kernel and
@@ -39,10 +47,17 @@ size_t fa_bwd_sm100_workspace_bytes(int B, int H, int G, int Tq, int Tk, int dk,
 int fa_bwd_sm100(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* L,
                  const float* M, void* dq, void* dk_out, void* dv_out, int B, int H, int G, int Tq, int Tk, int dk, int dv,
                  int mode, int window, int cmp_l, int cmp_d, int cmp_nb, float scale, const float* row_delta,
-                 void* workspace, size_t workspace_bytes, cudaStream_t st);
+                 const KvLayout& kv, void* workspace, size_t workspace_bytes, cudaStream_t st);
 
 // bf16 row-major [rows, cols] matrix -> tensor map with box [box_rows, 64 columns], 128-byte swizzle
-int make_tmap_bf16_2d(::CUtensorMap_st* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
+// (rows `ld` elements apart; 0: contiguous)
+int make_tmap_bf16_2d(::CUtensorMap_st* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint64_t ld = 0);
+// bf16 [planes, rows, cols], contiguous rows, planes `plane` elements apart; same box within one plane: a tile that reaches
+// past a plane's last row is filled with zeros instead of the next plane's rows
+int make_tmap_bf16_3d(::CUtensorMap_st* map, const void* base, uint64_t planes, uint64_t rows, uint64_t cols, uint64_t plane,
+                      uint32_t box_rows);
+// fp32 [rows, cols] -> bf16 hi / lo pair with rows `ld` >= cols elements apart, zeros behind each row
+int split_keys_padded(const float* x, void* hi, void* lo, int64_t rows, int cols, int ld, cudaStream_t st);
 
 // head-major bf16 rows [heads_total][T][width] -> rank-5 map, box = one token's rows of `heads` consecutive heads as
 // [heads/8][width/64][8][64], 128-byte swizzle; coordinates (0, 0, 0, first_head / 8, token)

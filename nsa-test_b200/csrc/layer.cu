@@ -11,6 +11,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "fa_sm100.cuh"
 
 namespace nsa {
 namespace {
@@ -24,6 +25,9 @@ int next_pow2(int n) {
 
 struct Sizes {
   int nb, nbp;
+  int ld_cmp;   // row distance of the compressed keys' I/O-type copies: whole 128-key tiles for the tensor-core kernels
+  int ld_time;  // row distance of the keys the tensor-core kernels read: T, or the next multiple of 8 (keys are copied then)
+  size_t pad_bytes;
   size_t es, rows, o_bytes, stat_bytes;
 };
 Sizes sizes_of(const nsa_layer_desc& d) {
@@ -31,6 +35,10 @@ Sizes sizes_of(const nsa_layer_desc& d) {
   s.nb = d.T >= d.l ? (d.T - d.l) / d.d + 1 : 0;
   s.nbp = next_pow2(s.nb < 1 ? 1 : s.nb);
   s.es = d.dtype == NSA_BF16 ? 2 : 4;
+  s.ld_cmp = d.dtype == NSA_BF16 && s.nb > 0 && nsa_cmp_attn_exact_supported(d.B, d.H, d.G, d.T, s.nbp, d.dk, d.dv, d.dtype)
+                 ? (s.nbp + 127) / 128 * 128 : s.nbp;
+  s.ld_time = d.dtype == NSA_BF16 ? (d.T + 7) / 8 * 8 : d.T;
+  s.pad_bytes = s.ld_time == d.T ? 0 : al256((size_t)d.B * d.G * d.dk * s.ld_time * 2);
   s.rows = (size_t)d.B * d.H * d.T;
   s.o_bytes = al256(s.rows * d.dv * s.es);
   s.stat_bytes = al256(s.rows * sizeof(float));
@@ -49,10 +57,10 @@ void ctx_layout(const nsa_layer_desc& d, size_t off[NSA_CTX_PIECES + 1]) {
   put(NSA_CTX_GATES, s.rows * 3 * sizeof(float));
   put(NSA_CTX_INDICES, BG * d.T * d.n * sizeof(int32_t));
   put(NSA_CTX_K_CMP, BG * d.dk * s.nbp * sizeof(float));
-  put(NSA_CTX_K_CMP_LP, BG * d.dk * s.nbp * s.es);
+  put(NSA_CTX_K_CMP_LP, BG * d.dk * s.ld_cmp * s.es);
   put(NSA_CTX_V_CMP, BG * s.nbp * d.dv * s.es);
   put(NSA_CTX_BLOCK_ENDS, (size_t)s.nbp * sizeof(int32_t));
-  put(NSA_CTX_K_CMP_LO, BG * d.dk * s.nbp * 2);
+  put(NSA_CTX_K_CMP_LO, BG * d.dk * s.ld_cmp * 2);
   put(NSA_CTX_LSE2_CMP, s.stat_bytes);
   put(NSA_CTX_PHI_SAVED, s.nb > 0 ? nsa_cmp_phi_saved_bytes(d.B, d.G, d.T, d.l, d.d, d.U) : 256);
   off[NSA_CTX_PIECES] = o;
@@ -69,10 +77,10 @@ int check_desc(const char* who, const nsa_layer_desc* d) {
   return NSA_OK;
 }
 
-// canonical contiguous strides of the attention entry points
-void fill_strides(const nsa_layer_desc& d, int Tk, int nslots, bool backward, bool selection, int64_t* s) {
+// canonical strides of the attention entry points (key rows `ld` elements apart)
+void fill_strides(const nsa_layer_desc& d, int Tk, int ld, int nslots, bool backward, bool selection, int64_t* s) {
   const int64_t H = d.H, G = d.G, T = d.T, dk = d.dk, dv = d.dv;
-  const int64_t q[4] = {H * T * dk, T * dk, dk, 1}, k[4] = {G * dk * Tk, dk * Tk, 1, Tk}, v[4] = {G * Tk * dv, Tk * dv, dv, 1};
+  const int64_t q[4] = {H * T * dk, T * dk, dk, 1}, k[4] = {G * dk * ld, dk * ld, 1, ld}, v[4] = {G * Tk * dv, Tk * dv, dv, 1};
   const int64_t o[4] = {H * T * dv, T * dv, dv, 1}, lm[3] = {H * T, T, 1};
   int i = 0;
   for (int j = 0; j < 4; ++j) s[i++] = q[j];
@@ -107,6 +115,20 @@ __global__ void selection_fallback_kernel(int32_t* idx, int64_t rows, int T, int
   if (!any) row[0] = (int32_t)((r % T) / lprime);
 }
 
+// rows of T values -> rows of `ld`, zeros behind (keys whose length is no multiple of 8: TMA rows start on 16-byte boundaries)
+__global__ void pad_keys_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int64_t n, int T, int ld) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int c = (int)(i % ld);
+  out[i] = c < T ? in[i / ld * T + c] : __float2bfloat16_rn(0.f);
+}
+const void* pad_keys(const nsa_layer_desc& d, const Sizes& s, const void* k, void* buf, cudaStream_t st) {
+  if (s.pad_bytes == 0) return k;
+  const int64_t n = (int64_t)d.B * d.G * d.dk * s.ld_time;
+  pad_keys_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)k, (__nv_bfloat16*)buf, n, d.T, s.ld_time);
+  return buf;
+}
+
 struct Scratch {
   char* base;
   size_t size, used;
@@ -133,7 +155,7 @@ size_t stage_scratch_bwd(const nsa_layer_desc& d, const Sizes& s) {
 size_t fixed_scratch_bwd(const nsa_layer_desc& d, const Sizes& s) {
   const size_t BG = (size_t)d.B * d.G;
   return 3 * s.o_bytes + 3 * s.stat_bytes + 2 * al256(s.rows * d.dk * s.es) + al256(BG * s.nbp * d.dk * s.es) +
-         al256(BG * s.nbp * d.dv * s.es);
+         al256(BG * s.nbp * d.dv * s.es) + 2 * s.pad_bytes;
 }
 
 }  // namespace
@@ -153,7 +175,7 @@ extern "C" NSA_API size_t nsa_layer_ctx_bytes(const nsa_layer_desc* d, size_t* o
 extern "C" NSA_API size_t nsa_layer_workspace_bytes(const nsa_layer_desc* d, int backward) {
   if (check_desc("layer_workspace_bytes", d)) return 0;
   const Sizes s = sizes_of(*d);
-  return backward ? fixed_scratch_bwd(*d, s) + stage_scratch_bwd(*d, s) + 256 : stage_scratch_fwd(*d, s) + 256;
+  return backward ? fixed_scratch_bwd(*d, s) + stage_scratch_bwd(*d, s) + 256 : stage_scratch_fwd(*d, s) + 2 * s.pad_bytes + 256;
 }
 
 extern "C" NSA_API int nsa_layer_fwd(const nsa_layer_desc* dp, const void* q, const void* k_slc, const void* v_slc, const void* k_cmp_src,
@@ -178,11 +200,16 @@ extern "C" NSA_API int nsa_layer_fwd(const nsa_layer_desc* dp, const void* q, co
   int32_t* be = (int32_t*)piece(NSA_CTX_BLOCK_ENDS);
   int32_t* idx = (int32_t*)piece(NSA_CTX_INDICES);
   const size_t BG = (size_t)d.B * d.G;
+  const void* k_win_p = pad_keys(d, s, k_win, workspace, st);
+  const void* k_slc_p = k_slc == k_win ? k_win_p : pad_keys(d, s, k_slc, (char*)workspace + s.pad_bytes, st);
+  workspace = (char*)workspace + 2 * s.pad_bytes;
+  workspace_bytes -= 2 * s.pad_bytes;
 
   // 1. block compression (a sequence shorter than one block leaves only the never-visible padding block)
+  const bool exact = s.nb > 0 && nsa_cmp_attn_exact_supported(d.B, d.H, d.G, d.T, s.nbp, d.dk, d.dv, d.dtype) != 0;
   block_ends_kernel<<<(s.nbp + 255) / 256, 256, 0, st>>>(be, s.nbp, s.nb, d.l, d.d);
   if (s.nb > 0) {
-    if (int rc = nsa_cmp_phi_fwd(k_cmp_src, v_cmp_src, pos_embed, w1, b1, w2, b2, k_cmp, piece(NSA_CTX_K_CMP_LP), piece(NSA_CTX_V_CMP),
+    if (int rc = nsa_cmp_phi_fwd(k_cmp_src, v_cmp_src, pos_embed, w1, b1, w2, b2, k_cmp, exact ? nullptr : piece(NSA_CTX_K_CMP_LP), piece(NSA_CTX_V_CMP),
                                  d.B, d.G, d.T, d.dk, d.dv, d.l, d.d, d.U, s.nbp, d.dtype, piece(NSA_CTX_PHI_SAVED),
                                  off[NSA_CTX_PHI_SAVED + 1] - off[NSA_CTX_PHI_SAVED], workspace, workspace_bytes, stream))
       return rc;
@@ -195,12 +222,11 @@ extern "C" NSA_API int nsa_layer_fwd(const nsa_layer_desc* dp, const void* q, co
   // 2. compressed attention.  On the tensor-core path it takes the keys as a bf16 pair hi + lo (the fp32 keys to 16
   //    mantissa bits) and also emits the log-sum-exp of its logits, the normaliser the scoring needs: the scoring
   //    kernel then makes one sweep over the compressed keys instead of two.
-  const bool exact = s.nb > 0 && nsa_cmp_attn_exact_supported(d.B, d.H, d.G, d.T, s.nbp, d.dk, d.dv, d.dtype) != 0;
   float* lse2 = exact ? (float*)piece(NSA_CTX_LSE2_CMP) : nullptr;
   void* k_lo = exact ? piece(NSA_CTX_K_CMP_LO) : nullptr;
   if (exact)
-    if (int rc = nsa_split_keys_hi_lo(k_cmp, piece(NSA_CTX_K_CMP_LP), k_lo, (int64_t)BG * d.dk * s.nbp, stream)) return rc;
-  fill_strides(d, s.nbp, 0, false, false, strides);
+    if (int rc = split_keys_padded(k_cmp, piece(NSA_CTX_K_CMP_LP), k_lo, (int64_t)BG * d.dk, s.nbp, s.ld_cmp, st)) return rc;
+  fill_strides(d, s.nbp, s.ld_cmp, 0, false, false, strides);
   if (int rc = nsa_cmp_attn_fwd(q, piece(NSA_CTX_K_CMP_LP), piece(NSA_CTX_V_CMP), be, piece(NSA_CTX_O_CMP), (float*)piece(NSA_CTX_L_CMP),
                                 (float*)piece(NSA_CTX_M_CMP), strides, d.B, d.H, d.G, d.T, s.nbp, d.dk, d.dv, d.scale, d.dtype, d.l, d.d,
                                 s.nb, 0, 0, k_lo, lse2, stream))
@@ -220,13 +246,13 @@ extern "C" NSA_API int nsa_layer_fwd(const nsa_layer_desc* dp, const void* q, co
   }
   if (int rc = check_launch("layer_fwd")) return rc;
   // 4. sliding window
-  fill_strides(d, d.T, 0, false, false, strides);
-  if (int rc = nsa_sliding_fwd(q, k_win, v_win, piece(NSA_CTX_O_WIN), (float*)piece(NSA_CTX_L_WIN), (float*)piece(NSA_CTX_M_WIN), strides,
+  fill_strides(d, d.T, s.ld_time, 0, false, false, strides);
+  if (int rc = nsa_sliding_fwd(q, k_win_p, v_win, piece(NSA_CTX_O_WIN), (float*)piece(NSA_CTX_L_WIN), (float*)piece(NSA_CTX_M_WIN), strides,
                                d.B, d.H, d.G, d.T, d.dk, d.dv, d.window, d.scale, d.dtype, 0, stream))
     return rc;
   // 5. selected-block attention with the gate + mix as its epilogue
-  fill_strides(d, d.T, d.n, false, true, strides);
-  return nsa_slc_fwd_mix(q, k_slc, v_slc, idx, piece(NSA_CTX_O_SLC), (float*)piece(NSA_CTX_L_SLC), (float*)piece(NSA_CTX_M_SLC), strides,
+  fill_strides(d, d.T, s.ld_time, d.n, false, true, strides);
+  return nsa_slc_fwd_mix(q, k_slc_p, v_slc, idx, piece(NSA_CTX_O_SLC), (float*)piece(NSA_CTX_L_SLC), (float*)piece(NSA_CTX_M_SLC), strides,
                          d.B, d.H, d.G, d.T, d.T, d.n, d.l_prime, d.dk, d.dv, d.scale, d.dtype, 0, 0, gate_logits,
                          piece(NSA_CTX_O_CMP), piece(NSA_CTX_O_WIN), out, (float*)piece(NSA_CTX_GATES), d.gate_mode,
                          d.out_token_major, workspace, workspace_bytes, stream);
@@ -257,6 +283,9 @@ extern "C" NSA_API int nsa_layer_bwd(const nsa_layer_desc* dp, const void* q, co
   float* delta = (float*)sc.take(3 * s.stat_bytes);
   void *dq_c = sc.take(s.rows * d.dk * s.es), *dq_w = sc.take(s.rows * d.dk * s.es);
   void *dkc = sc.take(BG * s.nbp * d.dk * s.es), *dvc = sc.take(BG * s.nbp * d.dv * s.es);
+  void *pad0 = sc.take(s.pad_bytes), *pad1 = sc.take(s.pad_bytes);
+  const void* k_win_p = pad_keys(d, s, k_win, pad0, st);
+  const void* k_slc_p = k_slc == k_win ? k_win_p : pad_keys(d, s, k_slc, pad1, st);
   void* stage = sc.base + sc.used;
   const size_t stage_bytes = workspace_bytes - sc.used;
   // delta holds three vectors of B*H*T floats back to back (the gate/mix backward's layout), not padded ones
@@ -270,18 +299,18 @@ extern "C" NSA_API int nsa_layer_bwd(const nsa_layer_desc* dp, const void* q, co
   const int32_t* be = (const int32_t*)piece(NSA_CTX_BLOCK_ENDS);
   cudaMemsetAsync(dkc, 0, BG * s.nbp * d.dk * s.es, st);
   cudaMemsetAsync(dvc, 0, BG * s.nbp * d.dv * s.es, st);
-  fill_strides(d, s.nbp, 0, true, false, strides);
+  fill_strides(d, s.nbp, s.ld_cmp, 0, true, false, strides);
   if (int rc = nsa_cmp_attn_bwd(q, piece(NSA_CTX_K_CMP_LP), piece(NSA_CTX_V_CMP), be, piece(NSA_CTX_O_CMP), d_cmp,
                                 (const float*)piece(NSA_CTX_L_CMP), (const float*)piece(NSA_CTX_M_CMP), dq_c, dkc, dvc, strides, d.B, d.H, d.G,
                                 d.T, s.nbp, d.dk, d.dv, d.scale, d.dtype, d.l, d.d, s.nb, 0, delta0, 0, stage, stage_bytes, stream))
     return rc;
-  fill_strides(d, d.T, 0, true, false, strides);
-  if (int rc = nsa_sliding_bwd(q, k_win, v_win, piece(NSA_CTX_O_WIN), d_win, (const float*)piece(NSA_CTX_L_WIN),
+  fill_strides(d, d.T, s.ld_time, 0, true, false, strides);
+  if (int rc = nsa_sliding_bwd(q, k_win_p, v_win, piece(NSA_CTX_O_WIN), d_win, (const float*)piece(NSA_CTX_L_WIN),
                                (const float*)piece(NSA_CTX_M_WIN), dq_w, dk_win, dv_win, strides, d.B, d.H, d.G, d.T, d.dk, d.dv, d.window,
                                d.scale, d.dtype, delta2, 0, stage, stage_bytes, stream))
     return rc;
-  fill_strides(d, d.T, d.n, true, true, strides);
-  if (int rc = nsa_slc_bwd(q, k_slc, v_slc, (const int32_t*)piece(NSA_CTX_INDICES), piece(NSA_CTX_O_SLC), d_slc,
+  fill_strides(d, d.T, s.ld_time, d.n, true, true, strides);
+  if (int rc = nsa_slc_bwd(q, k_slc_p, v_slc, (const int32_t*)piece(NSA_CTX_INDICES), piece(NSA_CTX_O_SLC), d_slc,
                            (const float*)piece(NSA_CTX_L_SLC), (const float*)piece(NSA_CTX_M_SLC), dq, dk_slc, dv_slc, strides, d.B, d.H, d.G,
                            d.T, d.T, d.n, d.l_prime, d.dk, d.dv, d.scale, d.dtype, 0, delta1, dq_c, dq_w, 0, stage, stage_bytes, stream))
     return rc;

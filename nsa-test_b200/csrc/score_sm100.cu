@@ -1,6 +1,6 @@
 // Selection scoring on tcgen05 tensor cores: Eq. 8 -> 9 -> 10/11 fused, nothing of size [B,H,T,n_cmp]
 // leaves the SM (replaces the torch code of nsa/kernels.py:2304-2343, 1920-1962, 1965-2040 for bf16
-// queries in the canonical layout, l = 2d, block counts that are multiples of 128).
+// queries in the canonical layout, l = 2d).
 //
 // Bit-exact top-n against an fp32 oracle needs logits far more accurate than bf16 keys give, so the fp32
 // compressed keys are split into bf16 hi + lo parts and every logit tile is S = Q K_hi^T + Q K_lo^T
@@ -37,11 +37,13 @@ struct ScoreParams {
   const float* lse2_ext;  // [B,H,T] log-sum-exp (log2 units) from the compressed attention's exact forward, or null (own first sweep)
 };
 
+// rows of `cols` values -> rows of `ld` >= cols, zeros behind
 __global__ void split_hi_lo_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo,
-                                   int64_t n) {
+                                   int64_t n, int cols, int ld) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const float v = x[i];
+  const int c = (int)(i % ld);
+  const float v = c < cols ? x[i / ld * cols + c] : 0.f;
   const __nv_bfloat16 h = __float2bfloat16_rn(v);
   hi[i] = h;
   lo[i] = __float2bfloat16_rn(v - __bfloat162float(h));
@@ -129,7 +131,7 @@ score_topn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (elect_one()) {
         mbar_arrive_expect_tx(&bar->q_full[s], kQ);
         for (int c = 0; c < DK / 64; ++c)
-          tma_load_2d(&tmQ, &bar->q_full[s], sQ + s * kQ + c * 16384, c * 64, (b * p.H + g * hpg + hh) * p.T + m0);
+          tma_load_3d(&tmQ, &bar->q_full[s], sQ + s * kQ + c * 16384, c * 64, m0, b * p.H + g * hpg + hh);
       }
       __syncwarp();
       qissued = step + 1;
@@ -240,7 +242,7 @@ score_topn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       } else {
         float lse2;
         if (p.lse2_ext) {
-          lse2 = p.lse2_ext[((int64_t)b * p.H + g * hpg + hh) * p.T + t];
+          lse2 = t < p.T ? p.lse2_ext[((int64_t)b * p.H + g * hpg + hh) * p.T + t] : CUDART_INF_F;
         } else {
           const float m_h = st_m[hh * 128 + r], l_h = st_l[hh * 128 + r];
           lse2 = l_h > 0.f ? m_h + log2f(l_h) : CUDART_INF_F;
@@ -298,11 +300,13 @@ score_topn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           // Streaming over the keys: key i ends the previous block when i % s_ == 0 and otherwise enters the
           // current block twice in a row; the block that straddles the tile end is finished by the next tile.
           float* sdst = srow + (n0 >> sshift) - 1;
+          // blocks of this tile that exist (fewer than per_tile only where all compressed blocks fit in one tile)
+          const int nblk = t < p.T ? min(per_tile, p.n_sel - (n0 >> sshift)) : -1;
 #pragma unroll
           for (int i = 0; i < 128; ++i) {
             const float av = agg[i];
             if ((i & smask) == 0) {
-              if (kt > 0 || i > 0) sdst[i >> sshift] = cur + av;
+              if ((kt > 0 || i > 0) && (i >> sshift) <= nblk) sdst[i >> sshift] = cur + av;
               cur = av;
             } else {
               cur = (cur + av) + av;
@@ -312,7 +316,7 @@ score_topn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
     }
     // the last block's final term lies beyond every visible key: + 0
-    if (ok && wg == 0) srow[ntiles * per_tile - 1] = cur;
+    if (ok && wg == 0 && t < p.T && ntiles * per_tile <= p.n_sel) srow[ntiles * per_tile - 1] = cur;
   }
   tc_fence_before();
   __syncthreads();
@@ -477,16 +481,23 @@ bool score_sm100_supported(int H, int G, int T, int dk, int nbp, int l, int d, i
   const int s_ = lprime / d;
   const size_t smem = 4 * (size_t)128 * dk * 2 + 2 * (size_t)hpg * 512 + 256 + 1024;
   const size_t rows_smem = 4 * (size_t)(nbp / (s_ > 0 ? s_ : 1)) * sizeof(float);
-  return smem <= 227 * 1024 && rows_smem <= 200 * 1024 && T % 128 == 0 && nbp % 128 == 0 && 128 % s_ == 0 && n >= 1 &&
+  return smem <= 227 * 1024 && rows_smem <= 200 * 1024 && T > 0 && nbp > 0 && 128 % s_ == 0 && n >= 1 &&
          n <= kScoreMaxN;
 }
 
 static size_t al256s(size_t x) { return (x + 255) & ~size_t(255); }
+static int key_ld(int nbp) { return (nbp + 127) / 128 * 128; }   // whole key tiles in the bf16 copies
 
 // bf16 hi and lo copies of the compressed keys + the [B,G,T,n_sel] block scores
 size_t score_sm100_workspace_bytes(int B, int G, int T, int dk, int nbp, int d, int lprime) {
-  const size_t n_sel = (size_t)nbp / (size_t)(lprime / d);
-  return 2 * al256s((size_t)B * G * dk * nbp * 2) + al256s((size_t)B * G * T * n_sel * sizeof(float));
+  const size_t s_ = lprime / d, n_sel = ((size_t)nbp + s_ - 1) / s_;
+  return 2 * al256s((size_t)B * G * dk * key_ld(nbp) * 2) + al256s((size_t)B * G * T * n_sel * sizeof(float));
+}
+
+int split_keys_padded(const float* x, void* hi, void* lo, int64_t rows, int cols, int ld, cudaStream_t st) {
+  const int64_t n = rows * ld;
+  split_hi_lo_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(x, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n, cols, ld);
+  return check_launch("split_hi_lo");
 }
 
 template <int DK>
@@ -502,7 +513,7 @@ static int launch_score_t(const CUtensorMap& tq, const CUtensorMap& thi, const C
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
     return fail(NSA_ERR_LAUNCH, "score_topn: cannot reserve shared memory");
   KernelTimer kt("score_topn_tc", st);
-  kern<<<dim3(p.T / 128, p.B * p.G), 384, dyn, st>>>(tq, thi, tlo, p, hpg, state_off, bar_off);
+  kern<<<dim3((p.T + 127) / 128, p.B * p.G), 384, dyn, st>>>(tq, thi, tlo, p, hpg, state_off, bar_off);
   return check_launch("score_topn_tc");
 }
 
@@ -513,21 +524,20 @@ int score_topn_sm100(const void* q, const float* k_cmp, int32_t* out, int B, int
   const size_t need = score_sm100_workspace_bytes(B, G, T, dk, nbp, d, lprime);
   if (!workspace || workspace_bytes < need)
     return fail(NSA_ERR_WORKSPACE, "scoring needs %zu workspace bytes, got %zu", need, workspace_bytes);
-  const size_t key_bytes = al256s((size_t)B * G * dk * nbp * 2);
+  const int ld = key_ld(nbp);
+  const size_t key_bytes = al256s((size_t)B * G * dk * ld * 2);
   __nv_bfloat16* hi = (__nv_bfloat16*)workspace;
   __nv_bfloat16* lo = (__nv_bfloat16*)((char*)workspace + key_bytes);
   float* sel = (float*)((char*)workspace + 2 * key_bytes);
-  const int64_t nk = (int64_t)B * G * dk * nbp;
   {
     KernelTimer kt("score_split_keys", st);
-    split_hi_lo_kernel<<<(unsigned)((nk + 255) / 256), 256, 0, st>>>(k_cmp, hi, lo, nk);
+    if (int rc = split_keys_padded(k_cmp, hi, lo, (int64_t)B * G * dk, nbp, ld, st)) return rc;
   }
-  if (int rc = check_launch("split_hi_lo")) return rc;
   CUtensorMap tq, thi, tlo;
-  if (int rc = make_tmap_bf16_2d(&tq, q, (uint64_t)B * H * T, dk, 128)) return rc;
-  if (int rc = make_tmap_bf16_2d(&thi, hi, (uint64_t)B * G * dk, nbp, dk)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tlo, lo, (uint64_t)B * G * dk, nbp, dk)) return rc;
-  const int s_ = lprime / d, n_sel = nbp / s_;
+  if (int rc = make_tmap_bf16_3d(&tq, q, (uint64_t)B * H, T, dk, (uint64_t)T * dk, 128)) return rc;
+  if (int rc = make_tmap_bf16_2d(&thi, hi, (uint64_t)B * G * dk, ld, dk)) return rc;
+  if (int rc = make_tmap_bf16_2d(&tlo, lo, (uint64_t)B * G * dk, ld, dk)) return rc;
+  const int s_ = lprime / d, n_sel = (nbp + s_ - 1) / s_;
   ScoreParams p;
   p.sel = sel;
   p.q0 = q0;
@@ -570,6 +580,6 @@ int score_topn_sm100(const void* q, const float* k_cmp, int32_t* out, int B, int
 extern "C" NSA_API int nsa_split_keys_hi_lo(const float* x, void* hi, void* lo, int64_t n, void* stream) {
   NSA_REQUIRE(x && hi && lo && n >= 0, "split_keys_hi_lo: bad arguments");
   if (n == 0) return NSA_OK;
-  nsa::split_hi_lo_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(x, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n);
+  nsa::split_hi_lo_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(x, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo, n, 1, 1);
   return nsa::check_launch("split_keys_hi_lo");
 }

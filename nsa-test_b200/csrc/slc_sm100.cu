@@ -201,7 +201,7 @@ slc_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
           mbar_arrive_expect_tx(&bar->kv_full[ks], SM::kK + SM::kV);
           tma_load_2d(&tmK, &bar->kv_full[ks], sK + ks * SM::kK, w.blk * 64, (b * p.G + g) * DK);
           for (int cc = 0; cc < DV / 64; ++cc)
-            tma_load_2d(&tmV, &bar->kv_full[ks], sV + ks * SM::kV + cc * 8192, cc * 64, (b * p.G + g) * p.Tk + w.blk * 64);
+            tma_load_3d(&tmV, &bar->kv_full[ks], sV + ks * SM::kV + cc * 8192, cc * 64, w.blk * 64, b * p.G + g);
         }
       }
       // this chunk's entries are fetched while the stage is still busy
@@ -328,7 +328,7 @@ slc_fwd_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
       tmem_ld32(tmem + lane_base + buf * 192, sv[0]);
       tmem_ld32(tmem + lane_base + buf * 192 + 32, sv[1]);
       tc_wait_ld();
-      const int chi = valid ? p.q0 + t - key0 : 63;  // causal: keys key0 + c <= position of the query
+      const int chi = valid ? min(p.q0 + t, p.Tk - 1) - key0 : 63;  // causal: keys key0 + c <= position of the query
       float mx = -CUDART_INF_F;
 #pragma unroll
       for (int cc = 0; cc < 2; ++cc)
@@ -835,7 +835,7 @@ slc_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
           mbar_arrive_expect_tx(&bar->kv_full, SM::kK + SM::kV);
           tma_load_2d(&tmK, &bar->kv_full, sK, w.blk * 64, (b * p.G + g) * DK);
           for (int cc = 0; cc < DV / 64; ++cc)
-            tma_load_2d(&tmV, &bar->kv_full, sV + cc * 8192, cc * 64, (b * p.G + g) * p.Tk + w.blk * 64);
+            tma_load_3d(&tmV, &bar->kv_full, sV + cc * 8192, cc * 64, w.blk * 64, b * p.G + g);
         }
       }
       const int s = c & 1;
@@ -1062,7 +1062,7 @@ slc_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
       const int entry = ent_next;
       const float lse2 = lse_next, Dr = D_next;
       const int t = entry < 0 ? -1 : (entry & 0xFFFFFF), slot = entry < 0 ? 0 : (entry >> 24);
-      const int chi = t < 0 ? -1 : p.q0 + t - w.blk * 64;
+      const int chi = t < 0 ? -1 : min(p.q0 + t, p.Tk - 1) - w.blk * 64;
       {  // this group's next chunk: fetch its statistics one chunk ahead
         ChunkWalker w2 = w;
         w2.next();
@@ -1182,6 +1182,7 @@ __global__ void slc_reduce_dkv_kernel(const float* __restrict__ dk_part, const f
       acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
     }
     const float mul = is_k ? scale : 1.f;
+    if (blk * 64 + r >= Tk) break;   // r only grows
     const int64_t krow = (int64_t)bg * Tk + blk * 64 + r;
     __nv_bfloat16* dst = (is_k ? dk : dv) + krow * width + col;
     uint2 raw = *reinterpret_cast<const uint2*>(dst);
@@ -1204,7 +1205,7 @@ bool slc_sm100_supported(int H, int G, int Tq, int Tk, int dk, int dv, int nslot
   const bool dims = (dk == 192 && dv == 128) || (dk == 128 && dv == 128) || (dk == 64 && dv == 64);
   if (!dims || G <= 0 || H % G != 0) return false;
   const int hpg = H / G;
-  return hpg <= 128 && 128 % hpg == 0 && lprime == 64 && Tk % 64 == 0 && Tk > 0 && Tq > 0 && Tq < (1 << 24) &&
+  return hpg <= 128 && 128 % hpg == 0 && lprime == 64 && Tk > 0 && Tq > 0 && Tq < (1 << 24) &&
          nslots > 0 && nslots <= 32;  // (the caller also keeps B*H*Tq below 2^31: rows are 32-bit TMA coordinates)
 }
 
@@ -1259,7 +1260,7 @@ static int launch_slc_fwd_t(const CUtensorMap& tk, const CUtensorMap& tv, const 
 
 int slc_fwd_sm100(const void* q, const void* k, const void* v, const int* indices, const int64_t* sidx, void* out, float* L,
                   float* M, int B, int H, int G, int Tq, int Tk, int dk, int dv, int nslots, int lprime, float scale, int q0,
-                  const SlcMix& mix, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+                  const SlcMix& mix, const KvLayout& kv, void* workspace, size_t workspace_bytes, cudaStream_t st) {
   if (!slc_sm100_supported(H, G, Tq, Tk, dk, dv, nslots, lprime)) return fail(NSA_ERR_UNSUPPORTED, "slc_fwd_sm100: unsupported shape");
   const size_t need = slc_fwd_sm100_workspace_bytes(B, H, G, Tq, Tk, dk, dv, nslots, lprime);
   if (!workspace || workspace_bytes < need)
@@ -1278,8 +1279,8 @@ int slc_fwd_sm100(const void* q, const void* k, const void* v, const int* indice
   p.scale = scale; p.scale_log2 = scale * kLog2ef;
   p.timeouts = fa_timeout_counter();
   CUtensorMap tk, tv;
-  if (int rc = make_tmap_bf16_2d(&tk, k, (uint64_t)B * G * dk, Tk, dk)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tv, v, (uint64_t)B * G * Tk, dv, 64)) return rc;
+  if (int rc = make_tmap_bf16_2d(&tk, k, (uint64_t)B * G * dk, Tk, dk, kv.k_ld)) return rc;
+  if (int rc = make_tmap_bf16_3d(&tv, v, (uint64_t)B * G, Tk, dv, kv.v_plane, 64)) return rc;
   CUtensorMap tqt;
   // heads of a group filling whole 8-row swizzle atoms: one rank-5 tile load per query straight from q; otherwise the
   // rows of a query are first made contiguous (token-major copy) and fetched with one 2-D tile per 64 columns
@@ -1363,7 +1364,8 @@ static int launch_slc_bwd_t(const CUtensorMap& tk, const CUtensorMap& tv, const 
 int slc_bwd_sm100(const void* q, const void* k, const void* v, const int* indices, const int64_t* sidx, const void* out,
                   const void* dout, const float* L, const float* M, void* dq, void* dk_out, void* dv_out, int B, int H, int G,
                   int Tq, int Tk, int dk, int dv, int nslots, int lprime, float scale, int q0, const float* row_delta,
-                  const void* dq_add0, const void* dq_add1, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+                  const void* dq_add0, const void* dq_add1, const KvLayout& kv, void* workspace, size_t workspace_bytes,
+                  cudaStream_t st) {
   if (!slc_sm100_supported(H, G, Tq, Tk, dk, dv, nslots, lprime)) return fail(NSA_ERR_UNSUPPORTED, "slc_bwd_sm100: unsupported shape");
   size_t o_stat, o_dq, o_dk, o_dv, o_qt, o_dot, need;
   slc_bwd_layout(B, H, G, Tq, Tk, dk, dv, nslots, lprime, &o_stat, &o_dq, &o_dk, &o_dv, &o_qt, &o_dot, &need);
@@ -1387,8 +1389,8 @@ int slc_bwd_sm100(const void* q, const void* k, const void* v, const int* indice
   p.scale = scale; p.scale_log2 = scale * kLog2ef;
   p.timeouts = fa_timeout_counter();
   CUtensorMap tk, tv;
-  if (int rc = make_tmap_bf16_2d(&tk, k, (uint64_t)B * G * dk, Tk, dk)) return rc;
-  if (int rc = make_tmap_bf16_2d(&tv, v, (uint64_t)B * G * Tk, dv, 64)) return rc;
+  if (int rc = make_tmap_bf16_2d(&tk, k, (uint64_t)B * G * dk, Tk, dk, kv.k_ld)) return rc;
+  if (int rc = make_tmap_bf16_3d(&tv, v, (uint64_t)B * G, Tk, dv, kv.v_plane, 64)) return rc;
   CUtensorMap tqt, tdot;
   p.g5 = (H / G) % 8 == 0 ? 1 : 0;  // whole 8-row swizzle atoms per query: one rank-5 tile load per query and tensor
   if (p.g5) {

@@ -3,9 +3,11 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fa_sm100.cuh"
+
 namespace nsa {
 
-// bf16, canonical contiguous layouts, 64-key selection blocks, heads-per-group dividing 128
+// bf16, canonical layouts (keys and values as KvLayout says), 64-key selection blocks, heads-per-group dividing 128
 bool slc_sm100_supported(int H, int G, int Tq, int Tk, int dk, int dv, int nslots, int lprime);
 
 // Gate + mix epilogue of the selection forward (out == null: none).  The kernel that merges a query's per-slot partials
@@ -23,7 +25,7 @@ struct SlcMix {
 size_t slc_fwd_sm100_workspace_bytes(int B, int H, int G, int Tq, int Tk, int dk, int dv, int nslots, int lprime);
 int slc_fwd_sm100(const void* q, const void* k, const void* v, const int* indices, const int64_t* sidx, void* out, float* L,
                   float* M, int B, int H, int G, int Tq, int Tk, int dk, int dv, int nslots, int lprime, float scale, int q0,
-                  const SlcMix& mix, void* workspace, size_t workspace_bytes, cudaStream_t st);
+                  const SlcMix& mix, const KvLayout& kv, void* workspace, size_t workspace_bytes, cudaStream_t st);
 
 
 // row_delta: row sums dO.O [B,H,Tq] fp32 or null (computed here); dq_add0/1: dQ of the other branches (bf16, laid out like
@@ -32,6 +34,7 @@ size_t slc_bwd_sm100_workspace_bytes(int B, int H, int G, int Tq, int Tk, int dk
 int slc_bwd_sm100(const void* q, const void* k, const void* v, const int* indices, const int64_t* sidx, const void* out,
                   const void* dout, const float* L, const float* M, void* dq, void* dk_out, void* dv_out, int B, int H, int G,
                   int Tq, int Tk, int dk, int dv, int nslots, int lprime, float scale, int q0, const float* row_delta,
-                  const void* dq_add0, const void* dq_add1, void* workspace, size_t workspace_bytes, cudaStream_t st);
+                  const void* dq_add0, const void* dq_add1, const KvLayout& kv, void* workspace, size_t workspace_bytes,
+                  cudaStream_t st);
 
 }  // namespace nsa

@@ -20,6 +20,17 @@ def _k_strides(k: torch.Tensor):
     return [k.stride(0), k.stride(1), k.stride(3), k.stride(2)]
 
 
+def _tc_keys(q, k, generic: bool = False):
+    """Keys the tensor-core kernels can fetch: bf16 rows start on 16-byte boundaries, so a length that is no multiple of 8
+    is served from a copy with padded rows (a view of the same shape)."""
+    T = k.shape[-1]
+    if generic or q.dtype != torch.bfloat16 or T % 8 == 0 or T == 0 or k.dtype != q.dtype:
+        return k
+    buf = k.new_zeros(*k.shape[:-1], (T + 7) // 8 * 8)
+    buf[..., :T] = k
+    return buf[..., :T]
+
+
 def _fwd_strides(q, k, v, o, L, M):
     return list(q.stride()) + _k_strides(k) + list(v.stride()) + list(o.stride()) + list(L.stride()) + list(M.stride())
 
@@ -38,6 +49,7 @@ def _stats(q, o_dv):
 
 def sliding_fwd(q, k, v, window: int, scale: float, generic: bool = False):
     """``generic=True`` forces the stride-generic kernels (cross-checks); same for the functions below."""
+    k = _tc_keys(q, k, generic)
     dev = require_cuda(q, k, v)
     B, H, T, dk = q.shape
     G, dv = k.shape[1], v.shape[-1]
@@ -53,6 +65,7 @@ def sliding_bwd(q, k, v, o, do, L, M, window: int, scale: float, row_delta=None,
                 recompute: bool = False):
     """``row_delta``: the row sums dO.O [B,H,T] (fp32) when the caller has them, else they are computed here.
     ``recompute``: small scratch; the dQ kernel recomputes S and dP instead of taking dS from the dK/dV kernel."""
+    k = _tc_keys(q, k, generic)
     dev = require_cuda(q, k, v, o, do, L, M)
     delta, dptr = _delta_ptr(row_delta, q)
     B, H, T, dk = q.shape
@@ -111,6 +124,8 @@ def cmp_attn_fwd(q, k_cmp, v_cmp, block_ends, scale: float, blocks=None, q_pos0:
     k_cmp being the high-order one) selects the exact-key form; a fourth result, the log-sum-exp of the logits in log2
     units (+inf on rows that see no block), is then returned for score_topn's ``cmp_lse2``."""
     bl, bd, bn = blocks if blocks is not None else (0, 0, 0)
+    k_cmp = _tc_keys(q, k_cmp, generic)
+    k_lo = None if k_lo is None else _tc_keys(q, k_lo, generic)
     dev = require_cuda(q, k_cmp, v_cmp, block_ends)
     B, H, T, dk = q.shape
     G, NB, dv = k_cmp.shape[1], k_cmp.shape[-1], v_cmp.shape[-1]
@@ -128,6 +143,7 @@ def cmp_attn_fwd(q, k_cmp, v_cmp, block_ends, scale: float, blocks=None, q_pos0:
 def cmp_attn_bwd(q, k_cmp, v_cmp, block_ends, o, do, L, M, scale: float, blocks=None, q_pos0: int = 0, row_delta=None,
                  generic: bool = False, recompute: bool = False):
     bl, bd, bn = blocks if blocks is not None else (0, 0, 0)
+    k_cmp = _tc_keys(q, k_cmp, generic)
     dev = require_cuda(q, k_cmp, v_cmp, block_ends, o, do, L, M)
     delta, dptr = _delta_ptr(row_delta, q)
     B, H, T, dk = q.shape
@@ -151,6 +167,7 @@ def cmp_attn_bwd(q, k_cmp, v_cmp, block_ends, o, do, L, M, scale: float, blocks=
 
 
 def slc_fwd(q, k, v, indices_i32, l_prime: int, scale: float, q_pos0: int = 0, generic: bool = False):
+    k = _tc_keys(q, k, generic)
     dev = require_cuda(q, k, v, indices_i32)
     B, H, Tq, dk = q.shape
     G, Tkv, dv = k.shape[1], k.shape[-1], v.shape[-1]
@@ -179,6 +196,7 @@ def _mixed_empty(like: torch.Tensor, token_major: bool) -> torch.Tensor:
 def slc_fwd_mix(q, k, v, indices_i32, l_prime: int, scale: float, gate_logits, o_cmp, o_win, gate_mode: str, q_pos0: int = 0,
                 token_major: bool = False, generic: bool = False):
     """Selection forward with the layer's gate + mix as its epilogue -> (o_slc, L, M, out_mixed, gates [B,H,T,3])."""
+    k = _tc_keys(q, k, generic)
     dev = require_cuda(q, k, v, indices_i32, gate_logits, o_cmp, o_win)
     B, H, Tq, dk = q.shape
     G, Tkv, dv = k.shape[1], k.shape[-1], v.shape[-1]
@@ -205,6 +223,7 @@ def slc_bwd(q, k, v, indices_i32, o, do, L, M, l_prime: int, scale: float, q_pos
             generic: bool = False):
     """``dq_addends``: up to two tensors shaped and typed like q (the dQ of the other branches) that the kernel adds
     to the selection branch's dQ before the one rounding of the sum."""
+    k = _tc_keys(q, k, generic)
     dev = require_cuda(q, k, v, indices_i32, o, do, L, M)
     delta, dptr = _delta_ptr(row_delta, q)
     B, H, Tq, dk = q.shape
@@ -471,7 +490,7 @@ def layer_ctx_views(desc, ctx: torch.Tensor):
                   o_slc=((B, H, T, dv), dt), L_slc=((B, H, T), torch.float32), M_slc=((B, H, T), torch.float32),
                   o_win=((B, H, T, dv), dt), L_win=((B, H, T), torch.float32), M_win=((B, H, T), torch.float32),
                   gates=((B, H, T, 3), torch.float32), indices=((B, G, T, n), torch.int32),
-                  k_cmp=((B, G, dk, nbp), torch.float32), k_cmp_lp=((B, G, dk, nbp), dt), v_cmp=((B, G, nbp, dv), dt),
+                  k_cmp=((B, G, dk, nbp), torch.float32), v_cmp=((B, G, nbp, dv), dt),
                   block_ends=((nbp,), torch.int32))
     out = {}
     for i, name in enumerate(_lib.CTX_PIECES):

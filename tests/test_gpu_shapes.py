@@ -33,3 +33,40 @@ def test_selection_over_ragged_chunks_and_short_ranges(dk, dv, H, G, T, n):
     _grad_close(dq, gq, "dq")
     _grad_close(dkey, gk.transpose(-1, -2), "dk")
     _grad_close(dval, gv, "dv")
+
+
+@pytest.mark.parametrize("T", [20, 33, 100, 129, 200, 637, 1030])
+@pytest.mark.parametrize("dk,dv,H,G", [(64, 64, 4, 2), (192, 128, 16, 1)])
+def test_bf16_layer_at_any_length(dk, dv, H, G, T):
+    """Sequences that are no multiple of a tile, of 64 or of 8, shorter than a key tile, and with fewer compressed blocks
+    than a tile holds run on the tensor-core kernels: ids, outputs and all gradients against the oracle."""
+    import nsa
+    from nsa import _lib
+    from nsa.kernels import nsa_layer
+    from tests.util import check_layer_against_oracle
+    c = dict(B=2, H=H, G=G, T=T, dk=dk, dv=dv, d_model=64, l=32, d=16, l_prime=64, n=16, w=150)
+    inp = O.make_inputs(2, H, G, T, dk, dv, 64, 32, seed=T, block_offset_std=0.5, dtype=torch.bfloat16)
+    check_layer_against_oracle(f"bf16 layer dk={dk} T={T}", nsa, c, inp, torch.bfloat16)
+    _no_timeouts()
+    if T >= 32:
+        cfg = nsa.NSAConfig(d_model=64, head_dim_qk=dk, head_dim_v=dv, n_heads=H, n_kv_groups=G, w=150)
+        q, k, v = (inp[x].to(DEV, torch.bfloat16).requires_grad_(True) for x in ("q", "k", "v"))
+        phi = tuple(getattr(inp["phi"], n_).to(DEV) for n_ in ("pos_embed", "w1", "b1", "w2", "b2"))
+        logits = torch.zeros(2, T, 3 * H, device=DEV)
+        ran = _lib.profile_kernels(lambda: torch.autograd.grad(nsa_layer(q, k, v, logits, phi, cfg).sum(), (q, k, v)))
+        assert {"fa_fwd_win", "fa_fwd_cmp_exact", "slc_bwd_fused", "fa_bwd_dkv_cmp", "fa_bwd_dqds_win"} <= set(ran), ran
+
+
+@pytest.mark.parametrize("Tk,lo", [(384, 128), (200, 72)])
+def test_keys_and_values_read_as_slices_of_a_longer_buffer(Tk, lo):
+    """Keys with padded rows and time slices of a longer key/value buffer are read where they lie."""
+    from nsa import ops
+    B, H, G, dk, dv = 2, 4, 2, 64, 64
+    q, _, _, _ = _inputs(B, H, G, Tk, dk, dv, seed=3)
+    _, k, v, _ = _inputs(B, H, G, 1024, dk, dv, seed=4)
+    ks, vs = k[..., lo:lo + Tk], v[:, :, lo:lo + Tk]
+    o, L, M = ops.sliding_fwd(q.to(DEV), k.to(DEV)[..., lo:lo + Tk], v.to(DEV)[:, :, lo:lo + Tk], 100, 0.125)
+    torch.cuda.synchronize()
+    _no_timeouts()
+    ref = O.sliding_window_attention(q.float(), ks.float().contiguous(), vs.float().contiguous(), 100, 0.125)
+    assert max_abs(o.float(), ref) < 2e-2
