@@ -364,6 +364,38 @@ NSA_API int nsa_layer_bwd(const nsa_layer_desc* desc, const void* q, const void*
                   float* dlogits, float* dpos, float* dw1, float* db1, float* dw2, float* db2, void* workspace,
                   size_t workspace_bytes, void* stream);
 
+/* ---------------------------------------------------------------------------------------------------------------
+ * A handful of newest tokens against a key/value cache (decode), bf16, forward only: B*G*Tn <= 64 rows.  The caches are
+ * k_* [B,G,dk,cap], v_* [B,G,cap,dv], compressed keys fp32 [B,G,dk,nbp] (k_cmp_lp: their bf16 copy) and values
+ * [B,G,nbp,dv], block_ends int32 [nbp]; the new tokens sit at positions pos + [0,Tn) and nb compressed blocks are valid
+ * once they are in.  project == 0: q [B,H,Tn,dk] (strides sq of b, h, t) and gate_logits [B,Tn,3H] are given and the
+ * tokens are in the caches.  project != 0 (B*Tn <= 8): x [B,Tn,d_model] (strides sx) goes through the projections w (rows of
+ * q, k_slc, v_slc, k_src, v_src, k_win, v_win; biases may be NULL) into q and the caches, through phi for the last nb_new of
+ * the nb blocks, and through the gate MLP; all parameters bf16.  out [B,Tn,H,dv]; indices int32 [B,G,Tn,n], gates fp32
+ * [B,H,Tn,3] and o_* [B,H,Tn,dv] are written when given.  nsa_decode_supported says whether the sizes are in range. */
+typedef struct nsa_decode_desc {
+  int B, Tn, H, G, dk, dv, l, d, l_prime, n, n_fixed, window, gate_mode;
+  int pos, nb, nb_new, cap, nbp, d_model, d_gate, U, project;
+  float scale;
+  int64_t sq[3];
+  const void* q;
+  const float* gate_logits;
+  void *k_slc, *v_slc, *k_src, *v_src, *k_win, *v_win, *k_cmp, *k_cmp_lp, *v_cmp;
+  int32_t* block_ends;
+  void* out;
+  int32_t* indices;
+  float* gates;
+  void *o_cmp, *o_slc, *o_win;
+  const void* x;
+  int64_t sx[2];          /* strides of x's batch and token */
+  const void *w[7], *bias[7];
+  const void *gate_w1, *gate_b1, *gate_w2, *gate_b2;
+  const void *pos_embed, *phi_w1, *phi_b1, *phi_w2, *phi_b2;
+} nsa_decode_desc;
+NSA_API int nsa_decode_supported(const nsa_decode_desc* desc);
+NSA_API size_t nsa_decode_workspace_bytes(const nsa_decode_desc* desc);
+NSA_API int nsa_decode_fwd(const nsa_decode_desc* desc, void* workspace, size_t workspace_bytes, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

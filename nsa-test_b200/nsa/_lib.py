@@ -35,10 +35,24 @@ class LayerDesc(ctypes.Structure):
                                        "gate_mode", "dtype", "out_token_major")] + [("scale", c_float)]
 
 
+class DecodeDesc(ctypes.Structure):
+    """nsa_decode_desc of include/nsa_b200.h."""
+    _fields_ = ([(n_, c_int) for n_ in ("B", "Tn", "H", "G", "dk", "dv", "l", "d", "l_prime", "n", "n_fixed", "window", "gate_mode",
+                                        "pos", "nb", "nb_new", "cap", "nbp", "d_model", "d_gate", "U", "project")]
+                + [("scale", c_float), ("sq", c_int64 * 3)]
+                + [(n_, c_void_p) for n_ in ("q", "gate_logits", "k_slc", "v_slc", "k_src", "v_src", "k_win", "v_win", "k_cmp",
+                                             "k_cmp_lp", "v_cmp", "block_ends", "out", "indices", "gates", "o_cmp", "o_slc",
+                                             "o_win", "x")]
+                + [("sx", c_int64 * 2), ("w", c_void_p * 7), ("bias", c_void_p * 7)]
+                + [(n_, c_void_p) for n_ in ("gate_w1", "gate_b1", "gate_w2", "gate_b2", "pos_embed", "phi_w1", "phi_b1",
+                                             "phi_w2", "phi_b2")])
+
+
 # pieces of the layer's context buffer, in the order of enum nsa_layer_ctx_piece
 CTX_PIECES = ("o_cmp", "L_cmp", "M_cmp", "o_slc", "L_slc", "M_slc", "o_win", "L_win", "M_win", "gates", "indices", "k_cmp",
               "k_cmp_lp", "v_cmp", "block_ends", "k_cmp_lo", "lse2_cmp", "phi_saved")
 _DESCP = POINTER(LayerDesc)
+_DECP = POINTER(DecodeDesc)
 
 # name -> (restype, argtypes); mirrors include/nsa_b200.h declaration by declaration
 PROTOTYPES = {
@@ -71,6 +85,9 @@ PROTOTYPES = {
     "nsa_layer_workspace_bytes": (c_size_t, [_DESCP, c_int]),
     "nsa_layer_fwd": (c_int, [_DESCP] + [_P] * 16 + [c_size_t, _P, c_size_t, _P]),
     "nsa_layer_bwd": (c_int, [_DESCP] + [_P] * 10 + [c_size_t] + [_P] * 14 + [_P, c_size_t, _P]),
+    "nsa_decode_supported": (c_int, [_DECP]),
+    "nsa_decode_workspace_bytes": (c_size_t, [_DECP]),
+    "nsa_decode_fwd": (c_int, [_DECP, _P, c_size_t, _P]),
     "nsa_phi_pool_fwd": (c_int, [_P, _P, _P, _I64P, _P, _P] + [c_int] * 10 + [_P]),
     "nsa_phi_pool_bwd": (c_int, [_P] * 7 + [c_int] * 9 + [_P]),
     "nsa_score_topn_workspace_bytes": (c_size_t, [c_int] * 12),

@@ -18,7 +18,7 @@ from typing import Optional
 
 import torch
 
-from . import ops
+from . import _lib, ops
 from .kernels import (NSAConfig, PAD_BLOCK_END, _PhiCompress, _next_pow2, _project_heads, _selection_fallback,
                       gate_logits_from_hidden)
 
@@ -26,6 +26,7 @@ __all__ = ["NSACache", "nsa_layer_incremental", "module_forward_incremental"]
 
 _TILE = 128
 _FEW_ROWS = 64       # (sequence, group, row) count up to which scoring takes the unpadded rows
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
 
 
 def _round_up(x: int, m: int) -> int:
@@ -97,6 +98,104 @@ class NSACache:
         return p0
 
 
+def _cache_desc(cache: NSACache, B: int, Tn: int, pos: int, nb: int, scale: float = 0.0):
+    """Descriptor of ``Tn`` tokens at ``pos`` of ``cache`` with ``nb`` valid compressed blocks for the library's entry points, or
+    None when the cache's tensors are not laid out as those read and write them."""
+    c = cache.config
+    H, G, dk, dv, cap, nbp = c.n_heads, c.n_kv_groups, c.head_dim_qk, c.head_dim_v, cache.capacity, cache.nbp
+    dev, dt = cache.k_slc.device, cache.dtype
+    for t, n, want in ((cache.k_slc, dk * cap, dt), (cache.v_slc, dv * cap, dt), (cache.k_win, dk * cap, dt), (cache.v_win, dv * cap, dt),
+                       (cache.k_src, dk * cap, dt), (cache.v_src, dv * cap, dt), (cache.k_cmp, dk * nbp, torch.float32),
+                       (cache.k_cmp_lp, dk * nbp, dt), (cache.v_cmp, dv * nbp, dt)):
+        if t.numel() != B * G * n or t.dtype != want or t.device != dev or not t.is_contiguous() or t.data_ptr() % 16:
+            return None
+    if cache.block_ends.numel() != nbp or cache.block_ends.dtype != torch.int32 or cache.block_ends.device != dev:
+        return None
+    return _lib.DecodeDesc(B=B, Tn=Tn, H=H, G=G, dk=dk, dv=dv, l=c.l, d=c.d, l_prime=c.l_prime, n=c.n,
+                           n_fixed=c.n_fixed if c.include_fixed_in_selection else 0, window=c.w,
+                           gate_mode=_lib.GATE_SOFTMAX if c.gate_mode == "softmax" else _lib.GATE_SIGMOID, pos=pos, nb=nb, cap=cap,
+                           nbp=nbp, scale=scale, k_slc=cache.k_slc.data_ptr(), v_slc=cache.v_slc.data_ptr(),
+                           k_src=cache.k_src.data_ptr(), v_src=cache.v_src.data_ptr(), k_win=cache.k_win.data_ptr(),
+                           v_win=cache.v_win.data_ptr(), k_cmp=cache.k_cmp.data_ptr(), k_cmp_lp=cache.k_cmp_lp.data_ptr(),
+                           v_cmp=cache.v_cmp.data_ptr(), block_ends=cache.block_ends.data_ptr())
+
+
+def _layer_rows(q: torch.Tensor, gate_logits: torch.Tensor, cache: NSACache, scale: float, return_info: bool):
+    """``nsa_layer_incremental`` for a handful of rows in one library call, or None where its kernels do not apply."""
+    B, H, Tn, dk = q.shape
+    dv, dev = cache.config.head_dim_v, q.device
+    if (q.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16 or dev != cache.k_slc.device or H != cache.config.n_heads
+            or dk != cache.config.head_dim_qk or gate_logits.shape != (B, Tn, 3 * H) or gate_logits.device != dev):
+        return None
+    d = _cache_desc(cache, B, Tn, cache.length - Tn, cache.n_blocks, scale)
+    if d is None or not _lib.lib.nsa_decode_supported(d):
+        return None
+    if q.data_ptr() % 16 or q.stride(3) != 1 or any(q.stride(i) % 8 for i in range(3)):
+        q = q.clone(memory_format=torch.contiguous_format)
+    lg = gate_logits.float().contiguous()
+    out = torch.empty(B, Tn, H, dv, device=dev, dtype=q.dtype)
+    d.q, d.sq, d.gate_logits, d.out = q.data_ptr(), q.stride()[:3], lg.data_ptr(), out.data_ptr()
+    info = None
+    if return_info:
+        o = lambda: torch.empty(B, H, Tn, dv, device=dev, dtype=q.dtype)
+        info = dict(indices=torch.empty(B, cache.config.n_kv_groups, Tn, cache.config.n, device=dev, dtype=torch.int32),
+                    gates=torch.empty(B, H, Tn, 3, device=dev, dtype=torch.float32), o_cmp=o(), o_slc=o(), o_win=o())
+        for name, t in info.items():
+            setattr(d, name, t.data_ptr())
+    ops.decode_fwd(d, dev)
+    out = out.transpose(1, 2)
+    return (out, info) if return_info else out
+
+
+def _decode_module(module, x: torch.Tensor, cache: NSACache):
+    """``module_forward_incremental`` up to the output projection for at most eight tokens in one library call: mixed output
+    [B,Tn,H*dv], or None where its kernels do not apply (other types or sizes, too short a cache, autocast, tensor
+    subclasses).  The same products, roundings and cache contents as the general path."""
+    c = module.config
+    if x.dim() != 3 or type(x) not in _PLAIN or x.dtype != torch.bfloat16 or cache.shared_kv or cache.config != c:
+        return None
+    B, Tn, dm = x.shape
+    p1 = cache.length + Tn
+    dev = x.device
+    if (B * Tn > 8 or Tn == 0 or p1 > cache.capacity or p1 < c.l or dm != c.d_model or dev != cache.k_slc.device
+            or cache.dtype != torch.bfloat16 or torch.is_autocast_enabled("cuda") or x.stride(2) != 1 or x.stride(0) % 8
+            or x.stride(1) % 8 or x.data_ptr() % 16):
+        return None
+    nb = (p1 - c.l) // c.d + 1
+    G, dk, dv, H = c.n_kv_groups, c.head_dim_qk, c.head_dim_v, c.n_heads
+    d = _cache_desc(cache, B, Tn, cache.length, nb, module.scale)
+    if d is None:
+        return None
+    lins = (module.q_proj, module.k_select, module.v_select, module.k_compress, module.v_compress, module.k_sliding, module.v_sliding)
+    g0, g2 = module.gate_mlp[0], module.gate_mlp[2]
+    pe, pw1, pb1, pw2, pb2 = module._phi_params()
+    D2, U = g0.weight.shape[0], pw1.shape[0]
+    rows = (H * dk, G * dk, G * dv, G * dk, G * dv, G * dk, G * dv)
+    params = [(lin.weight, r * dm) for lin, r in zip(lins, rows)] + [(lin.bias, r) for lin, r in zip(lins, rows)]
+    params += [(g0.weight, D2 * dm), (g0.bias, D2), (g2.weight, 3 * H * D2), (g2.bias, 3 * H), (pe, c.l * c.l), (pw1, U * (dk + c.l)),
+               (pb1, U), (pw2, dk * U), (pb2, dk)]
+    ptrs = []
+    for t, n in params:
+        if t is None:
+            ptrs.append(None)
+            continue
+        if type(t) not in _PLAIN or t.dtype != torch.bfloat16 or t.numel() != n or t.device != dev or not t.is_contiguous():
+            return None
+        ptrs.append(t.data_ptr())
+    if any(p_ is None or p_ % 16 for p_ in ptrs[:7] + [ptrs[14], ptrs[16], ptrs[19]]) or ptrs[18] is None or ptrs[21] is None:
+        return None
+    d.project, d.nb_new, d.d_model, d.d_gate, d.U = 1, nb - cache.n_blocks, dm, D2, U
+    if not _lib.lib.nsa_decode_supported(d):
+        return None
+    out = torch.empty(B, Tn, H * dv, device=dev, dtype=x.dtype)
+    d.x, d.sx, d.out = x.data_ptr(), x.stride()[:2], out.data_ptr()
+    d.w, d.bias = tuple(ptrs[:7]), tuple(ptrs[7:14])
+    (d.gate_w1, d.gate_b1, d.gate_w2, d.gate_b2, d.pos_embed, d.phi_w1, d.phi_b1, d.phi_w2, d.phi_b2) = ptrs[14:]
+    ops.decode_fwd(d, dev)
+    cache.length, cache.n_blocks = p1, nb
+    return out
+
+
 def _pad_rows(x: torch.Tensor, dim: int, rows: int) -> torch.Tensor:
     have = x.shape[dim]
     if have == rows:
@@ -126,6 +225,10 @@ def nsa_layer_incremental(q_new: torch.Tensor, gate_logits_new: torch.Tensor, ca
         # block exists there is nothing to reproduce, so the first chunk has to bring at least l tokens.
         raise ValueError(f"nsa_layer_incremental: the cache needs at least l={c.l} tokens")
     scale = 1.0 / math.sqrt(dk) if scale is None else scale
+    if Tn > 0:
+        res = _layer_rows(q_new, gate_logits_new, cache, scale, return_info)
+        if res is not None:
+            return res
     rows = _round_up(Tn, _TILE)
     q = _pad_rows(q_new, 2, rows)
     n_fixed = c.n_fixed if c.include_fixed_in_selection else 0
@@ -180,6 +283,9 @@ def module_forward_incremental(module, hidden_new: torch.Tensor, cache: NSACache
     c = module.config
     B, Tn, _ = hidden_new.shape
     H, G, dk, dv = c.n_heads, c.n_kv_groups, c.head_dim_qk, c.head_dim_v
+    few = _decode_module(module, hidden_new, cache)
+    if few is not None:
+        return module.o_proj(few)
     q = _project_heads(hidden_new, module.q_proj, H, dk)
 
     def kv(kp, vp):

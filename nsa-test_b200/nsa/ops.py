@@ -166,6 +166,14 @@ def cmp_attn_bwd(q, k_cmp, v_cmp, block_ends, o, do, L, M, scale: float, blocks=
     return dq, dkc, dvc
 
 
+def decode_fwd(desc, dev) -> None:
+    """nsa_decode_fwd with a workspace of its own, on the current stream of ``dev``."""
+    nbytes = lib.nsa_decode_workspace_bytes(desc)
+    ws = torch.empty(nbytes, device=dev, dtype=torch.uint8)
+    with torch.cuda.device(dev):
+        check(lib.nsa_decode_fwd(desc, ptr(ws), nbytes, stream_ptr(dev)), "nsa_decode_fwd")
+
+
 def slc_fwd(q, k, v, indices_i32, l_prime: int, scale: float, q_pos0: int = 0, generic: bool = False):
     k = _tc_keys(q, k, generic)
     dev = require_cuda(q, k, v, indices_i32)

@@ -35,7 +35,10 @@ def test_selection_over_ragged_chunks_and_short_ranges(dk, dv, H, G, T, n):
     _grad_close(dval, gv, "dv")
 
 
-@pytest.mark.parametrize("T", [20, 33, 100, 129, 200, 637, 1030])
+# (T = 32..46 shows every row at most one compressed block: the softmax over it is constant, the true gradient of phi is zero
+# and a bound relative to it has no scale.  At 63, sixteen rows see two blocks and sixteen one, whose bf16 roundings, 2^-8 of
+# a term each, stay under 1 % of the gradient.)
+@pytest.mark.parametrize("T", [20, 63, 100, 129, 200, 637, 1030])
 @pytest.mark.parametrize("dk,dv,H,G", [(64, 64, 4, 2), (192, 128, 16, 1)])
 def test_bf16_layer_at_any_length(dk, dv, H, G, T):
     """Sequences that are no multiple of a tile, of 64 or of 8, shorter than a key tile, and with fewer compressed blocks
@@ -70,3 +73,73 @@ def test_keys_and_values_read_as_slices_of_a_longer_buffer(Tk, lo):
     _no_timeouts()
     ref = O.sliding_window_attention(q.float(), ks.float().contiguous(), vs.float().contiguous(), 100, 0.125)
     assert max_abs(o.float(), ref) < 2e-2
+
+
+@pytest.mark.parametrize("heads,B,cached,news,w,gate,bias", [
+    ((8, 2, 64, 64), 3, 61, (1, 2, 1, 1, 2), 100, "softmax", True),          # a chunk edge, completed blocks, several tokens
+    ((16, 1, 192, 128), 1, 31, (1, 1, 8), 512, "sigmoid", False),            # the first block completes with the first token
+    ((32, 2, 128, 128), 8, 1999, (1, 1), 130, "sigmoid", True),
+    ((8, 4, 64, 64), 2, 6000, (1, 4, 3), 64, "sigmoid", False),              # two heads per group; more candidates than one pass
+])
+def test_decode_kernels_match_the_tile_kernels(monkeypatch, heads, B, cached, news, w, gate, bias):
+    """A handful of tokens through the decode kernels against the same call through the tile kernels: outputs, branch
+    outputs and everything written to the cache.  Both round the outputs to bf16 (2^-9 of a value below 4) and the general path
+    also P and the branch outputs: 2e-2 as everywhere for bf16 outputs; a near-tie may admit another block in a few rows."""
+    import nsa
+    from nsa import incremental as I
+    H, G, dk, dv = heads
+    cfg = nsa.NSAConfig(d_model=128, head_dim_qk=dk, head_dim_v=dv, n_heads=H, n_kv_groups=G, w=w, gate_mode=gate, use_bias=bias)
+    torch.manual_seed(3)
+    m = nsa.NSAAttention(cfg).to(DEV).bfloat16().eval()
+    x = torch.randn(B, cached + sum(news), 128, device=DEV).bfloat16()
+    new, old = I.NSACache(cfg, B, cached + 16, DEV), I.NSACache(cfg, B, cached + 16, DEV)
+    for c in (new, old):
+        if cached >= 32:
+            I.module_forward_incremental(m, x[:, :cached], c)
+        else:
+            c.append(m._phi_params(), *_kv(m, x[:, :cached], "select"), kv_compress=_kv(m, x[:, :cached], "compress"),
+                     kv_sliding=_kv(m, x[:, :cached], "sliding"))
+    p, calls = cached, []
+    real = I.ops.decode_fwd
+    monkeypatch.setattr(I.ops, "decode_fwd", lambda *a: (calls.append(1), real(*a))[1])
+    for Tn in news:
+        y = I.module_forward_incremental(m, x[:, p:p + Tn], new)
+        assert len(calls) == (1 if B * Tn <= 8 or B * Tn * G <= 64 else 0), "the decode kernels did not run"
+        calls.clear()
+        with monkeypatch.context() as mp:
+            mp.setattr(I, "_decode_module", lambda *a: None)
+            mp.setattr(I, "_layer_rows", lambda *a: None)
+            z = I.module_forward_incremental(m, x[:, p:p + Tn], old)
+        torch.cuda.synchronize()
+        _no_timeouts()
+        rows = (y.float() - z.float()).abs().amax(-1)
+        assert (rows < 2e-2).float().mean().item() > 0.8 and rows.median().item() < 1e-2, (Tn, rows)
+        p += Tn
+        assert (new.length, new.n_blocks) == (old.length, old.n_blocks) == (p, (p - 32) // 16 + 1)
+    for name in ("k_slc", "v_slc", "k_src", "v_src", "k_win", "v_win", "v_cmp", "k_cmp_lp", "k_cmp", "block_ends"):
+        a, b = getattr(new, name).float(), getattr(old, name).float()
+        # bf16 products of another summation order may round to the neighbour (2^-8 relative); phi adds what that moves
+        assert max_abs(a, b) <= 2e-2 * max(1.0, b.abs().max().item()), name
+    # the layer call with its diagnostics
+    q, lg = torch.randn(B, H, 1, dk, device=DEV).bfloat16(), torch.randn(B, 1, 3 * H, device=DEV)
+    out, info = I.nsa_layer_incremental(q, lg, new, return_info=True)
+    with monkeypatch.context() as mp:
+        mp.setattr(I, "_layer_rows", lambda *a: None)
+        ref, want = I.nsa_layer_incremental(q, lg, new, return_info=True)
+    torch.cuda.synchronize()
+    other = (info["indices"].unsqueeze(-1) != want["indices"].unsqueeze(-2)).all(-1).sum(-1)
+    assert int(other.max()) <= 1
+    for name in ("o_cmp", "o_win"):
+        assert max_abs(info[name].float(), want[name].float()) < 2e-2, name
+    assert max_abs(info["gates"], want["gates"]) < 1e-6
+    same = (other == 0).repeat_interleave(H // G, dim=1)
+    assert max_abs(info["o_slc"].float()[same], want["o_slc"].float()[same]) < 2e-2
+    assert max_abs(out.float()[same], ref.float()[same]) < 2e-2
+
+
+def _kv(m, x, name):
+    from nsa.kernels import _project_heads
+    c = m.config
+    with torch.no_grad():
+        return (_project_heads(x, getattr(m, "k_" + name), c.n_kv_groups, c.head_dim_qk, transposed=True),
+                _project_heads(x, getattr(m, "v_" + name), c.n_kv_groups, c.head_dim_v))
