@@ -396,6 +396,18 @@ NSA_API int nsa_decode_supported(const nsa_decode_desc* desc);
 NSA_API size_t nsa_decode_workspace_bytes(const nsa_decode_desc* desc);
 NSA_API int nsa_decode_fwd(const nsa_decode_desc* desc, void* workspace, size_t workspace_bytes, void* stream);
 
+/* Larger chunks of new tokens, same descriptor (project == 0, B*G*Tn > 64).  nsa_cache_append copies the tokens' keys and
+ * values into the caches and compresses the nb_new blocks they complete: src holds one pair (k_slc, v_slc: shared streams) or
+ * three (k_slc, v_slc, k_src, v_src, k_win, v_win), strides four element strides per tensor in the order (batch, group, time,
+ * channel); dtype is the caches', param_dtype the phi parameters'.  nsa_incremental_fwd then returns the new rows: q
+ * [B,H,Tn,dk] contiguous bf16, out [B,Tn,H,dv]. */
+NSA_API size_t nsa_cache_append_workspace_bytes(const nsa_decode_desc* desc, int dtype);
+NSA_API int nsa_cache_append(const nsa_decode_desc* desc, const void* const* src, const int64_t* strides, int n_tensors,
+                             int dtype, int param_dtype, void* workspace, size_t workspace_bytes, void* stream);
+NSA_API int nsa_incremental_supported(const nsa_decode_desc* desc);
+NSA_API size_t nsa_incremental_workspace_bytes(const nsa_decode_desc* desc);
+NSA_API int nsa_incremental_fwd(const nsa_decode_desc* desc, void* workspace, size_t workspace_bytes, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

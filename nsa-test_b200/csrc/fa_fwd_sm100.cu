@@ -59,8 +59,8 @@ struct FaBarriers {
 template <int MODE>
 __device__ __forceinline__ void row_bounds(const FaFwdParams& p, int t, int n0, int& clo, int& chi) {
   if (MODE == kWin) {
-    chi = t - n0;
-    clo = t - p.window - n0;
+    chi = p.win_q0 + t - n0;
+    clo = chi - p.window;
   } else {
     const int vis = t >= p.cmp_l - 1 ? min(p.cmp_nb - 1, (t - p.cmp_l + 1) / p.cmp_d) : -1;
     chi = vis - n0;
@@ -104,8 +104,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     w.g = w.h0 / hpg;
     int jhi;
     if (MODE == kWin) {
-      w.jlo = max(0, w.m0 - p.window + 1) / kBN;
-      jhi = min(w.m0 + kBM - 1, p.Tk - 1) / kBN;
+      w.jlo = max(0, p.win_q0 + w.m0 - p.window + 1) / kBN;
+      jhi = min(p.win_q0 + w.m0 + kBM - 1, p.Tk - 1) / kBN;
     } else {
       const int tl = w.m0 + kBM - 1;
       const int kmax = tl >= p.cmp_l - 1 ? min(p.cmp_nb - 1, (tl - p.cmp_l + 1) / p.cmp_d) : -1;
@@ -305,7 +305,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       // does this tile need element masks?
       bool full;
       if (MODE == kWin) {
-        full = (n0 + kBN - 1 <= m0) && (n0 > m0 + kBM - 1 - p.window);
+        full = (n0 + kBN - 1 <= p.win_q0 + m0) && (n0 > p.win_q0 + m0 + kBM - 1 - p.window);
       } else {
         full = (n0 + kBN - 1 < p.cmp_nb) && ((n0 + kBN - 1) * p.cmp_d + p.cmp_l - 1 <= m0);
       }
@@ -537,7 +537,7 @@ bool fa_fwd_sm100_supported(int H, int G, int Tq, int Tk, int dk, int dv) {
 
 int fa_fwd_sm100(const void* q, const void* k, const void* v, void* o, float* L, float* M, int B, int H, int G, int Tq,
                  int Tk, int dk, int dv, int mode, int window, int cmp_l, int cmp_d, int cmp_nb, float scale,
-                 const void* k_lo, float* lse2, const KvLayout& kv, cudaStream_t st) {
+                 const void* k_lo, float* lse2, const KvLayout& kv, cudaStream_t st, int win_q0) {
   if (!fa_fwd_sm100_supported(H, G, Tq, Tk, dk, dv)) return fail(NSA_ERR_UNSUPPORTED, "fa_fwd_sm100: unsupported shape");
   if (!fa_timeout_counter()) return fail(NSA_ERR_LAUNCH, "fa_fwd_sm100: cannot set up the time-out record of this device");
   if ((int64_t)B * (H / 2) * ((Tq + kBM - 1) / kBM) > 0x7fffffff) return fail(NSA_ERR_UNSUPPORTED, "fa_fwd_sm100: too many work items");
@@ -550,7 +550,7 @@ int fa_fwd_sm100(const void* q, const void* k, const void* v, void* o, float* L,
   FaFwdParams p;
   p.o = (__nv_bfloat16*)o; p.L = L; p.M = M;
   p.B = B; p.H = H; p.G = G; p.Tq = Tq; p.Tk = Tk;
-  p.window = window; p.cmp_l = cmp_l; p.cmp_d = cmp_d; p.cmp_nb = cmp_nb;
+  p.window = window; p.win_q0 = win_q0; p.cmp_l = cmp_l; p.cmp_d = cmp_d; p.cmp_nb = cmp_nb;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.lse2 = lse2;
 #define NSA_FA_CASE(DK_, DV_)                                                                                            \

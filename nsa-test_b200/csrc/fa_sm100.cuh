@@ -14,6 +14,7 @@ struct FaFwdParams {
   float* lse2;       // [B,H,Tq] log-sum-exp of the scaled logits in log2 units (+inf for rows that see nothing), may be null
   int B, H, G, Tq, Tk;
   int window;                // sliding window: keys (t-window, t]
+  int win_q0;                // sliding window: position of query row 0 among the keys
   int cmp_l, cmp_d, cmp_nb;  // compressed tokens: key i visible iff i < cmp_nb and i*cmp_d + cmp_l - 1 <= t
   float scale_log2;          // softmax scale times log2(e)
 };
@@ -31,10 +32,10 @@ struct KvLayout {
 // q [B,H,Tq,dk], o [B,H,Tq,dv]: contiguous bf16, any Tq and Tk (tiles reaching past them are filled with zeros by TMA and
 // their rows are not stored).  mode = kWin or kCmp.
 // k_lo (compressed branch, or null): low-order bf16 part of the keys, S = Q (k + k_lo)^T; lse2 (or null): receives the
-// log-sum-exp in log2 units.
+// log-sum-exp in log2 units.  win_q0: position of query row 0 among the keys of a sliding-window call.
 int fa_fwd_sm100(const void* q, const void* k, const void* v, void* o, float* L, float* M, int B, int H, int G, int Tq,
                  int Tk, int dk, int dv, int mode, int window, int cmp_l, int cmp_d, int cmp_nb, float scale,
-                 const void* k_lo, float* lse2, const KvLayout& kv, cudaStream_t st);
+                 const void* k_lo, float* lse2, const KvLayout& kv, cudaStream_t st, int win_q0 = 0);
 
 // Backward of the same two branches.  Adds into dk [B,G,Tk,dk] and dv [B,G,Tk,dv] (time-major, bf16),
 // overwrites dq [B,H,Tq,dk].  Three launches: delta/lse preparation, a query-stationary dQ kernel and

@@ -1,0 +1,14 @@
+// Block compression on strided inputs and outputs (see phi_mlp.cu).
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace nsa {
+
+// Scratch and saved sizes as for nsa_cmp_phi_fwd; v_cmp planes and k_cmp rows are nbp apart.
+int cmp_phi_fwd_strided(const void* k, int64_t k_ld, int64_t k_plane, const void* v, const int64_t* vs, const float* pos_embed,
+                        const float* w1, const float* b1, const float* w2, const float* b2, float* k_cmp, void* k_cmp_lp, void* v_cmp,
+                        int B, int G, int T, int dk, int dv, int l, int d, int U, int nbp, bool pad, int dtype, void* saved,
+                        size_t saved_bytes, void* workspace, size_t workspace_bytes, cudaStream_t st);
+
+}  // namespace nsa

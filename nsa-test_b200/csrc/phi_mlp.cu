@@ -21,6 +21,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "phi.cuh"
 
 namespace nsa {
 namespace {
@@ -108,18 +109,20 @@ __global__ void c_table_kernel(const float* __restrict__ pos, const float* __res
   for (int m = 0; m < l; ++m) acc = fmaf(pos[j * l + m], w1[(int64_t)u * (dk + l) + dk + m], acc);
   c[i] = acc;
 }
-// k_cmp[bg, c, i] += b2[c] for the real blocks; an optional copy in the I/O type is written alongside
+// k_cmp[bg, c, i] += b2[c] for the real blocks, zeros in the columns nb..cols behind them (rows are nbp apart); an optional
+// copy in the I/O type is written alongside
 template <typename T>
-__global__ void kcmp_finish_kernel(float* __restrict__ k_cmp, const float* __restrict__ b2, T* __restrict__ lp, int dk, int nb, int nbp,
-                                   int64_t total) {
+__global__ void kcmp_finish_kernel(float* __restrict__ k_cmp, const float* __restrict__ b2, T* __restrict__ lp, int dk, int nb, int cols,
+                                   int nbp, int64_t total) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
-  const int blk = i % nbp, c = (i / nbp) % dk;
-  float x = k_cmp[i];
+  const int blk = i % cols, c = (i / cols) % dk;
+  const int64_t at = i / cols * nbp + blk;
+  float x = k_cmp[at];
   if (blk < nb && b2) x += b2[c];
   if (blk >= nb) x = 0.f;
-  k_cmp[i] = x;
-  if (lp) Elem<T>::st(lp + i, x);
+  k_cmp[at] = x;
+  if (lp) Elem<T>::st(lp + at, x);
 }
 // rows [bg, i < nb] of a [BG, nbp, W] tensor of the I/O type -> fp32 [BG, nb_out, W] (rows beyond nb zero)
 template <typename T>
@@ -254,22 +257,18 @@ extern "C" NSA_API size_t nsa_cmp_phi_workspace_bytes(int B, int G, int T, int d
   return bwd_layout(B, G, T, dk, dv, l, d, U, nbp, dtype).total + 256;
 }
 
-extern "C" NSA_API int nsa_cmp_phi_fwd(const void* k, const void* v, const float* pos_embed, const float* w1, const float* b1,
-                                       const float* w2, const float* b2, float* k_cmp, void* k_cmp_lp, void* v_cmp, int B, int G,
-                                       int T, int dk, int dv, int l, int d, int U, int nbp, int dtype, void* saved,
-                                       size_t saved_bytes, void* workspace, size_t workspace_bytes, void* stream) {
-  NSA_REQUIRE(k && v && pos_embed && w1 && w2 && k_cmp && v_cmp && saved, "cmp_phi_fwd: null pointer");
-  NSA_REQUIRE(B > 0 && G > 0 && dk > 0 && dv > 0 && U > 0 && l > 0 && d > 0, "cmp_phi_fwd: bad sizes");
-  NSA_REQUIRE(dtype == NSA_F32 || dtype == NSA_BF16, "cmp_phi_fwd: unsupported dtype %d", dtype);
-  NSA_REQUIRE(T >= l, "cmp_phi_fwd: sequence length %d shorter than one compression block (%d)", T, l);
+// Forward on keys whose rows lie k_ld elements apart (planes k_plane) and values with strides vs; the nb blocks go to the first
+// columns of rows nbp apart and to rows of planes nbp apart.  `pad`: the rest of those rows and planes is cleared.
+int nsa::cmp_phi_fwd_strided(const void* k, int64_t k_ld, int64_t k_plane, const void* v, const int64_t* vs, const float* pos_embed,
+                             const float* w1, const float* b1, const float* w2, const float* b2, float* k_cmp, void* k_cmp_lp, void* v_cmp,
+                             int B, int G, int T, int dk, int dv, int l, int d, int U, int nbp, bool pad, int dtype, void* saved,
+                             size_t saved_bytes, void* workspace, size_t workspace_bytes, cudaStream_t st) {
   const int nb = (T - l) / d + 1, BG = B * G;
-  NSA_REQUIRE(nbp >= nb, "cmp_phi_fwd: nbp = %d holds fewer than the %d blocks of the sequence", nbp, nb);
   const SavedLayout sl = saved_layout(B, G, T, l, d, U);
   if (saved_bytes < sl.total) return fail(NSA_ERR_WORKSPACE, "cmp_phi_fwd needs %zu bytes for the backward's inputs, got %zu", sl.total, saved_bytes);
   const size_t need = nsa_cmp_phi_workspace_bytes(B, G, T, dk, dv, l, d, U, nbp, dtype, 0);
   if (dtype == NSA_BF16 && (!workspace || workspace_bytes < need))
     return fail(NSA_ERR_WORKSPACE, "cmp_phi_fwd needs %zu workspace bytes, got %zu", need, workspace_bytes);
-  cudaStream_t st = (cudaStream_t)stream;
   cublasHandle_t h;
   if (int rc = blas_handle(&h, st)) return rc;
   float* a = (float*)((char*)saved + sl.o_a);
@@ -279,42 +278,57 @@ extern "C" NSA_API int nsa_cmp_phi_fwd(const void* k, const void* v, const float
   {
     KernelTimer kt("phi_mlp_fwd", st);
     c_table_kernel<<<blocks_for((int64_t)l * U), 256, 0, st>>>(pos_embed, w1, b1, l, U, dk, c);
-    // A[bg] (T x U, row-major) = K[bg]^T W1k^T; column-major: C(U x T) = op_T(W (dk x U, ld)) op_T(K (T x dk, ld T))
+    // A[bg] (T x U, row-major) = K[bg]^T W1k^T; column-major: C(U x T) = op_T(W (dk x U, ld)) op_T(K (T x dk, ld k_ld))
     if (dtype == NSA_BF16) {
       __nv_bfloat16* hi = (__nv_bfloat16*)workspace;
       __nv_bfloat16 *mid = hi + (size_t)U * dk, *lo = mid + (size_t)U * dk;
       split3_kernel<<<blocks_for((int64_t)U * dk), 256, 0, st>>>(w1, U, dk, ld1, hi, mid, lo);
       const __nv_bfloat16* terms[3] = {hi, mid, lo};
       for (int t3 = 0; t3 < 3; ++t3)
-        if (int rc = gemm(h, CUBLAS_OP_T, CUBLAS_OP_T, U, T, dk, terms[t3], CUDA_R_16BF, dk, 0, k, CUDA_R_16BF, T, (long long)dk * T,
+        if (int rc = gemm(h, CUBLAS_OP_T, CUBLAS_OP_T, U, T, dk, terms[t3], CUDA_R_16BF, dk, 0, k, CUDA_R_16BF, (int)k_ld, k_plane,
                           t3 ? 1.f : 0.f, a, CUDA_R_32F, U, (long long)T * U, BG, "cmp_phi_fwd (K W1k^T)"))
           return rc;
     } else {
-      if (int rc = gemm(h, CUBLAS_OP_T, CUBLAS_OP_T, U, T, dk, w1, CUDA_R_32F, ld1, 0, k, CUDA_R_32F, T, (long long)dk * T, 0.f, a,
+      if (int rc = gemm(h, CUBLAS_OP_T, CUBLAS_OP_T, U, T, dk, w1, CUDA_R_32F, ld1, 0, k, CUDA_R_32F, (int)k_ld, k_plane, 0.f, a,
                         CUDA_R_32F, U, (long long)T * U, BG, "cmp_phi_fwd (K W1k^T)"))
         return rc;
     }
   }
   if (int rc = check_launch("cmp_phi_fwd")) return rc;
-  const int64_t vs[4] = {(int64_t)G * T * dv, (int64_t)T * dv, dv, 1};
-  if (int rc = nsa_phi_pool_fwd(a, c, v, vs, hbar, v_cmp, B, G, T, U, dv, l, d, nb, nbp, dtype, stream)) return rc;
+  if (int rc = nsa_phi_pool_fwd(a, c, v, vs, hbar, v_cmp, B, G, T, U, dv, l, d, nb, nbp, dtype, st)) return rc;
   {
     KernelTimer kt("phi_mlp_fwd", st);
     // pooled v_cmp rows beyond nb are the caller's zero padding: cleared here so that the caller need not
     const size_t es = dtype == NSA_BF16 ? 2 : 4;
-    if (nbp > nb)
+    if (pad && nbp > nb)
       cudaMemset2DAsync((char*)v_cmp + (size_t)nb * dv * es, (size_t)nbp * dv * es, 0, (size_t)(nbp - nb) * dv * es, BG, st);
     // k_cmp[bg] (dk x nbp, row-major) = (hbar[bg] W2^T)^T; column-major: C(nb x dk, ld nbp) = op_T(hbar (U x nb)) W2 (U x dk)
     if (int rc = gemm(h, CUBLAS_OP_T, CUBLAS_OP_N, nb, dk, U, hbar, CUDA_R_32F, U, (long long)nb * U, w2, CUDA_R_32F, U, 0, 0.f, k_cmp,
                       CUDA_R_32F, nbp, (long long)dk * nbp, BG, "cmp_phi_fwd (hbar W2^T)"))
       return rc;
-    const int64_t total = (int64_t)BG * dk * nbp;
+    const int cols = pad ? nbp : nb;
+    const int64_t total = (int64_t)BG * dk * cols;
     if (dtype == NSA_BF16)
-      kcmp_finish_kernel<__nv_bfloat16><<<blocks_for(total), 256, 0, st>>>(k_cmp, b2, (__nv_bfloat16*)k_cmp_lp, dk, nb, nbp, total);
+      kcmp_finish_kernel<__nv_bfloat16><<<blocks_for(total), 256, 0, st>>>(k_cmp, b2, (__nv_bfloat16*)k_cmp_lp, dk, nb, cols, nbp, total);
     else
-      kcmp_finish_kernel<float><<<blocks_for(total), 256, 0, st>>>(k_cmp, b2, (float*)k_cmp_lp, dk, nb, nbp, total);
+      kcmp_finish_kernel<float><<<blocks_for(total), 256, 0, st>>>(k_cmp, b2, (float*)k_cmp_lp, dk, nb, cols, nbp, total);
   }
   return check_launch("cmp_phi_fwd");
+}
+
+extern "C" NSA_API int nsa_cmp_phi_fwd(const void* k, const void* v, const float* pos_embed, const float* w1, const float* b1,
+                                       const float* w2, const float* b2, float* k_cmp, void* k_cmp_lp, void* v_cmp, int B, int G,
+                                       int T, int dk, int dv, int l, int d, int U, int nbp, int dtype, void* saved,
+                                       size_t saved_bytes, void* workspace, size_t workspace_bytes, void* stream) {
+  NSA_REQUIRE(k && v && pos_embed && w1 && w2 && k_cmp && v_cmp && saved, "cmp_phi_fwd: null pointer");
+  NSA_REQUIRE(B > 0 && G > 0 && dk > 0 && dv > 0 && U > 0 && l > 0 && d > 0, "cmp_phi_fwd: bad sizes");
+  NSA_REQUIRE(dtype == NSA_F32 || dtype == NSA_BF16, "cmp_phi_fwd: unsupported dtype %d", dtype);
+  NSA_REQUIRE(T >= l, "cmp_phi_fwd: sequence length %d shorter than one compression block (%d)", T, l);
+  const int nb = (T - l) / d + 1;
+  NSA_REQUIRE(nbp >= nb, "cmp_phi_fwd: nbp = %d holds fewer than the %d blocks of the sequence", nbp, nb);
+  const int64_t vs[4] = {(int64_t)G * T * dv, (int64_t)T * dv, dv, 1};
+  return cmp_phi_fwd_strided(k, T, (int64_t)dk * T, v, vs, pos_embed, w1, b1, w2, b2, k_cmp, k_cmp_lp, v_cmp, B, G, T, dk, dv, l, d, U,
+                             nbp, true, dtype, saved, saved_bytes, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 extern "C" NSA_API int nsa_cmp_phi_bwd(const void* k, const float* pos_embed, const float* w1, const float* w2, const void* dk_cmp,

@@ -88,6 +88,11 @@ PROTOTYPES = {
     "nsa_decode_supported": (c_int, [_DECP]),
     "nsa_decode_workspace_bytes": (c_size_t, [_DECP]),
     "nsa_decode_fwd": (c_int, [_DECP, _P, c_size_t, _P]),
+    "nsa_cache_append_workspace_bytes": (c_size_t, [_DECP, c_int]),
+    "nsa_cache_append": (c_int, [_DECP, POINTER(_P), _I64P, c_int, c_int, c_int, _P, c_size_t, _P]),
+    "nsa_incremental_supported": (c_int, [_DECP]),
+    "nsa_incremental_workspace_bytes": (c_size_t, [_DECP]),
+    "nsa_incremental_fwd": (c_int, [_DECP, _P, c_size_t, _P]),
     "nsa_phi_pool_fwd": (c_int, [_P, _P, _P, _I64P, _P, _P] + [c_int] * 10 + [_P]),
     "nsa_phi_pool_bwd": (c_int, [_P] * 7 + [c_int] * 9 + [_P]),
     "nsa_score_topn_workspace_bytes": (c_size_t, [c_int] * 12),

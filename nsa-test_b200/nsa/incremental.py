@@ -76,13 +76,44 @@ class NSACache:
             raise ValueError(f"NSACache: {p1} tokens exceed the capacity {self.capacity}")
         if not self.shared_kv and (kv_compress is None or kv_sliding is None):
             raise ValueError("NSACache: built with separate streams, kv_compress and kv_sliding are required")
+        nb_new = (p1 - c.l) // c.d + 1 if p1 >= c.l else 0
+        tensors = (k_slc, v_slc) if self.shared_kv else (k_slc, v_slc, *kv_compress, *kv_sliding)
+        if not self._append_in_place(phi_params, tensors, p0, Tn, max(nb_new, self.n_blocks)):
+            self._append_by_copies(phi_params, k_slc, v_slc, kv_compress, kv_sliding, p0, p1, nb_new)
+        self.length, self.n_blocks = p1, max(nb_new, self.n_blocks)
+        return p0
+
+    def _append_in_place(self, phi_params, tensors, p0: int, Tn: int, nb: int) -> bool:
+        """The append as one library call; False where a tensor is not of the cache's type, shape and device."""
+        c, dev = self.config, self.k_slc.device
+        B = self.k_slc.shape[0]
+        for i, t in enumerate(tensors):
+            want = (B, c.n_kv_groups, c.head_dim_qk, Tn) if i % 2 == 0 else (B, c.n_kv_groups, Tn, c.head_dim_v)
+            if type(t) not in _PLAIN or t.shape != want or t.dtype != self.dtype or t.device != dev:
+                return False
+        pe, w1, b1, w2, b2 = phi_params
+        U, dk, pdt = w1.shape[0], c.head_dim_qk, w1.dtype
+        for t, n in ((pe, c.l * c.l), (w1, U * (dk + c.l)), (b1, U), (w2, dk * U), (b2, dk)):
+            if t is not None and (type(t) not in _PLAIN or t.dtype != pdt or t.numel() != n or t.device != dev or not t.is_contiguous()):
+                return False
+        if Tn == 0 or self.dtype not in (torch.float32, torch.bfloat16) or pdt not in (torch.float32, torch.bfloat16):
+            return False
+        if B * c.n_kv_groups * len(tensors) > 65535:
+            return False
+        d = _cache_desc(self, B, Tn, p0, nb)
+        if d is None:
+            return False
+        d.nb_new, d.U = nb - self.n_blocks, U
+        ops.cache_append(d, tensors, phi_params)
+        return True
+
+    def _append_by_copies(self, phi_params, k_slc, v_slc, kv_compress, kv_sliding, p0: int, p1: int, nb_new: int) -> None:
+        c = self.config
         self.k_slc[..., p0:p1] = k_slc
         self.v_slc[:, :, p0:p1] = v_slc
         if not self.shared_kv:
             self.k_src[..., p0:p1], self.v_src[:, :, p0:p1] = kv_compress[0], kv_compress[1]
             self.k_win[..., p0:p1], self.v_win[:, :, p0:p1] = kv_sliding[0], kv_sliding[1]
-        self.length = p1
-        nb_new = (p1 - c.l) // c.d + 1 if p1 >= c.l else 0
         if nb_new > self.n_blocks:
             b0, cnt = self.n_blocks, nb_new - self.n_blocks
             lo, hi = b0 * c.d, (nb_new - 1) * c.d + c.l
@@ -94,8 +125,6 @@ class NSACache:
             self.v_cmp[:, :, b0:nb_new] = vc[:, :, :cnt].to(self.dtype)
             self.block_ends[b0:nb_new] = (torch.arange(b0, nb_new, device=self.block_ends.device, dtype=torch.int32)
                                           * c.d + (c.l - 1))
-            self.n_blocks = nb_new
-        return p0
 
 
 def _cache_desc(cache: NSACache, B: int, Tn: int, pos: int, nb: int, scale: float = 0.0):
@@ -121,20 +150,25 @@ def _cache_desc(cache: NSACache, B: int, Tn: int, pos: int, nb: int, scale: floa
 
 
 def _layer_rows(q: torch.Tensor, gate_logits: torch.Tensor, cache: NSACache, scale: float, return_info: bool):
-    """``nsa_layer_incremental`` for a handful of rows in one library call, or None where its kernels do not apply."""
+    """``nsa_layer_incremental`` in one library call: the decode kernels for a handful of rows, the tile kernels with a query
+    offset for more; None where neither applies."""
     B, H, Tn, dk = q.shape
     dv, dev = cache.config.head_dim_v, q.device
     if (q.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16 or dev != cache.k_slc.device or H != cache.config.n_heads
             or dk != cache.config.head_dim_qk or gate_logits.shape != (B, Tn, 3 * H) or gate_logits.device != dev):
         return None
     d = _cache_desc(cache, B, Tn, cache.length - Tn, cache.n_blocks, scale)
-    if d is None or not _lib.lib.nsa_decode_supported(d):
+    if d is None:
         return None
-    if q.data_ptr() % 16 or q.stride(3) != 1 or any(q.stride(i) % 8 for i in range(3)):
+    few = bool(_lib.lib.nsa_decode_supported(d))
+    if not few and not _lib.lib.nsa_incremental_supported(d):
+        return None
+    if q.data_ptr() % 16 or (q.stride(3) != 1 or any(q.stride(i) % 8 for i in range(3)) if few else not q.is_contiguous()):
         q = q.clone(memory_format=torch.contiguous_format)
     lg = gate_logits.float().contiguous()
     out = torch.empty(B, Tn, H, dv, device=dev, dtype=q.dtype)
-    d.q, d.sq, d.gate_logits, d.out = q.data_ptr(), q.stride()[:3], lg.data_ptr(), out.data_ptr()
+    d.q, d.gate_logits, d.out = q.data_ptr(), lg.data_ptr(), out.data_ptr()
+    d.sq = q.stride()[:3] if few else (H * Tn * dk, Tn * dk, dk)
     info = None
     if return_info:
         o = lambda: torch.empty(B, H, Tn, dv, device=dev, dtype=q.dtype)
@@ -142,7 +176,7 @@ def _layer_rows(q: torch.Tensor, gate_logits: torch.Tensor, cache: NSACache, sca
                     gates=torch.empty(B, H, Tn, 3, device=dev, dtype=torch.float32), o_cmp=o(), o_slc=o(), o_win=o())
         for name, t in info.items():
             setattr(d, name, t.data_ptr())
-    ops.decode_fwd(d, dev)
+    (ops.decode_fwd if few else ops.incremental_fwd)(d, dev)
     out = out.transpose(1, 2)
     return (out, info) if return_info else out
 

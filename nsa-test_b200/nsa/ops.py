@@ -174,6 +174,31 @@ def decode_fwd(desc, dev) -> None:
         check(lib.nsa_decode_fwd(desc, ptr(ws), nbytes, stream_ptr(dev)), "nsa_decode_fwd")
 
 
+def incremental_fwd(desc, dev) -> None:
+    """nsa_incremental_fwd likewise."""
+    nbytes = lib.nsa_incremental_workspace_bytes(desc)
+    ws = torch.empty(nbytes, device=dev, dtype=torch.uint8)
+    with torch.cuda.device(dev):
+        check(lib.nsa_incremental_fwd(desc, ptr(ws), nbytes, stream_ptr(dev)), "nsa_incremental_fwd")
+
+
+def cache_append(desc, tensors, params) -> None:
+    """nsa_cache_append: tensors are k [B,G,dk,Tn] and v [B,G,Tn,dv] alternating, of any strides; params (pos_embed, w1, b1, w2, b2)
+    contiguous and of one type."""
+    dev = require_cuda(*tensors, *params)
+    code = dtype_code(tensors[0])
+    strides = []
+    for i, t in enumerate(tensors):
+        strides += _k_strides(t) if i % 2 == 0 else list(t.stride())
+    src = (_lib.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
+    (desc.pos_embed, desc.phi_w1, desc.phi_b1, desc.phi_w2, desc.phi_b2) = [None if p is None else p.data_ptr() for p in params]
+    nbytes = lib.nsa_cache_append_workspace_bytes(desc, code)
+    ws = torch.empty(nbytes, device=dev, dtype=torch.uint8)
+    with torch.cuda.device(dev):
+        check(lib.nsa_cache_append(desc, src, i64(strides), len(tensors), code, dtype_code(params[0]), ptr(ws), nbytes, stream_ptr(dev)),
+              "nsa_cache_append")
+
+
 def slc_fwd(q, k, v, indices_i32, l_prime: int, scale: float, q_pos0: int = 0, generic: bool = False):
     k = _tc_keys(q, k, generic)
     dev = require_cuda(q, k, v, indices_i32)

@@ -143,3 +143,43 @@ def _kv(m, x, name):
     with torch.no_grad():
         return (_project_heads(x, getattr(m, "k_" + name), c.n_kv_groups, c.head_dim_qk, transposed=True),
                 _project_heads(x, getattr(m, "v_" + name), c.n_kv_groups, c.head_dim_v))
+
+
+@pytest.mark.parametrize("dtype,pdtype,shared", [(torch.bfloat16, torch.bfloat16, False), (torch.bfloat16, torch.float32, True),
+                                                 (torch.float32, torch.float32, False)])
+def test_append_kernel_matches_the_copies(dtype, pdtype, shared, monkeypatch):
+    """Appends of every alignment, from tensors of either order in memory, against the copies through tensor operations."""
+    import nsa
+    from nsa import incremental as I
+    H, G, dk, dv, B = 4, 2, 48, 40, 2
+    cfg = nsa.NSAConfig(d_model=64, head_dim_qk=dk, head_dim_v=dv, n_heads=H, n_kv_groups=G)
+    gen = torch.Generator().manual_seed(5)
+    rn = lambda *s: torch.randn(*s, generator=gen).to(DEV)
+    phi = (rn(32, 32), rn(2 * dk, dk + 32) * 0.1, rn(2 * dk), rn(dk, 2 * dk) * 0.1, rn(dk))
+    phi = tuple(p.to(pdtype) for p in phi)
+    a, b = (I.NSACache(cfg, B, 700, DEV, dtype=dtype, shared_kv=shared) for _ in range(2))
+    for i, Tn in enumerate((20, 11, 1, 33, 300, 1, 64)):
+        def kv():
+            k, v = rn(B, G, dk, Tn).to(dtype), rn(B, G, Tn, dv).to(dtype)
+            if i % 2:
+                k, v = k.transpose(2, 3).contiguous().transpose(2, 3), v.permute(0, 2, 1, 3).contiguous().permute(0, 2, 1, 3)
+            return k, v
+        args = kv()
+        more = {} if shared else dict(kv_compress=kv(), kv_sliding=kv())
+        calls = []
+        real = I.ops.cache_append
+        with monkeypatch.context() as mp:
+            mp.setattr(I.ops, "cache_append", lambda *x: (calls.append(1), real(*x)))
+            a.append(phi, *args, **more)
+        assert calls
+        with monkeypatch.context() as mp:
+            mp.setattr(I.NSACache, "_append_in_place", lambda *x: False)
+            b.append(phi, *args, **more)
+    torch.cuda.synchronize()
+    assert (a.length, a.n_blocks) == (b.length, b.n_blocks) == (430, 25)
+    for name in ("k_slc", "v_slc", "k_src", "v_src", "k_win", "v_win", "block_ends"):
+        assert torch.equal(getattr(a, name), getattr(b, name)), name
+    for name in ("k_cmp", "k_cmp_lp", "v_cmp"):          # the same products through other GEMM shapes: fp32 sums of 96 terms
+        x, y = getattr(a, name), getattr(b, name)
+        tol = 1e-5 if x.dtype == torch.float32 else 2 ** -8
+        assert max_abs(x.float(), y.float()) <= tol * max(1.0, y.float().abs().max().item()), name
