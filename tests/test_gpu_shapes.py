@@ -183,3 +183,78 @@ def test_append_kernel_matches_the_copies(dtype, pdtype, shared, monkeypatch):
         x, y = getattr(a, name), getattr(b, name)
         tol = 1e-5 if x.dtype == torch.float32 else 2 ** -8
         assert max_abs(x.float(), y.float()) <= tol * max(1.0, y.float().abs().max().item()), name
+
+
+@pytest.mark.parametrize("dk,dv,H,G,T,w,lp,n", [(40, 24, 6, 2, 65, 1, 48, 3), (64, 64, 3, 3, 129, 33, 16, 5), (100, 256, 34, 1, 40, 500, 64, 4),
+                                               (8, 8, 40, 2, 70, 64, 32, 30)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_generic_kernels_off_every_tile(dk, dv, H, G, T, w, lp, n, dtype):
+    """Head dims off the 32-channel columns, groups of 1, 3, 20 and 34 heads (a 32-row tile holds part of one, or several queries),
+    blocks that are no multiple of a 32-key tile, windows of one key and past the sequence; gradients included."""
+    from nsa import ops
+    q, k, v, do = (t.to(dtype) for t in _inputs(2, H, G, T, dk, dv, seed=T + dk))
+    gen = torch.Generator().manual_seed(n)
+    nblk = -(-T // lp)
+    idx = torch.randint(-1, nblk, (2, G, T, n), generator=gen, dtype=torch.int32)
+    idx[..., 0] = (torch.arange(T) // lp).int()
+    scale = dk ** -0.5
+    d = lambda t: t.to(DEV)
+    ends = torch.full((T,), 999999, dtype=torch.int32)
+    ends[:T // 2] = torch.randperm(T, generator=gen)[:T // 2].int()          # in no order
+    for name, fwd, bwd, ref in (
+            ("win", lambda *a: ops.sliding_fwd(*a, w, scale, generic=True), lambda *a: ops.sliding_bwd(*a, w, scale, generic=True),
+             lambda a, b, c: O.sliding_window_attention(a, b, c, w, scale)),
+            ("cmp", lambda *a: ops.cmp_attn_fwd(*a, d(ends), scale, generic=True),
+             lambda a, b, c, *r: ops.cmp_attn_bwd(a, b, c, d(ends), *r, scale, generic=True),
+             lambda a, b, c: _masked(a, b, c, ends[None, :] <= torch.arange(T)[:, None], scale)),
+            ("slc", lambda *a: ops.slc_fwd(*a, d(idx), lp, scale, generic=True),
+             lambda a, b, c, *r: ops.slc_bwd(a, b, c, d(idx), *r, lp, scale, generic=True),
+             lambda a, b, c: O.selection_attention(a, b, c, idx, lp, scale))):
+        o, L, M = fwd(d(q), d(k), d(v))
+        dq, dkey, dval = bwd(d(q), d(k), d(v), o, d(do), L, M)
+        torch.cuda.synchronize()
+        qf, kf, vf = (t.float().requires_grad_(True) for t in (q, k, v))
+        want = ref(qf, kf, vf)
+        gq, gk, gv = torch.autograd.grad(want, (qf, kf, vf), do.float())
+        if dtype == torch.float32:
+            # fp32 sums of at most 40 * T terms in another order: 1e-5 of the largest entry is 80 roundings in a row
+            for a, b in ((o, want), (dq, gq), (dkey, gk.transpose(-1, -2)), (dval, gv)):
+                assert max_abs(a, b) < 1e-5 * max(1.0, b.abs().max().item()), name
+        else:
+            assert max_abs(o.float(), want) < 2e-2, name
+            for a, b, what in ((dq, gq, "dq"), (dkey, gk.transpose(-1, -2), "dk"), (dval, gv, "dv")):
+                _grad_close(a, b, f"{name} {what}")
+
+
+def _masked(q, k, v, mask, scale):
+    """Attention under a [T, keys] mask; rows that see nothing give zeros."""
+    hpg = q.shape[1] // k.shape[1]
+    s = (q * scale) @ k.repeat_interleave(hpg, 1)
+    some = mask.any(-1)[:, None]
+    p = torch.softmax(torch.where(some, s.masked_fill(~mask, float("-inf")), torch.zeros_like(s)), -1)
+    return torch.where(mask, p, torch.zeros_like(p)) @ v.repeat_interleave(hpg, 1)
+
+
+def test_generic_kernels_ignore_what_a_row_does_not_see():
+    """Keys, values and upstream gradients of later positions that are not finite leave earlier rows and keys alone."""
+    from nsa import ops
+    B, H, G, T, D = 1, 4, 2, 96, 32
+    q, k, v, do = (t.float().to(DEV) for t in _inputs(B, H, G, T, D, D, seed=11))
+    idx = (torch.arange(T) // 16).int().view(1, 1, T, 1).expand(B, G, T, 1).contiguous().to(DEV)
+    be = torch.arange(T, dtype=torch.int32, device=DEV)
+    bad = T - 5
+    for fwd, bwd in ((lambda *a: ops.sliding_fwd(*a, 40, 0.2, generic=True), lambda *a: ops.sliding_bwd(*a, 40, 0.2, generic=True)),
+                     (lambda *a: ops.cmp_attn_fwd(*a, be, 0.2, generic=True), lambda a, b, c, *r: ops.cmp_attn_bwd(a, b, c, be, *r, 0.2, generic=True)),
+                     (lambda *a: ops.slc_fwd(*a, idx, 16, 0.2, generic=True), lambda a, b, c, *r: ops.slc_bwd(a, b, c, idx, *r, 16, 0.2, generic=True))):
+        kk, vv, dd = k.clone(), v.clone(), do.clone()
+        kk[..., bad:], vv[:, :, bad:] = float("nan"), float("inf")
+        dd[:, :, :8] = float("nan")                                  # keys from 8 on are seen by no such row
+        o, L, M = fwd(q, k, v)
+        dq, dkey, dval = bwd(q, k, v, o, do, L, M)
+        _, dkey2, dval2 = bwd(q, k, v, o, dd, L, M)
+        o2, L2, M2 = fwd(q, kk, vv)
+        dq2, _, _ = bwd(q, kk, vv, o2, do, L2, M2)
+        torch.cuda.synchronize()
+        for a, b in ((o[:, :, :bad], o2[:, :, :bad]), (dq[:, :, :bad], dq2[:, :, :bad]), (dkey[:, :, 8:], dkey2[:, :, 8:]),
+                     (dval[:, :, 8:], dval2[:, :, 8:])):
+            assert torch.isfinite(b).all() and max_abs(a, b) < 1e-5
