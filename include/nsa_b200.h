@@ -48,7 +48,10 @@ enum {
 /* `flags` argument of the attention and scoring entry points (testing / cross-checks): by default a call runs the
  * tensor-core (tcgen05) kernels when it qualifies (bf16, canonical contiguous layouts, supported head dims, T a
  * multiple of 128) and the stride-generic kernels otherwise; NSA_FLAG_GENERIC forces the stride-generic kernels. */
-enum { NSA_FLAG_GENERIC = 1, NSA_FLAG_RECOMPUTE = 2 };
+/* NSA_FLAG_ANY_LENGTH lets the tensor-core kernels, which round probabilities and dS to bf16 for their second products, take
+ * lengths that are no whole tiles and keys / values that are slices of longer buffers; without it such calls run on
+ * kernels that hold both in 32 bits.  The whole layer sets it for bf16 sequences of 2048 tokens and more. */
+enum { NSA_FLAG_GENERIC = 1, NSA_FLAG_RECOMPUTE = 2, NSA_FLAG_ANY_LENGTH = 4 };
 
 /* `q_pos0` argument (query-sharded long-context runs and incremental decoding; the reference has no counterpart, its
  * wrappers assume query row t sits at position t): position of query row 0 in the sequence.  The keys keep starting

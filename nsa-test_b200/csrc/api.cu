@@ -100,14 +100,33 @@ static bool canonical_fwd(const int64_t* s, int B, int H, int G, int Tq, int Tk,
   if (s[6] != 1 || kv->k_ld < Tk || kv->k_ld % 8 != 0 || (G > 1 && s[5] != dk * kv->k_ld) || (B > 1 && s[4] != G * dk * kv->k_ld)) return false;
   return s[11] == 1 && s[10] == dv && kv->v_plane >= (int64_t)Tk * dv && kv->v_plane % 8 == 0 && (B == 1 || s[8] == G * kv->v_plane);
 }
+// Without NSA_FLAG_ANY_LENGTH: whole tiles of whole tensors only, everything else keeps fp32 probabilities (generic kernels).
+static bool length_ok(int flags, int Tq, int q_tile, int Tk, int k_tile, int dv, const KvLayout& kv) {
+  return (flags & NSA_FLAG_ANY_LENGTH) || (Tq % q_tile == 0 && Tk % k_tile == 0 && kv.k_ld == Tk && kv.v_plane == (int64_t)Tk * dv);
+}
+static bool aligned16(const void* p);
+// bf16 in canonical layouts that the tcgen05 kernels do not take: 32-bit probabilities on mma.sync (attn_mma.cu)
+static bool mma_fwd_ok(const AttnArgs& a, const int64_t* s, int mode, int flags, int dtype) {
+  KvLayout kv;
+  return (flags & NSA_FLAG_GENERIC) == 0 && dtype == NSA_BF16 && a.Tk > 0 && attn_mma_supported(a.dk, a.dv, mode, a.lprime) &&
+         canonical_fwd(s, a.B, a.H, a.G, a.Tq, a.Tk, a.dk, a.dv, &kv) && aligned16(a.q) && aligned16(a.k) && aligned16(a.v);
+}
+static bool mma_bwd_ok(const AttnArgs& a, const int64_t* s, int mode, int flags, int dtype) {
+  if (!mma_fwd_ok(a, s, mode, flags, dtype) || !aligned16(a.o_in) || !aligned16(a.dout) || !aligned16(a.dq) || !aligned16(a.dk_out) || !aligned16(a.dv_out)) return false;
+  const int64_t g[12] = {(int64_t)a.H * a.Tq * a.dk, (int64_t)a.Tq * a.dk, a.dk, 1, (int64_t)a.G * a.Tk * a.dk, (int64_t)a.Tk * a.dk, a.dk, 1,
+                         (int64_t)a.G * a.Tk * a.dv, (int64_t)a.Tk * a.dv, a.dv, 1};
+  for (int i = 0; i < 12; ++i)
+    if (s[22 + i] != g[i]) return false;
+  return true;
+}
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // canonical contiguous gradients: dq like q, dk [B,G,Tk,dk], dv [B,G,Tk,dv]
-static bool tensor_core_bwd_ok(const int64_t* s, int dtype, int B, int H, int G, int Tq, int Tk, int dk, int dv,
+static bool tensor_core_bwd_ok(const int64_t* s, int flags, int dtype, int B, int H, int G, int Tq, int Tk, int dk, int dv,
                                const void* q, const void* k, const void* v, const void* o, const void* dout, const void* dq,
                                const void* dkey, const void* dval, KvLayout* kv) {
   if (dtype != NSA_BF16 || !fa_fwd_sm100_supported(H, G, Tq, Tk, dk, dv)) return false;
-  if (!canonical_fwd(s, B, H, G, Tq, Tk, dk, dv, kv) || (int64_t)B * H > 65535) return false;
+  if (!canonical_fwd(s, B, H, G, Tq, Tk, dk, dv, kv) || !length_ok(flags, Tq, 128, Tk, 128, dv, *kv) || (int64_t)B * H > 65535) return false;
   const int64_t gq[4] = {(int64_t)H * Tq * dk, (int64_t)Tq * dk, dk, 1};
   const int64_t gk[4] = {(int64_t)G * Tk * dk, (int64_t)Tk * dk, dk, 1};
   const int64_t gv[4] = {(int64_t)G * Tk * dv, (int64_t)Tk * dv, dv, 1};
@@ -117,10 +136,10 @@ static bool tensor_core_bwd_ok(const int64_t* s, int dtype, int B, int H, int G,
          aligned16(dkey) && aligned16(dval);
 }
 
-static bool tensor_core_bwd_ok_slc(const int64_t* s, int dtype, int B, int H, int G, int Tq, int Tk, int dk, int dv, const void* q,
+static bool tensor_core_bwd_ok_slc(const int64_t* s, int flags, int dtype, int B, int H, int G, int Tq, int Tk, int dk, int dv, const void* q,
                                    const void* k, const void* v, const void* o, const void* dout, const void* dq,
                                    const void* dkey, const void* dval, KvLayout* kv) {
-  if (dtype != NSA_BF16 || !canonical_fwd(s, B, H, G, Tq, Tk, dk, dv, kv)) return false;
+  if (dtype != NSA_BF16 || !canonical_fwd(s, B, H, G, Tq, Tk, dk, dv, kv) || !length_ok(flags, Tq, 1, Tk, 64, dv, *kv)) return false;
   const int64_t gq[4] = {(int64_t)H * Tq * dk, (int64_t)Tq * dk, dk, 1};
   const int64_t gk[4] = {(int64_t)G * Tk * dk, (int64_t)Tk * dk, dk, 1};
   const int64_t gv[4] = {(int64_t)G * Tk * dv, (int64_t)Tk * dv, dv, 1};
@@ -178,6 +197,7 @@ extern "C" NSA_API int nsa_profile_report(char* buf, size_t buf_bytes) {
   NSA_REQUIRE(q_pos0 == 0, what ": a query offset needs the bf16 tensor-core path of this call")
 
 static bool want_tc(int flags) { return (flags & NSA_FLAG_GENERIC) == 0; }
+static bool slc_sized_tc(int flags, int Tkv) { return want_tc(flags) && ((flags & NSA_FLAG_ANY_LENGTH) || Tkv % 64 == 0); }
 
 extern "C" NSA_API int nsa_selftest_wait_timeout(long long limit_clocks, void* stream) {
   NSA_REQUIRE(limit_clocks > 0 && limit_clocks <= (1ll << 24), "selftest: limit must be within 1..2^24 clocks");
@@ -212,13 +232,14 @@ extern "C" NSA_API int nsa_sliding_fwd(const void* q, const void* k, const void*
   NSA_REFUSE_AFTER_TIMEOUT("sliding_fwd");
   KvLayout kv;
   if (want_tc(flags) && dtype == NSA_BF16 && L && M && fa_fwd_sm100_supported(H, G, T, T, dk, dv) &&
-      canonical_fwd(strides, B, H, G, T, T, dk, dv, &kv) && aligned16(q) && aligned16(k) && aligned16(v) && aligned16(out) &&
+      canonical_fwd(strides, B, H, G, T, T, dk, dv, &kv) && length_ok(flags, T, 128, T, 128, dv, kv) && aligned16(q) && aligned16(k) && aligned16(v) && aligned16(out) &&
       (int64_t)B * (H / 2) <= 65535)
     return fa_fwd_sm100(q, k, v, out, L, M, B, H, G, T, T, dk, dv, kWin, window, 0, 0, 0, scale, nullptr, nullptr, kv, (cudaStream_t)stream);
   AttnArgs a = {};
   a.q = q; a.k = k; a.v = v; a.o = out; a.L = L; a.M = M;
   fill_fwd_strides(a, strides);
   a.B = B; a.H = H; a.G = G; a.Tq = T; a.Tk = T; a.dk = dk; a.dv = dv; a.window = window; a.scale = scale; a.causal = 1;
+  if (L && M && aligned16(out) && mma_fwd_ok(a, strides, kWin, flags, dtype)) return launch_attn_mma(a, kWin, false, (cudaStream_t)stream);
   return launch_attn_generic(a, kWin, dtype, false, (cudaStream_t)stream);
 }
 
@@ -232,13 +253,15 @@ extern "C" NSA_API int nsa_sliding_bwd(const void* q, const void* k, const void*
   NSA_REQUIRE(window > 0, "sliding_bwd: window must be positive");
   NSA_REFUSE_AFTER_TIMEOUT("sliding_bwd");
   KvLayout kv;
-  if (want_tc(flags) && tensor_core_bwd_ok(strides, dtype, B, H, G, T, T, dk, dv, q, k, v, out, dout, dq, dkey, dval, &kv))
+  if (want_tc(flags) && tensor_core_bwd_ok(strides, flags, dtype, B, H, G, T, T, dk, dv, q, k, v, out, dout, dq, dkey, dval, &kv))
     return fa_bwd_sm100(q, k, v, out, dout, L, M, dq, dkey, dval, B, H, G, T, T, dk, dv, kWin, window, 0, 0, 0, scale,
                         row_delta, kv, workspace, workspace_bytes, (cudaStream_t)stream);
   AttnArgs a = {};
   a.q = q; a.k = k; a.v = v; a.o_in = out; a.dout = dout; a.Lc = L; a.Mc = M; a.dq = dq; a.dk_out = dkey; a.dv_out = dval;
   fill_bwd_strides(a, strides);
   a.B = B; a.H = H; a.G = G; a.Tq = T; a.Tk = T; a.dk = dk; a.dv = dv; a.window = window; a.scale = scale; a.causal = 1;
+  a.row_delta = row_delta;
+  if (mma_bwd_ok(a, strides, kWin, flags, dtype)) return launch_attn_mma(a, kWin, true, (cudaStream_t)stream);
   return launch_attn_generic(a, kWin, dtype, true, (cudaStream_t)stream);
 }
 
@@ -255,7 +278,7 @@ extern "C" NSA_API int nsa_cmp_attn_fwd(const void* q, const void* k_cmp, const 
   NSA_REFUSE_AFTER_TIMEOUT("cmp_attn_fwd");
   KvLayout kv;
   if (want_tc(flags) && blocks_d > 0 && dtype == NSA_BF16 && L && M && fa_fwd_sm100_supported(H, G, T, NB, dk, dv) &&
-      canonical_fwd(strides, B, H, G, T, NB, dk, dv, &kv) && aligned16(q) && aligned16(k_cmp) && aligned16(v_cmp) &&
+      canonical_fwd(strides, B, H, G, T, NB, dk, dv, &kv) && length_ok(flags, T, 128, NB, 128, dv, kv) && aligned16(q) && aligned16(k_cmp) && aligned16(v_cmp) &&
       aligned16(out) && (int64_t)B * (H / 2) <= 65535)
     // block i is visible to the query at position q0 + t iff i*d + l - 1 <= q0 + t: the same rule with l - q0 for row t
     return fa_fwd_sm100(q, k_cmp, v_cmp, out, L, M, B, H, G, T, NB, dk, dv, kCmp, 0, blocks_l - q_pos0, blocks_d, blocks_n,
@@ -267,11 +290,12 @@ extern "C" NSA_API int nsa_cmp_attn_fwd(const void* q, const void* k_cmp, const 
   a.q = q; a.k = k_cmp; a.v = v_cmp; a.o = out; a.L = L; a.M = M; a.block_ends = block_ends;
   fill_fwd_strides(a, strides);
   a.B = B; a.H = H; a.G = G; a.Tq = T; a.Tk = NB; a.dk = dk; a.dv = dv; a.scale = scale; a.causal = 1;
+  if (L && M && aligned16(out) && mma_fwd_ok(a, strides, kCmp, flags, dtype)) return launch_attn_mma(a, kCmp, false, (cudaStream_t)stream);
   return launch_attn_generic(a, kCmp, dtype, false, (cudaStream_t)stream);
 }
 
 extern "C" NSA_API int nsa_cmp_attn_exact_supported(int B, int H, int G, int T, int NB, int dk, int dv, int dtype) {
-  return dtype == NSA_BF16 && B > 0 && fa_fwd_sm100_supported(H, G, T, NB, dk, dv) && (int64_t)B * (H / 2) <= 65535 ? 1 : 0;
+  return dtype == NSA_BF16 && B > 0 && T % 128 == 0 && NB % 128 == 0 && fa_fwd_sm100_supported(H, G, T, NB, dk, dv) && (int64_t)B * (H / 2) <= 65535 ? 1 : 0;
 }
 
 extern "C" NSA_API int nsa_cmp_attn_bwd(const void* q, const void* k_cmp, const void* v_cmp, const int32_t* block_ends,
@@ -289,7 +313,7 @@ extern "C" NSA_API int nsa_cmp_attn_bwd(const void* q, const void* k_cmp, const 
   NSA_REFUSE_AFTER_TIMEOUT("cmp_attn_bwd");
   KvLayout kv;
   if (want_tc(flags) && blocks_d > 0 &&
-      tensor_core_bwd_ok(strides, dtype, B, H, G, T, NB, dk, dv, q, k_cmp, v_cmp, out, dout, dq, dk_cmp, dv_cmp, &kv))
+      tensor_core_bwd_ok(strides, flags, dtype, B, H, G, T, NB, dk, dv, q, k_cmp, v_cmp, out, dout, dq, dk_cmp, dv_cmp, &kv))
     return fa_bwd_sm100(q, k_cmp, v_cmp, out, dout, L, M, dq, dk_cmp, dv_cmp, B, H, G, T, NB, dk, dv, kCmp, 0,
                         blocks_l - q_pos0, blocks_d, blocks_n, scale, row_delta, kv, workspace, workspace_bytes,
                         (cudaStream_t)stream);
@@ -299,6 +323,8 @@ extern "C" NSA_API int nsa_cmp_attn_bwd(const void* q, const void* k_cmp, const 
   a.dq = dq; a.dk_out = dk_cmp; a.dv_out = dv_cmp;
   fill_bwd_strides(a, strides);
   a.B = B; a.H = H; a.G = G; a.Tq = T; a.Tk = NB; a.dk = dk; a.dv = dv; a.scale = scale; a.causal = 1;
+  a.row_delta = row_delta;
+  if (mma_bwd_ok(a, strides, kCmp, flags, dtype)) return launch_attn_mma(a, kCmp, true, (cudaStream_t)stream);
   return launch_attn_generic(a, kCmp, dtype, true, (cudaStream_t)stream);
 }
 
@@ -315,7 +341,7 @@ static int slc_fwd_impl(const char* who, const void* q, const void* k, const voi
                 "then are invalid.  nsa_device_timeouts(1) reports and clears the condition", who);
   KvLayout kv;
   if (want_tc(flags) && dtype == NSA_BF16 && L && M && B > 0 && slc_sm100_supported(H, G, Tq, Tkv, dk, dv, n_slots, l_prime) &&
-      canonical_fwd(strides, B, H, G, Tq, Tkv, dk, dv, &kv) && aligned16(q) && aligned16(k) && aligned16(v) && aligned16(out) &&
+      canonical_fwd(strides, B, H, G, Tq, Tkv, dk, dv, &kv) && length_ok(flags, Tq, 1, Tkv, 64, dv, kv) && aligned16(q) && aligned16(k) && aligned16(v) && aligned16(out) &&
       (!mix.out || (aligned16(mix.out) && aligned16(mix.o_cmp) && aligned16(mix.o_win))))
     return slc_fwd_sm100(q, k, v, indices, strides + 22, out, L, M, B, H, G, Tq, Tkv, dk, dv, n_slots, l_prime, scale,
                          q_pos0, mix, kv, workspace, workspace_bytes, (cudaStream_t)stream);
@@ -326,7 +352,8 @@ static int slc_fwd_impl(const char* who, const void* q, const void* k, const voi
   for (int i = 0; i < 4; ++i) a.sidx[i] = strides[22 + i];
   a.B = B; a.H = H; a.G = G; a.Tq = Tq; a.Tk = Tkv; a.dk = dk; a.dv = dv; a.scale = scale; a.causal = 1;
   a.nslots = n_slots; a.lprime = l_prime; a.nblk = (Tkv + l_prime - 1) / l_prime;
-  if (int rc = launch_attn_generic(a, kSlc, dtype, false, (cudaStream_t)stream)) return rc;
+  const bool mma = L && M && aligned16(out) && mma_fwd_ok(a, strides, kSlc, flags, dtype);
+  if (int rc = mma ? launch_attn_mma(a, kSlc, false, (cudaStream_t)stream) : launch_attn_generic(a, kSlc, dtype, false, (cudaStream_t)stream)) return rc;
   if (!mix.out) return NSA_OK;
   // stride-generic kernels: the mix runs as its own pass over the three branch outputs (contiguous [B,H,Tq,dv])
   NSA_REQUIRE(strides[15] == 1 && strides[14] == dv && strides[13] == (int64_t)Tq * dv && strides[12] == (int64_t)H * Tq * dv,
@@ -361,14 +388,14 @@ extern "C" NSA_API int nsa_slc_fwd_mix(const void* q, const void* k, const void*
 
 extern "C" NSA_API size_t nsa_slc_fwd_workspace_bytes(int B, int H, int G, int Tq, int Tkv, int dk, int dv, int n_slots,
                                                       int l_prime, int dtype, int flags) {
-  if (!want_tc(flags) || dtype != NSA_BF16 || B <= 0 || !slc_sm100_supported(H, G, Tq, Tkv, dk, dv, n_slots, l_prime)) return 256;
+  if (!slc_sized_tc(flags, Tkv) || dtype != NSA_BF16 || B <= 0 || !slc_sm100_supported(H, G, Tq, Tkv, dk, dv, n_slots, l_prime)) return 256;
   return slc_fwd_sm100_workspace_bytes(B, H, G, Tq, Tkv, dk, dv, n_slots, l_prime);
 }
 
 extern "C" NSA_API size_t nsa_slc_bwd_workspace_bytes(int B, int H, int G, int Tq, int Tkv, int dk, int dv, int n_slots,
                                                       int l_prime, int dtype, int flags) {
   if (B <= 0 || G <= 0 || Tq <= 0 || Tkv <= 0 || n_slots <= 0 || l_prime <= 0) return 256;
-  if (want_tc(flags) && dtype == NSA_BF16 && slc_sm100_supported(H, G, Tq, Tkv, dk, dv, n_slots, l_prime))
+  if (slc_sized_tc(flags, Tkv) && dtype == NSA_BF16 && slc_sm100_supported(H, G, Tq, Tkv, dk, dv, n_slots, l_prime))
     return slc_bwd_sm100_workspace_bytes(B, H, G, Tq, Tkv, dk, dv, n_slots, l_prime);
   return slc_csr_workspace_bytes(B, G, Tq, Tkv, n_slots, l_prime);
 }
@@ -387,7 +414,7 @@ extern "C" NSA_API int nsa_slc_bwd(const void* q, const void* k, const void* v, 
   if (B == 0 || Tq == 0 || Tkv == 0) return NSA_OK;
   KvLayout kv;
   if (want_tc(flags) && slc_sm100_supported(H, G, Tq, Tkv, dk, dv, n_slots, l_prime) &&
-      tensor_core_bwd_ok_slc(strides, dtype, B, H, G, Tq, Tkv, dk, dv, q, k, v, out, dout, dq, dkey, dval, &kv))
+      tensor_core_bwd_ok_slc(strides, flags, dtype, B, H, G, Tq, Tkv, dk, dv, q, k, v, out, dout, dq, dkey, dval, &kv))
     return slc_bwd_sm100(q, k, v, indices, strides + 34, out, dout, L, M, dq, dkey, dval, B, H, G, Tq, Tkv, dk, dv, n_slots,
                          l_prime, scale, q_pos0, row_delta, dq_add0, dq_add1, kv, workspace, workspace_bytes,
                          (cudaStream_t)stream);
@@ -407,7 +434,8 @@ extern "C" NSA_API int nsa_slc_bwd(const void* q, const void* k, const void* v, 
   if (int rc = build_slc_csr(indices, a.sidx, B, G, Tq, Tkv, n_slots, l_prime, 1, 0, workspace, workspace_bytes,
                              &a.csr_off, &a.csr_t, st))
     return rc;
-  if (int rc = launch_attn_generic(a, kSlc, dtype, true, st)) return rc;
+  a.row_delta = row_delta;
+  if (int rc = mma_bwd_ok(a, strides, kSlc, flags, dtype) ? launch_attn_mma(a, kSlc, true, st) : launch_attn_generic(a, kSlc, dtype, true, st)) return rc;
   if (add0 || add1) {
     const int64_t n = (int64_t)B * H * Tq * dk;
     const unsigned blocks = (unsigned)((n + 255) / 256);

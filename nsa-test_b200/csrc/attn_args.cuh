@@ -15,6 +15,7 @@ struct AttnArgs {
   // backward
   const void *o_in, *dout;
   const float *Lc, *Mc;
+  const float* row_delta;  // row sums dO.O [B,H,Tq] when the caller has them (mma family only), else null
   void *dq, *dk_out, *dv_out;
   // masks
   const int* block_ends;  // kCmp: [Tk]
@@ -40,6 +41,9 @@ __device__ __forceinline__ int slot_block(const int* row, int64_t sn, int s, int
   return id;
 }
 
+// bf16 tensors in canonical layouts with 32-bit probabilities (attn_mma.cu); launch_attn_generic serves everything else
+bool attn_mma_supported(int dk, int dv, int mode, int lprime);
+int launch_attn_mma(const AttnArgs& a, int mode, bool backward, cudaStream_t st);
 int launch_attn_generic(const AttnArgs& a, int mode, int dtype, bool backward, cudaStream_t st);
 
 // Inverse index "key block -> queries that selected it" for the selection backward.

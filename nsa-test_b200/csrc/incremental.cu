@@ -124,8 +124,8 @@ ChunkLayout chunk_layout(const nsa_decode_desc& d) {
   L.o_win = take(R * d.dv * 2);
   L.o_gates = take(R * 3 * 4);
   L.o_idx = take(BG * d.Tn * d.n * 4);
-  L.stage = std::max(nsa_score_topn_workspace_bytes(d.B, d.H, d.G, d.Tn, d.dk, d.nbp, d.l, d.d, d.l_prime, d.n, NSA_BF16, 0),
-                     nsa_slc_fwd_workspace_bytes(d.B, d.H, d.G, d.Tn, L.Tk, d.dk, d.dv, d.n, d.l_prime, NSA_BF16, 0));
+  L.stage = std::max(nsa_score_topn_workspace_bytes(d.B, d.H, d.G, d.Tn, d.dk, d.nbp, d.l, d.d, d.l_prime, d.n, NSA_BF16, NSA_FLAG_ANY_LENGTH),
+                     nsa_slc_fwd_workspace_bytes(d.B, d.H, d.G, d.Tn, L.Tk, d.dk, d.dv, d.n, d.l_prime, NSA_BF16, NSA_FLAG_ANY_LENGTH));
   L.o_stage = take(L.stage);
   L.total = o;
   return L;
@@ -207,7 +207,7 @@ extern "C" NSA_API int nsa_incremental_supported(const nsa_decode_desc* dp) {
   const nsa_decode_desc& d = *dp;
   if (d.nb <= 0 || d.cap % 8 != 0 || d.n <= 0 || d.n_fixed < 0 || d.window <= 0 || (int64_t)d.B * d.H > 65535) return 0;
   if ((int64_t)d.B * d.G * d.Tn <= 64) return 0;      // (the scoring would take its few-rows form: decode_sm100.cu serves these)
-  return nsa_cmp_attn_exact_supported(d.B, d.H, d.G, d.Tn, d.nbp, d.dk, d.dv, NSA_BF16) &&
+  return fa_fwd_sm100_supported(d.H, d.G, d.Tn, d.nbp, d.dk, d.dv) &&
          score_sm100_supported(d.H, d.G, d.Tn, d.dk, d.nbp, d.l, d.d, d.l_prime, d.n) &&
          slc_sm100_supported(d.H, d.G, d.Tn, d.pos + d.Tn, d.dk, d.dv, d.n, d.l_prime);
 }
@@ -249,10 +249,10 @@ extern "C" NSA_API int nsa_incremental_fwd(const nsa_decode_desc* dp, void* work
   if (int rc = split_keys_padded((const float*)d.k_cmp, hi, lo, G * d.B * dk, d.nbp, L.ld, st)) return rc;
   strides(L.ld, (int64_t)d.nbp * dv);
   if (int rc = nsa_cmp_attn_fwd(d.q, hi, d.v_cmp, d.block_ends, o_cmp, Ls, Ms, s, d.B, d.H, d.G, d.Tn, d.nb, d.dk, d.dv, d.scale, NSA_BF16, d.l,
-                                d.d, d.nb, d.pos, 0, lo, lse2, stream))
+                                d.d, d.nb, d.pos, NSA_FLAG_ANY_LENGTH, lo, lse2, stream))
     return rc;
   if (int rc = nsa_score_topn(d.q, s, (const float*)d.k_cmp, d.block_ends, idx, d.B, d.H, d.G, d.Tn, d.dk, d.nbp, d.l, d.d, d.l_prime, d.n,
-                              d.n_fixed, d.scale, NSA_BF16, d.nb, d.pos, 0, lse2, w + L.o_stage, L.stage, stream))
+                              d.n_fixed, d.scale, NSA_BF16, d.nb, d.pos, NSA_FLAG_ANY_LENGTH, lse2, w + L.o_stage, L.stage, stream))
     return rc;
   const int64_t rows = (int64_t)d.B * G * T;
   fallback_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, st>>>(idx, rows, d.Tn, d.n, d.l_prime, d.pos);
@@ -262,5 +262,5 @@ extern "C" NSA_API int nsa_incremental_fwd(const nsa_decode_desc* dp, void* work
     return rc;
   strides(d.cap, (int64_t)d.cap * dv);
   return nsa_slc_fwd_mix(d.q, d.k_slc, d.v_slc, idx, o_slc, Ls, Ms, s, d.B, d.H, d.G, d.Tn, L.Tk, d.n, d.l_prime, d.dk, d.dv, d.scale,
-                         NSA_BF16, d.pos, 0, d.gate_logits, o_cmp, o_win, d.out, gates, d.gate_mode, 1, w + L.o_stage, L.stage, stream);
+                         NSA_BF16, d.pos, NSA_FLAG_ANY_LENGTH, d.gate_logits, o_cmp, o_win, d.out, gates, d.gate_mode, 1, w + L.o_stage, L.stage, stream);
 }

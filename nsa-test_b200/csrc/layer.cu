@@ -25,6 +25,9 @@ int next_pow2(int n) {
 
 struct Sizes {
   int nb, nbp;
+  int flags;    // NSA_FLAG_ANY_LENGTH from 2048 tokens on: what the tensor-core kernels gain over the generic ones grows with T
+                // while shorter ragged sequences keep their 32-bit probabilities (attn_mma.cu)
+  bool exact;   // the compressed attention takes its keys as a bf16 pair hi + lo
   int ld_cmp;   // row distance of the compressed keys' I/O-type copies: whole 128-key tiles for the tensor-core kernels
   int ld_time;  // row distance of the keys the tensor-core kernels read: T, or the next multiple of 8 (keys are copied then)
   size_t pad_bytes;
@@ -35,8 +38,10 @@ Sizes sizes_of(const nsa_layer_desc& d) {
   s.nb = d.T >= d.l ? (d.T - d.l) / d.d + 1 : 0;
   s.nbp = next_pow2(s.nb < 1 ? 1 : s.nb);
   s.es = d.dtype == NSA_BF16 ? 2 : 4;
-  s.ld_cmp = d.dtype == NSA_BF16 && s.nb > 0 && nsa_cmp_attn_exact_supported(d.B, d.H, d.G, d.T, s.nbp, d.dk, d.dv, d.dtype)
-                 ? (s.nbp + 127) / 128 * 128 : s.nbp;
+  s.flags = d.dtype == NSA_BF16 && d.T >= 2048 ? NSA_FLAG_ANY_LENGTH : 0;
+  s.exact = d.dtype == NSA_BF16 && s.nb > 0 && fa_fwd_sm100_supported(d.H, d.G, d.T, s.nbp, d.dk, d.dv) &&
+            (s.flags || (d.T % 128 == 0 && s.nbp % 128 == 0)) && (int64_t)d.B * (d.H / 2) <= 65535;
+  s.ld_cmp = s.exact ? (s.nbp + 127) / 128 * 128 : s.nbp;
   s.ld_time = d.dtype == NSA_BF16 ? (d.T + 7) / 8 * 8 : d.T;
   s.pad_bytes = s.ld_time == d.T ? 0 : al256((size_t)d.B * d.G * d.dk * s.ld_time * 2);
   s.rows = (size_t)d.B * d.H * d.T;
@@ -140,15 +145,15 @@ struct Scratch {
 };
 
 size_t stage_scratch_fwd(const nsa_layer_desc& d, const Sizes& s) {
-  size_t m = nsa_score_topn_workspace_bytes(d.B, d.H, d.G, d.T, d.dk, s.nbp, d.l, d.d, d.l_prime, d.n, d.dtype, 0);
-  m = std::max(m, nsa_slc_fwd_workspace_bytes(d.B, d.H, d.G, d.T, d.T, d.dk, d.dv, d.n, d.l_prime, d.dtype, 0));
+  size_t m = nsa_score_topn_workspace_bytes(d.B, d.H, d.G, d.T, d.dk, s.nbp, d.l, d.d, d.l_prime, d.n, d.dtype, s.flags);
+  m = std::max(m, nsa_slc_fwd_workspace_bytes(d.B, d.H, d.G, d.T, d.T, d.dk, d.dv, d.n, d.l_prime, d.dtype, s.flags));
   if (s.nb > 0) m = std::max(m, nsa_cmp_phi_workspace_bytes(d.B, d.G, d.T, d.dk, d.dv, d.l, d.d, d.U, s.nbp, d.dtype, 0));
   return al256(m);
 }
 size_t stage_scratch_bwd(const nsa_layer_desc& d, const Sizes& s) {
   size_t m = nsa_attn_bwd_workspace_bytes(d.B, d.H, d.G, d.T, s.nbp, d.dk, d.dv, 1, 0, 0);
   m = std::max(m, nsa_attn_bwd_workspace_bytes(d.B, d.H, d.G, d.T, d.T, d.dk, d.dv, 0, d.window, 0));
-  m = std::max(m, nsa_slc_bwd_workspace_bytes(d.B, d.H, d.G, d.T, d.T, d.dk, d.dv, d.n, d.l_prime, d.dtype, 0));
+  m = std::max(m, nsa_slc_bwd_workspace_bytes(d.B, d.H, d.G, d.T, d.T, d.dk, d.dv, d.n, d.l_prime, d.dtype, s.flags));
   if (s.nb > 0) m = std::max(m, nsa_cmp_phi_workspace_bytes(d.B, d.G, d.T, d.dk, d.dv, d.l, d.d, d.U, s.nbp, d.dtype, 1));
   return al256(m);
 }
@@ -206,7 +211,7 @@ extern "C" NSA_API int nsa_layer_fwd(const nsa_layer_desc* dp, const void* q, co
   workspace_bytes -= 2 * s.pad_bytes;
 
   // 1. block compression (a sequence shorter than one block leaves only the never-visible padding block)
-  const bool exact = s.nb > 0 && nsa_cmp_attn_exact_supported(d.B, d.H, d.G, d.T, s.nbp, d.dk, d.dv, d.dtype) != 0;
+  const bool exact = s.exact;
   block_ends_kernel<<<(s.nbp + 255) / 256, 256, 0, st>>>(be, s.nbp, s.nb, d.l, d.d);
   if (s.nb > 0) {
     if (int rc = nsa_cmp_phi_fwd(k_cmp_src, v_cmp_src, pos_embed, w1, b1, w2, b2, k_cmp, exact ? nullptr : piece(NSA_CTX_K_CMP_LP), piece(NSA_CTX_V_CMP),
@@ -229,7 +234,7 @@ extern "C" NSA_API int nsa_layer_fwd(const nsa_layer_desc* dp, const void* q, co
   fill_strides(d, s.nbp, s.ld_cmp, 0, false, false, strides);
   if (int rc = nsa_cmp_attn_fwd(q, piece(NSA_CTX_K_CMP_LP), piece(NSA_CTX_V_CMP), be, piece(NSA_CTX_O_CMP), (float*)piece(NSA_CTX_L_CMP),
                                 (float*)piece(NSA_CTX_M_CMP), strides, d.B, d.H, d.G, d.T, s.nbp, d.dk, d.dv, d.scale, d.dtype, d.l, d.d,
-                                s.nb, 0, 0, k_lo, lse2, stream))
+                                s.nb, 0, s.flags, k_lo, lse2, stream))
     return rc;
   // 3. Eq. 8-11: which blocks every query attends
   if (indices_in) {
@@ -237,7 +242,7 @@ extern "C" NSA_API int nsa_layer_fwd(const nsa_layer_desc* dp, const void* q, co
   } else {
     const int64_t qs[4] = {(int64_t)d.H * d.T * d.dk, (int64_t)d.T * d.dk, d.dk, 1};
     if (int rc = nsa_score_topn(q, qs, k_cmp, be, idx, d.B, d.H, d.G, d.T, d.dk, s.nbp, d.l, d.d, d.l_prime, d.n, d.n_fixed, d.scale,
-                                d.dtype, s.nb, 0, 0, lse2, workspace, workspace_bytes, stream))
+                                d.dtype, s.nb, 0, s.flags, lse2, workspace, workspace_bytes, stream))
       return rc;
   }
   {
@@ -248,12 +253,12 @@ extern "C" NSA_API int nsa_layer_fwd(const nsa_layer_desc* dp, const void* q, co
   // 4. sliding window
   fill_strides(d, d.T, s.ld_time, 0, false, false, strides);
   if (int rc = nsa_sliding_fwd(q, k_win_p, v_win, piece(NSA_CTX_O_WIN), (float*)piece(NSA_CTX_L_WIN), (float*)piece(NSA_CTX_M_WIN), strides,
-                               d.B, d.H, d.G, d.T, d.dk, d.dv, d.window, d.scale, d.dtype, 0, stream))
+                               d.B, d.H, d.G, d.T, d.dk, d.dv, d.window, d.scale, d.dtype, s.flags, stream))
     return rc;
   // 5. selected-block attention with the gate + mix as its epilogue
   fill_strides(d, d.T, s.ld_time, d.n, false, true, strides);
   return nsa_slc_fwd_mix(q, k_slc_p, v_slc, idx, piece(NSA_CTX_O_SLC), (float*)piece(NSA_CTX_L_SLC), (float*)piece(NSA_CTX_M_SLC), strides,
-                         d.B, d.H, d.G, d.T, d.T, d.n, d.l_prime, d.dk, d.dv, d.scale, d.dtype, 0, 0, gate_logits,
+                         d.B, d.H, d.G, d.T, d.T, d.n, d.l_prime, d.dk, d.dv, d.scale, d.dtype, 0, s.flags, gate_logits,
                          piece(NSA_CTX_O_CMP), piece(NSA_CTX_O_WIN), out, (float*)piece(NSA_CTX_GATES), d.gate_mode,
                          d.out_token_major, workspace, workspace_bytes, stream);
 }
@@ -302,17 +307,17 @@ extern "C" NSA_API int nsa_layer_bwd(const nsa_layer_desc* dp, const void* q, co
   fill_strides(d, s.nbp, s.ld_cmp, 0, true, false, strides);
   if (int rc = nsa_cmp_attn_bwd(q, piece(NSA_CTX_K_CMP_LP), piece(NSA_CTX_V_CMP), be, piece(NSA_CTX_O_CMP), d_cmp,
                                 (const float*)piece(NSA_CTX_L_CMP), (const float*)piece(NSA_CTX_M_CMP), dq_c, dkc, dvc, strides, d.B, d.H, d.G,
-                                d.T, s.nbp, d.dk, d.dv, d.scale, d.dtype, d.l, d.d, s.nb, 0, delta0, 0, stage, stage_bytes, stream))
+                                d.T, s.nbp, d.dk, d.dv, d.scale, d.dtype, d.l, d.d, s.nb, 0, delta0, s.flags, stage, stage_bytes, stream))
     return rc;
   fill_strides(d, d.T, s.ld_time, 0, true, false, strides);
   if (int rc = nsa_sliding_bwd(q, k_win_p, v_win, piece(NSA_CTX_O_WIN), d_win, (const float*)piece(NSA_CTX_L_WIN),
                                (const float*)piece(NSA_CTX_M_WIN), dq_w, dk_win, dv_win, strides, d.B, d.H, d.G, d.T, d.dk, d.dv, d.window,
-                               d.scale, d.dtype, delta2, 0, stage, stage_bytes, stream))
+                               d.scale, d.dtype, delta2, s.flags, stage, stage_bytes, stream))
     return rc;
   fill_strides(d, d.T, s.ld_time, d.n, true, true, strides);
   if (int rc = nsa_slc_bwd(q, k_slc_p, v_slc, (const int32_t*)piece(NSA_CTX_INDICES), piece(NSA_CTX_O_SLC), d_slc,
                            (const float*)piece(NSA_CTX_L_SLC), (const float*)piece(NSA_CTX_M_SLC), dq, dk_slc, dv_slc, strides, d.B, d.H, d.G,
-                           d.T, d.T, d.n, d.l_prime, d.dk, d.dv, d.scale, d.dtype, 0, delta1, dq_c, dq_w, 0, stage, stage_bytes, stream))
+                           d.T, d.T, d.n, d.l_prime, d.dk, d.dv, d.scale, d.dtype, 0, delta1, dq_c, dq_w, s.flags, stage, stage_bytes, stream))
     return rc;
   if (s.nb > 0)
     return nsa_cmp_phi_bwd(k_cmp_src, pos_embed, w1, w2, dkc, dvc, piece(NSA_CTX_PHI_SAVED), off[NSA_CTX_PHI_SAVED + 1] - off[NSA_CTX_PHI_SAVED],

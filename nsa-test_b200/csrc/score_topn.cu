@@ -231,10 +231,13 @@ static size_t few_rows_logit_bytes(int B, int H, int G, int T, int nbp) {
   return (size_t)B * G * T * hpg * nbp * sizeof(float);
 }
 
+// whole tiles, unless the caller asks for the tensor-core kernel at any length
+static bool score_length_ok(int flags, int T, int nbp) { return (flags & NSA_FLAG_ANY_LENGTH) || (T % 128 == 0 && nbp % 128 == 0); }
 static bool score_tc_ok(const void* q, const int64_t* qs, int B, int H, int G, int T, int dk, int nbp, int l, int d, int l_prime,
                         int n, int n_real_blocks, int dtype, int flags) {
   if ((flags & NSA_FLAG_GENERIC) || dtype != NSA_BF16 || n_real_blocks < 0 || n_real_blocks > nbp) return false;
   if (!score_sm100_supported(H, G, T, dk, nbp, l, d, l_prime, n) || (int64_t)B * G > 65535) return false;
+  if (!score_length_ok(flags, T, nbp)) return false;
   if (few_rows_logit_bytes(B, H, G, T, nbp) > 0) return false;   // (a 128-row tile would leave most of the GPU idle)
   const int64_t cq[4] = {(int64_t)H * T * dk, (int64_t)T * dk, dk, 1};
   for (int i = 0; i < 4; ++i)
@@ -245,7 +248,7 @@ static bool score_tc_ok(const void* q, const int64_t* qs, int B, int H, int G, i
 extern "C" NSA_API size_t nsa_score_topn_workspace_bytes(int B, int H, int G, int T, int dk, int nbp, int l, int d, int l_prime,
                                                          int n, int dtype, int flags) {
   const size_t few = few_rows_logit_bytes(B, H, G, T, nbp);
-  if (few > 0 || B <= 0 || G <= 0 || dtype != NSA_BF16 || (flags & NSA_FLAG_GENERIC) ||
+  if (few > 0 || B <= 0 || G <= 0 || dtype != NSA_BF16 || (flags & NSA_FLAG_GENERIC) || !score_length_ok(flags, T, nbp) ||
       !score_sm100_supported(H, G, T, dk, nbp, l, d, l_prime, n))
     return std::max<size_t>(256, few);
   return score_sm100_workspace_bytes(B, G, T, dk, nbp, d, l_prime);

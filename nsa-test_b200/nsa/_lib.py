@@ -16,7 +16,7 @@ LIB_PATH = os.path.join(_HERE, "libnsa_b200.so")
 
 F32, BF16 = 0, 1
 GATE_SIGMOID, GATE_SOFTMAX = 0, 1
-FLAG_GENERIC, FLAG_RECOMPUTE = 1, 2
+FLAG_GENERIC, FLAG_RECOMPUTE, FLAG_ANY_LENGTH = 1, 2, 4
 
 if not os.path.exists(LIB_PATH):
     raise ImportError(

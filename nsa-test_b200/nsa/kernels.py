@@ -195,16 +195,18 @@ class _BranchesAndMix(torch.autograd.Function):
         # tensor-core kernels apply, the compressed attention runs on the keys as a bf16 pair hi + lo and hands its
         # log-sum-exp to the scoring kernel, which then sweeps the compressed keys once instead of twice.
         lse2 = None
-        if indices is None and k_cmp_f32 is not None and blocks is not None and ops.cmp_exact_supported(q, k_cmp, v_cmp):
+        # long ragged sequences run on the tensor-core kernels, as in the library's own layer calls
+        any_length = q.dtype == torch.bfloat16 and q_pos0 == 0 and Tq >= 2048 and k_slc.shape[-1] == Tq and k_win.shape[-1] == Tq
+        if indices is None and k_cmp_f32 is not None and blocks is not None and ops.cmp_exact_supported(q, k_cmp, v_cmp, any_length):
             hi, lo = ops.split_keys(k_cmp_f32)
-            o_cmp, Lc, Mc, lse2 = ops.cmp_attn_fwd(q, hi, v_cmp, block_ends, scale, blocks, q_pos0, k_lo=lo)
+            o_cmp, Lc, Mc, lse2 = ops.cmp_attn_fwd(q, hi, v_cmp, block_ends, scale, blocks, q_pos0, k_lo=lo, any_length=any_length)
             k_cmp = hi
         else:
-            o_cmp, Lc, Mc = ops.cmp_attn_fwd(q, k_cmp, v_cmp, block_ends, scale, blocks, q_pos0)
+            o_cmp, Lc, Mc = ops.cmp_attn_fwd(q, k_cmp, v_cmp, block_ends, scale, blocks, q_pos0, any_length=any_length)
         if indices is None:
             n_fixed = config.n_fixed if config.include_fixed_in_selection else 0
             indices = ops.score_topn(q, k_cmp_f32, block_ends, config.l, config.d, config.l_prime, config.n, n_fixed, scale,
-                                     blocks[2], q_pos0, cmp_lse2=lse2)
+                                     blocks[2], q_pos0, cmp_lse2=lse2, any_length=any_length)
         ctx.chosen = indices
         idx = _selection_fallback(indices, config.l_prime, q_pos0).to(torch.int32).contiguous()
         lo, hi, pad = _window_slice(q_pos0, Tq, k_win.shape[-1], config.w)
@@ -213,14 +215,15 @@ class _BranchesAndMix(torch.autograd.Function):
             qw = torch.cat([q.new_zeros(q.shape[0], q.shape[1], pad, q.shape[3]), q], dim=2) if pad else q
         else:
             kw_s, vw_s, qw = k_win, v_win, q
-        o_wp, Lw, Mw = ops.sliding_fwd(qw, kw_s, vw_s, config.w, scale)
+        o_wp, Lw, Mw = ops.sliding_fwd(qw, kw_s, vw_s, config.w, scale, any_length=any_length)
         o_win = o_wp[:, :, pad:] if pad else o_wp
         o_slc, Ls, Ms, out, gates = ops.slc_fwd_mix(q, k_slc, v_slc, idx, config.l_prime, scale, gate_logits, o_cmp, o_win,
-                                                    config.gate_mode, q_pos0, token_major)
+                                                    config.gate_mode, q_pos0, token_major, any_length=any_length)
         ctx.save_for_backward(q, k_cmp, v_cmp, block_ends, k_slc, v_slc, idx, kw_s, vw_s, qw, o_cmp, Lc, Mc, o_slc, Ls, Ms,
                               o_wp, Lw, Mw, gates)
         ctx.scale, ctx.l_prime, ctx.w, ctx.blocks = scale, config.l_prime, config.w, blocks
         ctx.gate_mode, ctx.ldtype = config.gate_mode, gate_logits.dtype
+        ctx.any_length = any_length
         ctx.q_pos0, ctx.win = q_pos0, (lo, hi, pad, tuple(k_win.shape), tuple(v_win.shape))
         # one k/v pair feeding both the selection and the sliding-window branch: their dK/dV are summed in the backward
         ctx.shared_win = (k_win.data_ptr() == k_slc.data_ptr() and v_win.data_ptr() == v_slc.data_ptr()
@@ -238,18 +241,18 @@ class _BranchesAndMix(torch.autograd.Function):
         d_cmp, d_slc, d_win, dlogits, delta = ops.gate_mix_bwd(gates, o_cmp, o_slc, o_win, dout, ctx.gate_mode,
                                                                want_delta=True)
         dq_c, dkc, dvc = ops.cmp_attn_bwd(q, k_cmp, v_cmp, block_ends, o_cmp, d_cmp, Lc, Mc, ctx.scale, ctx.blocks,
-                                          ctx.q_pos0, row_delta=delta[0])
+                                          ctx.q_pos0, row_delta=delta[0], any_length=ctx.any_length)
         if pad:
             # the zero query rows in front get a zero upstream gradient and zero row sums: they add nothing to dK/dV
             F = torch.nn.functional
             d_wp, delta_w = F.pad(d_win, (0, 0, pad, 0)), F.pad(delta[2], (pad, 0))
         else:
             d_wp, delta_w = d_win, delta[2]
-        dq_w, dkw, dvw = ops.sliding_bwd(qw, kw_s, vw_s, o_wp, d_wp, Lw, Mw, ctx.w, ctx.scale, row_delta=delta_w)
+        dq_w, dkw, dvw = ops.sliding_bwd(qw, kw_s, vw_s, o_wp, d_wp, Lw, Mw, ctx.w, ctx.scale, row_delta=delta_w, any_length=ctx.any_length)
         if pad:
             dq_w = dq_w[:, :, pad:].contiguous()
         dq, dks, dvs = ops.slc_bwd(q, k_slc, v_slc, idx, o_slc, d_slc, Ls, Ms, ctx.l_prime, ctx.scale, ctx.q_pos0,
-                                   dq_addends=(dq_c, dq_w), row_delta=delta[1])
+                                   dq_addends=(dq_c, dq_w), row_delta=delta[1], any_length=ctx.any_length)
         if ctx.shared_win:
             # the window's gradients (time-major, for the key slice [lo, hi)) go straight into the selection branch's
             # full-length buffers: no zero-filled full-length copies, no separate full-length additions by autograd

@@ -20,11 +20,11 @@ def _k_strides(k: torch.Tensor):
     return [k.stride(0), k.stride(1), k.stride(3), k.stride(2)]
 
 
-def _tc_keys(q, k, generic: bool = False):
-    """Keys the tensor-core kernels can fetch: bf16 rows start on 16-byte boundaries, so a length that is no multiple of 8
-    is served from a copy with padded rows (a view of the same shape)."""
+def _tc_keys(q, k, any_length: bool = False):
+    """Keys the tensor-core kernels can fetch at any length: bf16 rows start on 16-byte boundaries, so a length that is no
+    multiple of 8 is served from a copy with padded rows (a view of the same shape)."""
     T = k.shape[-1]
-    if generic or q.dtype != torch.bfloat16 or T % 8 == 0 or T == 0 or k.dtype != q.dtype:
+    if not any_length or q.dtype != torch.bfloat16 or T % 8 == 0 or T == 0 or k.dtype != q.dtype:
         return k
     buf = k.new_zeros(*k.shape[:-1], (T + 7) // 8 * 8)
     buf[..., :T] = k
@@ -47,25 +47,26 @@ def _stats(q, o_dv):
 # the three branches
 # ------------------------------------------------------------------------------------------------
 
-def sliding_fwd(q, k, v, window: int, scale: float, generic: bool = False):
-    """``generic=True`` forces the stride-generic kernels (cross-checks); same for the functions below."""
-    k = _tc_keys(q, k, generic)
+def sliding_fwd(q, k, v, window: int, scale: float, generic: bool = False, any_length: bool = False):
+    """``generic=True`` forces the stride-generic kernels (cross-checks), ``any_length=True`` admits the tensor-core kernels at
+    lengths that are no whole tiles; same for the functions below."""
+    k = _tc_keys(q, k, any_length)
     dev = require_cuda(q, k, v)
     B, H, T, dk = q.shape
     G, dv = k.shape[1], v.shape[-1]
     o, L, M = _stats(q, dv)
     with torch.cuda.device(dev):
         check(lib.nsa_sliding_fwd(ptr(q), ptr(k), ptr(v), ptr(o), ptr(L), ptr(M), i64(_fwd_strides(q, k, v, o, L, M)),
-                                  B, H, G, T, dk, dv, int(window), float(scale), dtype_code(q), _flags(generic),
+                                  B, H, G, T, dk, dv, int(window), float(scale), dtype_code(q), _flags(generic, any_length=any_length),
                                   stream_ptr(dev)), "nsa_sliding_fwd")
     return o, L, M
 
 
 def sliding_bwd(q, k, v, o, do, L, M, window: int, scale: float, row_delta=None, generic: bool = False,
-                recompute: bool = False):
+                recompute: bool = False, any_length: bool = False):
     """``row_delta``: the row sums dO.O [B,H,T] (fp32) when the caller has them, else they are computed here.
     ``recompute``: small scratch; the dQ kernel recomputes S and dP instead of taking dS from the dK/dV kernel."""
-    k = _tc_keys(q, k, generic)
+    k = _tc_keys(q, k, any_length)
     dev = require_cuda(q, k, v, o, do, L, M)
     delta, dptr = _delta_ptr(row_delta, q)
     B, H, T, dk = q.shape
@@ -77,17 +78,18 @@ def sliding_bwd(q, k, v, o, do, L, M, window: int, scale: float, row_delta=None,
     dkey = torch.zeros(B, G, T, dk, device=dev, dtype=q.dtype)
     dval = torch.zeros(B, G, T, dv, device=dev, dtype=q.dtype)
     s = _fwd_strides(q, k, v, o, L, M) + list(dq.stride()) + list(dkey.stride()) + list(dval.stride())
-    nbytes = lib.nsa_attn_bwd_workspace_bytes(B, H, G, T, T, dk, dv, 0, int(window), _flags(generic, recompute))
+    nbytes = lib.nsa_attn_bwd_workspace_bytes(B, H, G, T, T, dk, dv, 0, int(window), _flags(generic, recompute, any_length))
     ws = torch.empty(nbytes, device=dev, dtype=torch.uint8)
     with torch.cuda.device(dev):
         check(lib.nsa_sliding_bwd(ptr(q), ptr(k), ptr(v), ptr(o), ptr(do), ptr(L), ptr(M), ptr(dq), ptr(dkey), ptr(dval),
-                                  i64(s), B, H, G, T, dk, dv, int(window), float(scale), dtype_code(q), dptr, _flags(generic),
+                                  i64(s), B, H, G, T, dk, dv, int(window), float(scale), dtype_code(q), dptr, _flags(generic, any_length=any_length),
                                   ptr(ws), nbytes, stream_ptr(dev)), "nsa_sliding_bwd")
     return dq, dkey, dval
 
 
-def _flags(generic: bool, recompute: bool = False) -> int:
-    return (_lib.FLAG_GENERIC if generic else 0) | (_lib.FLAG_RECOMPUTE if recompute else 0)
+def _flags(generic: bool, recompute: bool = False, any_length: bool = False) -> int:
+    return ((_lib.FLAG_GENERIC if generic else 0) | (_lib.FLAG_RECOMPUTE if recompute else 0)
+            | (_lib.FLAG_ANY_LENGTH if any_length else 0))
 
 
 def _delta_ptr(row_delta, q):
@@ -100,11 +102,14 @@ def _delta_ptr(row_delta, q):
     return d, ptr(d)
 
 
-def cmp_exact_supported(q, k_cmp, v_cmp) -> bool:
+def cmp_exact_supported(q, k_cmp, v_cmp, any_length: bool = False) -> bool:
     """Does this shape admit the hi + lo key form of the compressed attention's forward (bf16 tensor-core path)?"""
     B, H, T, dk = q.shape
-    return q.dtype == torch.bfloat16 and bool(lib.nsa_cmp_attn_exact_supported(B, H, k_cmp.shape[1], T, k_cmp.shape[-1], dk,
-                                                                              v_cmp.shape[-1], dtype_code(q)))
+    NB = k_cmp.shape[-1]
+    if any_length:
+        T, NB = (T + 127) // 128 * 128, (NB + 127) // 128 * 128
+    return q.dtype == torch.bfloat16 and bool(lib.nsa_cmp_attn_exact_supported(B, H, k_cmp.shape[1], T, NB, dk, v_cmp.shape[-1],
+                                                                              dtype_code(q)))
 
 
 def split_keys(k_cmp_f32):
@@ -118,14 +123,14 @@ def split_keys(k_cmp_f32):
     return hi, lo
 
 
-def cmp_attn_fwd(q, k_cmp, v_cmp, block_ends, scale: float, blocks=None, q_pos0: int = 0, generic: bool = False, k_lo=None):
+def cmp_attn_fwd(q, k_cmp, v_cmp, block_ends, scale: float, blocks=None, q_pos0: int = 0, generic: bool = False, any_length: bool = False, k_lo=None):
     """``blocks=(l, d, n_blocks)`` asserts block_ends[i] == i*d + l - 1 for i < n_blocks and no later block
     ever visible; it lets the tensor-core kernel bound its key loop.  ``k_lo`` (the low-order bf16 part of the keys,
     k_cmp being the high-order one) selects the exact-key form; a fourth result, the log-sum-exp of the logits in log2
     units (+inf on rows that see no block), is then returned for score_topn's ``cmp_lse2``."""
     bl, bd, bn = blocks if blocks is not None else (0, 0, 0)
-    k_cmp = _tc_keys(q, k_cmp, generic)
-    k_lo = None if k_lo is None else _tc_keys(q, k_lo, generic)
+    k_cmp = _tc_keys(q, k_cmp, any_length)
+    k_lo = None if k_lo is None else _tc_keys(q, k_lo, any_length)
     dev = require_cuda(q, k_cmp, v_cmp, block_ends)
     B, H, T, dk = q.shape
     G, NB, dv = k_cmp.shape[1], k_cmp.shape[-1], v_cmp.shape[-1]
@@ -135,15 +140,15 @@ def cmp_attn_fwd(q, k_cmp, v_cmp, block_ends, scale: float, blocks=None, q_pos0:
     with torch.cuda.device(dev):
         check(lib.nsa_cmp_attn_fwd(ptr(q), ptr(k_cmp), ptr(v_cmp), ptr(be), ptr(o), ptr(L), ptr(M),
                                    i64(_fwd_strides(q, k_cmp, v_cmp, o, L, M)), B, H, G, T, NB, dk, dv, float(scale),
-                                   dtype_code(q), int(bl), int(bd), int(bn), int(q_pos0), _flags(generic), ptr(k_lo), ptr(lse2),
+                                   dtype_code(q), int(bl), int(bd), int(bn), int(q_pos0), _flags(generic, any_length=any_length), ptr(k_lo), ptr(lse2),
                                    stream_ptr(dev)), "nsa_cmp_attn_fwd")
     return (o, L, M) if k_lo is None else (o, L, M, lse2)
 
 
 def cmp_attn_bwd(q, k_cmp, v_cmp, block_ends, o, do, L, M, scale: float, blocks=None, q_pos0: int = 0, row_delta=None,
-                 generic: bool = False, recompute: bool = False):
+                 generic: bool = False, recompute: bool = False, any_length: bool = False):
     bl, bd, bn = blocks if blocks is not None else (0, 0, 0)
-    k_cmp = _tc_keys(q, k_cmp, generic)
+    k_cmp = _tc_keys(q, k_cmp, any_length)
     dev = require_cuda(q, k_cmp, v_cmp, block_ends, o, do, L, M)
     delta, dptr = _delta_ptr(row_delta, q)
     B, H, T, dk = q.shape
@@ -156,12 +161,12 @@ def cmp_attn_bwd(q, k_cmp, v_cmp, block_ends, o, do, L, M, scale: float, blocks=
     dkc = torch.zeros(B, G, NB, dk, device=dev, dtype=q.dtype)
     dvc = torch.zeros(B, G, NB, dv, device=dev, dtype=q.dtype)
     s = _fwd_strides(q, k_cmp, v_cmp, o, L, M) + list(dq.stride()) + list(dkc.stride()) + list(dvc.stride())
-    nbytes = lib.nsa_attn_bwd_workspace_bytes(B, H, G, T, NB, dk, dv, 1, 0, _flags(generic, recompute))
+    nbytes = lib.nsa_attn_bwd_workspace_bytes(B, H, G, T, NB, dk, dv, 1, 0, _flags(generic, recompute, any_length))
     ws = torch.empty(nbytes, device=dev, dtype=torch.uint8)
     with torch.cuda.device(dev):
         check(lib.nsa_cmp_attn_bwd(ptr(q), ptr(k_cmp), ptr(v_cmp), ptr(be), ptr(o), ptr(do), ptr(L), ptr(M), ptr(dq),
                                    ptr(dkc), ptr(dvc), i64(s), B, H, G, T, NB, dk, dv, float(scale), dtype_code(q),
-                                   int(bl), int(bd), int(bn), int(q_pos0), dptr, _flags(generic), ptr(ws), nbytes,
+                                   int(bl), int(bd), int(bn), int(q_pos0), dptr, _flags(generic, any_length=any_length), ptr(ws), nbytes,
                                    stream_ptr(dev)), "nsa_cmp_attn_bwd")
     return dq, dkc, dvc
 
@@ -199,8 +204,8 @@ def cache_append(desc, tensors, params) -> None:
               "nsa_cache_append")
 
 
-def slc_fwd(q, k, v, indices_i32, l_prime: int, scale: float, q_pos0: int = 0, generic: bool = False):
-    k = _tc_keys(q, k, generic)
+def slc_fwd(q, k, v, indices_i32, l_prime: int, scale: float, q_pos0: int = 0, generic: bool = False, any_length: bool = False):
+    k = _tc_keys(q, k, any_length)
     dev = require_cuda(q, k, v, indices_i32)
     B, H, Tq, dk = q.shape
     G, Tkv, dv = k.shape[1], k.shape[-1], v.shape[-1]
@@ -208,11 +213,11 @@ def slc_fwd(q, k, v, indices_i32, l_prime: int, scale: float, q_pos0: int = 0, g
     o, L, M = _stats(q, dv)
     s = _fwd_strides(q, k, v, o, L, M) + list(indices_i32.stride())
     n = indices_i32.shape[-1]
-    nbytes = lib.nsa_slc_fwd_workspace_bytes(B, H, G, Tq, Tkv, dk, dv, n, int(l_prime), dtype_code(q), _flags(generic))
+    nbytes = lib.nsa_slc_fwd_workspace_bytes(B, H, G, Tq, Tkv, dk, dv, n, int(l_prime), dtype_code(q), _flags(generic, any_length=any_length))
     ws = torch.empty(nbytes, device=dev, dtype=torch.uint8)
     with torch.cuda.device(dev):
         check(lib.nsa_slc_fwd(ptr(q), ptr(k), ptr(v), ptr(indices_i32), ptr(o), ptr(L), ptr(M), i64(s), B, H, G, Tq, Tkv,
-                              n, int(l_prime), dk, dv, float(scale), dtype_code(q), int(q_pos0), _flags(generic), ptr(ws),
+                              n, int(l_prime), dk, dv, float(scale), dtype_code(q), int(q_pos0), _flags(generic, any_length=any_length), ptr(ws),
                               nbytes, stream_ptr(dev)), "nsa_slc_fwd")
     return o, L, M
 
@@ -227,9 +232,9 @@ def _mixed_empty(like: torch.Tensor, token_major: bool) -> torch.Tensor:
 
 
 def slc_fwd_mix(q, k, v, indices_i32, l_prime: int, scale: float, gate_logits, o_cmp, o_win, gate_mode: str, q_pos0: int = 0,
-                token_major: bool = False, generic: bool = False):
+                token_major: bool = False, generic: bool = False, any_length: bool = False):
     """Selection forward with the layer's gate + mix as its epilogue -> (o_slc, L, M, out_mixed, gates [B,H,T,3])."""
-    k = _tc_keys(q, k, generic)
+    k = _tc_keys(q, k, any_length)
     dev = require_cuda(q, k, v, indices_i32, gate_logits, o_cmp, o_win)
     B, H, Tq, dk = q.shape
     G, Tkv, dv = k.shape[1], k.shape[-1], v.shape[-1]
@@ -242,21 +247,21 @@ def slc_fwd_mix(q, k, v, indices_i32, l_prime: int, scale: float, gate_logits, o
     out = _mixed_empty(o, token_major)
     gates = torch.empty(B, H, Tq, 3, device=dev, dtype=torch.float32)
     mode = _lib.GATE_SOFTMAX if gate_mode == "softmax" else _lib.GATE_SIGMOID
-    nbytes = lib.nsa_slc_fwd_workspace_bytes(B, H, G, Tq, Tkv, dk, dv, n, int(l_prime), dtype_code(q), _flags(generic))
+    nbytes = lib.nsa_slc_fwd_workspace_bytes(B, H, G, Tq, Tkv, dk, dv, n, int(l_prime), dtype_code(q), _flags(generic, any_length=any_length))
     ws = torch.empty(nbytes, device=dev, dtype=torch.uint8)
     with torch.cuda.device(dev):
         check(lib.nsa_slc_fwd_mix(ptr(q), ptr(k), ptr(v), ptr(indices_i32), ptr(o), ptr(L), ptr(M), i64(s), B, H, G, Tq, Tkv,
-                                  n, int(l_prime), dk, dv, float(scale), dtype_code(q), int(q_pos0), _flags(generic), ptr(lg),
+                                  n, int(l_prime), dk, dv, float(scale), dtype_code(q), int(q_pos0), _flags(generic, any_length=any_length), ptr(lg),
                                   ptr(o_cmp), ptr(o_win), ptr(out), ptr(gates), mode, 1 if token_major else 0, ptr(ws), nbytes,
                                   stream_ptr(dev)), "nsa_slc_fwd_mix")
     return o, L, M, out, gates
 
 
 def slc_bwd(q, k, v, indices_i32, o, do, L, M, l_prime: int, scale: float, q_pos0: int = 0, dq_addends=(), row_delta=None,
-            generic: bool = False):
+            generic: bool = False, any_length: bool = False):
     """``dq_addends``: up to two tensors shaped and typed like q (the dQ of the other branches) that the kernel adds
     to the selection branch's dQ before the one rounding of the sum."""
-    k = _tc_keys(q, k, generic)
+    k = _tc_keys(q, k, any_length)
     dev = require_cuda(q, k, v, indices_i32, o, do, L, M)
     delta, dptr = _delta_ptr(row_delta, q)
     B, H, Tq, dk = q.shape
@@ -268,7 +273,7 @@ def slc_bwd(q, k, v, indices_i32, o, do, L, M, l_prime: int, scale: float, q_pos
     dq = torch.empty_like(q, memory_format=torch.contiguous_format)
     dkey = torch.zeros(B, G, Tkv, dk, device=dev, dtype=q.dtype)
     dval = torch.zeros(B, G, Tkv, dv, device=dev, dtype=q.dtype)
-    nbytes = lib.nsa_slc_bwd_workspace_bytes(B, H, G, Tq, Tkv, dk, dv, n, int(l_prime), dtype_code(q), _flags(generic))
+    nbytes = lib.nsa_slc_bwd_workspace_bytes(B, H, G, Tq, Tkv, dk, dv, n, int(l_prime), dtype_code(q), _flags(generic, any_length=any_length))
     ws = torch.empty(nbytes, device=dev, dtype=torch.uint8)
     s = (_fwd_strides(q, k, v, o, L, M) + list(dq.stride()) + list(dkey.stride()) + list(dval.stride())
          + list(indices_i32.stride()))
@@ -280,7 +285,7 @@ def slc_bwd(q, k, v, indices_i32, o, do, L, M, l_prime: int, scale: float, q_pos
     with torch.cuda.device(dev):
         check(lib.nsa_slc_bwd(ptr(q), ptr(k), ptr(v), ptr(indices_i32), ptr(o), ptr(do), ptr(L), ptr(M), ptr(dq),
                               ptr(dkey), ptr(dval), i64(s), B, H, G, Tq, Tkv, n, int(l_prime), dk, dv, float(scale),
-                              dtype_code(q), int(q_pos0), dptr, add0, add1, _flags(generic), ptr(ws), nbytes,
+                              dtype_code(q), int(q_pos0), dptr, add0, add1, _flags(generic, any_length=any_length), ptr(ws), nbytes,
                               stream_ptr(dev)), "nsa_slc_bwd")
     return dq, dkey, dval
 
@@ -369,7 +374,7 @@ def phi_pool_bwd(a, c, dhbar, dv_cmp, l: int, d: int, n_blocks: int):
 
 
 def score_topn(q, k_cmp_f32, block_ends, l: int, d: int, l_prime: int, n: int, n_fixed: int, scale: float,
-               n_real_blocks: int = -1, q_pos0: int = 0, generic: bool = False, cmp_lse2=None):
+               n_real_blocks: int = -1, q_pos0: int = 0, generic: bool = False, any_length: bool = False, cmp_lse2=None):
     """q [B,H,T,dk], k_cmp fp32 [B,G,dk,nbp] -> int32 indices [B,G,T,n].  ``n_real_blocks >= 0`` asserts the
     canonical block ends (block i ends at i*d + l - 1 for i < n_real_blocks, later blocks never visible)."""
     dev = require_cuda(q, k_cmp_f32, block_ends)
@@ -379,12 +384,12 @@ def score_topn(q, k_cmp_f32, block_ends, l: int, d: int, l_prime: int, n: int, n
     be = block_ends.to(torch.int32).contiguous()
     out = torch.empty(B, G, T, n, device=dev, dtype=torch.int32)
     nbytes = lib.nsa_score_topn_workspace_bytes(B, H, G, T, dk, nbp, int(l), int(d), int(l_prime), int(n), dtype_code(q),
-                                                _flags(generic))
+                                                _flags(generic, any_length=any_length))
     ws = torch.empty(nbytes, device=dev, dtype=torch.uint8)
     with torch.cuda.device(dev):
         check(lib.nsa_score_topn(ptr(q), i64(q.stride()), ptr(kc), ptr(be), ptr(out), B, H, G, T, dk, nbp, int(l), int(d),
                                  int(l_prime), int(n), int(n_fixed), float(scale), dtype_code(q), int(n_real_blocks),
-                                 int(q_pos0), _flags(generic), ptr(cmp_lse2), ptr(ws), nbytes, stream_ptr(dev)), "nsa_score_topn")
+                                 int(q_pos0), _flags(generic, any_length=any_length), ptr(cmp_lse2), ptr(ws), nbytes, stream_ptr(dev)), "nsa_score_topn")
     return out
 
 

@@ -35,29 +35,29 @@ def test_selection_over_ragged_chunks_and_short_ranges(dk, dv, H, G, T, n):
     _grad_close(dval, gv, "dv")
 
 
-# (T = 32..46 shows every row at most one compressed block: the softmax over it is constant, the true gradient of phi is zero
-# and a bound relative to it has no scale.  At 63, sixteen rows see two blocks and sixteen one, whose bf16 roundings, 2^-8 of
-# a term each, stay under 1 % of the gradient.)
-@pytest.mark.parametrize("T", [20, 63, 100, 129, 200, 637, 1030])
+@pytest.mark.parametrize("T", [20, 100, 129, 200, 637, 1030, 2061])
 @pytest.mark.parametrize("dk,dv,H,G", [(64, 64, 4, 2), (192, 128, 16, 1)])
 def test_bf16_layer_at_any_length(dk, dv, H, G, T):
     """Sequences that are no multiple of a tile, of 64 or of 8, shorter than a key tile, and with fewer compressed blocks
-    than a tile holds run on the tensor-core kernels: ids, outputs and all gradients against the oracle."""
+    than a tile holds: ids, outputs and all gradients against the oracle.  From 2048 tokens on the tensor-core kernels run,
+    whose probabilities are bf16; shorter ones keep fp32 probabilities."""
     import nsa
     from nsa import _lib
     from nsa.kernels import nsa_layer
     from tests.util import check_layer_against_oracle
-    c = dict(B=2, H=H, G=G, T=T, dk=dk, dv=dv, d_model=64, l=32, d=16, l_prime=64, n=16, w=150)
-    inp = O.make_inputs(2, H, G, T, dk, dv, 64, 32, seed=T, block_offset_std=0.5, dtype=torch.bfloat16)
+    B = 1 if T > 2000 else 2
+    c = dict(B=B, H=H, G=G, T=T, dk=dk, dv=dv, d_model=64, l=32, d=16, l_prime=64, n=16, w=150)
+    inp = O.make_inputs(B, H, G, T, dk, dv, 64, 32, seed=T, block_offset_std=0.5, dtype=torch.bfloat16)
     check_layer_against_oracle(f"bf16 layer dk={dk} T={T}", nsa, c, inp, torch.bfloat16)
     _no_timeouts()
     if T >= 32:
         cfg = nsa.NSAConfig(d_model=64, head_dim_qk=dk, head_dim_v=dv, n_heads=H, n_kv_groups=G, w=150)
         q, k, v = (inp[x].to(DEV, torch.bfloat16).requires_grad_(True) for x in ("q", "k", "v"))
         phi = tuple(getattr(inp["phi"], n_).to(DEV) for n_ in ("pos_embed", "w1", "b1", "w2", "b2"))
-        logits = torch.zeros(2, T, 3 * H, device=DEV)
-        ran = _lib.profile_kernels(lambda: torch.autograd.grad(nsa_layer(q, k, v, logits, phi, cfg).sum(), (q, k, v)))
-        assert {"fa_fwd_win", "fa_fwd_cmp_exact", "slc_bwd_fused", "fa_bwd_dkv_cmp", "fa_bwd_dqds_win"} <= set(ran), ran
+        logits = torch.zeros(B, T, 3 * H, device=DEV)
+        ran = set(_lib.profile_kernels(lambda: torch.autograd.grad(nsa_layer(q, k, v, logits, phi, cfg).sum(), (q, k, v))))
+        tc = {"fa_fwd_win", "fa_fwd_cmp_exact", "slc_bwd_fused", "fa_bwd_dkv_cmp", "fa_bwd_dqds_win"}
+        assert tc <= ran if T >= 2048 else not tc & ran and {"attn_fwd_mma", "attn_bwd_mma"} <= ran, ran
 
 
 @pytest.mark.parametrize("Tk,lo", [(384, 128), (200, 72)])
@@ -68,7 +68,7 @@ def test_keys_and_values_read_as_slices_of_a_longer_buffer(Tk, lo):
     q, _, _, _ = _inputs(B, H, G, Tk, dk, dv, seed=3)
     _, k, v, _ = _inputs(B, H, G, 1024, dk, dv, seed=4)
     ks, vs = k[..., lo:lo + Tk], v[:, :, lo:lo + Tk]
-    o, L, M = ops.sliding_fwd(q.to(DEV), k.to(DEV)[..., lo:lo + Tk], v.to(DEV)[:, :, lo:lo + Tk], 100, 0.125)
+    o, L, M = ops.sliding_fwd(q.to(DEV), k.to(DEV)[..., lo:lo + Tk], v.to(DEV)[:, :, lo:lo + Tk], 100, 0.125, any_length=True)
     torch.cuda.synchronize()
     _no_timeouts()
     ref = O.sliding_window_attention(q.float(), ks.float().contiguous(), vs.float().contiguous(), 100, 0.125)
@@ -258,3 +258,59 @@ def test_generic_kernels_ignore_what_a_row_does_not_see():
         for a, b in ((o[:, :, :bad], o2[:, :, :bad]), (dq[:, :, :bad], dq2[:, :, :bad]), (dkey[:, :, 8:], dkey2[:, :, 8:]),
                      (dval[:, :, 8:], dval2[:, :, 8:])):
             assert torch.isfinite(b).all() and max_abs(a, b) < 1e-5
+
+
+@pytest.mark.parametrize("dk,dv,H,G,T,w,n", [(64, 64, 3, 1, 72, 1, 3), (192, 128, 16, 1, 200, 100, 4), (128, 128, 80, 1, 40, 512, 1),
+                                             (64, 64, 4, 4, 1000, 333, 16)])
+def test_mma_kernels_keep_32_bit_probabilities(dk, dv, H, G, T, w, n):
+    """Ragged bf16 calls (groups of 1, 3, 16 and 80 heads, windows of one key and past the sequence, ends in no order) against the
+    oracle on the same inputs; their error against it is that of the fp32-probability FMA kernels: what rounding the results to bf16
+    leaves, with a tenth of room for sums in another order.  (A window of one key has a zero gradient, a difference of two equal
+    sums of dv products in 32 bits: 1e-6 of what the products alone would give.)"""
+    from nsa import _lib, ops
+    q, k, v, do = _inputs(2, H, G, T, dk, dv, seed=T + dk)
+    gen = torch.Generator().manual_seed(n)
+    idx = torch.randint(-1, -(-T // 64), (2, G, T, n), generator=gen, dtype=torch.int32)
+    idx[..., 0] = (torch.arange(T) // 64).int()
+    ends = torch.full((T,), 999999, dtype=torch.int32)
+    ends[:T // 2] = torch.randperm(T, generator=gen)[:T // 2].int()
+    scale = dk ** -0.5
+    d = lambda t: t.to(DEV)
+    for name, fwd, bwd, ref in (
+            ("win", lambda *a, **k_: ops.sliding_fwd(*a, w, scale, **k_), lambda *a, **k_: ops.sliding_bwd(*a, w, scale, **k_),
+             lambda a, b, c: O.sliding_window_attention(a, b, c, w, scale)),
+            ("cmp", lambda *a, **k_: ops.cmp_attn_fwd(*a, d(ends), scale, **k_),
+             lambda a, b, c, *r, **k_: ops.cmp_attn_bwd(a, b, c, d(ends), *r, scale, **k_),
+             lambda a, b, c: _masked(a, b, c, ends[None, :] <= torch.arange(T)[:, None], scale)),
+            ("slc", lambda *a, **k_: ops.slc_fwd(*a, d(idx), 64, scale, **k_),
+             lambda a, b, c, *r, **k_: ops.slc_bwd(a, b, c, d(idx), *r, 64, scale, **k_),
+             lambda a, b, c: O.selection_attention(a, b, c, idx, 64, scale))):
+        got = []
+        for generic in (False, True):
+            def run():
+                o, L, M = fwd(d(q), d(k), d(v), generic=generic)
+                got.append((o, *bwd(d(q), d(k), d(v), o, d(do), L, M, generic=generic), L, M))
+            ran = set(_lib.profile_kernels(run))
+            assert ("attn_fwd_mma" in ran and "attn_bwd_mma" in ran) != generic, ran
+        qf, kf, vf = (t.double().requires_grad_(True) for t in (q, k, v))
+        want = ref(qf, kf, vf)
+        gq, gk, gv = torch.autograd.grad(want, (qf, kf, vf), do.double())
+        for what, a, b, r in zip(("o", "dq", "dk", "dv"), *got, (want, gq, gk.transpose(-1, -2), gv)):
+            ea, eb = (a.double().cpu() - r).norm().item(), (b.double().cpu() - r).norm().item()
+            floor = do.double().norm() * v.double().norm(dim=-1).max() * max(k.double().norm(dim=-2).max(), q.double().norm(dim=-1).max()) * scale
+            assert ea <= 1.1 * eb + 1e-6 * floor.item(), (name, what, ea, eb)
+        for a, b in zip(got[0][4:], got[1][4:]):
+            assert torch.equal(torch.isfinite(a), torch.isfinite(b)) and max_abs(a.nan_to_num(0, 0, 0), b.nan_to_num(0, 0, 0)) < 1e-4, name
+    # values that are not finite behind what a row sees
+    kk, vv = d(k).clone(), d(v).clone()
+    kk[..., T - 5:], vv[:, :, T - 5:] = float("nan"), float("inf")
+    dd = d(do).clone()
+    dd[:, :, :8] = float("nan")
+    o, L, M = ops.sliding_fwd(d(q), d(k), d(v), w, scale)
+    dq, dkey, dval = ops.sliding_bwd(d(q), d(k), d(v), o, d(do), L, M, w, scale)
+    _, dkey2, dval2 = ops.sliding_bwd(d(q), d(k), d(v), o, dd, L, M, w, scale)
+    o2, L2, M2 = ops.sliding_fwd(d(q), kk, vv, w, scale)
+    dq2, _, _ = ops.sliding_bwd(d(q), kk, vv, o2, d(do), L2, M2, w, scale)
+    torch.cuda.synchronize()
+    for a, b in ((o[:, :, :T - 5], o2[:, :, :T - 5]), (dq[:, :, :T - 5], dq2[:, :, :T - 5]), (dkey[:, :, 8:], dkey2[:, :, 8:]), (dval[:, :, 8:], dval2[:, :, 8:])):
+        assert torch.isfinite(b).all() and max_abs(a.float(), b.float()) <= 2 ** -7 * max(1.0, a.float().abs().max().item())
