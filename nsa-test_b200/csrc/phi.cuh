@@ -11,4 +11,11 @@ int cmp_phi_fwd_strided(const void* k, int64_t k_ld, int64_t k_plane, const void
                         int B, int G, int T, int dk, int dv, int l, int d, int U, int nbp, bool pad, int dtype, void* saved,
                         size_t saved_bytes, void* workspace, size_t workspace_bytes, cudaStream_t st);
 
+// Pooling backward for l = 32, d = 16 in one pass: da in the I/O type, dv_out += dv, dc_part [phi_pool_bwd_parts() * BG, l, U].
+bool phi_pool_bwd_fused_ok(int l, int d);
+int phi_pool_bwd_parts(int BG, int T);
+template <typename T>
+int phi_pool_bwd_fused(const float* a, const float* c, const float* dhbar, const float* dv_cmp, T* da, float* dc_part, T* dv_out, int BG, int Tn,
+                       int U, int dv, int nb, int nbp, cudaStream_t st);
+
 }  // namespace nsa

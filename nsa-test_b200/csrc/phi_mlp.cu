@@ -18,6 +18,7 @@
 #include <dlfcn.h>
 
 #include <algorithm>
+#include <initializer_list>
 #include <mutex>
 
 #include "common.cuh"
@@ -106,6 +107,7 @@ __global__ void c_table_kernel(const float* __restrict__ pos, const float* __res
   if (i >= l * U) return;
   const int j = i / U, u = i % U;
   float acc = b1 ? b1[u] : 0.f;
+#pragma unroll 16
   for (int m = 0; m < l; ++m) acc = fmaf(pos[j * l + m], w1[(int64_t)u * (dk + l) + dk + m], acc);
   c[i] = acc;
 }
@@ -133,16 +135,21 @@ __global__ void rows_to_f32_kernel(const T* __restrict__ in, float* __restrict__
   const int64_t bg = i / ((int64_t)W * nb_out);
   out[i] = r < nb ? Elem<T>::ld(in + (bg * nbp + r) * W + c) : 0.f;
 }
-// Column sums out[c] = sum over rows of in[row, c] in a fixed order: 1024-row chunks are summed by 8 row lanes per column
-// (stage 1, partial sums to scratch), the chunks then one after the other (stage 2).
-constexpr int kColsumChunk = 1024;
+// Column sums out[c] = sum over rows of in[row, c] in a fixed order: chunks of rows are summed by 8 row lanes per column
+// (stage 1, partial sums to scratch), the chunks then one after the other (stage 2).  A chunk has up to 1024 rows, fewer as
+// long as the grid is short of four CTAs per SM: 1024 rows of a 1280-wide matrix were 40 CTAs and 15 us.
+int colsum_chunk(int64_t rows, int W) {
+  const int64_t want = (4 * 148 + (W + 31) / 32 - 1) / ((W + 31) / 32);      // chunks
+  return (int)std::min<int64_t>(1024, std::max<int64_t>(32, (rows + want - 1) / want));
+}
 template <typename T>
-__global__ void colsum_stage1_kernel(const T* __restrict__ in, int64_t rows, int W, float* __restrict__ part) {
+__global__ void colsum_stage1_kernel(const T* __restrict__ in, int64_t rows, int W, int chunk, float* __restrict__ part) {
   __shared__ float sh[8][32];
   const int c = blockIdx.x * 32 + (threadIdx.x & 31), rl = threadIdx.x >> 5;
-  const int64_t r0 = (int64_t)blockIdx.y * kColsumChunk, r1 = min(rows, r0 + kColsumChunk);
+  const int64_t r0 = (int64_t)blockIdx.y * chunk, r1 = min(rows, r0 + chunk);
   float acc = 0.f;
   if (c < W)
+#pragma unroll 8
     for (int64_t r = r0 + rl; r < r1; r += 8) acc += Elem<T>::ld(in + r * W + c);
   sh[rl][threadIdx.x & 31] = acc;
   __syncthreads();
@@ -157,6 +164,7 @@ __global__ void colsum_stage2_kernel(const float* __restrict__ part, int chunks,
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= W) return;
   float acc = 0.f;
+#pragma unroll 16
   for (int i = 0; i < chunks; ++i) acc += part[(int64_t)i * W + c];
   out[c] = acc;
 }
@@ -175,6 +183,7 @@ __global__ void dc_sum_kernel(const float* __restrict__ part, int BG, int n, flo
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float acc = 0.f;
+#pragma unroll 16
   for (int b = 0; b < BG; ++b) acc += part[(int64_t)b * n + i];
   dc[i] = acc;
 }
@@ -184,30 +193,37 @@ __global__ void table_grads_kernel(const float* __restrict__ dc, const float* __
   const int ld = dk + l;
   if (i < U) {
     float acc = 0.f;
+#pragma unroll 16
     for (int j = 0; j < l; ++j) acc += dc[j * U + i];
     db1[i] = acc;
   }
   if (i < U * l) {
     const int u = i / l, m = i % l;
     float acc = 0.f;
+#pragma unroll 16
     for (int j = 0; j < l; ++j) acc = fmaf(dc[j * U + u], pos[j * l + m], acc);
     dw1[(int64_t)u * ld + dk + m] = acc;
   }
-  if (i < l * l) {
-    const int j = i / l, m = i % l;
+  // (a warp per entry: U products one after the other by one thread were 30 us at U = 384)
+  const int w = i >> 5, lane = threadIdx.x & 31;
+  if (w < l * l) {
+    const int j = w / l, m = w % l;
     float acc = 0.f;
-    for (int u = 0; u < U; ++u) acc = fmaf(dc[j * U + u], w1[(int64_t)u * ld + dk + m], acc);
-    dpos[i] = acc;
+#pragma unroll 4
+    for (int u = lane; u < U; u += 32) acc = fmaf(dc[j * U + u], w1[(int64_t)u * ld + dk + m], acc);
+    acc = warp_sum(acc);
+    if (lane == 0) dpos[w] = acc;
   }
 }
 
 unsigned blocks_for(int64_t n) { return (unsigned)((n + 255) / 256); }
 
-size_t colsum_scratch_bytes(int64_t rows, int W) { return al256((size_t)((rows + kColsumChunk - 1) / kColsumChunk) * W * sizeof(float)); }
+int colsum_chunks(int64_t rows, int W) { return (int)((rows + colsum_chunk(rows, W) - 1) / colsum_chunk(rows, W)); }
+size_t colsum_scratch_bytes(int64_t rows, int W) { return al256((size_t)colsum_chunks(rows, W) * W * sizeof(float)); }
 template <typename T>
 void colsum(const T* in, int64_t rows, int W, float* out, float* scratch, cudaStream_t st) {
-  const int chunks = (int)((rows + kColsumChunk - 1) / kColsumChunk);
-  colsum_stage1_kernel<T><<<dim3((W + 31) / 32, chunks), 256, 0, st>>>(in, rows, W, scratch);
+  const int chunks = colsum_chunks(rows, W);
+  colsum_stage1_kernel<T><<<dim3((W + 31) / 32, chunks), 256, 0, st>>>(in, rows, W, colsum_chunk(rows, W), scratch);
   colsum_stage2_kernel<<<blocks_for(W), 256, 0, st>>>(scratch, chunks, W, out);
 }
 
@@ -221,7 +237,7 @@ SavedLayout saved_layout(int B, int G, int T, int l, int d, int U) {
   s.total = s.o_hbar + al256(BG * nb * U * sizeof(float));
   return s;
 }
-struct BwdLayout { size_t o_dkc, o_dhbar, o_dvc, o_da, o_dalp, o_dcpart, o_dc, o_dvt, o_w1k, o_cs, total; };
+struct BwdLayout { size_t o_dkc, o_dhbar, o_dvc, o_da, o_dalp, o_dcpart, o_dc, o_dvt, o_w1k, o_cs, parts, total; };
 BwdLayout bwd_layout(int B, int G, int T, int dk, int dv, int l, int d, int U, int nbp, int dtype) {
   const size_t BG = (size_t)B * G, nb = T >= l ? (size_t)(T - l) / d + 1 : 0, es = dtype == NSA_BF16 ? 2 : 4;
   BwdLayout w;
@@ -229,11 +245,13 @@ BwdLayout bwd_layout(int B, int G, int T, int dk, int dv, int l, int d, int U, i
   w.o_dkc = o;    o += al256(BG * nb * dk * sizeof(float));
   w.o_dhbar = o;  o += al256(BG * nb * U * sizeof(float));
   w.o_dvc = o;    o += al256(BG * nbp * dv * sizeof(float));
-  w.o_da = o;     o += al256(BG * T * U * sizeof(float));
-  w.o_dalp = o;   o += dtype == NSA_BF16 ? al256(BG * T * U * es) : 0;
-  w.o_dcpart = o; o += al256(BG * l * U * sizeof(float));
+  const bool fused = phi_pool_bwd_fused_ok(l, d);      // da leaves the pooling kernel in the I/O type, dv is added in place
+  w.parts = fused ? phi_pool_bwd_parts((int)BG, T) : 1;
+  w.o_da = o;     o += fused ? 0 : al256(BG * T * U * sizeof(float));
+  w.o_dalp = o;   o += dtype == NSA_BF16 || fused ? al256(BG * T * U * es) : 0;
+  w.o_dcpart = o; o += al256(w.parts * BG * l * U * sizeof(float));
   w.o_dc = o;     o += al256((size_t)l * U * sizeof(float));
-  w.o_dvt = o;    o += al256(BG * T * dv * sizeof(float));
+  w.o_dvt = o;    o += fused ? 0 : al256(BG * T * dv * sizeof(float));
   w.o_w1k = o;    o += al256((size_t)U * dk * es);
   w.o_cs = o;     o += colsum_scratch_bytes((int64_t)BG * nb, dk);
   w.total = o;
@@ -379,18 +397,24 @@ extern "C" NSA_API int nsa_cmp_phi_bwd(const void* k, const float* pos_embed, co
       return rc;
   }
   if (int rc = check_launch("cmp_phi_bwd")) return rc;
-  if (int rc = nsa_phi_pool_bwd(a, c, dhbar, dvc, da, dcpart, dvt, B, G, T, U, dv, l, d, nb, nbp, stream)) return rc;
+  const bool fused = phi_pool_bwd_fused_ok(l, d);
+  int rc_pool;
+  if (!fused) rc_pool = nsa_phi_pool_bwd(a, c, dhbar, dvc, da, dcpart, dvt, B, G, T, U, dv, l, d, nb, nbp, stream);
+  else if (dtype == NSA_BF16)
+    rc_pool = phi_pool_bwd_fused(a, c, dhbar, dvc, (__nv_bfloat16*)(w + wl.o_dalp), dcpart, (__nv_bfloat16*)dv_out, BG, T, U, dv, nb, nbp, st);
+  else rc_pool = phi_pool_bwd_fused(a, c, dhbar, dvc, (float*)(w + wl.o_dalp), dcpart, (float*)dv_out, BG, T, U, dv, nb, nbp, st);
+  if (rc_pool) return rc_pool;
   {
     KernelTimer kt("phi_mlp_bwd", st);
     const int64_t na = (int64_t)BG * T * U;
-    const void* da_op = da;
+    const void* da_op = fused ? (const void*)(w + wl.o_dalp) : da;
     const void* w1k_op = w1;
     cudaDataType ot = CUDA_R_32F;
     int ldw = ld1;
     if (dtype == NSA_BF16) {
       __nv_bfloat16* dalp = (__nv_bfloat16*)(w + wl.o_dalp);
       __nv_bfloat16* w1k = (__nv_bfloat16*)(w + wl.o_w1k);
-      cast_kernel<__nv_bfloat16><<<blocks_for(na), 256, 0, st>>>(da, dalp, na);
+      if (!fused) cast_kernel<__nv_bfloat16><<<blocks_for(na), 256, 0, st>>>(da, dalp, na);
       w1k_cast_kernel<__nv_bfloat16><<<blocks_for((int64_t)U * dk), 256, 0, st>>>(w1, U, dk, ld1, w1k);
       da_op = dalp; w1k_op = w1k; ot = CUDA_R_16BF; ldw = dk;
     }
@@ -408,11 +432,13 @@ extern "C" NSA_API int nsa_cmp_phi_bwd(const void* k, const float* pos_embed, co
                         "cmp_phi_bwd (dW1k)"))
         return rc;
     }
-    dc_sum_kernel<<<blocks_for((int64_t)l * U), 256, 0, st>>>(dcpart, BG, l * U, dc);
-    const int64_t nt = std::max<int64_t>((int64_t)U * l, (int64_t)l * l);
+    dc_sum_kernel<<<blocks_for((int64_t)l * U), 256, 0, st>>>(dcpart, (int)wl.parts * BG, l * U, dc);
+    const int64_t nt = std::max<int64_t>((int64_t)U * l, (int64_t)l * l * 32);
     table_grads_kernel<<<blocks_for(nt), 256, 0, st>>>(dc, pos_embed, w1, l, U, dk, db1, dw1, dpos);
     const int64_t nvt = (int64_t)BG * T * dv;
-    if (dtype == NSA_BF16) add_into_kernel<__nv_bfloat16><<<blocks_for(nvt), 256, 0, st>>>((__nv_bfloat16*)dv_out, dvt, nvt);
+    if (fused) {
+      // dv was added by the pooling kernel
+    } else if (dtype == NSA_BF16) add_into_kernel<__nv_bfloat16><<<blocks_for(nvt), 256, 0, st>>>((__nv_bfloat16*)dv_out, dvt, nvt);
     else add_into_kernel<float><<<blocks_for(nvt), 256, 0, st>>>((float*)dv_out, dvt, nvt);
   }
   return check_launch("cmp_phi_bwd");
@@ -426,23 +452,53 @@ extern "C" NSA_API int nsa_cmp_phi_bwd(const void* k, const float* pos_embed, co
 // ================================================================================================================
 namespace nsa {
 namespace {
-template <typename T>
+// V consecutive elements per thread (16 bytes when the row width and the pointers allow it: one element per thread moved
+// 1 TB/s of the 6.5 there are), W a multiple of V
+template <typename T, int V> struct alignas(sizeof(T) * V) Pack { T v[V]; };
+template <typename T, int V>
 __global__ void bias_relu_kernel(T* __restrict__ h, const T* __restrict__ b, int W, int64_t n) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * V;
   if (i >= n) return;
-  const float x = Elem<T>::ld(h + i) + (b ? Elem<T>::ld(b + i % W) : 0.f);
-  Elem<T>::st(h + i, x > 0.f ? x : 0.f);
+  Pack<T, V> x = *reinterpret_cast<const Pack<T, V>*>(h + i);
+  const int c = (int)(i % W);
+#pragma unroll
+  for (int e = 0; e < V; ++e) {
+    const float y = Elem<T>::ld(&x.v[e]) + (b ? Elem<T>::ld(b + c + e) : 0.f);
+    Elem<T>::st(&x.v[e], y > 0.f ? y : 0.f);
+  }
+  *reinterpret_cast<Pack<T, V>*>(h + i) = x;
 }
-template <typename T>
+template <typename T, int V>
 __global__ void bias_add_f32_kernel(float* __restrict__ y, const T* __restrict__ b, int W, int64_t n) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) y[i] += Elem<T>::ld(b + i % W);
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * V;
+  if (i >= n) return;
+  Pack<float, V> x = *reinterpret_cast<const Pack<float, V>*>(y + i);
+  const int c = (int)(i % W);
+#pragma unroll
+  for (int e = 0; e < V; ++e) x.v[e] += Elem<T>::ld(b + c + e);
+  *reinterpret_cast<Pack<float, V>*>(y + i) = x;
 }
-template <typename T>
+template <typename T, int V>
 __global__ void relu_mask_kernel(T* __restrict__ dh, const T* __restrict__ h, int64_t n) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && !(Elem<T>::ld(h + i) > 0.f)) Elem<T>::st(dh + i, 0.f);
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * V;
+  if (i >= n) return;
+  const Pack<T, V> x = *reinterpret_cast<const Pack<T, V>*>(h + i);
+  Pack<T, V> d = *reinterpret_cast<const Pack<T, V>*>(dh + i);
+#pragma unroll
+  for (int e = 0; e < V; ++e)
+    if (!(Elem<T>::ld(&x.v[e]) > 0.f)) Elem<T>::st(&d.v[e], 0.f);
+  *reinterpret_cast<Pack<T, V>*>(dh + i) = d;
 }
+bool wide(int W, std::initializer_list<const void*> ps) {      // 16-byte accesses: 8 elements of 16 bits, 4 of 32
+  uintptr_t all = 0;
+  for (const void* p : ps) all |= reinterpret_cast<uintptr_t>(p);
+  return W % 8 == 0 && (all & 15) == 0;
+}
+#define NSA_WIDE(KERNEL, TYPE, VEC, WIDE, N, ...)                                            \
+  do {                                                                                       \
+    if (WIDE) KERNEL<TYPE, VEC><<<blocks_for((N) / VEC), 256, 0, st>>>(__VA_ARGS__, N);      \
+    else KERNEL<TYPE, 1><<<blocks_for(N), 256, 0, st>>>(__VA_ARGS__, N);                     \
+  } while (0)
 }  // namespace
 }  // namespace nsa
 
@@ -450,7 +506,7 @@ extern "C" NSA_API size_t nsa_gate_mlp_workspace_bytes(int64_t N, int Dm, int D2
   if (N <= 0 || Dm <= 0 || D2 <= 0 || O <= 0) return 256;
   const size_t es = dtype == NSA_BF16 ? 2 : 4;
   if (!backward) return 256;
-  return al256((size_t)N * O * es) + al256((size_t)N * D2 * es) + colsum_scratch_bytes(N, std::max(O, D2)) + 256;
+  return al256((size_t)N * O * es) + al256((size_t)N * D2 * es) + std::max(colsum_scratch_bytes(N, O), colsum_scratch_bytes(N, D2)) + 256;
 }
 
 extern "C" NSA_API int nsa_gate_mlp_fwd(const void* x, const void* w1, const void* b1, const void* w2, const void* b2, void* hidden,
@@ -467,12 +523,13 @@ extern "C" NSA_API int nsa_gate_mlp_fwd(const void* x, const void* w1, const voi
   // hidden (N x D2, row-major) = x W1^T; column-major: C(D2 x N) = op_T(W1 (Dm x D2)) x (Dm x N)
   if (int rc = gemm(h, CUBLAS_OP_T, CUBLAS_OP_N, D2, (int)N, Dm, w1, t, Dm, 0, x, t, Dm, 0, 0.f, hidden, t, D2, 0, 1, "gate_mlp_fwd (x W1^T)")) return rc;
   const int64_t nh = N * D2, nl = N * O;
-  if (dtype == NSA_BF16) bias_relu_kernel<__nv_bfloat16><<<blocks_for(nh), 256, 0, st>>>((__nv_bfloat16*)hidden, (const __nv_bfloat16*)b1, D2, nh);
-  else bias_relu_kernel<float><<<blocks_for(nh), 256, 0, st>>>((float*)hidden, (const float*)b1, D2, nh);
+  const bool wh = wide(D2, {hidden}), wl = wide(O, {logits});
+  if (dtype == NSA_BF16) NSA_WIDE(bias_relu_kernel, __nv_bfloat16, 8, wh, nh, (__nv_bfloat16*)hidden, (const __nv_bfloat16*)b1, D2);
+  else NSA_WIDE(bias_relu_kernel, float, 4, wh, nh, (float*)hidden, (const float*)b1, D2);
   if (int rc = gemm(h, CUBLAS_OP_T, CUBLAS_OP_N, O, (int)N, D2, w2, t, D2, 0, hidden, t, D2, 0, 0.f, logits, CUDA_R_32F, O, 0, 1, "gate_mlp_fwd (h W2^T)")) return rc;
   if (b2) {
-    if (dtype == NSA_BF16) bias_add_f32_kernel<__nv_bfloat16><<<blocks_for(nl), 256, 0, st>>>(logits, (const __nv_bfloat16*)b2, O, nl);
-    else bias_add_f32_kernel<float><<<blocks_for(nl), 256, 0, st>>>(logits, (const float*)b2, O, nl);
+    if (dtype == NSA_BF16) NSA_WIDE(bias_add_f32_kernel, __nv_bfloat16, 4, wl, nl, logits, (const __nv_bfloat16*)b2, O);
+    else NSA_WIDE(bias_add_f32_kernel, float, 4, wl, nl, logits, (const float*)b2, O);
   }
   return check_launch("gate_mlp_fwd");
 }
@@ -507,10 +564,10 @@ extern "C" NSA_API int nsa_gate_mlp_bwd(const void* x, const void* w1, const voi
   // dh (N x D2) = dl W2; column-major: C(D2 x N) = W2 (D2 x O) dl (O x N)
   if (int rc = gemm(h, CUBLAS_OP_N, CUBLAS_OP_N, D2, (int)N, O, w2, t, D2, 0, dl_op, t, O, 0, 0.f, dh, t, D2, 0, 1, "gate_mlp_bwd (dh)")) return rc;
   if (dtype == NSA_BF16) {
-    relu_mask_kernel<__nv_bfloat16><<<blocks_for(nh), 256, 0, st>>>((__nv_bfloat16*)dh, (const __nv_bfloat16*)hidden, nh);
+    NSA_WIDE(relu_mask_kernel, __nv_bfloat16, 8, wide(D2, {dh, hidden}), nh, (__nv_bfloat16*)dh, (const __nv_bfloat16*)hidden);
     colsum<__nv_bfloat16>((const __nv_bfloat16*)dh, N, D2, db1, cs, st);
   } else {
-    relu_mask_kernel<float><<<blocks_for(nh), 256, 0, st>>>((float*)dh, (const float*)hidden, nh);
+    NSA_WIDE(relu_mask_kernel, float, 4, wide(D2, {dh, hidden}), nh, (float*)dh, (const float*)hidden);
     colsum<float>((const float*)dh, N, D2, db1, cs, st);
   }
   // dW1 (D2 x Dm, row-major) = dh^T x; column-major: C(Dm x D2) = x (Dm x N) op_T(dh (D2 x N))
