@@ -12,6 +12,7 @@
 //          TMEM: dK 192 + dV 128 + S^T 64 + dP^T 64 columns.  Heads may be split over several CTAs
 //          (compressed branch, few key tiles): partial sums go to scratch and are added in head order.
 #include <algorithm>
+#include <cooperative_groups.h>
 #include <cuda.h>
 
 #include <mutex>
@@ -24,6 +25,7 @@
 namespace nsa {
 
 using namespace ptx;
+namespace cg = cooperative_groups;
 
 static int bwd_sm_count() {
   static int cached[64] = {0};
@@ -46,7 +48,8 @@ struct FaBwdParams {
   float *dk_part, *dv_part;  // [hsplit, B, G, Tk, dk|dv] when hsplit > 1
   int B, H, G, Tq, Tk;
   int window, cmp_l, cmp_d, cmp_nb;
-  int hsplit;
+  int hsplit;                // chunks of heads that share a key tile's dK/dV: partial sums in scratch (compressed branch), or
+                             // the CTAs of a cluster that add theirs through distributed shared memory (window)
   float scale, scale_log2;
   int* timeouts;
   // dS^T tiles handed from the dK/dV kernel to the dQ kernel (null: the dQ kernel recomputes S and dP itself):
@@ -86,25 +89,42 @@ static int ds_slots_per_key_tile(int mode, int Tq, int window) { return mode == 
 
 
 // ------------------------------------------------------------------------------------------------
-// prep: one warp per (b,h,t)
+// prep: row sums dO.O and log-sum-exp of every (b,h,t)
 // ------------------------------------------------------------------------------------------------
-__global__ void fa_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
-                                   const float* __restrict__ L, const float* __restrict__ M, float* __restrict__ D,
-                                   float* __restrict__ lse2, int64_t rows, int dv) {
-  const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= rows) return;
-  float acc = 0.f;
-  for (int c = lane * 2; c < dv; c += 64) {
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(o + row * dv + c));
-    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(dout + row * dv + c));
-    acc = fmaf(a.x, b.x, fmaf(a.y, b.y, acc));
+// dv / 8 lanes per row (16-byte loads), kPrepRows rows each: one 4-byte load per lane and row moved 2.6 TB/s of the 6.5 there are
+// (B=4, H=64, T=8192, dv=128: 406 -> 172 us)
+constexpr int kPrepRows = 4;
+template <int DV>
+__global__ void __launch_bounds__(256) fa_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
+                                                          const float* __restrict__ L, const float* __restrict__ M, float* __restrict__ D,
+                                                          float* __restrict__ lse2, int64_t rows) {
+  constexpr int LPR = DV / 8, RPW = 32 / LPR;
+  const int lane = threadIdx.x & 31, sub = lane / LPR, c = lane % LPR * 8;
+  const int64_t row0 = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * (RPW * kPrepRows) + sub;
+  uint4 a[kPrepRows], b[kPrepRows];
+#pragma unroll
+  for (int i = 0; i < kPrepRows; ++i) {
+    const int64_t row = row0 + i * RPW < rows ? row0 + i * RPW : rows - 1;
+    a[i] = *reinterpret_cast<const uint4*>(o + row * DV + c);
+    b[i] = *reinterpret_cast<const uint4*>(dout + row * DV + c);
   }
-  acc = warp_sum(acc);
-  if (lane == 0) {
-    D[row] = acc;
-    const float lse = M[row] + L[row];
-    lse2[row] = isfinite(lse) ? lse * kLog2e : CUDART_INF_F;  // +inf: exp2(x - inf) = 0 for rows that saw nothing
+#pragma unroll
+  for (int i = 0; i < kPrepRows; ++i) {
+    const __nv_bfloat162 *x = reinterpret_cast<const __nv_bfloat162*>(&a[i]), *y = reinterpret_cast<const __nv_bfloat162*>(&b[i]);
+    float acc = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 f = __bfloat1622float2(x[e]), g = __bfloat1622float2(y[e]);
+      acc = fmaf(f.x, g.x, fmaf(f.y, g.y, acc));
+    }
+#pragma unroll
+    for (int k = LPR / 2; k > 0; k >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, k);
+    const int64_t row = row0 + i * RPW;
+    if (c == 0 && row < rows) {
+      D[row] = acc;
+      const float lse = M[row] + L[row];
+      lse2[row] = isfinite(lse) ? lse * kLog2e : CUDART_INF_F;  // +inf: exp2(x - inf) = 0 for rows that saw nothing
+    }
   }
 }
 
@@ -123,9 +143,12 @@ void launch_bwd_prep(const void* o, const void* dout, const float* L, const floa
   KernelTimer kt("bwd_prep", st);
   if (delta)
     fa_bwd_prep_given_delta_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, st>>>(delta, L, M, D, lse2, rows);
-  else
-    fa_bwd_prep_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, L, M, D, lse2,
-                                                                 rows, dv);
+  else if (dv == 128)
+    fa_bwd_prep_kernel<128><<<(unsigned)((rows + 16 * kPrepRows - 1) / (16 * kPrepRows)), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
+                                                                                                  L, M, D, lse2, rows);
+  else      // (the tensor-core kernels cover dv = 128 and 64)
+    fa_bwd_prep_kernel<64><<<(unsigned)((rows + 32 * kPrepRows - 1) / (32 * kPrepRows)), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout,
+                                                                                                 L, M, D, lse2, rows);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -646,6 +669,9 @@ struct DkvSmem {
   static constexpr int kDsTile = 128 * 64 * 2;  // one dS^T tile on its way to global memory (128-byte-swizzled rows)
   static constexpr int oK = 0, oV = oK + kK, oStage = oV + kV, oDs = oStage + kStages * kStage, oBar = oDs + kDsTile;
   static constexpr int kDynamic = oBar + 256 + 1024;
+  // a CTA's sums for its cluster, over the tiles: rows of float padded by 4, so that neighbouring keys lie 4 banks apart
+  static constexpr int kLdK = DK + 4, kLdV = DV + 4;
+  static_assert(128 * (kLdK + kLdV) * 4 <= oDs, "the sums of a CTA lie over its tiles");
 };
 struct DkvBarriers {
   uint64_t kv_full, full[3], empty[3], stp_full, st_free, pds_full, pds_free, acc_done, dst_ready, dst_free;
@@ -942,6 +968,14 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 #pragma unroll
             for (int e = 0; e < 32; ++e) ov[e] = 0;
           }
+          if (MODE == kWin && p.hsplit > 1) {
+            float* dst = reinterpret_cast<float*>(smem) + (width == DK && out_bf == p.dk ? r * SM::kLdK : 128 * SM::kLdK + r * SM::kLdV) + c * 32;
+#pragma unroll
+            for (int e = 0; e < 32; e += 4)
+              *reinterpret_cast<float4*>(dst + e) = make_float4(__uint_as_float(ov[e]) * mul, __uint_as_float(ov[e + 1]) * mul,
+                                                                __uint_as_float(ov[e + 2]) * mul, __uint_as_float(ov[e + 3]) * mul);
+            continue;
+          }
           if (key >= p.Tk) continue;
           if (out_part) {
             float* dst = out_part + ((int64_t)hc * p.B * p.G * p.Tk + krow) * width + c * 32;
@@ -966,6 +1000,34 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     }
   }
   tc_fence_before();
+  if (MODE == kWin && p.hsplit > 1) {
+    // CTA c of the cluster finishes every hsplit-th share of the 128 keys: the chunks' sums in chunk order, added to the outputs
+    cg::cluster_group cluster = cg::this_cluster();
+    __syncwarp();
+    cluster.sync();
+    if (warp < 8 && n_it > 0) {
+      const int per = 128 / p.hsplit, w4 = (DK + DV) / 4;
+      float* sums = reinterpret_cast<float*>(smem);
+      for (int i = threadIdx.x; i < per * w4; i += 256) {
+        const int row = hc * per + i / w4, c = i % w4 * 4;
+        if (n0 + row >= p.Tk) break;
+        const bool isk = c < DK;
+        float* at = sums + (isk ? row * SM::kLdK + c : 128 * SM::kLdK + row * SM::kLdV + c - DK);
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < p.hsplit; ++k) {
+          const float4 x = *reinterpret_cast<const float4*>(cluster.map_shared_rank(at, k));
+          t.x += x.x; t.y += x.y; t.z += x.z; t.w += x.w;
+        }
+        const int64_t krow = ((int64_t)b * p.G + g) * p.Tk + n0 + row;
+        __nv_bfloat162* dst = reinterpret_cast<__nv_bfloat162*>(isk ? p.dk + krow * DK + c : p.dv + krow * DV + c - DK);
+        const float2 u = __bfloat1622float2(dst[0]), v = __bfloat1622float2(dst[1]);
+        dst[0] = __floats2bfloat162_rn(u.x + t.x, u.y + t.y);
+        dst[1] = __floats2bfloat162_rn(v.x + t.z, v.y + t.w);
+      }
+    }
+    __syncwarp();
+    cluster.sync();      // nobody leaves while its sums are being read
+  }
   __syncthreads();
   if (threadIdx.x == 0 && bar->abort) ptx::report_timeout(p.timeouts);
   if (warp == 9) {
@@ -993,17 +1055,30 @@ __global__ void dkv_reduce_kernel(const float* __restrict__ part, __nv_bfloat16*
 // ------------------------------------------------------------------------------------------------
 static size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 
-static int pick_hsplit(int B, int G, int H, int Tk, int mode) {
-  if (mode == kWin) return 1;
+// Chunks of heads that share a key tile's dK/dV (a CTA holds its SM alone).  The compressed branch, whose key tiles differ in
+// length, splits until there are four waves; its partial sums go through scratch.  The window, whose tiles are alike, takes the
+// split with the smallest estimate: 1.5 us per 64-query sub-tile and head, 8 us for a cluster's merge, and the SMs that
+// clusters of that size can fill (a cluster stays inside one of the chip's GPCs).  Unsplit, 32 CTAs took 202 us at T = 1024 (G = 4).
+static int pick_hsplit(int B, int G, int H, int Tk, int mode, int window) {
   const int hpg = H / G;
-  const long ctas = (long)B * G * ((Tk + 127) / 128);
+  const int64_t ctas = (int64_t)B * G * ((Tk + 127) / 128);
   int hs = 1;
+  if (mode == kWin) {
+    const int room[4] = {148, 144, 136, 128};      // CTAs at a time in clusters of 1, 2, 4, 8
+    double best_ns = 0.;
+    for (int i = 0; i < 4 && hpg % (1 << i) == 0; ++i) {
+      const double tile_ns = 1500. * (hpg >> i) * ((std::min(window, Tk) + 127) / 64 + 1);
+      const double ns = (double)(((ctas << i) + room[i] - 1) / room[i]) * (tile_ns + (i ? 8000. : 0.));
+      if (i == 0 || ns < 0.95 * best_ns) { hs = 1 << i; best_ns = ns; }
+    }
+    return hs;
+  }
   while (hs < hpg && ctas * hs < 4 * 148 && hpg % (hs * 2) == 0) hs *= 2;
   return hs;
 }
 
 static size_t bwd_base_bytes(int B, int H, int G, int Tq, int Tk, int dk, int dv, int mode) {
-  const int hs = pick_hsplit(B, G, H, Tk, mode);
+  const int hs = mode == kWin ? 1 : pick_hsplit(B, G, H, Tk, mode, 0);      // (the window's chunks need no scratch)
   size_t n = 2 * al256((size_t)B * H * Tq * sizeof(float));
   if (hs > 1) n += al256((size_t)hs * B * G * Tk * dk * sizeof(float)) + al256((size_t)hs * B * G * Tk * dv * sizeof(float));
   return n;
@@ -1035,12 +1110,22 @@ static int launch_bwd_t(const CUtensorMap& tq128, const CUtensorMap& tdo128, con
       cudaFuncSetAttribute(kkv, cudaFuncAttributeMaxDynamicSharedMemorySize, DkvSmem<DK, DV>::kDynamic) != cudaSuccess)
     return fail(NSA_ERR_LAUNCH, "fa_bwd: cannot reserve shared memory");
   const dim3 qgrid((unsigned)std::min(((p.Tq + 127) / 128) * p.B * p.H, bwd_sm_count()));
-  const dim3 kvgrid((p.Tk + 127) / 128, p.hsplit, p.B * p.G);
+  cudaLaunchConfig_t kv_cfg = {};
+  kv_cfg.gridDim = dim3((p.Tk + 127) / 128, p.hsplit, p.B * p.G);
+  kv_cfg.blockDim = dim3(384);
+  kv_cfg.dynamicSmemBytes = DkvSmem<DK, DV>::kDynamic;
+  kv_cfg.stream = st;
+  cudaLaunchAttribute kv_attr[1];
+  kv_attr[0].id = cudaLaunchAttributeClusterDimension;
+  kv_attr[0].val.clusterDim.x = kv_attr[0].val.clusterDim.z = 1;
+  kv_attr[0].val.clusterDim.y = MODE == kWin ? p.hsplit : 1;
+  kv_cfg.attrs = kv_attr;
+  kv_cfg.numAttrs = 1;
   if (p.ds) {
     // key-stationary kernel first: it leaves dS^T behind, from which the dQ kernel only has one product left to do
     {
       KernelTimer kt(MODE == kWin ? "fa_bwd_dkv_win" : "fa_bwd_dkv_cmp", st);
-      kkv<<<kvgrid, 384, DkvSmem<DK, DV>::kDynamic, st>>>(tq64, tdo64, tk, tv, tds, p);
+      if (cudaLaunchKernelEx(&kv_cfg, kkv, tq64, tdo64, tk, tv, tds, p) != cudaSuccess) return check_launch("fa_bwd_dkv_sm100");
     }
     if (int rc = check_launch("fa_bwd_dkv_sm100")) return rc;
     KernelTimer kt(MODE == kWin ? "fa_bwd_dqds_win" : "fa_bwd_dqds_cmp", st);
@@ -1053,7 +1138,7 @@ static int launch_bwd_t(const CUtensorMap& tq128, const CUtensorMap& tdo128, con
   }
   if (int rc = check_launch("fa_bwd_dq_sm100")) return rc;
   KernelTimer kt(MODE == kWin ? "fa_bwd_dkv_win" : "fa_bwd_dkv_cmp", st);
-  kkv<<<kvgrid, 384, DkvSmem<DK, DV>::kDynamic, st>>>(tq64, tdo64, tk, tv, tds, p);
+  if (cudaLaunchKernelEx(&kv_cfg, kkv, tq64, tdo64, tk, tv, tds, p) != cudaSuccess) return check_launch("fa_bwd_dkv_sm100");
   return check_launch("fa_bwd_dkv_sm100");
 }
 
@@ -1077,9 +1162,9 @@ int fa_bwd_sm100(const void* q, const void* k, const void* v, const void* o, con
   float* D = (float*)w;
   float* lse2 = (float*)(w + al256(rows * sizeof(float)));
   p.D = D; p.lse2 = lse2;
-  p.hsplit = pick_hsplit(B, G, H, Tk, mode);
+  p.hsplit = pick_hsplit(B, G, H, Tk, mode, window);
   p.dk_part = p.dv_part = nullptr;
-  if (p.hsplit > 1) {
+  if (p.hsplit > 1 && mode == kCmp) {
     p.dk_part = (float*)(w + 2 * al256(rows * sizeof(float)));
     p.dv_part = (float*)((char*)p.dk_part + al256((size_t)p.hsplit * B * G * Tk * dk * sizeof(float)));
   }
@@ -1112,7 +1197,7 @@ int fa_bwd_sm100(const void* q, const void* k, const void* v, const void* o, con
   NSA_BWD_CASE(64, 64)
 #undef NSA_BWD_CASE
   if (rc) return rc == NSA_ERR_UNSUPPORTED ? fail(rc, "fa_bwd_sm100: unsupported head dims") : rc;
-  if (p.hsplit > 1) {
+  if (p.hsplit > 1 && mode == kCmp) {
     const int64_t nk = (int64_t)B * G * Tk * dk, nv = (int64_t)B * G * Tk * dv;
     KernelTimer kt("fa_dkv_reduce", st);
     dkv_reduce_kernel<<<(unsigned)((nk / 2 + 255) / 256), 256, 0, st>>>(p.dk_part, p.dk, nk, p.hsplit);

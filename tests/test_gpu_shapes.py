@@ -314,3 +314,22 @@ def test_mma_kernels_keep_32_bit_probabilities(dk, dv, H, G, T, w, n):
     torch.cuda.synchronize()
     for a, b in ((o[:, :, :T - 5], o2[:, :, :T - 5]), (dq[:, :, :T - 5], dq2[:, :, :T - 5]), (dkey[:, :, 8:], dkey2[:, :, 8:]), (dval[:, :, 8:], dval2[:, :, 8:])):
         assert torch.isfinite(b).all() and max_abs(a.float(), b.float()) <= 2 ** -7 * max(1.0, a.float().abs().max().item())
+
+
+@pytest.mark.parametrize("dk,dv,H,G,T,w", [(64, 64, 8, 2, 128, 150), (192, 128, 16, 1, 640, 512), (128, 128, 4, 2, 896, 30), (192, 128, 6, 1, 256, 600)])
+def test_window_backward_with_heads_split_over_a_cluster(dk, dv, H, G, T, w):
+    """Few key tiles: clusters of 2, 4 and 8 CTAs share a tile's heads (and none where the heads are odd in number).  The row sums
+    dO.O are computed here; the outputs are added into."""
+    from nsa import ops
+    q, k, v, do = _inputs(2, H, G, T, dk, dv, seed=T)
+    qd, kd, vd, dd = (t.to(DEV) for t in (q, k, v, do))
+    scale = dk ** -0.5
+    o, L, M = ops.sliding_fwd(qd, kd, vd, w, scale)
+    qf, kf, vf = (t.float().requires_grad_(True) for t in (q, k, v))
+    want = torch.autograd.grad(O.sliding_window_attention(qf, kf, vf, w, scale), (qf, kf, vf), do.float())
+    dq, dkey, dval = ops.sliding_bwd(qd, kd, vd, o, dd, L, M, w, scale)
+    torch.cuda.synchronize()
+    _no_timeouts()
+    _grad_close(dq, want[0], "dq")
+    _grad_close(dkey, want[1].transpose(-1, -2), "dk")
+    _grad_close(dval, want[2], "dv")
