@@ -118,47 +118,65 @@ __global__ void gate_mix_fwd_bf16x4_kernel(const float* __restrict__ logits, con
   }
 }
 
-__global__ void gate_mix_bwd_bf16x4_kernel(const float* __restrict__ gates, const __nv_bfloat16* __restrict__ oc,
+// Half a warp per row, kMixRows rows each whose loads go out together.
+constexpr int kMixRows = 2;
+__global__ void __launch_bounds__(256) gate_mix_bwd_bf16x4_kernel(const float* __restrict__ gates, const __nv_bfloat16* __restrict__ oc,
                                            const __nv_bfloat16* __restrict__ os, const __nv_bfloat16* __restrict__ ow,
                                            const __nv_bfloat16* __restrict__ dout, __nv_bfloat16* __restrict__ doc,
                                            __nv_bfloat16* __restrict__ dos, __nv_bfloat16* __restrict__ dow, float* __restrict__ dlogits,
                                            int B, int H, int T_, int dv, int mode, float* __restrict__ delta, int dout_tm) {
   const int lane = threadIdx.x & 31, hl = lane & 15;
-  int64_t row = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 2 + (lane >> 4);
-  const bool live = row < (int64_t)B * H * T_;  // both halves stay for the shuffles
-  if (!live) row = 0;
-  const int t = row % T_, h = (row / T_) % H, b = row / ((int64_t)T_ * H);
-  const float g0 = gates[row * 3], g1 = gates[row * 3 + 1], g2 = gates[row * 3 + 2];
-  const int64_t base = row * dv, dbase = mixed_row(row, b, h, t, H, T_, dout_tm) * dv;
-  float d0 = 0.f, d1 = 0.f, d2 = 0.f;
+  const int64_t rows = (int64_t)B * H * T_;
+  const int64_t row0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (2 * kMixRows) + (lane >> 4);
+  int t[kMixRows], h[kMixRows], b[kMixRows];
+  int64_t row[kMixRows], dbase[kMixRows];
+  float g[kMixRows][3], d[kMixRows][3];
+#pragma unroll
+  for (int k = 0; k < kMixRows; ++k) {
+    row[k] = row0 + 2 * k < rows ? row0 + 2 * k : 0;      // both halves stay for the shuffles
+    t[k] = row[k] % T_; h[k] = (row[k] / T_) % H; b[k] = row[k] / ((int64_t)T_ * H);
+    dbase[k] = mixed_row(row[k], b[k], h[k], t[k], H, T_, dout_tm) * dv;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) { g[k][i] = gates[row[k] * 3 + i]; d[k][i] = 0.f; }
+  }
   for (int c = hl * 8; c < dv; c += 128) {
-    float dy[8], a[8], s_[8], w[8], r0[8], r1[8], r2[8];
-    const uint4 qd = *reinterpret_cast<const uint4*>(dout + dbase + c), qa = *reinterpret_cast<const uint4*>(oc + base + c);
-    const uint4 qs = *reinterpret_cast<const uint4*>(os + base + c), qw = *reinterpret_cast<const uint4*>(ow + base + c);
-    unpack8(qd, dy); unpack8(qa, a); unpack8(qs, s_); unpack8(qw, w);
+    uint4 qd[kMixRows], qb[kMixRows][3];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      d0 = fmaf(dy[i], a[i], d0); d1 = fmaf(dy[i], s_[i], d1); d2 = fmaf(dy[i], w[i], d2);
-      r0[i] = dy[i] * g0; r1[i] = dy[i] * g1; r2[i] = dy[i] * g2;
+    for (int k = 0; k < kMixRows; ++k) {
+      qd[k] = *reinterpret_cast<const uint4*>(dout + dbase[k] + c);
+      qb[k][0] = *reinterpret_cast<const uint4*>(oc + row[k] * dv + c);
+      qb[k][1] = *reinterpret_cast<const uint4*>(os + row[k] * dv + c);
+      qb[k][2] = *reinterpret_cast<const uint4*>(ow + row[k] * dv + c);
     }
-    if (live) {
-      *reinterpret_cast<uint4*>(doc + base + c) = pack8(r0);
-      *reinterpret_cast<uint4*>(dos + base + c) = pack8(r1);
-      *reinterpret_cast<uint4*>(dow + base + c) = pack8(r2);
+#pragma unroll
+    for (int k = 0; k < kMixRows; ++k) {
+      float dy[8];
+      unpack8(qd[k], dy);
+#pragma unroll
+      for (int br = 0; br < 3; ++br) {
+        float x[8], r[8];
+        unpack8(qb[k][br], x);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          d[k][br] = fmaf(dy[i], x[i], d[k][br]);
+          r[i] = dy[i] * g[k][br];
+        }
+        if (row0 + 2 * k < rows) *reinterpret_cast<uint4*>((br == 0 ? doc : br == 1 ? dos : dow) + row[k] * dv + c) = pack8(r);
+      }
     }
   }
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1) {  // sums inside each half-warp
-    d0 += __shfl_xor_sync(0xffffffffu, d0, o);
-    d1 += __shfl_xor_sync(0xffffffffu, d1, o);
-    d2 += __shfl_xor_sync(0xffffffffu, d2, o);
-  }
-  if (hl == 0 && live) {
+  for (int k = 0; k < kMixRows; ++k) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)  // sums inside each half-warp
+#pragma unroll
+      for (int br = 0; br < 3; ++br) d[k][br] += __shfl_xor_sync(0xffffffffu, d[k][br], o);
+    if (hl != 0 || row0 + 2 * k >= rows) continue;
+    const float g0 = g[k][0], g1 = g[k][1], g2 = g[k][2], d0 = d[k][0], d1 = d[k][1], d2 = d[k][2];
     if (delta) {  // row sums dO_b . O_b of the three branches, dO_b = g_b dO
-      const int64_t rows = (int64_t)B * H * T_;
-      delta[row] = g0 * d0; delta[rows + row] = g1 * d1; delta[2 * rows + row] = g2 * d2;
+      delta[row[k]] = g0 * d0; delta[rows + row[k]] = g1 * d1; delta[2 * rows + row[k]] = g2 * d2;
     }
-    float* dl = dlogits + ((int64_t)b * T_ + t) * 3 * H + 3 * h;
+    float* dl = dlogits + ((int64_t)b[k] * T_ + t[k]) * 3 * H + 3 * h[k];
     if (mode == NSA_GATE_SOFTMAX) {
       const float dot = g0 * d0 + g1 * d1 + g2 * d2;
       dl[0] = g0 * (d0 - dot); dl[1] = g1 * (d1 - dot); dl[2] = g2 * (d2 - dot);
@@ -214,7 +232,7 @@ extern "C" NSA_API int nsa_gate_mix_bwd_delta(const float* gates, const void* o_
                                                       (const float*)dout, (float*)do_cmp, (float*)do_slc, (float*)do_win,
                                                       dlogits, B, H, T, dv, gate_mode, delta, dout_tm);
   else if (dtype == NSA_BF16 && dv % 128 == 0)
-    gate_mix_bwd_bf16x4_kernel<<<(unsigned)((rows + 15) / 16), 256, 0, st>>>(gates, (const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)o_slc,
+    gate_mix_bwd_bf16x4_kernel<<<(unsigned)((rows + 16 * kMixRows - 1) / (16 * kMixRows)), 256, 0, st>>>(gates, (const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)o_slc,
                                                      (const __nv_bfloat16*)o_win, (const __nv_bfloat16*)dout, (__nv_bfloat16*)do_cmp,
                                                      (__nv_bfloat16*)do_slc, (__nv_bfloat16*)do_win, dlogits, B, H, T, dv, gate_mode, delta, dout_tm);
   else if (dtype == NSA_BF16)

@@ -16,6 +16,9 @@
 // query (block 0) is spread over many CTAs.
 #include <cuda.h>
 
+#include <cstring>
+#include <type_traits>
+
 #include "attn_args.cuh"
 #include "common.cuh"
 #include "fa_sm100.cuh"
@@ -415,28 +418,35 @@ __device__ __forceinline__ unsigned valid_slot_mask(const int* irow, int64_t s3,
 
 // Gate + mix epilogue of the merge kernels: the warp holds the finished (rounded) O_slc row of (b,h,t), lane owning VPL
 // consecutive columns; the mixed row is (o_cmp g0 + o_slc g1) + o_win g2, the operation order of the stand-alone pass.
+// The inputs are loaded apart from the arithmetic, so that a kernel can start them before it waits for the partials.
 template <int VPL>
-__device__ __forceinline__ void slc_mix_row(const SlcMix& mix, const __nv_bfloat162 (&oslc)[VPL / 2], int64_t row, int b, int h, int t,
-                                            int H, int Tq, int dv, int lane) {
-  const __nv_bfloat16* oc = (const __nv_bfloat16*)mix.o_cmp + row * dv + lane * VPL;
-  const __nv_bfloat16* ow = (const __nv_bfloat16*)mix.o_win + row * dv + lane * VPL;
+struct MixRow {
   __nv_bfloat162 a[VPL / 2], w[VPL / 2];
+  float lg[3];
+  __device__ __forceinline__ void load(const SlcMix& mix, int64_t row, int b, int h, int t, int H, int Tq, int dv, int lane) {
+    using Vec = typename std::conditional<VPL == 4, uint2, uint32_t>::type;
+    const Vec va = *reinterpret_cast<const Vec*>((const __nv_bfloat16*)mix.o_cmp + row * dv + lane * VPL);
+    const Vec vw = *reinterpret_cast<const Vec*>((const __nv_bfloat16*)mix.o_win + row * dv + lane * VPL);
+    memcpy(a, &va, sizeof(a));
+    memcpy(w, &vw, sizeof(w));
+    const float* src = mix.logits + ((int64_t)b * Tq + t) * 3 * H + 3 * h;
 #pragma unroll
-  for (int c = 0; c < VPL / 2; ++c) {
-    a[c] = *reinterpret_cast<const __nv_bfloat162*>(oc + 2 * c);
-    w[c] = *reinterpret_cast<const __nv_bfloat162*>(ow + 2 * c);
+    for (int i = 0; i < 3; ++i) lg[i] = src[i];
   }
-  float g[3];
-  gates3(mix.logits + ((int64_t)b * Tq + t) * 3 * H + 3 * h, mix.mode, g);
-  if (lane < 3) mix.gates[row * 3 + lane] = g[lane];
-  __nv_bfloat16* dst = (__nv_bfloat16*)mix.out + mixed_row(row, b, h, t, H, Tq, mix.token_major) * dv + lane * VPL;
+  __device__ __forceinline__ void store(const SlcMix& mix, const __nv_bfloat162 (&oslc)[VPL / 2], int64_t row, int b, int h, int t, int H,
+                                        int Tq, int dv, int lane) const {
+    float g[3];
+    gates3(lg, mix.mode, g);
+    if (lane < 3) mix.gates[row * 3 + lane] = lane == 0 ? g[0] : lane == 1 ? g[1] : g[2];
+    __nv_bfloat16* dst = (__nv_bfloat16*)mix.out + mixed_row(row, b, h, t, H, Tq, mix.token_major) * dv + lane * VPL;
 #pragma unroll
-  for (int c = 0; c < VPL / 2; ++c) {
-    const float2 fa = __bfloat1622float2(a[c]), fs = __bfloat1622float2(oslc[c]), fw = __bfloat1622float2(w[c]);
-    *reinterpret_cast<__nv_bfloat162*>(dst + 2 * c) =
-        __floats2bfloat162_rn((fa.x * g[0] + fs.x * g[1]) + fw.x * g[2], (fa.y * g[0] + fs.y * g[1]) + fw.y * g[2]);
+    for (int c = 0; c < VPL / 2; ++c) {
+      const float2 fa = __bfloat1622float2(a[c]), fs = __bfloat1622float2(oslc[c]), fw = __bfloat1622float2(w[c]);
+      *reinterpret_cast<__nv_bfloat162*>(dst + 2 * c) =
+          __floats2bfloat162_rn((fa.x * g[0] + fs.x * g[1]) + fw.x * g[2], (fa.y * g[0] + fs.y * g[1]) + fw.y * g[2]);
+    }
   }
-}
+};
 
 // merge the partials of a query in slot order: one warp per (b,h,t).  Every load of the row (index row, statistics,
 // all slots' partial outputs) is issued before the first value is used; slots that turn out not to contribute were
@@ -508,14 +518,19 @@ __global__ void slc_combine_fwd_kernel(const __nv_bfloat16* __restrict__ o_part,
     L[row] = lsum > 0.f ? logf(lsum) : -CUDART_INF_F;
     M[row] = lsum > 0.f ? mx * kLn2f : -CUDART_INF_F;
   }
-  if (mix.out) slc_mix_row<VPL>(mix, rounded, row, b, h, t, H, Tq, DV, lane);
+  if (mix.out) {
+    MixRow<VPL> mr;
+    mr.load(mix, row, b, h, t, H, Tq, DV, lane);
+    mr.store(mix, rounded, row, b, h, t, H, Tq, DV, lane);
+  }
 }
 
 // Same merge with the whole contiguous block of a query's partials ([slots][heads][dv]) brought into shared memory by
 // one bulk copy: one thread block per (group, query), one warp per head.  No registers are spent on loads in flight,
 // so several blocks per SM keep enough bytes on their way to saturate HBM.
+// (40 registers: three blocks of 16 heads per SM; 44 let in two and took a quarter longer)
 template <int DV>
-__global__ void slc_combine_fwd_bulk_kernel(const __nv_bfloat16* __restrict__ o_part, const float2* __restrict__ st_part,
+__global__ void __maxnreg__(40) slc_combine_fwd_bulk_kernel(const __nv_bfloat16* __restrict__ o_part, const float2* __restrict__ st_part,
                                             const int* __restrict__ indices, int64_t s0, int64_t s1, int64_t s2, int64_t s3,
                                             __nv_bfloat16* __restrict__ out, float* __restrict__ L, float* __restrict__ M, int B,
                                             int H, int G, int Tq, int Tk, int nslots, int lprime, int q0, int* timeouts,
@@ -528,16 +543,14 @@ __global__ void slc_combine_fwd_bulk_kernel(const __nv_bfloat16* __restrict__ o_
   const int64_t q = blockIdx.x;  // (batch, group, query)
   const int t = q % Tq, bgi = q / Tq, b = bgi / G, g = bgi % G, h = g * hpg + hh;
   const uint32_t bytes = (uint32_t)nslots * hpg * DV * 2;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0) {      // (the thread that set the barrier up may use it at once)
     mbar_init(&bar, 1);
     abort_flag = 0;
     fence_barrier_init();
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
     mbar_arrive_expect_tx(&bar, bytes);
     bulk_load_1d(sm_part, o_part + q * (int64_t)nslots * hpg * DV, bytes, &bar);
   }
+  __syncthreads();
   const int64_t row = ((int64_t)b * H + h) * Tq + t;
   const int* irow = indices + b * s0 + g * s1 + (int64_t)t * s2;
   const int64_t base = (q * nslots) * hpg + hh;
@@ -551,6 +564,8 @@ __global__ void slc_combine_fwd_bulk_kernel(const __nv_bfloat16* __restrict__ o_
   float lsum = 0.f, acc[VPL];
 #pragma unroll
   for (int c = 0; c < VPL; ++c) acc[c] = 0.f;
+  MixRow<VPL> mr;      // the other branches' rows arrive while the partials do
+  if (mix.out) mr.load(mix, row, b, h, t, H, Tq, DV, lane);
   const bool ok = mbar_wait_warp(&bar, 0, &abort_flag);
   if (ok) {
     for (int s = 0; s < nslots; ++s) {
@@ -580,7 +595,7 @@ __global__ void slc_combine_fwd_bulk_kernel(const __nv_bfloat16* __restrict__ o_
       L[row] = lsum > 0.f ? logf(lsum) : -CUDART_INF_F;
       M[row] = lsum > 0.f ? mx * kLn2f : -CUDART_INF_F;
     }
-    if (mix.out) slc_mix_row<VPL>(mix, rounded, row, b, h, t, H, Tq, DV, lane);
+    if (mix.out) mr.store(mix, rounded, row, b, h, t, H, Tq, DV, lane);
   }
   __syncthreads();  // the copy has landed (or was given up on) before shared memory is handed back
   if (threadIdx.x == 0 && abort_flag) ptx::report_timeout(timeouts);
@@ -592,19 +607,12 @@ __global__ void slc_combine_fwd_bulk_kernel(const __nv_bfloat16* __restrict__ o_
 // dQ[b,h,t,:] = scale * sum of the contributing slots' partials, slot order: one warp per row; the loads of 8 slots
 // are in flight together and do not wait for the index row
 // dQ of the selection branch plus, when given, the dQ of the two other branches (same layout): one rounding of the sum
-__device__ __forceinline__ __nv_bfloat162 slc_dq_total(float x, float y, const __nv_bfloat16* add0, const __nv_bfloat16* add1,
-                                                       int64_t at) {
-  if (add0) {
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(add0 + at));
-    x += a.x;
-    y += a.y;
-  }
-  if (add1) {
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(add1 + at));
-    x += a.x;
-    y += a.y;
-  }
-  return __floats2bfloat162_rn(x, y);
+__device__ __forceinline__ __nv_bfloat162 slc_dq_total(float x, float y, __nv_bfloat162 add0, __nv_bfloat162 add1) {
+  const float2 a = __bfloat1622float2(add0), c = __bfloat1622float2(add1);
+  return __floats2bfloat162_rn((x + a.x) + c.x, (y + a.y) + c.y);
+}
+__device__ __forceinline__ __nv_bfloat162 ld_pair(const __nv_bfloat16* p, int64_t at) {     // a missing addend changes nothing
+  return p ? *reinterpret_cast<const __nv_bfloat162*>(p + at) : __floats2bfloat162_rn(-0.f, -0.f);
 }
 
 template <int DK>
@@ -649,7 +657,7 @@ __global__ void slc_combine_dq_kernel(const __nv_bfloat16* __restrict__ dq_part,
 #pragma unroll
   for (int c = 0; c < DK / 64; ++c) {
     const int64_t at = row * DK + c * 64 + lane * 2;
-    *reinterpret_cast<__nv_bfloat162*>(dq + at) = slc_dq_total(acc[2 * c] * scale, acc[2 * c + 1] * scale, add0, add1, at);
+    *reinterpret_cast<__nv_bfloat162*>(dq + at) = slc_dq_total(acc[2 * c] * scale, acc[2 * c + 1] * scale, ld_pair(add0, at), ld_pair(add1, at));
   }
 }
 
@@ -667,19 +675,23 @@ __global__ void slc_combine_dq_bulk_kernel(const __nv_bfloat16* __restrict__ dq_
   const int64_t q = blockIdx.x;
   const int t = q % Tq, bgi = q / Tq, b = bgi / G, g = bgi % G, h = g * hpg + hh;
   const uint32_t bytes = (uint32_t)nslots * hpg * DK * 2;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0) {      // (the thread that set the barrier up may use it at once)
     mbar_init(&bar, 1);
     abort_flag = 0;
     fence_barrier_init();
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
     mbar_arrive_expect_tx(&bar, bytes);
     bulk_load_1d(sm_part, dq_part + q * (int64_t)nslots * hpg * DK, bytes, &bar);
   }
+  __syncthreads();
   const int64_t row = ((int64_t)b * H + h) * Tq + t;
   const int* irow = indices + b * s0 + g * s1 + (int64_t)t * s2;
   const unsigned validmask = valid_slot_mask(irow, s3, nslots, q0 + t, Tk, lprime, lane);
+  __nv_bfloat162 ad0[DK / 64], ad1[DK / 64];      // the other branches' dQ arrives while the partials do
+#pragma unroll
+  for (int c = 0; c < DK / 64; ++c) {
+    ad0[c] = ld_pair(add0, row * DK + c * 64 + lane * 2);
+    ad1[c] = ld_pair(add1, row * DK + c * 64 + lane * 2);
+  }
   float acc[DK / 32];
 #pragma unroll
   for (int c = 0; c < DK / 32; ++c) acc[c] = 0.f;
@@ -698,7 +710,7 @@ __global__ void slc_combine_dq_bulk_kernel(const __nv_bfloat16* __restrict__ dq_
 #pragma unroll
     for (int c = 0; c < DK / 64; ++c) {
       const int64_t at = row * DK + c * 64 + lane * 2;
-      *reinterpret_cast<__nv_bfloat162*>(dq + at) = slc_dq_total(acc[2 * c] * scale, acc[2 * c + 1] * scale, add0, add1, at);
+      *reinterpret_cast<__nv_bfloat162*>(dq + at) = slc_dq_total(acc[2 * c] * scale, acc[2 * c + 1] * scale, ad0[c], ad1[c]);
     }
   }
   __syncthreads();

@@ -333,3 +333,22 @@ def test_window_backward_with_heads_split_over_a_cluster(dk, dv, H, G, T, w):
     _grad_close(dq, want[0], "dq")
     _grad_close(dkey, want[1].transpose(-1, -2), "dk")
     _grad_close(dval, want[2], "dv")
+
+
+@pytest.mark.parametrize("rows,dv", [((1, 2, 33), 128), ((2, 3, 21), 64), ((1, 1, 1), 128)])
+def test_row_kernels_at_any_row_count(rows, dv):
+    """Rows that do not fill a warp's share: gate/mix backward with its row sums, against the formulas."""
+    from nsa import ops
+    B, H, T = rows
+    gen = torch.Generator().manual_seed(T)
+    oc, os_, ow, do = (torch.randn(B, H, T, dv, generator=gen).bfloat16() for _ in range(4))
+    lg = torch.randn(B, T, 3 * H, generator=gen)
+    out, gates = ops.gate_mix_fwd(lg.to(DEV), oc.to(DEV), os_.to(DEV), ow.to(DEV), "sigmoid")
+    dc, ds, dw, dlog, delta = ops.gate_mix_bwd(gates, oc.to(DEV), os_.to(DEV), ow.to(DEV), do.to(DEV), "sigmoid", want_delta=True)
+    torch.cuda.synchronize()
+    g = torch.sigmoid(lg.view(B, T, H, 3).permute(0, 2, 1, 3))
+    for i, (o, d) in enumerate(((oc, dc), (os_, ds), (ow, dw))):
+        dot = (do.float() * o.float()).sum(-1)
+        assert max_abs(d.float(), (g[..., i:i + 1] * do.float()).bfloat16().float()) <= 2 ** -8 * 4      # one rounding apart
+        assert max_abs(delta[i], g[..., i] * dot) < 1e-4 * max(1.0, dot.abs().max().item())            # fp32 sums of dv terms
+        assert max_abs(dlog.view(B, T, H, 3)[..., i], (dot * g[..., i] * (1 - g[..., i])).transpose(1, 2)) < 1e-4 * max(1.0, dot.abs().max().item())
