@@ -118,7 +118,9 @@ __global__ void gate_mix_fwd_bf16x4_kernel(const float* __restrict__ logits, con
   }
 }
 
-// Half a warp per row, kMixRows rows each whose loads go out together.
+// A block owns 16 heads x kMixRows consecutive tokens, half a warp a head: its loads go out together, and the 12 bytes a row has of
+// dlogits [B,T,3H] make whole sectors.  Memory bound: 64 heads x 65536 x 128 went from 1.64 ms, walking the tokens of one head, to
+// 1.36 ms (5.5 TB/s); two tokens in flight without this order gained nothing (1.72 ms).
 constexpr int kMixRows = 2;
 __global__ void __launch_bounds__(256) gate_mix_bwd_bf16x4_kernel(const float* __restrict__ gates, const __nv_bfloat16* __restrict__ oc,
                                            const __nv_bfloat16* __restrict__ os, const __nv_bfloat16* __restrict__ ow,
@@ -127,15 +129,17 @@ __global__ void __launch_bounds__(256) gate_mix_bwd_bf16x4_kernel(const float* _
                                            int B, int H, int T_, int dv, int mode, float* __restrict__ delta, int dout_tm) {
   const int lane = threadIdx.x & 31, hl = lane & 15;
   const int64_t rows = (int64_t)B * H * T_;
-  const int64_t row0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (2 * kMixRows) + (lane >> 4);
-  int t[kMixRows], h[kMixRows], b[kMixRows];
+  const int nhb = (H + 15) / 16, ntb = (T_ + kMixRows - 1) / kMixRows, g16 = blockIdx.x / ntb, b = g16 / nhb;
+  const int h = (g16 - b * nhb) * 16 + (threadIdx.x >> 4), t0 = (blockIdx.x - g16 * ntb) * kMixRows;
   int64_t row[kMixRows], dbase[kMixRows];
+  bool live[kMixRows];
   float g[kMixRows][3], d[kMixRows][3];
 #pragma unroll
   for (int k = 0; k < kMixRows; ++k) {
-    row[k] = row0 + 2 * k < rows ? row0 + 2 * k : 0;      // both halves stay for the shuffles
-    t[k] = row[k] % T_; h[k] = (row[k] / T_) % H; b[k] = row[k] / ((int64_t)T_ * H);
-    dbase[k] = mixed_row(row[k], b[k], h[k], t[k], H, T_, dout_tm) * dv;
+    live[k] = h < H && t0 + k < T_;      // (both halves stay for the shuffles)
+    const int hh = live[k] ? h : 0, t = live[k] ? t0 + k : 0;
+    row[k] = ((int64_t)b * H + hh) * T_ + t;
+    dbase[k] = mixed_row(row[k], b, hh, t, H, T_, dout_tm) * dv;
 #pragma unroll
     for (int i = 0; i < 3; ++i) { g[k][i] = gates[row[k] * 3 + i]; d[k][i] = 0.f; }
   }
@@ -161,7 +165,7 @@ __global__ void __launch_bounds__(256) gate_mix_bwd_bf16x4_kernel(const float* _
           d[k][br] = fmaf(dy[i], x[i], d[k][br]);
           r[i] = dy[i] * g[k][br];
         }
-        if (row0 + 2 * k < rows) *reinterpret_cast<uint4*>((br == 0 ? doc : br == 1 ? dos : dow) + row[k] * dv + c) = pack8(r);
+        if (live[k]) *reinterpret_cast<uint4*>((br == 0 ? doc : br == 1 ? dos : dow) + row[k] * dv + c) = pack8(r);
       }
     }
   }
@@ -171,12 +175,12 @@ __global__ void __launch_bounds__(256) gate_mix_bwd_bf16x4_kernel(const float* _
     for (int o = 8; o > 0; o >>= 1)  // sums inside each half-warp
 #pragma unroll
       for (int br = 0; br < 3; ++br) d[k][br] += __shfl_xor_sync(0xffffffffu, d[k][br], o);
-    if (hl != 0 || row0 + 2 * k >= rows) continue;
+    if (hl != 0 || !live[k]) continue;
     const float g0 = g[k][0], g1 = g[k][1], g2 = g[k][2], d0 = d[k][0], d1 = d[k][1], d2 = d[k][2];
     if (delta) {  // row sums dO_b . O_b of the three branches, dO_b = g_b dO
       delta[row[k]] = g0 * d0; delta[rows + row[k]] = g1 * d1; delta[2 * rows + row[k]] = g2 * d2;
     }
-    float* dl = dlogits + ((int64_t)b[k] * T_ + t[k]) * 3 * H + 3 * h[k];
+    float* dl = dlogits + ((int64_t)b * T_ + t0 + k) * 3 * H + 3 * h;
     if (mode == NSA_GATE_SOFTMAX) {
       const float dot = g0 * d0 + g1 * d1 + g2 * d2;
       dl[0] = g0 * (d0 - dot); dl[1] = g1 * (d1 - dot); dl[2] = g2 * (d2 - dot);
@@ -232,7 +236,7 @@ extern "C" NSA_API int nsa_gate_mix_bwd_delta(const float* gates, const void* o_
                                                       (const float*)dout, (float*)do_cmp, (float*)do_slc, (float*)do_win,
                                                       dlogits, B, H, T, dv, gate_mode, delta, dout_tm);
   else if (dtype == NSA_BF16 && dv % 128 == 0)
-    gate_mix_bwd_bf16x4_kernel<<<(unsigned)((rows + 16 * kMixRows - 1) / (16 * kMixRows)), 256, 0, st>>>(gates, (const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)o_slc,
+    gate_mix_bwd_bf16x4_kernel<<<(unsigned)((int64_t)B * ((H + 15) / 16) * ((T + kMixRows - 1) / kMixRows)), 256, 0, st>>>(gates, (const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)o_slc,
                                                      (const __nv_bfloat16*)o_win, (const __nv_bfloat16*)dout, (__nv_bfloat16*)do_cmp,
                                                      (__nv_bfloat16*)do_slc, (__nv_bfloat16*)do_win, dlogits, B, H, T, dv, gate_mode, delta, dout_tm);
   else if (dtype == NSA_BF16)

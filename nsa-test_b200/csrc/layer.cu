@@ -25,8 +25,8 @@ int next_pow2(int n) {
 
 struct Sizes {
   int nb, nbp;
-  int flags;    // NSA_FLAG_ANY_LENGTH from 2048 tokens on: what the tensor-core kernels gain over the generic ones grows with T
-                // while shorter ragged sequences keep their 32-bit probabilities (attn_mma.cu)
+  int flags;    // NSA_FLAG_ANY_LENGTH for bf16 from 2048 tokens on: ragged tensor-core kernels with bf16 probabilities (3.7 ms a step
+                // of 5001 tokens).  Shorter ragged sequences hold 32-bit probabilities, so they stay on attn_mma.cu (3.8 ms at 1000)
   bool exact;   // the compressed attention takes its keys as a bf16 pair hi + lo
   int ld_cmp;   // row distance of the compressed keys' I/O-type copies: whole 128-key tiles for the tensor-core kernels
   int ld_time;  // row distance of the keys the tensor-core kernels read: T, or the next multiple of 8 (keys are copied then)

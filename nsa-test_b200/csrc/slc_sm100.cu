@@ -16,9 +16,6 @@
 // query (block 0) is spread over many CTAs.
 #include <cuda.h>
 
-#include <cstring>
-#include <type_traits>
-
 #include "attn_args.cuh"
 #include "common.cuh"
 #include "fa_sm100.cuh"
@@ -418,35 +415,28 @@ __device__ __forceinline__ unsigned valid_slot_mask(const int* irow, int64_t s3,
 
 // Gate + mix epilogue of the merge kernels: the warp holds the finished (rounded) O_slc row of (b,h,t), lane owning VPL
 // consecutive columns; the mixed row is (o_cmp g0 + o_slc g1) + o_win g2, the operation order of the stand-alone pass.
-// The inputs are loaded apart from the arithmetic, so that a kernel can start them before it waits for the partials.
 template <int VPL>
-struct MixRow {
+__device__ __forceinline__ void slc_mix_row(const SlcMix& mix, const __nv_bfloat162 (&oslc)[VPL / 2], int64_t row, int b, int h, int t,
+                                            int H, int Tq, int dv, int lane) {
+  const __nv_bfloat16* oc = (const __nv_bfloat16*)mix.o_cmp + row * dv + lane * VPL;
+  const __nv_bfloat16* ow = (const __nv_bfloat16*)mix.o_win + row * dv + lane * VPL;
   __nv_bfloat162 a[VPL / 2], w[VPL / 2];
-  float lg[3];
-  __device__ __forceinline__ void load(const SlcMix& mix, int64_t row, int b, int h, int t, int H, int Tq, int dv, int lane) {
-    using Vec = typename std::conditional<VPL == 4, uint2, uint32_t>::type;
-    const Vec va = *reinterpret_cast<const Vec*>((const __nv_bfloat16*)mix.o_cmp + row * dv + lane * VPL);
-    const Vec vw = *reinterpret_cast<const Vec*>((const __nv_bfloat16*)mix.o_win + row * dv + lane * VPL);
-    memcpy(a, &va, sizeof(a));
-    memcpy(w, &vw, sizeof(w));
-    const float* src = mix.logits + ((int64_t)b * Tq + t) * 3 * H + 3 * h;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) lg[i] = src[i];
+  for (int c = 0; c < VPL / 2; ++c) {
+    a[c] = *reinterpret_cast<const __nv_bfloat162*>(oc + 2 * c);
+    w[c] = *reinterpret_cast<const __nv_bfloat162*>(ow + 2 * c);
   }
-  __device__ __forceinline__ void store(const SlcMix& mix, const __nv_bfloat162 (&oslc)[VPL / 2], int64_t row, int b, int h, int t, int H,
-                                        int Tq, int dv, int lane) const {
-    float g[3];
-    gates3(lg, mix.mode, g);
-    if (lane < 3) mix.gates[row * 3 + lane] = lane == 0 ? g[0] : lane == 1 ? g[1] : g[2];
-    __nv_bfloat16* dst = (__nv_bfloat16*)mix.out + mixed_row(row, b, h, t, H, Tq, mix.token_major) * dv + lane * VPL;
+  float g[3];
+  gates3(mix.logits + ((int64_t)b * Tq + t) * 3 * H + 3 * h, mix.mode, g);
+  if (lane < 3) mix.gates[row * 3 + lane] = g[lane];
+  __nv_bfloat16* dst = (__nv_bfloat16*)mix.out + mixed_row(row, b, h, t, H, Tq, mix.token_major) * dv + lane * VPL;
 #pragma unroll
-    for (int c = 0; c < VPL / 2; ++c) {
-      const float2 fa = __bfloat1622float2(a[c]), fs = __bfloat1622float2(oslc[c]), fw = __bfloat1622float2(w[c]);
-      *reinterpret_cast<__nv_bfloat162*>(dst + 2 * c) =
-          __floats2bfloat162_rn((fa.x * g[0] + fs.x * g[1]) + fw.x * g[2], (fa.y * g[0] + fs.y * g[1]) + fw.y * g[2]);
-    }
+  for (int c = 0; c < VPL / 2; ++c) {
+    const float2 fa = __bfloat1622float2(a[c]), fs = __bfloat1622float2(oslc[c]), fw = __bfloat1622float2(w[c]);
+    *reinterpret_cast<__nv_bfloat162*>(dst + 2 * c) =
+        __floats2bfloat162_rn((fa.x * g[0] + fs.x * g[1]) + fw.x * g[2], (fa.y * g[0] + fs.y * g[1]) + fw.y * g[2]);
   }
-};
+}
 
 // merge the partials of a query in slot order: one warp per (b,h,t).  Every load of the row (index row, statistics,
 // all slots' partial outputs) is issued before the first value is used; slots that turn out not to contribute were
@@ -518,19 +508,16 @@ __global__ void slc_combine_fwd_kernel(const __nv_bfloat16* __restrict__ o_part,
     L[row] = lsum > 0.f ? logf(lsum) : -CUDART_INF_F;
     M[row] = lsum > 0.f ? mx * kLn2f : -CUDART_INF_F;
   }
-  if (mix.out) {
-    MixRow<VPL> mr;
-    mr.load(mix, row, b, h, t, H, Tq, DV, lane);
-    mr.store(mix, rounded, row, b, h, t, H, Tq, DV, lane);
-  }
+  if (mix.out) slc_mix_row<VPL>(mix, rounded, row, b, h, t, H, Tq, DV, lane);
 }
 
 // Same merge with the whole contiguous block of a query's partials ([slots][heads][dv]) brought into shared memory by
 // one bulk copy: one thread block per (group, query), one warp per head.  No registers are spent on loads in flight,
 // so several blocks per SM keep enough bytes on their way to saturate HBM.
-// (40 registers: three blocks of 16 heads per SM; 44 let in two and took a quarter longer)
+// (40 registers, three blocks of 16 heads per SM: loading the other branches' rows before the wait took 44, two blocks and a
+// quarter more time; held to 40 it gained nothing.)
 template <int DV>
-__global__ void __maxnreg__(40) slc_combine_fwd_bulk_kernel(const __nv_bfloat16* __restrict__ o_part, const float2* __restrict__ st_part,
+__global__ void slc_combine_fwd_bulk_kernel(const __nv_bfloat16* __restrict__ o_part, const float2* __restrict__ st_part,
                                             const int* __restrict__ indices, int64_t s0, int64_t s1, int64_t s2, int64_t s3,
                                             __nv_bfloat16* __restrict__ out, float* __restrict__ L, float* __restrict__ M, int B,
                                             int H, int G, int Tq, int Tk, int nslots, int lprime, int q0, int* timeouts,
@@ -564,8 +551,6 @@ __global__ void __maxnreg__(40) slc_combine_fwd_bulk_kernel(const __nv_bfloat16*
   float lsum = 0.f, acc[VPL];
 #pragma unroll
   for (int c = 0; c < VPL; ++c) acc[c] = 0.f;
-  MixRow<VPL> mr;      // the other branches' rows arrive while the partials do
-  if (mix.out) mr.load(mix, row, b, h, t, H, Tq, DV, lane);
   const bool ok = mbar_wait_warp(&bar, 0, &abort_flag);
   if (ok) {
     for (int s = 0; s < nslots; ++s) {
@@ -595,7 +580,7 @@ __global__ void __maxnreg__(40) slc_combine_fwd_bulk_kernel(const __nv_bfloat16*
       L[row] = lsum > 0.f ? logf(lsum) : -CUDART_INF_F;
       M[row] = lsum > 0.f ? mx * kLn2f : -CUDART_INF_F;
     }
-    if (mix.out) mr.store(mix, rounded, row, b, h, t, H, Tq, DV, lane);
+    if (mix.out) slc_mix_row<VPL>(mix, rounded, row, b, h, t, H, Tq, DV, lane);
   }
   __syncthreads();  // the copy has landed (or was given up on) before shared memory is handed back
   if (threadIdx.x == 0 && abort_flag) ptx::report_timeout(timeouts);
