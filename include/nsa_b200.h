@@ -297,6 +297,11 @@ NSA_API int nsa_gate_mix_bwd(const float* gates, const void* o_cmp, const void* 
                      int B, int H, int T, int dv, int gate_mode, int dtype, int dout_token_major,
                      void* stream);
 
+/* Rows of `D` channels between the head-major layout [B,N,T,D] and the token-major one [B,T,N,D] (contiguous, D * element size a
+ * multiple of 16 bytes): what lies between the branch kernels' gradients and the projections' GEMMs. */
+NSA_API int nsa_permute_heads(const void* in, void* out, int B, int N, int T, int D, int dtype, int to_token_major,
+                              void* stream);
+
 /* Branch-gate MLP (nsa/kernels.py:2105-2109): logits = W2 relu(W1 x + b1) + b2 for N = B*T tokens.  x [N,Dm], w1 [D2,Dm],
  * b1 [D2], w2 [O,D2], b2 [O] (O = 3H) in dtype (biases may be NULL); logits [N,O] fp32, the input of the gate/mix entry
  * points; hidden [N,D2] in dtype receives the activation the backward needs.  GEMMs on cuBLAS (see nsa_cmp_phi_fwd).

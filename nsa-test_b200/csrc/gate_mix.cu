@@ -255,3 +255,48 @@ extern "C" NSA_API int nsa_gate_mix_bwd(const float* gates, const void* o_cmp, c
   return nsa_gate_mix_bwd_delta(gates, o_cmp, o_slc, o_win, dout, do_cmp, do_slc, do_win, dlogits, nullptr, B, H, T, dv,
                                 gate_mode, dtype, dout_token_major, stream);
 }
+
+// ------------------------------------------------------------------------------------------------
+// head-major <-> token-major rows: 16-byte copies, four per thread in flight, whole rows contiguous on both sides (the generic
+// strided copy moves 2 bytes per thread)
+// ------------------------------------------------------------------------------------------------
+namespace nsa {
+constexpr int kPermuteVecs = 4;
+__global__ void __launch_bounds__(256) permute_heads_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, int N, int T, int vpr,
+                                                            int64_t total, int to_token) {
+  const int64_t i0 = (int64_t)blockIdx.x * (256 * kPermuteVecs) + threadIdx.x;
+  uint4 v[kPermuteVecs];
+#pragma unroll
+  for (int k = 0; k < kPermuteVecs; ++k)
+    if (i0 + k * 256 < total) v[k] = in[i0 + k * 256];
+#pragma unroll
+  for (int k = 0; k < kPermuteVecs; ++k) {
+    const int64_t i = i0 + k * 256;
+    if (i >= total) continue;
+    const int64_t row = i / vpr;
+    const int c = (int)(i - row * vpr);
+    const int inner = to_token ? T : N, outer = to_token ? N : T;      // row = (b * outer + y) * inner + x
+    const int64_t q = row / inner;
+    const int x = (int)(row - q * inner);
+    const int64_t b = q / outer;
+    const int y = (int)(q - b * outer);
+    out[((b * inner + x) * outer + y) * vpr + c] = v[k];
+  }
+}
+}  // namespace nsa
+
+extern "C" NSA_API int nsa_permute_heads(const void* in, void* out, int B, int N, int T, int D, int dtype, int to_token_major, void* stream) {
+  NSA_REQUIRE(in && out && in != out, "permute_heads: null pointer or in-place call");
+  NSA_REQUIRE(B >= 0 && N >= 0 && T >= 0 && D > 0, "permute_heads: bad sizes");
+  NSA_REQUIRE(dtype == NSA_F32 || dtype == NSA_BF16, "permute_heads: unsupported dtype %d", dtype);
+  const int64_t bytes = (int64_t)D * (dtype == NSA_F32 ? 4 : 2);
+  NSA_REQUIRE(bytes % 16 == 0 && ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0,
+              "permute_heads: rows must be multiples of 16 bytes on 16-byte boundaries");
+  const int vpr = (int)(bytes / 16);
+  const int64_t total = (int64_t)B * N * T * vpr;
+  if (total == 0) return NSA_OK;
+  KernelTimer kt("permute_heads", (cudaStream_t)stream);
+  permute_heads_kernel<<<(unsigned)((total + 256 * kPermuteVecs - 1) / (256 * kPermuteVecs)), 256, 0, (cudaStream_t)stream>>>(
+      (const uint4*)in, (uint4*)out, N, T, vpr, total, to_token_major ? 1 : 0);
+  return check_launch("permute_heads");
+}

@@ -78,6 +78,7 @@ PROTOTYPES = {
     "nsa_cmp_phi_workspace_bytes": (c_size_t, [c_int] * 11),
     "nsa_cmp_phi_fwd": (c_int, [_P] * 10 + [c_int] * 10 + [_P, c_size_t, _P, c_size_t, _P]),
     "nsa_cmp_phi_bwd": (c_int, [_P] * 7 + [c_size_t] + [_P] * 7 + [c_int] * 10 + [_P, c_size_t, _P]),
+    "nsa_permute_heads": (c_int, [_P, _P] + [c_int] * 6 + [_P]),
     "nsa_gate_mlp_workspace_bytes": (c_size_t, [c_int64, c_int, c_int, c_int, c_int, c_int]),
     "nsa_gate_mlp_fwd": (c_int, [_P] * 7 + [c_int64, c_int, c_int, c_int, c_int, _P]),
     "nsa_gate_mlp_bwd": (c_int, [_P] * 10 + [c_int64, c_int, c_int, c_int, c_int, _P, c_size_t, _P]),

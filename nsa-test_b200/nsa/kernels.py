@@ -524,6 +524,67 @@ def _project_heads(x: torch.Tensor, linear: torch.nn.Linear, heads: int, dim: in
     return y if b is None else y + b.view(heads, 1, dim)
 
 
+def _fused_projections(x: torch.Tensor, lins, layouts) -> bool:
+    """Whether ``_Projections`` covers these linears: plain contiguous weights of x's type without biases, no autocast."""
+    plain = (torch.Tensor, torch.nn.Parameter)
+    if type(x) not in plain or not x.is_cuda or x.dim() != 3 or x.numel() == 0 or torch.is_autocast_enabled("cuda"):
+        return False
+    return all(type(lin.weight) in plain and lin.bias is None and lin.weight.dtype == x.dtype and lin.weight.device == x.device
+               and lin.weight.shape == (heads * dim, x.shape[2]) and lin.weight.is_contiguous()
+               for lin, (heads, dim, _) in zip(lins, layouts))
+
+
+class _Projections(torch.autograd.Function):
+    """``apply(x [B,T,d_model], (heads, dim, transposed) per weight, *weights)`` -> the projections in the kernels' layouts:
+    [B,heads,T,dim], or [B,heads,dim,T] where ``transposed``.
+
+    The values of ``_project_heads`` without biases.  A GEMM batched over the heads with x shared by a zero batch stride writes
+    [B,heads,T,dim] itself (``matmul`` of a 2-d by a 3-d tensor folds them into one product and leaves its transpose).  The
+    backward reads the keys' gradients as they lie and the others as token-major rows: one product per weight and one added
+    onto dx; through autograd's own formulas it went through strided copies of every gradient."""
+
+    @staticmethod
+    def forward(ctx, x, layouts, *weights):
+        ctx.save_for_backward(x, *weights)
+        ctx.layouts = layouts
+        out = []
+        for (heads, dim, transposed), w in zip(layouts, weights):
+            if transposed:
+                out.append(torch.matmul(w, x.transpose(1, 2)).view(x.shape[0], heads, dim, x.shape[1]))
+                continue
+            y = x.new_empty(x.shape[0], heads, x.shape[1], dim)
+            wt = w.view(heads, dim, -1).transpose(1, 2)
+            for b in range(x.shape[0]):
+                torch.bmm(x[b].unsqueeze(0).expand(heads, -1, -1), wt, out=y[b])
+            out.append(y)
+        return tuple(out)
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, *grads):
+        x, *weights = ctx.saved_tensors
+        B, T, dm = x.shape
+        dx, dws = None, []
+        x2 = x.reshape(B * T, dm)
+        for i, ((heads, dim, transposed), w, g) in enumerate(zip(ctx.layouts, weights, grads)):
+            dw = None
+            if transposed:
+                gt = g.reshape(B, heads * dim, T)
+                if ctx.needs_input_grad[2 + i]:
+                    dw = torch.mm(gt[0], x2) if B == 1 else torch.bmm(gt, x).sum(0)
+                if ctx.needs_input_grad[0]:
+                    gt = gt.transpose(1, 2)
+                    dx = torch.matmul(gt, w) if dx is None else dx.baddbmm_(gt, w.expand(B, -1, -1))
+            else:
+                g2 = ops.token_major(g).view(B * T, heads * dim)
+                if ctx.needs_input_grad[2 + i]:
+                    dw = torch.mm(g2.t(), x2)
+                if ctx.needs_input_grad[0]:
+                    dx = torch.mm(g2, w).view(B, T, dm) if dx is None else dx.view(B * T, dm).addmm_(g2, w).view(B, T, dm)
+            dws.append(dw)
+        return (dx, None, *dws)
+
+
 class NSAAttention(torch.nn.Module):
     """Drop-in for the reference's ``NSAAttention``: same parameter names (so its state_dicts load),
     same ``forward(hidden_states, attention_mask=None, output_attentions=False) -> (out, info)``."""
@@ -572,17 +633,16 @@ class NSAAttention(torch.nn.Module):
         c = self.config
         B, T, _ = hidden_states.shape
         H, G, dk, dv = c.n_heads, c.n_kv_groups, c.head_dim_qk, c.head_dim_v
-        q = _project_heads(hidden_states, self.q_proj, H, dk)                                    # [B,H,T,dk]
-
-        def kv(kp, vp):
-            return (_project_heads(hidden_states, kp, G, dk, transposed=True),                   # [B,G,dk,T]
-                    _project_heads(hidden_states, vp, G, dv))                                    # [B,G,T,dv]
-
-        k_sel, v_sel = kv(self.k_select, self.v_select)
+        # q [B,H,T,dk]; k [B,G,dk,T]; v [B,G,T,dv]
+        lins = (self.q_proj, self.k_select, self.v_select, self.k_compress, self.v_compress, self.k_sliding, self.v_sliding)
+        layouts = ((H, dk, False),) + ((G, dk, True), (G, dv, False)) * 3
+        if _fused_projections(hidden_states, lins, layouts):
+            q, k_sel, v_sel, *other = _Projections.apply(hidden_states, layouts, *[lin.weight for lin in lins])
+        else:
+            q, k_sel, v_sel, *other = [_project_heads(hidden_states, lin, *lay) for lin, lay in zip(lins, layouts)]
         gate_logits = gate_logits_from_hidden(hidden_states, self.gate_mlp)                      # [B,T,3H] fp32
         out, info = nsa_layer(q, k_sel, v_sel, gate_logits, self._phi_params(), c,
-                              kv_compress=kv(self.k_compress, self.v_compress),
-                              kv_sliding=kv(self.k_sliding, self.v_sliding), scale=self.scale, return_info=True,
+                              kv_compress=tuple(other[:2]), kv_sliding=tuple(other[2:]), scale=self.scale, return_info=True,
                               token_major_out=True)
         # the mix epilogue wrote [B,T,H,dv] in memory: this reshape is a view, not the copy of nsa/kernels.py:2466-2467
         y = self.o_proj(out.permute(0, 2, 1, 3).reshape(B, T, H * dv))

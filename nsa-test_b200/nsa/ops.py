@@ -301,6 +301,21 @@ def _next_pow2(n: int) -> int:
     return p
 
 
+def token_major(x):
+    """[B,N,T,D] -> a contiguous [B,T,N,D] tensor: a view where it lies so already, one copy otherwise."""
+    y = x.transpose(1, 2)
+    if y.is_contiguous():
+        return y
+    B, N, T, D = x.shape
+    if not x.is_contiguous() or x.dtype not in (torch.float32, torch.bfloat16) or D * x.element_size() % 16 or x.data_ptr() % 16:
+        return y.contiguous()
+    dev = require_cuda(x)
+    out = torch.empty(B, T, N, D, device=dev, dtype=x.dtype)
+    with torch.cuda.device(dev):
+        check(lib.nsa_permute_heads(ptr(x), ptr(out), B, N, T, D, dtype_code(x), 1, stream_ptr(dev)), "nsa_permute_heads")
+    return out
+
+
 def cmp_phi_fwd(k, v, pos_embed, w1, b1, w2, b2, l: int, d: int):
     """Block compression phi through the C ABI.  k [B,G,dk,T], v [B,G,T,dv] (contiguous, one dtype); fp32 parameters.
     -> k_cmp fp32 [B,G,dk,nbp], v_cmp [B,G,nbp,dv], and the buffer the backward needs."""

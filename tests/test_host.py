@@ -115,3 +115,21 @@ def test_launcher_checks_every_tensor_before_launching():
     view = t[:, :, 2:]                                                   # storage offset counts against the room left
     with pytest.raises(ValueError):
         _Launcher._fits("dQ", view, t.stride(), t.shape)
+
+
+def test_projections_match_the_per_linear_products(monkeypatch):
+    """The one autograd node of the seven projections against one product per linear: values and gradients in 64 bits."""
+    import torch
+    from nsa import kernels as K, ops
+    monkeypatch.setattr(ops, "token_major", lambda x: x.transpose(1, 2).contiguous())
+    torch.manual_seed(0)
+    x = torch.randn(2, 5, 8, dtype=torch.double, requires_grad=True)
+    layouts = ((4, 3, False), (2, 3, True), (2, 2, False))
+    lins = [torch.nn.Linear(8, h * d, bias=False, dtype=torch.double) for h, d, _ in layouts]
+    ws = [lin.weight for lin in lins]
+    a = K._Projections.apply(x, layouts, *ws)
+    b = [K._project_heads(x, lin, *lay) for lin, lay in zip(lins, layouts)]
+    gs = [torch.randn_like(t) for t in b]
+    for p, q in zip((*a, *torch.autograd.grad(a, [x, *ws], gs)), (*b, *torch.autograd.grad(b, [x, *ws], gs))):
+        assert p.shape == q.shape and (p - q).abs().max().item() < 1e-12
+    assert all(t.is_contiguous() for t in a)
