@@ -155,6 +155,16 @@ NSA_API int nsa_sliding_bwd_noalloc(const void* q, const void* k, const void* v,
  * the logits are q (k_cmp + k_cmp_lo), i.e. those of the fp32 keys to 16 mantissa bits, and lse2_out [B,H,T] fp32
  * receives their log-sum-exp in log2 units (+inf for rows that see no block).  That is the normaliser of Eq. 8, so
  * nsa_score_topn given it as cmp_lse2 skips its own first sweep over the compressed keys. */
+/* The exact-key form of the compressed attention and the Eq. 8-11 block choice in one call (k_cmp: the fp32 keys whose halves
+ * k_hi, k_lo [B,G,dk,ld] are; arguments otherwise as for nsa_cmp_attn_fwd and nsa_score_topn): where the scratch it asks for
+ * holds them, the forward leaves the sums of its probabilities and the choice only adds those up. */
+NSA_API size_t nsa_cmp_attn_topn_workspace_bytes(int B, int H, int G, int T, int NB, int dk, int dv, int l, int d, int l_prime,
+                                                 int n, int n_real_blocks, int flags);
+NSA_API int nsa_cmp_attn_topn_fwd(const void* q, const void* k_hi, const void* k_lo, const float* k_cmp, const void* v_cmp,
+                                  const int32_t* block_ends, void* out, float* L, float* M, float* lse2_out,
+                                  int32_t* indices_out, const int64_t* strides, int B, int H, int G, int T, int NB, int nbp,
+                                  int dk, int dv, int l, int d, int l_prime, int n, int n_fixed, int n_real_blocks,
+                                  float scale, int q_pos0, int flags, void* workspace, size_t workspace_bytes, void* stream);
 NSA_API int nsa_cmp_attn_exact_supported(int B, int H, int G, int T, int NB, int dk, int dv, int dtype);
 NSA_API int nsa_split_keys_hi_lo(const float* x, void* hi, void* lo, int64_t n, void* stream);
 NSA_API int nsa_cmp_attn_fwd(const void* q, const void* k_cmp, const void* v_cmp, const int32_t* block_ends,

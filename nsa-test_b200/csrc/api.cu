@@ -294,6 +294,42 @@ extern "C" NSA_API int nsa_cmp_attn_fwd(const void* q, const void* k_cmp, const 
   return launch_attn_generic(a, kCmp, dtype, false, (cudaStream_t)stream);
 }
 
+static size_t topn_partials(int B, int H, int G, int T, int NB, int dk, int dv, int l, int d, int l_prime, int n, int nb, int flags) {
+  if (!want_tc(flags) || !fa_fwd_sm100_supported(H, G, T, NB, dk, dv) || (int64_t)B * (H / 2) > 65535) return 0;
+  return score_partials_bytes(B, H, G, T, dk, NB, nb, l, d, l_prime, n);
+}
+extern "C" NSA_API size_t nsa_cmp_attn_topn_workspace_bytes(int B, int H, int G, int T, int NB, int dk, int dv, int l, int d, int l_prime,
+                                                            int n, int n_real_blocks, int flags) {
+  const size_t parts = topn_partials(B, H, G, T, NB, dk, dv, l, d, l_prime, n, n_real_blocks, flags);
+  return parts ? parts : nsa_score_topn_workspace_bytes(B, H, G, T, dk, NB, l, d, l_prime, n, NSA_BF16, flags);
+}
+extern "C" NSA_API int nsa_cmp_attn_topn_fwd(const void* q, const void* k_hi, const void* k_lo, const float* k_cmp, const void* v_cmp,
+                                             const int32_t* block_ends, void* out, float* L, float* M, float* lse2_out, int32_t* indices_out,
+                                             const int64_t* strides, int B, int H, int G, int T, int NB, int nbp, int dk, int dv, int l, int d,
+                                             int l_prime, int n, int n_fixed, int n_real_blocks, float scale, int q_pos0, int flags,
+                                             void* workspace, size_t workspace_bytes, void* stream) {
+  if (int rc = check_common("cmp_attn_topn_fwd", B, H, G, T, NB, dk, dv, NSA_BF16)) return rc;
+  NSA_REQUIRE(q && k_hi && k_lo && k_cmp && v_cmp && block_ends && out && L && M && lse2_out && indices_out && strides, "cmp_attn_topn_fwd: null pointer");
+  NSA_REQUIRE(NB > 0 && nbp >= NB && n_real_blocks > 0 && n_real_blocks <= NB && l > 0 && d > 0 && q_pos0 >= 0, "cmp_attn_topn_fwd: bad block layout");
+  NSA_REFUSE_AFTER_TIMEOUT("cmp_attn_topn_fwd");
+  KvLayout kv;
+  const size_t parts = topn_partials(B, H, G, T, nbp, dk, dv, l, d, l_prime, n, n_real_blocks, flags);
+  if (parts && canonical_fwd(strides, B, H, G, T, NB, dk, dv, &kv) && length_ok(flags, T, 128, NB, 128, dv, kv) && aligned16(q) && aligned16(k_hi) &&
+      aligned16(k_lo) && aligned16(v_cmp) && aligned16(out) && workspace && workspace_bytes >= parts) {
+    const ScorePartials sp = score_partials_at(workspace, B, H, T, n_real_blocks);
+    if (int rc = fa_fwd_sm100(q, k_hi, v_cmp, out, L, M, B, H, G, T, NB, dk, dv, kCmp, 0, l - q_pos0, d, n_real_blocks, scale, k_lo, lse2_out, kv,
+                              (cudaStream_t)stream, 0, &sp))
+      return rc;
+    return score_topn_from_partials(sp, q, k_hi, k_lo, NB, kv, lse2_out, indices_out, B, H, G, T, dk, nbp, l, d, l_prime, n_real_blocks, n, n_fixed,
+                                    scale, q_pos0, workspace, (cudaStream_t)stream);
+  }
+  if (int rc = nsa_cmp_attn_fwd(q, k_hi, v_cmp, block_ends, out, L, M, strides, B, H, G, T, NB, dk, dv, scale, NSA_BF16, l, d, n_real_blocks, q_pos0,
+                                flags, k_lo, lse2_out, stream))
+    return rc;
+  return nsa_score_topn(q, strides, k_cmp, block_ends, indices_out, B, H, G, T, dk, nbp, l, d, l_prime, n, n_fixed, scale, NSA_BF16, n_real_blocks,
+                        q_pos0, flags, lse2_out, workspace, workspace_bytes, stream);
+}
+
 extern "C" NSA_API int nsa_cmp_attn_exact_supported(int B, int H, int G, int T, int NB, int dk, int dv, int dtype) {
   return dtype == NSA_BF16 && B > 0 && T % 128 == 0 && NB % 128 == 0 && fa_fwd_sm100_supported(H, G, T, NB, dk, dv) && (int64_t)B * (H / 2) <= 65535 ? 1 : 0;
 }

@@ -2,7 +2,7 @@
 // block choice, the three attention branches and the gate mix, for up to 64 (sequence, group, token) rows.
 //
 // The tile kernels pad such a call to 128 query rows and need an inverse index, padded copies and one launch per piece:
-// 45 launches and 760 us per token at B=1, 2K cached; 80 launches and 1400 us at B=8, 32K.  What the work cannot do without
+// 45 launches and 760 us per token at B=1, 2K cached; 80 launches and 1400 us at B=8, 32K (91 and 138 us here).  What the work cannot do without
 // is reading the weights once (131 MB for the 64-head configuration, 20 us) and the visible keys and values once, so here
 // the keys of a row are cut into 64-key chunks, one CTA each, that serve all heads of the group, and everything between
 // two grid-wide dependencies is one launch:

@@ -72,7 +72,10 @@ __device__ __forceinline__ void row_bounds(const FaFwdParams& p, int t, int n0, 
 // Q K_hi^T + Q K_lo^T, so the log-sum-exp this kernel emits (lse2, log2 units) is the one the selection scoring needs and
 // that kernel can skip its own first sweep.  The two K stages then hold the hi and the lo part of ONE tile (the next
 // tile's keys are fetched while the softmax warps work, once both heads' S MMAs have read the current ones).
-template <int DK, int DV, int MODE, bool EXACT>
+// SCORE: the softmax warps have every p in registers, so they also leave the Eq. 9 sums of 4 + 1 consecutive keys behind (a
+// column of 128 rows per block: coalesced stores, 3 additions per 2 keys).  The block choice then reads 1/4 of the logits' bytes
+// instead of computing S a second time; at T = 65536 this kernel takes 9.1 instead of 8.0 ms, the scores 3.5 instead of 7.3.
+template <int DK, int DV, int MODE, bool EXACT, bool SCORE>
 __global__ void __launch_bounds__(kFaThreads, 1)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
               const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmKlo, const FaFwdParams p) {
@@ -355,7 +358,9 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       }
       if (grow) m_ref = m_true;
       const float mref_use = m_ref == -CUDART_INF_F ? 0.f : m_ref;
-      float rs = 0.f;
+      float rs = 0.f, blk = 0.f;
+      const int64_t qtile = ((int64_t)b * p.H + h0 + i) * ((p.Tq + kBM - 1) / kBM) + m0 / kBM;
+      float* sel = SCORE ? p.sel + ((qtile * p.sel_tiles + jlo + j) * 32) * 128 + r : nullptr;
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t pk[32];
@@ -365,11 +370,22 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
           const float p0 = ex2(__uint_as_float(sv[cc][ee]) - mref_use);
           const float p1 = ex2(__uint_as_float(sv[cc][ee + 1]) - mref_use);
           rs += p0 + p1;
+          if (SCORE) {
+            const int jj = cc * 8 + (ee >> 2);
+            if ((ee & 2) == 0) {
+              if (jj == 0) p.sel_aux[(qtile * p.sel_tiles + jlo + j) * 128 + r] = make_float2(m_ref, p0);
+              else sel[(jj - 1) * 128] = blk + p0;
+              blk = fmaf(2.f, p1, p0);
+            } else {
+              blk = fmaf(2.f, p0 + p1, blk);
+            }
+          }
           __nv_bfloat162 v2 = __floats2bfloat162_rn(p0, p1);  // .x (low half) = even key
           pk[e] = *reinterpret_cast<uint32_t*>(&v2);
         }
         tmem_st32(tS + c * 32, pk);
       }
+      if (SCORE) sel[31 * 128] = blk;
       l += rs;
       tc_wait_st();
       tc_fence_before();
@@ -516,11 +532,11 @@ static int sm_count() {
   return cached[dev];
 }
 
-template <int DK, int DV, int MODE, bool EXACT>
+template <int DK, int DV, int MODE, bool EXACT, bool SCORE>
 static int launch_fa_fwd_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tklo,
                            const FaFwdParams& p, cudaStream_t st) {
   using SM = FaSmem<DK, DV>;
-  auto kern = fa_fwd_kernel<DK, DV, MODE, EXACT>;
+  auto kern = fa_fwd_kernel<DK, DV, MODE, EXACT, SCORE>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::kDynamic);
   if (e != cudaSuccess) return fail(NSA_ERR_LAUNCH, "fa_fwd: cannot reserve %d bytes of shared memory: %s", SM::kDynamic, cudaGetErrorString(e));
   const int nitems = ((p.Tq + kBM - 1) / kBM) * p.B * (p.H / 2);
@@ -537,7 +553,8 @@ bool fa_fwd_sm100_supported(int H, int G, int Tq, int Tk, int dk, int dv) {
 
 int fa_fwd_sm100(const void* q, const void* k, const void* v, void* o, float* L, float* M, int B, int H, int G, int Tq,
                  int Tk, int dk, int dv, int mode, int window, int cmp_l, int cmp_d, int cmp_nb, float scale,
-                 const void* k_lo, float* lse2, const KvLayout& kv, cudaStream_t st, int win_q0) {
+                 const void* k_lo, float* lse2, const KvLayout& kv, cudaStream_t st, int win_q0,
+                 const ScorePartials* sp) {
   if (!fa_fwd_sm100_supported(H, G, Tq, Tk, dk, dv)) return fail(NSA_ERR_UNSUPPORTED, "fa_fwd_sm100: unsupported shape");
   if (!fa_timeout_counter()) return fail(NSA_ERR_LAUNCH, "fa_fwd_sm100: cannot set up the time-out record of this device");
   if ((int64_t)B * (H / 2) * ((Tq + kBM - 1) / kBM) > 0x7fffffff) return fail(NSA_ERR_UNSUPPORTED, "fa_fwd_sm100: too many work items");
@@ -553,11 +570,15 @@ int fa_fwd_sm100(const void* q, const void* k, const void* v, void* o, float* L,
   p.window = window; p.win_q0 = win_q0; p.cmp_l = cmp_l; p.cmp_d = cmp_d; p.cmp_nb = cmp_nb;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.lse2 = lse2;
+  p.sel = sp ? sp->sel : nullptr;
+  p.sel_aux = sp ? sp->aux : nullptr;
+  p.sel_tiles = sp ? sp->tiles : 0;
 #define NSA_FA_CASE(DK_, DV_)                                                                                            \
   if (dk == DK_ && dv == DV_)                                                                                            \
-    return mode == kWin ? launch_fa_fwd_t<DK_, DV_, kWin, false>(tq, tk, tv, tklo, p, st)                               \
-                        : (k_lo ? launch_fa_fwd_t<DK_, DV_, kCmp, true>(tq, tk, tv, tklo, p, st)                          \
-                                : launch_fa_fwd_t<DK_, DV_, kCmp, false>(tq, tk, tv, tklo, p, st));
+    return mode == kWin ? launch_fa_fwd_t<DK_, DV_, kWin, false, false>(tq, tk, tv, tklo, p, st)                        \
+           : !k_lo      ? launch_fa_fwd_t<DK_, DV_, kCmp, false, false>(tq, tk, tv, tklo, p, st)                        \
+           : !sp        ? launch_fa_fwd_t<DK_, DV_, kCmp, true, false>(tq, tk, tv, tklo, p, st)                         \
+                        : launch_fa_fwd_t<DK_, DV_, kCmp, true, true>(tq, tk, tv, tklo, p, st);
   NSA_FA_CASE(192, 128)
   NSA_FA_CASE(128, 128)
   NSA_FA_CASE(64, 64)

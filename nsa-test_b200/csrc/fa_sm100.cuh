@@ -17,8 +17,25 @@ struct FaFwdParams {
   int win_q0;                // sliding window: position of query row 0 among the keys
   int cmp_l, cmp_d, cmp_nb;  // compressed tokens: key i visible iff i < cmp_nb and i*cmp_d + cmp_l - 1 <= t
   float scale_log2;          // softmax scale times log2(e)
+  // what the block choice needs from the compressed branch, or null (see ScorePartials)
+  float* sel;
+  float2* sel_aux;
+  int sel_tiles;
 };
 
+// Eq. 9 sums that the compressed attention's exact forward leaves for the block choice (l = 2 d, l' = 4 d): sel [B*H][query
+// tile][4-key block][128 rows] holds p[4j] + 2 (p[4j+1] + p[4j+2] + p[4j+3]) + p[4j+4] relative to the row's reference maximum at
+// that key tile (without the last term for a tile's last block), aux [B*H][query tile][key tile][128 rows] that maximum (log2
+// units) and the tile's first p.
+struct ScorePartials {
+  float* sel;
+  float2* aux;
+  int tiles;       // key tiles the buffers have room for
+};
+// Bytes of the buffers and of the block scores behind them; 0: not available for these sizes (other block shapes, or more than
+// kMaxScorePartials), the stand-alone scoring kernel does it then.
+size_t score_partials_bytes(int B, int H, int G, int T, int dk, int nbp, int nb, int l, int d, int lprime, int n);
+ScorePartials score_partials_at(void* workspace, int B, int H, int T, int nb);
 // True when the tensor-core forward covers this shape (bf16, canonical contiguous layouts assumed).
 bool fa_fwd_sm100_supported(int H, int G, int Tq, int Tk, int dk, int dv);
 
@@ -28,6 +45,11 @@ bool fa_fwd_sm100_supported(int H, int G, int Tq, int Tk, int dk, int dv);
 struct KvLayout {
   int64_t k_ld, v_plane;
 };
+// The block choice from them: scores added up, the top n taken, and the rows where rounding could move the cut scored again by the
+// scoring kernel, so the blocks are the ones it picks.
+int score_topn_from_partials(const ScorePartials& sp, const void* q, const void* k_hi, const void* k_lo, int NB, const KvLayout& kv, const float* lse2,
+                             int32_t* out, int B, int H, int G, int T, int dk, int nbp, int l, int d, int lprime, int nb, int n, int n_fixed,
+                             float scale, int q0, void* workspace, cudaStream_t st);
 
 // q [B,H,Tq,dk], o [B,H,Tq,dv]: contiguous bf16, any Tq and Tk (tiles reaching past them are filled with zeros by TMA and
 // their rows are not stored).  mode = kWin or kCmp.
@@ -35,7 +57,8 @@ struct KvLayout {
 // log-sum-exp in log2 units.  win_q0: position of query row 0 among the keys of a sliding-window call.
 int fa_fwd_sm100(const void* q, const void* k, const void* v, void* o, float* L, float* M, int B, int H, int G, int Tq,
                  int Tk, int dk, int dv, int mode, int window, int cmp_l, int cmp_d, int cmp_nb, float scale,
-                 const void* k_lo, float* lse2, const KvLayout& kv, cudaStream_t st, int win_q0 = 0);
+                 const void* k_lo, float* lse2, const KvLayout& kv, cudaStream_t st, int win_q0 = 0,
+                 const ScorePartials* sp = nullptr);
 
 // Backward of the same two branches.  Adds into dk [B,G,Tk,dk] and dv [B,G,Tk,dv] (time-major, bf16),
 // overwrites dq [B,H,Tq,dk].  Three launches: delta/lse preparation, a query-stationary dQ kernel and

@@ -124,7 +124,7 @@ ChunkLayout chunk_layout(const nsa_decode_desc& d) {
   L.o_win = take(R * d.dv * 2);
   L.o_gates = take(R * 3 * 4);
   L.o_idx = take(BG * d.Tn * d.n * 4);
-  L.stage = std::max(nsa_score_topn_workspace_bytes(d.B, d.H, d.G, d.Tn, d.dk, d.nbp, d.l, d.d, d.l_prime, d.n, NSA_BF16, NSA_FLAG_ANY_LENGTH),
+  L.stage = std::max(nsa_cmp_attn_topn_workspace_bytes(d.B, d.H, d.G, d.Tn, d.nbp, d.dk, d.dv, d.l, d.d, d.l_prime, d.n, d.nb, NSA_FLAG_ANY_LENGTH),
                      nsa_slc_fwd_workspace_bytes(d.B, d.H, d.G, d.Tn, L.Tk, d.dk, d.dv, d.n, d.l_prime, NSA_BF16, NSA_FLAG_ANY_LENGTH));
   L.o_stage = take(L.stage);
   L.total = o;
@@ -248,11 +248,9 @@ extern "C" NSA_API int nsa_incremental_fwd(const nsa_decode_desc* dp, void* work
   // compressed attention on the fp32 keys as a bf16 pair hi + lo; its log-sum-exp normalises the scoring
   if (int rc = split_keys_padded((const float*)d.k_cmp, hi, lo, G * d.B * dk, d.nbp, L.ld, st)) return rc;
   strides(L.ld, (int64_t)d.nbp * dv);
-  if (int rc = nsa_cmp_attn_fwd(d.q, hi, d.v_cmp, d.block_ends, o_cmp, Ls, Ms, s, d.B, d.H, d.G, d.Tn, d.nb, d.dk, d.dv, d.scale, NSA_BF16, d.l,
-                                d.d, d.nb, d.pos, NSA_FLAG_ANY_LENGTH, lo, lse2, stream))
-    return rc;
-  if (int rc = nsa_score_topn(d.q, s, (const float*)d.k_cmp, d.block_ends, idx, d.B, d.H, d.G, d.Tn, d.dk, d.nbp, d.l, d.d, d.l_prime, d.n,
-                              d.n_fixed, d.scale, NSA_BF16, d.nb, d.pos, NSA_FLAG_ANY_LENGTH, lse2, w + L.o_stage, L.stage, stream))
+  if (int rc = nsa_cmp_attn_topn_fwd(d.q, hi, lo, (const float*)d.k_cmp, d.v_cmp, d.block_ends, o_cmp, Ls, Ms, lse2, idx, s, d.B, d.H, d.G, d.Tn, d.nb,
+                                     d.nbp, d.dk, d.dv, d.l, d.d, d.l_prime, d.n, d.n_fixed, d.nb, d.scale, d.pos, NSA_FLAG_ANY_LENGTH, w + L.o_stage,
+                                     L.stage, stream))
     return rc;
   const int64_t rows = (int64_t)d.B * G * T;
   fallback_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, st>>>(idx, rows, d.Tn, d.n, d.l_prime, d.pos);

@@ -10,6 +10,7 @@
 // k/v pair that feeds several branches needs no extra accumulation pass.
 #include <algorithm>
 
+#include "attn_args.cuh"
 #include "common.cuh"
 #include "fa_sm100.cuh"
 
@@ -146,6 +147,7 @@ struct Scratch {
 
 size_t stage_scratch_fwd(const nsa_layer_desc& d, const Sizes& s) {
   size_t m = nsa_score_topn_workspace_bytes(d.B, d.H, d.G, d.T, d.dk, s.nbp, d.l, d.d, d.l_prime, d.n, d.dtype, s.flags);
+  if (s.exact) m = std::max(m, nsa_cmp_attn_topn_workspace_bytes(d.B, d.H, d.G, d.T, s.nbp, d.dk, d.dv, d.l, d.d, d.l_prime, d.n, s.nb, s.flags));
   m = std::max(m, nsa_slc_fwd_workspace_bytes(d.B, d.H, d.G, d.T, d.T, d.dk, d.dv, d.n, d.l_prime, d.dtype, s.flags));
   if (s.nb > 0) m = std::max(m, nsa_cmp_phi_workspace_bytes(d.B, d.G, d.T, d.dk, d.dv, d.l, d.d, d.U, s.nbp, d.dtype, 0));
   return al256(m);
@@ -232,14 +234,22 @@ extern "C" NSA_API int nsa_layer_fwd(const nsa_layer_desc* dp, const void* q, co
   if (exact)
     if (int rc = split_keys_padded(k_cmp, piece(NSA_CTX_K_CMP_LP), k_lo, (int64_t)BG * d.dk, s.nbp, s.ld_cmp, st)) return rc;
   fill_strides(d, s.nbp, s.ld_cmp, 0, false, false, strides);
-  if (int rc = nsa_cmp_attn_fwd(q, piece(NSA_CTX_K_CMP_LP), piece(NSA_CTX_V_CMP), be, piece(NSA_CTX_O_CMP), (float*)piece(NSA_CTX_L_CMP),
-                                (float*)piece(NSA_CTX_M_CMP), strides, d.B, d.H, d.G, d.T, s.nbp, d.dk, d.dv, d.scale, d.dtype, d.l, d.d,
-                                s.nb, 0, s.flags, k_lo, lse2, stream))
-    return rc;
+  const bool chosen = exact && !indices_in;      // the block choice comes with the attention
+  if (chosen) {
+    if (int rc = nsa_cmp_attn_topn_fwd(q, piece(NSA_CTX_K_CMP_LP), k_lo, k_cmp, piece(NSA_CTX_V_CMP), be, piece(NSA_CTX_O_CMP), (float*)piece(NSA_CTX_L_CMP),
+                                       (float*)piece(NSA_CTX_M_CMP), lse2, idx, strides, d.B, d.H, d.G, d.T, s.nbp, s.nbp, d.dk, d.dv, d.l, d.d,
+                                       d.l_prime, d.n, d.n_fixed, s.nb, d.scale, 0, s.flags, workspace, workspace_bytes, stream))
+      return rc;
+  } else {
+    if (int rc = nsa_cmp_attn_fwd(q, piece(NSA_CTX_K_CMP_LP), piece(NSA_CTX_V_CMP), be, piece(NSA_CTX_O_CMP), (float*)piece(NSA_CTX_L_CMP),
+                                  (float*)piece(NSA_CTX_M_CMP), strides, d.B, d.H, d.G, d.T, s.nbp, d.dk, d.dv, d.scale, d.dtype, d.l, d.d,
+                                  s.nb, 0, s.flags, k_lo, lse2, stream))
+      return rc;
+  }
   // 3. Eq. 8-11: which blocks every query attends
   if (indices_in) {
     cudaMemcpyAsync(idx, indices_in, BG * d.T * d.n * sizeof(int32_t), cudaMemcpyDeviceToDevice, st);
-  } else {
+  } else if (!chosen) {
     const int64_t qs[4] = {(int64_t)d.H * d.T * d.dk, (int64_t)d.T * d.dk, d.dk, 1};
     if (int rc = nsa_score_topn(q, qs, k_cmp, be, idx, d.B, d.H, d.G, d.T, d.dk, s.nbp, d.l, d.d, d.l_prime, d.n, d.n_fixed, d.scale,
                                 d.dtype, s.nb, 0, s.flags, lse2, workspace, workspace_bytes, stream))

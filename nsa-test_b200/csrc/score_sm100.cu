@@ -15,6 +15,8 @@
 // forced blocks in, drops repeats, cuts the list to n and pads it with -1.
 #include <cuda.h>
 
+#include <algorithm>
+
 #include "attn_args.cuh"
 #include "common.cuh"
 #include "fa_sm100.cuh"
@@ -35,6 +37,8 @@ struct ScoreParams {
   float scale_log2;
   int* timeouts;
   const float* lse2_ext;  // [B,H,T] log-sum-exp (log2 units) from the compressed attention's exact forward, or null (own first sweep)
+  const int* list;        // LISTED: [B*G][T] query rows to score, count[B*G] of them; q holds them compacted
+  const int* count;
 };
 
 // rows of `cols` values -> rows of `ld` >= cols, zeros behind
@@ -55,7 +59,9 @@ struct ScoreBarriers {
   int abort;
 };
 
-template <int DK>
+// LISTED: the 128 rows of a tile are rows of a list (their queries compacted beforehand).  A row's logits and sums do not depend on
+// the rows beside it, so its scores are bit for bit those of the plain form.
+template <int DK, bool LISTED>
 __global__ void __launch_bounds__(384, 1)
 score_topn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKhi,
                      const __grid_constant__ CUtensorMap tmKlo, const ScoreParams p, int hpg, int smem_state_off,
@@ -72,7 +78,16 @@ score_topn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = (gridDim.x - 1 - blockIdx.x) * 128;
   const int bg = blockIdx.y, b = bg / p.G, g = bg % p.G;
-  const int tl = p.q0 + m0 + 127;
+  __shared__ int s_last;
+  const int nlist = LISTED ? p.count[bg] : 0;
+  if (LISTED) {
+    if (m0 >= nlist) return;
+    if (threadIdx.x == 0) s_last = 0;
+    __syncthreads();
+    if (threadIdx.x < 128 && m0 + threadIdx.x < nlist) atomicMax(&s_last, p.list[(int64_t)bg * p.T + m0 + threadIdx.x]);
+    __syncthreads();
+  }
+  const int tl = p.q0 + (LISTED ? s_last : m0 + 127);
   const int kmax = tl >= p.l - 1 ? min(p.nb - 1, (tl - p.l + 1) / p.d) : -1;
   const int ntiles = max(1, kmax / 128 + 1);
   const int steps_per_pass = ntiles * hpg;
@@ -182,10 +197,11 @@ score_topn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // own, applies the stencil and feeds the top-n list, while group 1 is already on the next tile.
     asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
     const int wg = warp >> 2;
-    const int r = (warp & 3) * 32 + lane, t = m0 + r;
+    const int r = (warp & 3) * 32 + lane;
+    const int t = !LISTED ? m0 + r : m0 + r < nlist ? p.list[(int64_t)bg * p.T + m0 + r] : p.T;
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const int tp = p.q0 + t;  // position in the sequence
-    const int vis = tp >= p.l - 1 ? min(p.nb - 1, (tp - p.l + 1) / p.d) : -1;  // last visible compressed block
+    const int vis = tp >= p.l - 1 && !(LISTED && t >= p.T) ? min(p.nb - 1, (tp - p.l + 1) / p.d) : -1;  // last visible compressed block
     const int s_ = p.lprime / p.d;   // keys per selection block (a power of two on this path); l / d == 2
     const int smask = s_ - 1, sshift = 31 - __clz(s_);
     const int per_tile = 128 >> sshift;
@@ -331,14 +347,24 @@ score_topn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // forced blocks first, repeats dropped, cut to n, padded with -1.  Scores of blocks past the last key tile of the
 // row's query tile were never written and count as 0.  Lane i owns the ids i, i + 32, ...: PER of them in registers
 // (PER * 32 >= n_sel), or the row in shared memory when PER == 0 (any n_sel).
-template <int PER>
-__global__ void __launch_bounds__(128)
-topn_rows_kernel(const float* __restrict__ sel, int32_t* __restrict__ out, int64_t rows, int T, int n_sel, int per_tile, int l,
-                 int d, int nb, int lprime, int n, int n_fixed, int q0) {
+// How far apart two scores' difference may come out from the forward's sums and from the scoring kernel, relative to the score v: rows
+// whose choice that leaves open are settled by the latter.  u = 2^-24, s a logit in log2 units, x = s - lse.  A term p = 2^x is off by
+//   there, one fma and ex2.approx: (0.7 |x| + 4) u
+//   here, s, s - m and m - lse rounded and two powers: 0.7 (|s| + |s - m| + |m - lse|) u + 9 u, where |s| <= |lse| + |x|, and
+//   m <= lse, s <= m + 8 (the reference's slack) make it at most (0.7 |lse| + 1.4 |x| + 21) u,
+// the sums on the way by 1.5 hpg + 17 additions.  Over a score the mean of |x| = -log2 p, weighted by p, is at most
+// log2(number of terms / v) (concavity), with 8 hpg terms.  Two scores: twice that.
+__device__ __forceinline__ float score_tolerance(int hpg, float lse, float v) {
+  return 5.9605e-8f * (84.f + 3.f * hpg + 4.2f * log2f(8.f * hpg / v) + 1.4f * lse);
+}
+
+// CHECK: the scores come from the forward's sums; returns whether the scoring kernel's could cut elsewhere between the last block taken
+// and the first one left out.
+template <int PER, bool CHECK>
+__device__ __forceinline__ bool topn_row(const float* __restrict__ sel, int32_t* __restrict__ out, int64_t row, int T, int n_sel, int per_tile, int l,
+                 int d, int nb, int lprime, int n, int n_fixed, int q0, int hpg, float lse) {
   extern __shared__ float sm_rows[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t row = (int64_t)blockIdx.x * 4 + warp;
-  if (row >= rows) return;  // warps are independent: no block-wide barrier below
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;   // warps are independent: no block-wide barrier below
   const int tloc = (int)(row % T), t = q0 + tloc;  // row of the launch, position in the sequence
   const int tl = q0 + (tloc / 128) * 128 + 127;
   const int kmax = tl >= l - 1 ? min(nb - 1, (tl - l + 1) / d) : -1;
@@ -348,6 +374,7 @@ topn_rows_kernel(const float* __restrict__ sel, int32_t* __restrict__ out, int64
   float vr[PER > 0 ? PER : 1];        // PER > 0 only
   const int k_actual = min(n, n_sel);
   int mytop = -1;  // lane r keeps the r-th pick
+  float mytopv = 0.f;
   if (PER > 0) {
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
@@ -382,16 +409,13 @@ topn_rows_kernel(const float* __restrict__ sel, int32_t* __restrict__ out, int64
       cnt = min(cnt, 4);
     };
     refill();
-    for (int r = 0; r < k_actual; ++r) {
-      float wv = b0;
-      int wi = i0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, wv, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, wi, o);
-        if (ov > wv || (ov == wv && oi < wi)) { wv = ov; wi = oi; }
-      }
-      if (lane == r) mytop = wi;
+    const int rounds = CHECK ? min(n + 1, n_sel) : k_actual;   // (one more to see the first score left out)
+    for (int r = 0; r < rounds; ++r) {
+      // scores are >= 0, so their bits order like integers: two warp-wide integer reductions instead of ten shuffles
+      const unsigned key = i0 != 0x7fffffff ? __float_as_uint(b0) + 1u : 0u;
+      const unsigned top = __reduce_max_sync(0xffffffffu, key);
+      const int wi = (int)__reduce_min_sync(0xffffffffu, key == top ? (unsigned)i0 : 0x7fffffffu);
+      if (lane == r) { mytop = wi; mytopv = __uint_as_float(top - 1u); }
       const bool mine = (wi & 31) == lane && wi == i0;
       if (mine) {
         last_v = b0; last_i = i0;
@@ -435,6 +459,21 @@ topn_rows_kernel(const float* __restrict__ sel, int32_t* __restrict__ out, int64
   }
   int32_t* dst = out + row * n;
   const int nf = n_fixed > 0 ? 3 : 0;
+  bool close = false;
+  if (CHECK) {
+    const int f1 = t < lprime ? 0 : (t - lprime) / lprime, f2 = t / lprime;
+    const int nforced = nf ? 1 + (f1 != 0) + (f2 != 0 && f2 != f1) : 0;
+    const bool free_ = lane < min(n + 1, n_sel) && !(nf && (mytop == 0 || mytop == f1 || mytop == f2));
+    const unsigned mask = __ballot_sync(0xffffffffu, free_);
+    const int rank = __popc(mask & ((1u << lane) - 1u)), take = n - nforced;     // of the picks that no forced block repeats
+    const unsigned at = __ballot_sync(0xffffffffu, free_ && rank == take - 1), nx = __ballot_sync(0xffffffffu, free_ && rank == take);
+    if (at && nx) {      // (the smallest and the next score; where either is missing nothing is cut)
+      const float va = __shfl_sync(0xffffffffu, mytopv, __ffs(at) - 1), vb = __shfl_sync(0xffffffffu, mytopv, __ffs(nx) - 1);
+      const int ida = __shfl_sync(0xffffffffu, mytop, __ffs(at) - 1);
+      const bool seen = (int64_t)ida * lprime + l - 1 <= t;       // a block with no visible key scores exactly 0 either way
+      close = seen && (!(va - vb > score_tolerance(hpg, lse, va) * va) || va < 1e-25f);
+    }
+  }
   if (nf + k_actual <= 32) {
     // lane i holds candidate i: the forced blocks, then the picks in order; a candidate equal to an earlier one is dropped
     int cand = -1;
@@ -469,7 +508,49 @@ topn_rows_kernel(const float* __restrict__ sel, int32_t* __restrict__ out, int64
     if (lane == 0)
       for (int i = 0; i < n; ++i) dst[i] = i < nres ? res[i] : -1;
   }
+  return close;
 }
+
+template <int PER>
+__global__ void __launch_bounds__(128)
+topn_rows_kernel(const float* __restrict__ sel, int32_t* __restrict__ out, int64_t rows, int T, int n_sel, int per_tile, int l,
+                 int d, int nb, int lprime, int n, int n_fixed, int q0) {
+  const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (row < rows) topn_row<PER, false>(sel, out, row, T, n_sel, per_tile, l, d, nb, lprime, n, n_fixed, q0, 0, 0.f);
+}
+
+// the same from approximate scores; rows whose cut they leave open go on their group's list
+template <int PER>
+__global__ void __launch_bounds__(128)
+topn_check_kernel(const float* __restrict__ sel, int32_t* __restrict__ out, int64_t rows, int T, int n_sel, int per_tile, int l, int d, int nb,
+                  int lprime, int n, int n_fixed, int q0, int hpg, const float* __restrict__ big_lse, int* __restrict__ list, int* __restrict__ count) {
+  const int64_t row = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const bool close = topn_row<PER, true>(sel, out, row, T, n_sel, per_tile, l, d, nb, lprime, n, n_fixed, q0, hpg, big_lse[row]);
+  if (close && (threadIdx.x & 31) == 0) list[row / T * T + atomicAdd(&count[row / T], 1)] = (int)(row % T);
+}
+
+template <int PER>
+__global__ void __launch_bounds__(128)
+topn_listed_kernel(const float* __restrict__ sel, int32_t* __restrict__ out, int T, int n_sel, int per_tile, int l, int d, int nb, int lprime,
+                   int n, int n_fixed, int q0, const int* __restrict__ list, const int* __restrict__ count) {
+  const int bg = blockIdx.y, cnt = count[bg];
+  for (int i = blockIdx.x * 4 + (threadIdx.x >> 5); i < cnt; i += gridDim.x * 4)
+    topn_row<PER, false>(sel, out, (int64_t)bg * T + list[(int64_t)bg * T + i], T, n_sel, per_tile, l, d, nb, lprime, n, n_fixed, q0, 0, 0.f);
+}
+
+// listed queries of a group, all its heads, packed to the front of the head's rows
+__global__ void __launch_bounds__(256) pack_rows_kernel(const uint4* __restrict__ q, uint4* __restrict__ out, int H, int G, int T, int vpr,
+                                                        const int* __restrict__ list, const int* __restrict__ count) {
+  const int bg = blockIdx.y, hpg = H / G;
+  const int64_t n = (int64_t)count[bg] * vpr, plane = (int64_t)T * vpr;
+  const int64_t h0 = ((int64_t)(bg / G) * H + (bg % G) * hpg + blockIdx.z) * plane;
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
+    const int r = (int)(i / vpr), c = (int)(i - (int64_t)r * vpr);
+    out[h0 + i] = q[h0 + (int64_t)list[(int64_t)bg * T + r] * vpr + c];
+  }
+}
+
 
 // ------------------------------------------------------------------------------------------------
 // host side
@@ -500,7 +581,7 @@ int split_keys_padded(const float* x, void* hi, void* lo, int64_t rows, int cols
   return check_launch("split_hi_lo");
 }
 
-template <int DK>
+template <int DK, bool LISTED = false>
 static int launch_score_t(const CUtensorMap& tq, const CUtensorMap& thi, const CUtensorMap& tlo, const ScoreParams& p,
                           cudaStream_t st) {
   const int hpg = p.H / p.G;
@@ -509,12 +590,35 @@ static int launch_score_t(const CUtensorMap& tq, const CUtensorMap& thi, const C
   const int bar_off = state_off + state_bytes;
   const int dyn = bar_off + 256 + 1024;
   if (dyn > 227 * 1024) return fail(NSA_ERR_UNSUPPORTED, "score_topn: %d bytes of shared memory needed", dyn);
-  auto kern = score_topn_tc_kernel<DK>;
+  auto kern = score_topn_tc_kernel<DK, LISTED>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
     return fail(NSA_ERR_LAUNCH, "score_topn: cannot reserve shared memory");
   KernelTimer kt("score_topn_tc", st);
   kern<<<dim3((p.T + 127) / 128, p.B * p.G), 384, dyn, st>>>(tq, thi, tlo, p, hpg, state_off, bar_off);
   return check_launch("score_topn_tc");
+}
+
+static int launch_topn_rows(const float* sel, int32_t* out, int B, int G, int T, int n_sel, int s_, int l, int d, int nb, int lprime, int n,
+                            int n_fixed, int q0, cudaStream_t st) {
+  const int64_t rows = (int64_t)B * G * T;
+  KernelTimer kt("score_topn_rows", st);
+  const unsigned grid = (unsigned)((rows + 3) / 4);
+#define NSA_ROWS_CASE(PER_)                                                                                                   \
+  topn_rows_kernel<PER_><<<grid, 128, 0, st>>>(sel, out, rows, T, n_sel, 128 / s_, l, d, nb, lprime, n, n_fixed, q0)
+  if (n_sel <= 8 * 32) {
+    NSA_ROWS_CASE(8);
+  } else if (n_sel <= 16 * 32) {
+    NSA_ROWS_CASE(16);
+  } else if (n_sel <= 32 * 32) {
+    NSA_ROWS_CASE(32);
+  } else {
+    const size_t sm = 4 * (size_t)n_sel * sizeof(float);
+    if (cudaFuncSetAttribute(topn_rows_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
+      return fail(NSA_ERR_LAUNCH, "score_topn: cannot reserve shared memory for the row selection");
+    topn_rows_kernel<0><<<grid, 128, sm, st>>>(sel, out, rows, T, n_sel, 128 / s_, l, d, nb, lprime, n, n_fixed, q0);
+  }
+#undef NSA_ROWS_CASE
+  return check_launch("score_topn_rows");
 }
 
 int score_topn_sm100(const void* q, const float* k_cmp, int32_t* out, int B, int H, int G, int T, int dk, int nbp, int l, int d,
@@ -545,30 +649,145 @@ int score_topn_sm100(const void* q, const float* k_cmp, int32_t* out, int B, int
   p.scale_log2 = scale * 1.4426950408889634f;
   p.timeouts = fa_timeout_counter();
   p.lse2_ext = lse2;
+  p.list = p.count = nullptr;
   int rc;
   if (dk == 192) rc = launch_score_t<192>(tq, thi, tlo, p, st);
   else if (dk == 128) rc = launch_score_t<128>(tq, thi, tlo, p, st);
   else rc = launch_score_t<64>(tq, thi, tlo, p, st);
   if (rc) return rc;
-  const int64_t rows = (int64_t)B * G * T;
-  KernelTimer kt("score_topn_rows", st);
+  return launch_topn_rows(sel, out, B, G, T, n_sel, s_, l, d, nb, lprime, n, n_fixed, q0, st);
+}
+
+// ------------------------------------------------------------------------------------------------
+// Block scores from the sums the compressed attention's forward left (ScorePartials)
+// ------------------------------------------------------------------------------------------------
+constexpr size_t kMaxScorePartials = (size_t)24 << 30;
+// Query tiles (of all groups) from which the forward's sums pay: the re-scored rows are a few tiles per group with the whole sweep of
+// their keys, so with fewer than three waves of tiles they take as long as scoring everything.  Sums + choice + re-scored rows against
+// scoring + choice, 16 heads a group: 0.23 ms against 0.10 at 16 tiles (512 queries on 7000 keys), 0.18 against 0.09 at 128
+// (T = 4096), 0.55 against 0.66 at 512 (T = 16384), 2.0 against 4.0 at 2 x 32768, 4.4 against 8.1 at 65536; the forward itself
+// takes 0.03, 0.5 and 1.1 ms longer at the last three.
+constexpr int kMinPartialTiles = 3 * 148;
+
+static size_t partial_sel_bytes(int B, int H, int T, int nb) {
+  return al256s((size_t)B * H * ((T + 127) / 128) * ((nb + 127) / 128) * 32 * 128 * sizeof(float));
+}
+static size_t partial_aux_bytes(int B, int H, int T, int nb) {
+  return al256s((size_t)B * H * ((T + 127) / 128) * ((nb + 127) / 128) * 128 * sizeof(float2));
+}
+static size_t partial_q_bytes(int B, int H, int T, int dk) { return al256s((size_t)B * H * T * dk * 2); }
+size_t score_partials_bytes(int B, int H, int G, int T, int dk, int nbp, int nb, int l, int d, int lprime, int n) {
+  if (nb <= 0 || nb > nbp || lprime != 4 * d || !score_sm100_supported(H, G, T, dk, nbp, l, d, lprime, n)) return 0;
+  if ((int64_t)B * G > 65535 || (T + 127) / 128 > 65535 || H / G > 64 || n > 28 || (nbp + 3) / 4 > 32 * 32) return 0;
+  if ((int64_t)B * G * ((T + 127) / 128) < kMinPartialTiles) return 0;
+  const size_t parts = partial_sel_bytes(B, H, T, nb) + partial_aux_bytes(B, H, T, nb);
+  if (parts > kMaxScorePartials) return 0;
+  const size_t rows = (size_t)B * G * T;
+  return parts + al256s(rows * (nbp / 4 + 1) * sizeof(float)) + partial_q_bytes(B, H, T, dk) + 2 * al256s(rows * 4) + al256s((size_t)B * G * 4);
+}
+ScorePartials score_partials_at(void* workspace, int B, int H, int T, int nb) {
+  return {(float*)workspace, (float2*)((char*)workspace + partial_sel_bytes(B, H, T, nb)), (nb + 127) / 128};
+}
+
+// A CTA owns 128 rows x 32 blocks (one key tile) of a group and adds the heads in order, a thread per row: every load is a
+// 128-byte line per warp, 32 of them in flight per thread.  HBM-bound: 4 bytes per (head, query, block).
+__global__ void __launch_bounds__(128) score_reduce_kernel(const float* __restrict__ part, const float2* __restrict__ aux, const float* __restrict__ lse2,
+                                                           float* __restrict__ sel, int H, int G, int T, int l, int d, int nb, int n_sel,
+                                                           int tiles, int q0, float* __restrict__ big_lse, int* __restrict__ count) {
+  __shared__ float tr[128][33];
+  const int jt = blockIdx.x, qt = blockIdx.y, bg = blockIdx.z, b = bg / G, hpg = H / G, h0 = (bg % G) * hpg, r = threadIdx.x;
+  const int tl = q0 + qt * 128 + 127, kmax = tl >= l - 1 ? min(nb - 1, (tl - l + 1) / d) : -1, ntiles = max(1, kmax / 128 + 1);
+  if (jt >= ntiles) return;
+  const int t = qt * 128 + r;
+  float acc[32], big = 0.f;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) acc[j] = 0.f;
+  for (int h = h0; h < h0 + hpg; ++h) {
+    const float lse = t < T ? lse2[((int64_t)b * H + h) * T + t] : CUDART_INF_F;
+    if (lse != CUDART_INF_F) big = fabsf(lse) < big ? big : fabsf(lse);
+    if (lse == CUDART_INF_F) {      // the row sees no block: block 0 alone (and nothing was written for it where no row does)
+      if (jt == 0) acc[0] += 1.f;
+      continue;
+    }
+    const int64_t tile = (((int64_t)b * H + h) * gridDim.y + qt) * tiles + jt;
+    const float w = exp2f(aux[tile * 128 + r].x - lse);
+    const float* src = part + tile * 32 * 128 + r;
+    float x[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) x[j] = src[j * 128];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) acc[j] = fmaf(x[j], w, acc[j]);
+    if (jt + 1 < ntiles) {
+      const float2 nx = aux[(tile + 1) * 128 + r];
+      acc[31] = fmaf(nx.y, exp2f(nx.x - lse), acc[31]);
+    }
+  }
+  if (jt == 0 && t < T) big_lse[(int64_t)bg * T + t] = big;
+  if (jt == 0 && qt == 0 && r == 0) count[bg] = 0;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) tr[r][j] = acc[j];
+  __syncthreads();
+  const int j = jt * 32 + (r & 31);
+  for (int k = r >> 5; k < 128; k += 4)
+    if (qt * 128 + k < T && j < n_sel) sel[((int64_t)bg * T + qt * 128 + k) * n_sel + j] = tr[k][r & 31];
+}
+
+int score_topn_from_partials(const ScorePartials& sp, const void* q, const void* k_hi, const void* k_lo, int NB, const KvLayout& kv, const float* lse2,
+                             int32_t* out, int B, int H, int G, int T, int dk, int nbp, int l, int d, int lprime, int nb, int n, int n_fixed,
+                             float scale, int q0, void* workspace, cudaStream_t st) {
+  const int n_sel = (nbp + 3) / 4;
+  const size_t rows = (size_t)B * G * T;
+  char* at = (char*)workspace + partial_sel_bytes(B, H, T, nb) + partial_aux_bytes(B, H, T, nb);
+  float* sel = (float*)at;
+  void* qp = at += al256s(rows * (nbp / 4 + 1) * sizeof(float));
+  float* big_lse = (float*)(at += partial_q_bytes(B, H, T, dk));
+  int* list = (int*)(at += al256s(rows * 4));
+  int* count = (int*)(at + al256s(rows * 4));
+  {
+    KernelTimer kt("score_topn_tc", st);   // the family name of the tensor-core path's block scores, whichever kernel makes them
+    score_reduce_kernel<<<dim3(sp.tiles, (T + 127) / 128, B * G), 128, 0, st>>>(sp.sel, sp.aux, lse2, sel, H, G, T, l, d, nb, n_sel, sp.tiles, q0,
+                                                                                big_lse, count);
+  }
+  if (int rc = check_launch("score_reduce")) return rc;
   const unsigned grid = (unsigned)((rows + 3) / 4);
-#define NSA_ROWS_CASE(PER_)                                                                                                   \
-  topn_rows_kernel<PER_><<<grid, 128, 0, st>>>(sel, out, rows, T, n_sel, 128 / s_, l, d, nb, lprime, n, n_fixed, q0)
-  if (n_sel <= 8 * 32) {
-    NSA_ROWS_CASE(8);
-  } else if (n_sel <= 16 * 32) {
-    NSA_ROWS_CASE(16);
-  } else if (n_sel <= 32 * 32) {
-    NSA_ROWS_CASE(32);
-  } else {
-    const size_t sm = 4 * (size_t)n_sel * sizeof(float);
-    if (cudaFuncSetAttribute(topn_rows_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
-      return fail(NSA_ERR_LAUNCH, "score_topn: cannot reserve shared memory for the row selection");
-    topn_rows_kernel<0><<<grid, 128, sm, st>>>(sel, out, rows, T, n_sel, 128 / s_, l, d, nb, lprime, n, n_fixed, q0);
+  const dim3 lgrid((unsigned)std::min((T + 3) / 4, 592), B * G);
+#define NSA_ROWS_CASE(KERNEL_, GRID_, ...)                                                                                    \
+  if (n_sel <= 8 * 32) KERNEL_<8><<<GRID_, 128, 0, st>>>(__VA_ARGS__);                                                         \
+  else if (n_sel <= 16 * 32) KERNEL_<16><<<GRID_, 128, 0, st>>>(__VA_ARGS__);                                                  \
+  else KERNEL_<32><<<GRID_, 128, 0, st>>>(__VA_ARGS__);
+  {
+    KernelTimer kt("score_topn_rows", st);
+    NSA_ROWS_CASE(topn_check_kernel, grid, sel, out, (int64_t)rows, T, n_sel, 32, l, d, nb, lprime, n, n_fixed, q0, H / G, big_lse, list, count)
+  }
+  if (int rc = check_launch("score_topn_check")) return rc;
+  // the rows whose cut is open: their scores once more, by the scoring kernel
+  pack_rows_kernel<<<dim3((unsigned)std::min(((int64_t)T * dk / 8 + 255) / 256, (int64_t)64), B * G, H / G), 256, 0, st>>>(
+      (const uint4*)q, (uint4*)qp, H, G, T, dk / 8, list, count);
+  if (int rc = check_launch("score_pack_rows")) return rc;
+  CUtensorMap tq, thi, tlo;
+  if (int rc = make_tmap_bf16_3d(&tq, qp, (uint64_t)B * H, T, dk, (uint64_t)T * dk, 128)) return rc;
+  if (int rc = make_tmap_bf16_2d(&thi, k_hi, (uint64_t)B * G * dk, NB, dk, kv.k_ld)) return rc;
+  if (int rc = make_tmap_bf16_2d(&tlo, k_lo, (uint64_t)B * G * dk, NB, dk, kv.k_ld)) return rc;
+  ScoreParams p;
+  p.sel = sel;
+  p.q0 = q0;
+  p.B = B; p.H = H; p.G = G; p.T = T; p.nbp = nbp; p.l = l; p.d = d; p.lprime = lprime; p.nb = nb; p.n_sel = n_sel;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  p.timeouts = fa_timeout_counter();
+  p.lse2_ext = lse2;
+  p.list = list;
+  p.count = count;
+  int rc;
+  if (dk == 192) rc = launch_score_t<192, true>(tq, thi, tlo, p, st);
+  else if (dk == 128) rc = launch_score_t<128, true>(tq, thi, tlo, p, st);
+  else rc = launch_score_t<64, true>(tq, thi, tlo, p, st);
+  if (rc) return rc;
+  {
+    KernelTimer kt("score_topn_rows", st);
+    NSA_ROWS_CASE(topn_listed_kernel, lgrid, sel, out, T, n_sel, 32, l, d, nb, lprime, n, n_fixed, q0, list, count)
   }
 #undef NSA_ROWS_CASE
-  return check_launch("score_topn_rows");
+  return check_launch("score_topn_listed");
 }
 
 }  // namespace nsa

@@ -67,6 +67,8 @@ PROTOTYPES = {
     "nsa_sliding_bwd": (c_int, [_P] * 10 + [_I64P] + [c_int] * 7 + [c_float, c_int, _P, c_int, _P, c_size_t, _P]),
     "nsa_sliding_bwd_noalloc": (c_int, [_P] * 10 + [c_int] * 7 + [c_float, _P]),
     "nsa_cmp_attn_fwd": (c_int, [_P] * 7 + [_I64P] + [c_int] * 7 + [c_float] + [c_int] * 6 + [_P, _P, _P]),
+    "nsa_cmp_attn_topn_workspace_bytes": (c_size_t, [c_int] * 13),
+    "nsa_cmp_attn_topn_fwd": (c_int, [_P] * 11 + [_I64P] + [c_int] * 14 + [c_float, c_int, c_int, _P, c_size_t, _P]),
     "nsa_cmp_attn_exact_supported": (c_int, [c_int] * 8),
     "nsa_split_keys_hi_lo": (c_int, [_P, _P, _P, c_int64, _P]),
     "nsa_cmp_attn_bwd": (c_int, [_P] * 11 + [_I64P] + [c_int] * 7 + [c_float] + [c_int] * 5 + [_P, c_int, _P, c_size_t, _P]),

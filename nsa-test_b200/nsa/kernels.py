@@ -192,21 +192,21 @@ class _BranchesAndMix(torch.autograd.Function):
                 q_pos0=0, token_major=False, k_cmp_f32=None):
         Tq = q.shape[2]
         # ``indices`` None: the blocks are chosen here (Eq. 8-11) from the fp32 compressed keys ``k_cmp_f32``.  Where the
-        # tensor-core kernels apply, the compressed attention runs on the keys as a bf16 pair hi + lo and hands its
-        # log-sum-exp to the scoring kernel, which then sweeps the compressed keys once instead of twice.
-        lse2 = None
+        # tensor-core kernels apply, the compressed attention runs on the keys as a bf16 pair hi + lo and leaves
+        # what the block choice needs.
         # long ragged sequences run on the tensor-core kernels, as in the library's own layer calls
+        n_fixed = config.n_fixed if config.include_fixed_in_selection else 0
         any_length = q.dtype == torch.bfloat16 and q_pos0 == 0 and Tq >= 2048 and k_slc.shape[-1] == Tq and k_win.shape[-1] == Tq
         if indices is None and k_cmp_f32 is not None and blocks is not None and ops.cmp_exact_supported(q, k_cmp, v_cmp, any_length):
             hi, lo = ops.split_keys(k_cmp_f32)
-            o_cmp, Lc, Mc, lse2 = ops.cmp_attn_fwd(q, hi, v_cmp, block_ends, scale, blocks, q_pos0, k_lo=lo, any_length=any_length)
+            o_cmp, Lc, Mc, _, indices = ops.cmp_attn_topn_fwd(q, hi, lo, k_cmp_f32, v_cmp, block_ends, config.l, config.d, config.l_prime,
+                                                              config.n, n_fixed, blocks[2], scale, q_pos0, any_length=any_length)
             k_cmp = hi
         else:
             o_cmp, Lc, Mc = ops.cmp_attn_fwd(q, k_cmp, v_cmp, block_ends, scale, blocks, q_pos0, any_length=any_length)
         if indices is None:
-            n_fixed = config.n_fixed if config.include_fixed_in_selection else 0
             indices = ops.score_topn(q, k_cmp_f32, block_ends, config.l, config.d, config.l_prime, config.n, n_fixed, scale,
-                                     blocks[2], q_pos0, cmp_lse2=lse2, any_length=any_length)
+                                     blocks[2], q_pos0, any_length=any_length)
         ctx.chosen = indices
         idx = _selection_fallback(indices, config.l_prime, q_pos0).to(torch.int32).contiguous()
         lo, hi, pad = _window_slice(q_pos0, Tq, k_win.shape[-1], config.w)

@@ -145,6 +145,32 @@ def cmp_attn_fwd(q, k_cmp, v_cmp, block_ends, scale: float, blocks=None, q_pos0:
     return (o, L, M) if k_lo is None else (o, L, M, lse2)
 
 
+def cmp_attn_topn_fwd(q, k_hi, k_lo, k_cmp, v_cmp, block_ends, l: int, d: int, l_prime: int, n: int, n_fixed: int, nb: int, scale: float,
+                      q_pos0: int = 0, any_length: bool = False):
+    """The exact-key form of ``cmp_attn_fwd`` with the Eq. 8-11 block choice -> (o, L, M, lse2, indices); k_cmp the fp32 keys."""
+    k_hi, k_lo = _tc_keys(q, k_hi, any_length), _tc_keys(q, k_lo, any_length)
+    dev = require_cuda(q, k_hi, k_lo, k_cmp, v_cmp, block_ends)
+    B, H, T, dk = q.shape
+    G, NB, dv = k_hi.shape[1], k_hi.shape[-1], v_cmp.shape[-1]
+    k_cmp, be = k_cmp.float().contiguous(), block_ends.to(torch.int32).contiguous()
+    o, L, M = _stats(q, dv)
+    lse2 = torch.empty(B, H, T, device=dev, dtype=torch.float32)
+    idx = torch.empty(B, G, T, n, device=dev, dtype=torch.int32)
+    flags = _flags(False, any_length=any_length)
+    nbytes = lib.nsa_cmp_attn_topn_workspace_bytes(B, H, G, T, NB, dk, dv, int(l), int(d), int(l_prime), int(n), int(nb), flags)
+    try:
+        ws = torch.empty(nbytes, device=dev, dtype=torch.uint8)
+    except torch.OutOfMemoryError:      # the same choice from the scoring kernel's own, smaller scratch
+        nbytes = lib.nsa_score_topn_workspace_bytes(B, H, G, T, dk, NB, int(l), int(d), int(l_prime), int(n), dtype_code(q), flags)
+        ws = torch.empty(nbytes, device=dev, dtype=torch.uint8)
+    with torch.cuda.device(dev):
+        check(lib.nsa_cmp_attn_topn_fwd(ptr(q), ptr(k_hi), ptr(k_lo), ptr(k_cmp), ptr(v_cmp), ptr(be), ptr(o), ptr(L), ptr(M), ptr(lse2), ptr(idx),
+                                        i64(_fwd_strides(q, k_hi, v_cmp, o, L, M)), B, H, G, T, NB, NB, dk, dv, int(l), int(d), int(l_prime), int(n),
+                                        int(n_fixed), int(nb), float(scale), int(q_pos0), flags, ptr(ws), nbytes, stream_ptr(dev)),
+              "nsa_cmp_attn_topn_fwd")
+    return o, L, M, lse2, idx
+
+
 def cmp_attn_bwd(q, k_cmp, v_cmp, block_ends, o, do, L, M, scale: float, blocks=None, q_pos0: int = 0, row_delta=None,
                  generic: bool = False, recompute: bool = False, any_length: bool = False):
     bl, bd, bn = blocks if blocks is not None else (0, 0, 0)

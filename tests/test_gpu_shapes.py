@@ -260,6 +260,87 @@ def test_generic_kernels_ignore_what_a_row_does_not_see():
             assert torch.isfinite(b).all() and max_abs(a, b) < 1e-5
 
 
+@pytest.mark.parametrize("dk,dv,H,G,T,w", [(64, 64, 8, 2, 128, 150), (192, 128, 16, 1, 640, 512), (128, 128, 4, 2, 896, 30), (192, 128, 6, 1, 256, 600)])
+def test_window_backward_with_heads_split_over_a_cluster(dk, dv, H, G, T, w):
+    """Few key tiles: clusters of 2, 4 and 8 CTAs share a tile's heads (and none where the heads are odd in number).  The row sums
+    dO.O are computed here; the outputs are added into."""
+    from nsa import ops
+    q, k, v, do = _inputs(2, H, G, T, dk, dv, seed=T)
+    qd, kd, vd, dd = (t.to(DEV) for t in (q, k, v, do))
+    scale = dk ** -0.5
+    o, L, M = ops.sliding_fwd(qd, kd, vd, w, scale)
+    qf, kf, vf = (t.float().requires_grad_(True) for t in (q, k, v))
+    want = torch.autograd.grad(O.sliding_window_attention(qf, kf, vf, w, scale), (qf, kf, vf), do.float())
+    dq, dkey, dval = ops.sliding_bwd(qd, kd, vd, o, dd, L, M, w, scale)
+    torch.cuda.synchronize()
+    _no_timeouts()
+    _grad_close(dq, want[0], "dq")
+    _grad_close(dkey, want[1].transpose(-1, -2), "dk")
+    _grad_close(dval, want[2], "dv")
+
+
+@pytest.mark.parametrize("dk,dv,H,G,T,pos", [(64, 64, 4, 2, 4500, 0), (64, 64, 16, 8, 7201, 0), (192, 128, 32, 8, 7200, 0), (128, 128, 16, 8, 7130, 600)])
+def test_block_scores_from_the_forward_match_the_scoring_kernel(dk, dv, H, G, T, pos):
+    """Keys that grow along the sequence move the softmax reference from key tile to key tile; sums cross tile edges.  Ids of the
+    layer (and of a chunk against a cache), whose scores come out of the compressed forward, against the scoring kernel on the
+    same compressed keys: the same blocks but for near-ties at the cut."""
+    import nsa
+    from nsa import incremental as I, ops
+    from nsa.kernels import nsa_layer
+    cfg = nsa.NSAConfig(d_model=64, head_dim_qk=dk, head_dim_v=dv, n_heads=H, n_kv_groups=G, w=128)
+    Tk = pos + T
+    inp = O.make_inputs(1, H, G, Tk, dk, dv, 64, 32, seed=T, block_offset_std=0.5, dtype=torch.bfloat16)
+    grow = torch.linspace(0.2, 6.0, Tk).view(1, 1, 1, Tk)
+    q, k, v = inp["q"].to(DEV, torch.bfloat16), (inp["k"] * grow).to(DEV, torch.bfloat16), inp["v"].to(DEV, torch.bfloat16)
+    phi = tuple(getattr(inp["phi"], n_).to(DEV) * (20.0 if n_ in ("w1", "w2") else 1.0) for n_ in ("pos_embed", "w1", "b1", "w2", "b2"))
+    logits = torch.zeros(1, Tk, 3 * H, device=DEV)
+    qn = q[:, :, pos:].contiguous()
+    if pos == 0:
+        _, info = nsa_layer(q, k, v, logits, phi, cfg, return_info=True)
+        k_cmp, nb = info["k_cmp"], (Tk - 32) // 16 + 1
+    else:
+        cache = I.NSACache(cfg, 1, Tk, DEV, shared_kv=True)
+        cache.append(phi, k, v)
+        _, info = I.nsa_layer_incremental(qn, logits[:, pos:], cache, return_info=True)
+        k_cmp, nb = cache.k_cmp, cache.n_blocks
+    be = torch.full((k_cmp.shape[-1],), 999999, device=DEV, dtype=torch.int32)
+    be[:nb] = torch.arange(nb, device=DEV, dtype=torch.int32) * 16 + 31
+    want = ops.score_topn(qn, k_cmp, be, 32, 16, 64, 16, 3, dk ** -0.5, nb, pos, any_length=True)
+    torch.cuda.synchronize()
+    _no_timeouts()
+    other = (info["indices"].unsqueeze(-1) != want.unsqueeze(-2)).all(-1).sum(-1)
+    assert int(other.max()) <= 1 and (other > 0).float().mean().item() < 0.02, (int(other.max()), (other > 0).float().mean().item())
+    # on one log-sum-exp the two choose the same blocks: rows whose cut rounding could move go to the scoring kernel itself.  So do
+    # rows of equal scores (constant keys): every row of that call.
+    for keys in (k_cmp.float(), torch.ones_like(k_cmp, dtype=torch.float32)):
+        hi, lo = ops.split_keys(keys)
+        val = torch.randn(1, G, keys.shape[-1], dv, device=DEV, dtype=torch.bfloat16)
+        _, _, _, lse2, got = ops.cmp_attn_topn_fwd(qn, hi, lo, keys, val, be, 32, 16, 64, 16, 3, nb, dk ** -0.5, pos, any_length=True)
+        want = ops.score_topn(qn, keys, be, 32, 16, 64, 16, 3, dk ** -0.5, nb, pos, any_length=True, cmp_lse2=lse2)
+        torch.cuda.synchronize()
+        _no_timeouts()
+        assert torch.equal(got.sort(-1).values, want.sort(-1).values)
+
+
+@pytest.mark.parametrize("rows,dv", [((1, 2, 33), 128), ((2, 3, 21), 64), ((1, 1, 1), 128)])
+def test_row_kernels_at_any_row_count(rows, dv):
+    """Rows that do not fill a warp's share: gate/mix backward with its row sums, against the formulas."""
+    from nsa import ops
+    B, H, T = rows
+    gen = torch.Generator().manual_seed(T)
+    oc, os_, ow, do = (torch.randn(B, H, T, dv, generator=gen).bfloat16() for _ in range(4))
+    lg = torch.randn(B, T, 3 * H, generator=gen)
+    out, gates = ops.gate_mix_fwd(lg.to(DEV), oc.to(DEV), os_.to(DEV), ow.to(DEV), "sigmoid")
+    dc, ds, dw, dlog, delta = ops.gate_mix_bwd(gates, oc.to(DEV), os_.to(DEV), ow.to(DEV), do.to(DEV), "sigmoid", want_delta=True)
+    torch.cuda.synchronize()
+    g = torch.sigmoid(lg.view(B, T, H, 3).permute(0, 2, 1, 3))
+    for i, (o, d) in enumerate(((oc, dc), (os_, ds), (ow, dw))):
+        dot = (do.float() * o.float()).sum(-1)
+        assert max_abs(d.float(), (g[..., i:i + 1] * do.float()).bfloat16().float()) <= 2 ** -8 * 4      # one rounding apart
+        assert max_abs(delta[i], g[..., i] * dot) < 1e-4 * max(1.0, dot.abs().max().item())            # fp32 sums of dv terms
+        assert max_abs(dlog.view(B, T, H, 3)[..., i], (dot * g[..., i] * (1 - g[..., i])).transpose(1, 2)) < 1e-4 * max(1.0, dot.abs().max().item())
+
+
 @pytest.mark.parametrize("dk,dv,H,G,T,w,n", [(64, 64, 3, 1, 72, 1, 3), (192, 128, 16, 1, 200, 100, 4), (128, 128, 80, 1, 40, 512, 1),
                                              (64, 64, 4, 4, 1000, 333, 16)])
 def test_mma_kernels_keep_32_bit_probabilities(dk, dv, H, G, T, w, n):
@@ -314,41 +395,3 @@ def test_mma_kernels_keep_32_bit_probabilities(dk, dv, H, G, T, w, n):
     torch.cuda.synchronize()
     for a, b in ((o[:, :, :T - 5], o2[:, :, :T - 5]), (dq[:, :, :T - 5], dq2[:, :, :T - 5]), (dkey[:, :, 8:], dkey2[:, :, 8:]), (dval[:, :, 8:], dval2[:, :, 8:])):
         assert torch.isfinite(b).all() and max_abs(a.float(), b.float()) <= 2 ** -7 * max(1.0, a.float().abs().max().item())
-
-
-@pytest.mark.parametrize("dk,dv,H,G,T,w", [(64, 64, 8, 2, 128, 150), (192, 128, 16, 1, 640, 512), (128, 128, 4, 2, 896, 30), (192, 128, 6, 1, 256, 600)])
-def test_window_backward_with_heads_split_over_a_cluster(dk, dv, H, G, T, w):
-    """Few key tiles: clusters of 2, 4 and 8 CTAs share a tile's heads (and none where the heads are odd in number).  The row sums
-    dO.O are computed here; the outputs are added into."""
-    from nsa import ops
-    q, k, v, do = _inputs(2, H, G, T, dk, dv, seed=T)
-    qd, kd, vd, dd = (t.to(DEV) for t in (q, k, v, do))
-    scale = dk ** -0.5
-    o, L, M = ops.sliding_fwd(qd, kd, vd, w, scale)
-    qf, kf, vf = (t.float().requires_grad_(True) for t in (q, k, v))
-    want = torch.autograd.grad(O.sliding_window_attention(qf, kf, vf, w, scale), (qf, kf, vf), do.float())
-    dq, dkey, dval = ops.sliding_bwd(qd, kd, vd, o, dd, L, M, w, scale)
-    torch.cuda.synchronize()
-    _no_timeouts()
-    _grad_close(dq, want[0], "dq")
-    _grad_close(dkey, want[1].transpose(-1, -2), "dk")
-    _grad_close(dval, want[2], "dv")
-
-
-@pytest.mark.parametrize("rows,dv", [((1, 2, 33), 128), ((2, 3, 21), 64), ((1, 1, 1), 128)])
-def test_row_kernels_at_any_row_count(rows, dv):
-    """Rows that do not fill a warp's share: gate/mix backward with its row sums, against the formulas."""
-    from nsa import ops
-    B, H, T = rows
-    gen = torch.Generator().manual_seed(T)
-    oc, os_, ow, do = (torch.randn(B, H, T, dv, generator=gen).bfloat16() for _ in range(4))
-    lg = torch.randn(B, T, 3 * H, generator=gen)
-    out, gates = ops.gate_mix_fwd(lg.to(DEV), oc.to(DEV), os_.to(DEV), ow.to(DEV), "sigmoid")
-    dc, ds, dw, dlog, delta = ops.gate_mix_bwd(gates, oc.to(DEV), os_.to(DEV), ow.to(DEV), do.to(DEV), "sigmoid", want_delta=True)
-    torch.cuda.synchronize()
-    g = torch.sigmoid(lg.view(B, T, H, 3).permute(0, 2, 1, 3))
-    for i, (o, d) in enumerate(((oc, dc), (os_, ds), (ow, dw))):
-        dot = (do.float() * o.float()).sum(-1)
-        assert max_abs(d.float(), (g[..., i:i + 1] * do.float()).bfloat16().float()) <= 2 ** -8 * 4      # one rounding apart
-        assert max_abs(delta[i], g[..., i] * dot) < 1e-4 * max(1.0, dot.abs().max().item())            # fp32 sums of dv terms
-        assert max_abs(dlog.view(B, T, H, 3)[..., i], (dot * g[..., i] * (1 - g[..., i])).transpose(1, 2)) < 1e-4 * max(1.0, dot.abs().max().item())
