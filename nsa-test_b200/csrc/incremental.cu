@@ -198,7 +198,7 @@ extern "C" NSA_API int nsa_cache_append(const nsa_decode_desc* dp, const void* c
   const char* vs = (const char*)(n_tensors == 2 ? d.v_slc : d.v_src) + (size_t)L.lo * d.dv * es;
   const int64_t vst[4] = {(int64_t)d.G * d.cap * d.dv, (int64_t)d.cap * d.dv, d.dv, 1};
   return cmp_phi_fwd_strided(ks, d.cap, (int64_t)d.dk * d.cap, vs, vst, par[0], par[1], par[2], par[3], par[4], (float*)d.k_cmp + b0,
-                             d.k_cmp_lp ? (char*)d.k_cmp_lp + b0 * es : nullptr, (char*)d.v_cmp + (size_t)b0 * d.dv * es, d.B, d.G, L.T, d.dk,
+                             d.k_cmp_lp ? (char*)d.k_cmp_lp + b0 * es : nullptr, (char*)d.v_cmp + (size_t)b0 * d.dv * es, d.B, d.G, L.T, L.T, d.dk,
                              d.dv, d.l, d.d, d.U, d.nbp, false, dtype, w + L.o_saved, L.saved, w + L.o_ws, L.ws, st);
 }
 

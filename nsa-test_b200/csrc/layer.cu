@@ -13,6 +13,7 @@
 #include "attn_args.cuh"
 #include "common.cuh"
 #include "fa_sm100.cuh"
+#include "phi.cuh"
 
 namespace nsa {
 namespace {
@@ -32,6 +33,8 @@ struct Sizes {
   int ld_cmp;   // row distance of the compressed keys' I/O-type copies: whole 128-key tiles for the tensor-core kernels
   int ld_time;  // row distance of the keys the tensor-core kernels read: T, or the next multiple of 8 (keys are copied then)
   size_t pad_bytes;
+  bool k_pad;   // the compression reads the aligned copy of its keys too: its products then add in the order that whole tiles do
+  int phi_rows; // and form this many rows (T = 5001: 5008; the step takes 3.78 ms, 3.86 from rows off the 16-byte boundaries)
   size_t es, rows, o_bytes, stat_bytes;
 };
 Sizes sizes_of(const nsa_layer_desc& d) {
@@ -45,6 +48,8 @@ Sizes sizes_of(const nsa_layer_desc& d) {
   s.ld_cmp = s.exact ? (s.nbp + 127) / 128 * 128 : s.nbp;
   s.ld_time = d.dtype == NSA_BF16 ? (d.T + 7) / 8 * 8 : d.T;
   s.pad_bytes = s.ld_time == d.T ? 0 : al256((size_t)d.B * d.G * d.dk * s.ld_time * 2);
+  s.k_pad = s.flags && s.pad_bytes && phi_pool_bwd_fused_ok(d.l, d.d);
+  s.phi_rows = s.k_pad ? s.ld_time : d.T;
   s.rows = (size_t)d.B * d.H * d.T;
   s.o_bytes = al256(s.rows * d.dv * s.es);
   s.stat_bytes = al256(s.rows * sizeof(float));
@@ -68,7 +73,7 @@ void ctx_layout(const nsa_layer_desc& d, size_t off[NSA_CTX_PIECES + 1]) {
   put(NSA_CTX_BLOCK_ENDS, (size_t)s.nbp * sizeof(int32_t));
   put(NSA_CTX_K_CMP_LO, BG * d.dk * s.ld_cmp * 2);
   put(NSA_CTX_LSE2_CMP, s.stat_bytes);
-  put(NSA_CTX_PHI_SAVED, s.nb > 0 ? nsa_cmp_phi_saved_bytes(d.B, d.G, d.T, d.l, d.d, d.U) : 256);
+  put(NSA_CTX_PHI_SAVED, s.nb > 0 ? nsa_cmp_phi_saved_bytes(d.B, d.G, s.phi_rows, d.l, d.d, d.U) : 256);
   off[NSA_CTX_PIECES] = o;
 }
 
@@ -149,20 +154,20 @@ size_t stage_scratch_fwd(const nsa_layer_desc& d, const Sizes& s) {
   size_t m = nsa_score_topn_workspace_bytes(d.B, d.H, d.G, d.T, d.dk, s.nbp, d.l, d.d, d.l_prime, d.n, d.dtype, s.flags);
   if (s.exact) m = std::max(m, nsa_cmp_attn_topn_workspace_bytes(d.B, d.H, d.G, d.T, s.nbp, d.dk, d.dv, d.l, d.d, d.l_prime, d.n, s.nb, s.flags));
   m = std::max(m, nsa_slc_fwd_workspace_bytes(d.B, d.H, d.G, d.T, d.T, d.dk, d.dv, d.n, d.l_prime, d.dtype, s.flags));
-  if (s.nb > 0) m = std::max(m, nsa_cmp_phi_workspace_bytes(d.B, d.G, d.T, d.dk, d.dv, d.l, d.d, d.U, s.nbp, d.dtype, 0));
+  if (s.nb > 0) m = std::max(m, nsa_cmp_phi_workspace_bytes(d.B, d.G, s.phi_rows, d.dk, d.dv, d.l, d.d, d.U, s.nbp, d.dtype, 0));
   return al256(m);
 }
 size_t stage_scratch_bwd(const nsa_layer_desc& d, const Sizes& s) {
   size_t m = nsa_attn_bwd_workspace_bytes(d.B, d.H, d.G, d.T, s.nbp, d.dk, d.dv, 1, 0, 0);
   m = std::max(m, nsa_attn_bwd_workspace_bytes(d.B, d.H, d.G, d.T, d.T, d.dk, d.dv, 0, d.window, 0));
   m = std::max(m, nsa_slc_bwd_workspace_bytes(d.B, d.H, d.G, d.T, d.T, d.dk, d.dv, d.n, d.l_prime, d.dtype, s.flags));
-  if (s.nb > 0) m = std::max(m, nsa_cmp_phi_workspace_bytes(d.B, d.G, d.T, d.dk, d.dv, d.l, d.d, d.U, s.nbp, d.dtype, 1));
+  if (s.nb > 0) m = std::max(m, nsa_cmp_phi_workspace_bytes(d.B, d.G, s.phi_rows, d.dk, d.dv, d.l, d.d, d.U, s.nbp, d.dtype, 1));
   return al256(m);
 }
 size_t fixed_scratch_bwd(const nsa_layer_desc& d, const Sizes& s) {
   const size_t BG = (size_t)d.B * d.G;
   return 3 * s.o_bytes + 3 * s.stat_bytes + 2 * al256(s.rows * d.dk * s.es) + al256(BG * s.nbp * d.dk * s.es) +
-         al256(BG * s.nbp * d.dv * s.es) + 2 * s.pad_bytes;
+         al256(BG * s.nbp * d.dv * s.es) + 3 * s.pad_bytes;
 }
 
 }  // namespace
@@ -182,7 +187,7 @@ extern "C" NSA_API size_t nsa_layer_ctx_bytes(const nsa_layer_desc* d, size_t* o
 extern "C" NSA_API size_t nsa_layer_workspace_bytes(const nsa_layer_desc* d, int backward) {
   if (check_desc("layer_workspace_bytes", d)) return 0;
   const Sizes s = sizes_of(*d);
-  return backward ? fixed_scratch_bwd(*d, s) + stage_scratch_bwd(*d, s) + 256 : stage_scratch_fwd(*d, s) + 2 * s.pad_bytes + 256;
+  return backward ? fixed_scratch_bwd(*d, s) + stage_scratch_bwd(*d, s) + 256 : stage_scratch_fwd(*d, s) + 3 * s.pad_bytes + 256;
 }
 
 extern "C" NSA_API int nsa_layer_fwd(const nsa_layer_desc* dp, const void* q, const void* k_slc, const void* v_slc, const void* k_cmp_src,
@@ -209,16 +214,20 @@ extern "C" NSA_API int nsa_layer_fwd(const nsa_layer_desc* dp, const void* q, co
   const size_t BG = (size_t)d.B * d.G;
   const void* k_win_p = pad_keys(d, s, k_win, workspace, st);
   const void* k_slc_p = k_slc == k_win ? k_win_p : pad_keys(d, s, k_slc, (char*)workspace + s.pad_bytes, st);
-  workspace = (char*)workspace + 2 * s.pad_bytes;
-  workspace_bytes -= 2 * s.pad_bytes;
+  const void* k_phi = !s.k_pad ? k_cmp_src : k_cmp_src == k_win ? k_win_p : k_cmp_src == k_slc ? k_slc_p
+                      : pad_keys(d, s, k_cmp_src, (char*)workspace + 2 * s.pad_bytes, st);
+  workspace = (char*)workspace + 3 * s.pad_bytes;
+  workspace_bytes -= 3 * s.pad_bytes;
 
   // 1. block compression (a sequence shorter than one block leaves only the never-visible padding block)
   const bool exact = s.exact;
   block_ends_kernel<<<(s.nbp + 255) / 256, 256, 0, st>>>(be, s.nbp, s.nb, d.l, d.d);
   if (s.nb > 0) {
-    if (int rc = nsa_cmp_phi_fwd(k_cmp_src, v_cmp_src, pos_embed, w1, b1, w2, b2, k_cmp, exact ? nullptr : piece(NSA_CTX_K_CMP_LP), piece(NSA_CTX_V_CMP),
-                                 d.B, d.G, d.T, d.dk, d.dv, d.l, d.d, d.U, s.nbp, d.dtype, piece(NSA_CTX_PHI_SAVED),
-                                 off[NSA_CTX_PHI_SAVED + 1] - off[NSA_CTX_PHI_SAVED], workspace, workspace_bytes, stream))
+    const int64_t vs[4] = {(int64_t)d.G * d.T * d.dv, (int64_t)d.T * d.dv, d.dv, 1};
+    if (int rc = cmp_phi_fwd_strided(k_phi, s.phi_rows, (int64_t)d.dk * s.phi_rows, v_cmp_src, vs, pos_embed, w1, b1, w2, b2, k_cmp,
+                                     exact ? nullptr : piece(NSA_CTX_K_CMP_LP), piece(NSA_CTX_V_CMP), d.B, d.G, d.T, s.phi_rows, d.dk, d.dv, d.l, d.d, d.U, s.nbp,
+                                     true, d.dtype, piece(NSA_CTX_PHI_SAVED), off[NSA_CTX_PHI_SAVED + 1] - off[NSA_CTX_PHI_SAVED], workspace,
+                                     workspace_bytes, st))
       return rc;
   } else {
     cudaMemsetAsync(k_cmp, 0, BG * d.dk * s.nbp * sizeof(float), st);
@@ -298,9 +307,10 @@ extern "C" NSA_API int nsa_layer_bwd(const nsa_layer_desc* dp, const void* q, co
   float* delta = (float*)sc.take(3 * s.stat_bytes);
   void *dq_c = sc.take(s.rows * d.dk * s.es), *dq_w = sc.take(s.rows * d.dk * s.es);
   void *dkc = sc.take(BG * s.nbp * d.dk * s.es), *dvc = sc.take(BG * s.nbp * d.dv * s.es);
-  void *pad0 = sc.take(s.pad_bytes), *pad1 = sc.take(s.pad_bytes);
+  void *pad0 = sc.take(s.pad_bytes), *pad1 = sc.take(s.pad_bytes), *pad2 = sc.take(s.pad_bytes);
   const void* k_win_p = pad_keys(d, s, k_win, pad0, st);
   const void* k_slc_p = k_slc == k_win ? k_win_p : pad_keys(d, s, k_slc, pad1, st);
+  const void* k_phi = !s.k_pad ? k_cmp_src : k_cmp_src == k_win ? k_win_p : k_cmp_src == k_slc ? k_slc_p : pad_keys(d, s, k_cmp_src, pad2, st);
   void* stage = sc.base + sc.used;
   const size_t stage_bytes = workspace_bytes - sc.used;
   // delta holds three vectors of B*H*T floats back to back (the gate/mix backward's layout), not padded ones
@@ -330,9 +340,9 @@ extern "C" NSA_API int nsa_layer_bwd(const nsa_layer_desc* dp, const void* q, co
                            d.T, d.T, d.n, d.l_prime, d.dk, d.dv, d.scale, d.dtype, 0, delta1, dq_c, dq_w, s.flags, stage, stage_bytes, stream))
     return rc;
   if (s.nb > 0)
-    return nsa_cmp_phi_bwd(k_cmp_src, pos_embed, w1, w2, dkc, dvc, piece(NSA_CTX_PHI_SAVED), off[NSA_CTX_PHI_SAVED + 1] - off[NSA_CTX_PHI_SAVED],
-                           dk_cmp_src, dv_cmp_src, dpos, dw1, db1, dw2, db2, d.B, d.G, d.T, d.dk, d.dv, d.l, d.d, d.U, s.nbp, d.dtype,
-                           stage, stage_bytes, stream);
+    return cmp_phi_bwd_ld(k_phi, s.phi_rows, pos_embed, w1, w2, dkc, dvc, piece(NSA_CTX_PHI_SAVED),
+                          off[NSA_CTX_PHI_SAVED + 1] - off[NSA_CTX_PHI_SAVED], dk_cmp_src, dv_cmp_src, dpos, dw1, db1, dw2, db2, d.B, d.G, d.T, s.phi_rows, d.dk,
+                          d.dv, d.l, d.d, d.U, s.nbp, d.dtype, stage, stage_bytes, st);
   // no compression block exists: phi took no part in the forward
   cudaMemsetAsync(dpos, 0, (size_t)d.l * d.l * sizeof(float), st);
   cudaMemsetAsync(dw1, 0, (size_t)d.U * (d.dk + d.l) * sizeof(float), st);

@@ -5,17 +5,22 @@
 
 namespace nsa {
 
-// Scratch and saved sizes as for nsa_cmp_phi_fwd; v_cmp planes and k_cmp rows are nbp apart.
+// Scratch and saved sizes as for nsa_cmp_phi_fwd with `arows` tokens, the rows of W1 K that are formed per plane: T, or where
+// phi_pool_bwd_fused_ok more, the keys' rows being zero there (T no multiple of 8 lets the products choose a slower kernel).  v_cmp planes and k_cmp rows are nbp apart.
 int cmp_phi_fwd_strided(const void* k, int64_t k_ld, int64_t k_plane, const void* v, const int64_t* vs, const float* pos_embed,
                         const float* w1, const float* b1, const float* w2, const float* b2, float* k_cmp, void* k_cmp_lp, void* v_cmp,
-                        int B, int G, int T, int dk, int dv, int l, int d, int U, int nbp, bool pad, int dtype, void* saved,
+                        int B, int G, int T, int arows, int dk, int dv, int l, int d, int U, int nbp, bool pad, int dtype, void* saved,
                         size_t saved_bytes, void* workspace, size_t workspace_bytes, cudaStream_t st);
+int cmp_phi_bwd_ld(const void* k, int64_t k_ld, const float* pos_embed, const float* w1, const float* w2, const void* dk_cmp,
+                   const void* dv_cmp, const void* saved, size_t saved_bytes, void* dk_out, void* dv_out, float* dpos, float* dw1, float* db1,
+                   float* dw2, float* db2, int B, int G, int T, int arows, int dk, int dv, int l, int d, int U, int nbp, int dtype, void* workspace,
+                   size_t workspace_bytes, cudaStream_t st);
 
-// Pooling backward for l = 32, d = 16 in one pass: da in the I/O type, dv_out += dv, dc_part [phi_pool_bwd_parts() * BG, l, U].
+// Pooling backward for l = 32, d = 16 in one pass: da in the I/O type (planes of a and da arows rows apart), dv_out += dv, dc_part [phi_pool_bwd_parts() * BG, l, U].
 bool phi_pool_bwd_fused_ok(int l, int d);
 int phi_pool_bwd_parts(int BG, int T);
 template <typename T>
 int phi_pool_bwd_fused(const float* a, const float* c, const float* dhbar, const float* dv_cmp, T* da, float* dc_part, T* dv_out, int BG, int Tn,
-                       int U, int dv, int nb, int nbp, cudaStream_t st);
+                       int arows, int U, int dv, int nb, int nbp, cudaStream_t st);
 
 }  // namespace nsa

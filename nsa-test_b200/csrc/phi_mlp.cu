@@ -279,12 +279,12 @@ extern "C" NSA_API size_t nsa_cmp_phi_workspace_bytes(int B, int G, int T, int d
 // columns of rows nbp apart and to rows of planes nbp apart.  `pad`: the rest of those rows and planes is cleared.
 int nsa::cmp_phi_fwd_strided(const void* k, int64_t k_ld, int64_t k_plane, const void* v, const int64_t* vs, const float* pos_embed,
                              const float* w1, const float* b1, const float* w2, const float* b2, float* k_cmp, void* k_cmp_lp, void* v_cmp,
-                             int B, int G, int T, int dk, int dv, int l, int d, int U, int nbp, bool pad, int dtype, void* saved,
+                             int B, int G, int T, int arows, int dk, int dv, int l, int d, int U, int nbp, bool pad, int dtype, void* saved,
                              size_t saved_bytes, void* workspace, size_t workspace_bytes, cudaStream_t st) {
   const int nb = (T - l) / d + 1, BG = B * G;
-  const SavedLayout sl = saved_layout(B, G, T, l, d, U);
+  const SavedLayout sl = saved_layout(B, G, arows, l, d, U);
   if (saved_bytes < sl.total) return fail(NSA_ERR_WORKSPACE, "cmp_phi_fwd needs %zu bytes for the backward's inputs, got %zu", sl.total, saved_bytes);
-  const size_t need = nsa_cmp_phi_workspace_bytes(B, G, T, dk, dv, l, d, U, nbp, dtype, 0);
+  const size_t need = nsa_cmp_phi_workspace_bytes(B, G, arows, dk, dv, l, d, U, nbp, dtype, 0);
   if (dtype == NSA_BF16 && (!workspace || workspace_bytes < need))
     return fail(NSA_ERR_WORKSPACE, "cmp_phi_fwd needs %zu workspace bytes, got %zu", need, workspace_bytes);
   cublasHandle_t h;
@@ -303,17 +303,17 @@ int nsa::cmp_phi_fwd_strided(const void* k, int64_t k_ld, int64_t k_plane, const
       split3_kernel<<<blocks_for((int64_t)U * dk), 256, 0, st>>>(w1, U, dk, ld1, hi, mid, lo);
       const __nv_bfloat16* terms[3] = {hi, mid, lo};
       for (int t3 = 0; t3 < 3; ++t3)
-        if (int rc = gemm(h, CUBLAS_OP_T, CUBLAS_OP_T, U, T, dk, terms[t3], CUDA_R_16BF, dk, 0, k, CUDA_R_16BF, (int)k_ld, k_plane,
-                          t3 ? 1.f : 0.f, a, CUDA_R_32F, U, (long long)T * U, BG, "cmp_phi_fwd (K W1k^T)"))
+        if (int rc = gemm(h, CUBLAS_OP_T, CUBLAS_OP_T, U, arows, dk, terms[t3], CUDA_R_16BF, dk, 0, k, CUDA_R_16BF, (int)k_ld, k_plane,
+                          t3 ? 1.f : 0.f, a, CUDA_R_32F, U, (long long)arows * U, BG, "cmp_phi_fwd (K W1k^T)"))
           return rc;
     } else {
-      if (int rc = gemm(h, CUBLAS_OP_T, CUBLAS_OP_T, U, T, dk, w1, CUDA_R_32F, ld1, 0, k, CUDA_R_32F, (int)k_ld, k_plane, 0.f, a,
-                        CUDA_R_32F, U, (long long)T * U, BG, "cmp_phi_fwd (K W1k^T)"))
+      if (int rc = gemm(h, CUBLAS_OP_T, CUBLAS_OP_T, U, arows, dk, w1, CUDA_R_32F, ld1, 0, k, CUDA_R_32F, (int)k_ld, k_plane, 0.f, a,
+                        CUDA_R_32F, U, (long long)arows * U, BG, "cmp_phi_fwd (K W1k^T)"))
         return rc;
     }
   }
   if (int rc = check_launch("cmp_phi_fwd")) return rc;
-  if (int rc = nsa_phi_pool_fwd(a, c, v, vs, hbar, v_cmp, B, G, T, U, dv, l, d, nb, nbp, dtype, st)) return rc;
+  if (int rc = nsa_phi_pool_fwd(a, c, v, vs, hbar, v_cmp, B, G, arows, U, dv, l, d, nb, nbp, dtype, st)) return rc;
   {
     KernelTimer kt("phi_mlp_fwd", st);
     // pooled v_cmp rows beyond nb are the caller's zero padding: cleared here so that the caller need not
@@ -345,7 +345,7 @@ extern "C" NSA_API int nsa_cmp_phi_fwd(const void* k, const void* v, const float
   const int nb = (T - l) / d + 1;
   NSA_REQUIRE(nbp >= nb, "cmp_phi_fwd: nbp = %d holds fewer than the %d blocks of the sequence", nbp, nb);
   const int64_t vs[4] = {(int64_t)G * T * dv, (int64_t)T * dv, dv, 1};
-  return cmp_phi_fwd_strided(k, T, (int64_t)dk * T, v, vs, pos_embed, w1, b1, w2, b2, k_cmp, k_cmp_lp, v_cmp, B, G, T, dk, dv, l, d, U,
+  return cmp_phi_fwd_strided(k, T, (int64_t)dk * T, v, vs, pos_embed, w1, b1, w2, b2, k_cmp, k_cmp_lp, v_cmp, B, G, T, T, dk, dv, l, d, U,
                              nbp, true, dtype, saved, saved_bytes, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
@@ -354,18 +354,26 @@ extern "C" NSA_API int nsa_cmp_phi_bwd(const void* k, const float* pos_embed, co
                                        float* dpos, float* dw1, float* db1, float* dw2, float* db2, int B, int G, int T, int dk,
                                        int dv, int l, int d, int U, int nbp, int dtype, void* workspace, size_t workspace_bytes,
                                        void* stream) {
+  return cmp_phi_bwd_ld(k, T, pos_embed, w1, w2, dk_cmp, dv_cmp, saved, saved_bytes, dk_out, dv_out, dpos, dw1, db1, dw2, db2, B, G, T, T, dk, dv,
+                        l, d, U, nbp, dtype, workspace, workspace_bytes, (cudaStream_t)stream);
+}
+
+// keys whose rows lie k_ld elements apart
+int nsa::cmp_phi_bwd_ld(const void* k, int64_t k_ld, const float* pos_embed, const float* w1, const float* w2, const void* dk_cmp,
+                        const void* dv_cmp, const void* saved, size_t saved_bytes, void* dk_out, void* dv_out, float* dpos, float* dw1,
+                        float* db1, float* dw2, float* db2, int B, int G, int T, int arows, int dk, int dv, int l, int d, int U, int nbp, int dtype,
+                        void* workspace, size_t workspace_bytes, cudaStream_t st) {
   NSA_REQUIRE(k && pos_embed && w1 && w2 && dk_cmp && dv_cmp && saved && dk_out && dv_out && dpos && dw1 && db1 && dw2 && db2,
               "cmp_phi_bwd: null pointer");
   NSA_REQUIRE(B > 0 && G > 0 && dk > 0 && dv > 0 && U > 0 && l > 0 && d > 0 && T >= l, "cmp_phi_bwd: bad sizes");
   NSA_REQUIRE(dtype == NSA_F32 || dtype == NSA_BF16, "cmp_phi_bwd: unsupported dtype %d", dtype);
   const int nb = (T - l) / d + 1, BG = B * G;
   NSA_REQUIRE(nbp >= nb, "cmp_phi_bwd: nbp = %d holds fewer than the %d blocks of the sequence", nbp, nb);
-  const SavedLayout sl = saved_layout(B, G, T, l, d, U);
+  const SavedLayout sl = saved_layout(B, G, arows, l, d, U);
   if (saved_bytes < sl.total) return fail(NSA_ERR_WORKSPACE, "cmp_phi_bwd: the forward's saved buffer has %zu bytes, got %zu", sl.total, saved_bytes);
-  const BwdLayout wl = bwd_layout(B, G, T, dk, dv, l, d, U, nbp, dtype);
+  const BwdLayout wl = bwd_layout(B, G, arows, dk, dv, l, d, U, nbp, dtype);
   if (!workspace || workspace_bytes < wl.total)
     return fail(NSA_ERR_WORKSPACE, "cmp_phi_bwd needs %zu workspace bytes, got %zu", wl.total, workspace_bytes);
-  cudaStream_t st = (cudaStream_t)stream;
   cublasHandle_t h;
   if (int rc = blas_handle(&h, st)) return rc;
   const float* a = (const float*)((const char*)saved + sl.o_a);
@@ -399,10 +407,10 @@ extern "C" NSA_API int nsa_cmp_phi_bwd(const void* k, const float* pos_embed, co
   if (int rc = check_launch("cmp_phi_bwd")) return rc;
   const bool fused = phi_pool_bwd_fused_ok(l, d);
   int rc_pool;
-  if (!fused) rc_pool = nsa_phi_pool_bwd(a, c, dhbar, dvc, da, dcpart, dvt, B, G, T, U, dv, l, d, nb, nbp, stream);
+  if (!fused) rc_pool = nsa_phi_pool_bwd(a, c, dhbar, dvc, da, dcpart, dvt, B, G, T, U, dv, l, d, nb, nbp, st);
   else if (dtype == NSA_BF16)
-    rc_pool = phi_pool_bwd_fused(a, c, dhbar, dvc, (__nv_bfloat16*)(w + wl.o_dalp), dcpart, (__nv_bfloat16*)dv_out, BG, T, U, dv, nb, nbp, st);
-  else rc_pool = phi_pool_bwd_fused(a, c, dhbar, dvc, (float*)(w + wl.o_dalp), dcpart, (float*)dv_out, BG, T, U, dv, nb, nbp, st);
+    rc_pool = phi_pool_bwd_fused(a, c, dhbar, dvc, (__nv_bfloat16*)(w + wl.o_dalp), dcpart, (__nv_bfloat16*)dv_out, BG, T, arows, U, dv, nb, nbp, st);
+  else rc_pool = phi_pool_bwd_fused(a, c, dhbar, dvc, (float*)(w + wl.o_dalp), dcpart, (float*)dv_out, BG, T, arows, U, dv, nb, nbp, st);
   if (rc_pool) return rc_pool;
   {
     KernelTimer kt("phi_mlp_bwd", st);
@@ -419,16 +427,16 @@ extern "C" NSA_API int nsa_cmp_phi_bwd(const void* k, const float* pos_embed, co
       da_op = dalp; w1k_op = w1k; ot = CUDA_R_16BF; ldw = dk;
     }
     // dK[bg] (T x dk, row-major) += da[bg] W1k; column-major: C(dk x T) = W1k (dk x U, ld) da (U x T)
-    if (int rc = gemm(h, CUBLAS_OP_N, CUBLAS_OP_N, dk, T, U, w1k_op, ot, ldw, 0, da_op, ot, U, (long long)T * U, 1.f, dk_out, ot, dk,
+    if (int rc = gemm(h, CUBLAS_OP_N, CUBLAS_OP_N, dk, T, U, w1k_op, ot, ldw, 0, da_op, ot, U, (long long)arows * U, 1.f, dk_out, ot, dk,
                       (long long)T * dk, BG, "cmp_phi_bwd (dK)"))
       return rc;
     // dW1[:, :dk] (U x dk inside rows of dk + l, row-major) = sum_bg da[bg]^T K[bg]^T; column-major: C(dk x U, ld dk+l) =
-    // op_T(K[bg] (T x dk, ld T)) op_T(da[bg] (U x T)), accumulated over bg in order
+    // op_T(K[bg] (T x dk, ld k_ld)) op_T(da[bg] (U x T)), accumulated over bg in order
     for (int bg = 0; bg < BG; ++bg) {
       const size_t es = dtype == NSA_BF16 ? 2 : 4;
-      const void* kb = (const char*)k + (size_t)bg * dk * T * es;
-      const void* dab = (const char*)da_op + (size_t)bg * T * U * es;
-      if (int rc = gemm(h, CUBLAS_OP_T, CUBLAS_OP_T, dk, U, T, kb, ot, T, 0, dab, ot, U, 0, bg ? 1.f : 0.f, dw1, CUDA_R_32F, ld1, 0, 1,
+      const void* kb = (const char*)k + (size_t)bg * dk * k_ld * es;
+      const void* dab = (const char*)da_op + (size_t)bg * arows * U * es;
+      if (int rc = gemm(h, CUBLAS_OP_T, CUBLAS_OP_T, dk, U, T, kb, ot, (int)k_ld, 0, dab, ot, U, 0, bg ? 1.f : 0.f, dw1, CUDA_R_32F, ld1, 0, 1,
                         "cmp_phi_bwd (dW1k)"))
         return rc;
     }

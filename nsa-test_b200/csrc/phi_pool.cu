@@ -141,7 +141,7 @@ template <typename T>
 __global__ void __launch_bounds__(512) phi_pool_bwd_seg_kernel(const float* __restrict__ a, const float* __restrict__ c,
                                                                const float* __restrict__ dhbar, const float* __restrict__ dv_cmp,
                                                                T* __restrict__ da, float* __restrict__ dc_part, T* __restrict__ dv_out, int T_,
-                                                               int U, int dvd, int nb, int nbp, int cs) {
+                                                               int arows, int U, int dvd, int nb, int nbp, int cs) {
   const int nseg = (T_ + kSeg - 1) / kSeg, s0 = blockIdx.x * cs, s1 = min(nseg, s0 + cs), bg = blockIdx.y;
   const float inv = 1.f / (2 * kSeg);
   const int nv = seg_value_threads(dvd), nu = blockDim.x - nv;
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(512) phi_pool_bwd_seg_kernel(const float* __re
     const float* dh = dhbar + (int64_t)bg * nb * U + u;
     float before = s0 > 0 && s0 - 1 < nb ? dh[(int64_t)(s0 - 1) * U] : 0.f;
     for (int s = s0; s < s1; ++s) {
-      const int64_t at = ((int64_t)bg * T_ + (int64_t)s * kSeg) * U + u;
+      const int64_t at = ((int64_t)bg * arows + (int64_t)s * kSeg) * U + u;
       const float here = s < nb ? dh[(int64_t)s * U] : 0.f;
 #pragma unroll
       for (int j = 0; j < kSeg; ++j) x[j] = s * kSeg + j < T_ ? a[at + (int64_t)j * U] : 0.f;
@@ -199,16 +199,16 @@ int phi_pool_bwd_parts(int BG, int T) {
 }
 template <typename T>
 int phi_pool_bwd_fused(const float* a, const float* c, const float* dhbar, const float* dv_cmp, T* da, float* dc_part, T* dv_out, int BG, int Tn,
-                       int U, int dv, int nb, int nbp, cudaStream_t st) {
+                       int arows, int U, int dv, int nb, int nbp, cudaStream_t st) {
   KernelTimer kt("phi_pool_bwd", st);
-  phi_pool_bwd_seg_kernel<T><<<dim3(phi_pool_bwd_parts(BG, Tn), BG), seg_threads(U, dv), 0, st>>>(a, c, dhbar, dv_cmp, da, dc_part, dv_out, Tn, U,
+  phi_pool_bwd_seg_kernel<T><<<dim3(phi_pool_bwd_parts(BG, Tn), BG), seg_threads(U, dv), 0, st>>>(a, c, dhbar, dv_cmp, da, dc_part, dv_out, Tn, arows, U,
                                                                                                   dv, nb, nbp, bwd_seg_chunk(BG, Tn));
   return check_launch("phi_pool_bwd");
 }
-template int phi_pool_bwd_fused<float>(const float*, const float*, const float*, const float*, float*, float*, float*, int, int, int, int, int, int,
+template int phi_pool_bwd_fused<float>(const float*, const float*, const float*, const float*, float*, float*, float*, int, int, int, int, int, int, int,
                                        cudaStream_t);
 template int phi_pool_bwd_fused<__nv_bfloat16>(const float*, const float*, const float*, const float*, __nv_bfloat16*, float*, __nv_bfloat16*, int,
-                                               int, int, int, int, int, cudaStream_t);
+                                               int, int, int, int, int, int, cudaStream_t);
 
 }  // namespace nsa
 
