@@ -386,10 +386,11 @@ NSA_API int nsa_layer_bwd(const nsa_layer_desc* desc, const void* q, const void*
  * A handful of newest tokens against a key/value cache (decode), bf16, forward only: B*G*Tn <= 64 rows.  The caches are
  * k_* [B,G,dk,cap], v_* [B,G,cap,dv], compressed keys fp32 [B,G,dk,nbp] (k_cmp_lp: their bf16 copy) and values
  * [B,G,nbp,dv], block_ends int32 [nbp]; the new tokens sit at positions pos + [0,Tn) and nb compressed blocks are valid
- * once they are in.  project == 0: q [B,H,Tn,dk] (strides sq of b, h, t) and gate_logits [B,Tn,3H] are given and the
+ * once they are in; q [B,H,Tn,dk] has strides sq (b, h, t).  project == 0: gate_logits [B,Tn,3H] are given and the
  * tokens are in the caches.  project != 0 (B*Tn <= 8): x [B,Tn,d_model] (strides sx) goes through the projections w (rows of
- * q, k_slc, v_slc, k_src, v_src, k_win, v_win; biases may be NULL) into q and the caches, through phi for the last nb_new of
- * the nb blocks, and through the gate MLP; all parameters bf16.  out [B,Tn,H,dv]; indices int32 [B,G,Tn,n], gates fp32
+ * k_slc, v_slc, v_src, k_win, v_win; biases may be NULL) into the caches, k_new [B,G,dk,Tn] (strides sk) into k_src, both
+ * through phi for the last nb_new of the nb blocks, and x through the gate MLP; all parameters bf16.  (q and k_new decide which
+ * blocks are chosen: the caller forms them with the products of its other paths, so that all choose alike.)  out [B,Tn,H,dv]; indices int32 [B,G,Tn,n], gates fp32
  * [B,H,Tn,3] and o_* [B,H,Tn,dv] are written when given.  nsa_decode_supported says whether the sizes are in range. */
 typedef struct nsa_decode_desc {
   int B, Tn, H, G, dk, dv, l, d, l_prime, n, n_fixed, window, gate_mode;
@@ -406,9 +407,11 @@ typedef struct nsa_decode_desc {
   void *o_cmp, *o_slc, *o_win;
   const void* x;
   int64_t sx[2];          /* strides of x's batch and token */
-  const void *w[7], *bias[7];
+  const void *w[5], *bias[5];
   const void *gate_w1, *gate_b1, *gate_w2, *gate_b2;
   const void *pos_embed, *phi_w1, *phi_b1, *phi_w2, *phi_b2;
+  const void* k_new;
+  int64_t sk[4];          /* strides of k_new's batch, group, channel and token */
 } nsa_decode_desc;
 NSA_API int nsa_decode_supported(const nsa_decode_desc* desc);
 NSA_API size_t nsa_decode_workspace_bytes(const nsa_decode_desc* desc);

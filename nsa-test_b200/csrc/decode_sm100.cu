@@ -2,24 +2,33 @@
 // block choice, the three attention branches and the gate mix, for up to 64 (sequence, group, token) rows.
 //
 // The tile kernels pad such a call to 128 query rows and need an inverse index, padded copies and one launch per piece:
-// 45 launches and 760 us per token at B=1, 2K cached; 80 launches and 1400 us at B=8, 32K (91 and 138 us here).  What the work cannot do without
-// is reading the weights once (131 MB for the 64-head configuration, 20 us) and the visible keys and values once, so here
-// the keys of a row are cut into 64-key chunks, one CTA each, that serve all heads of the group, and everything between
-// two grid-wide dependencies is one launch:
+// 45 launches and 760 us per token at B=1, 2K cached; 80 launches and 1400 us at B=8, 32K.  What the work
+// cannot do without is reading the weights once (131 MB for the 64-head configuration, 20 us) and the visible keys and values
+// once, so here the keys of a row are cut into 64-key chunks, one CTA each, that serve all heads of the group, and everything
+// between two grid-wide dependencies is one launch:
 //   1 project     weights x tokens on mma.sync (8 tokens are one n tile; the weights stream through once), written straight
-//                 into q and the caches; the gate MLP's hidden layer is one more row range
-//   2 phi         only when the tokens complete compression blocks: fp32 sums over the bf16 weights
+//                 into the caches; the gate MLP's hidden layer is one more row range
+//   2 phi         only when the tokens complete compression blocks: the block compression of every other path
 //   3 chunks      compressed and sliding-window chunks + the gate logits
 //   4 top-n       Eq. 8-11 from the fp32 logits the chunks left
 //   5 chunks      the selected blocks
 //   6 combine     merge of the chunk partials, gates, mix
-// Launches overlap their ramp-up by programmatic dependent launch.  Keys of the compressed blocks stay fp32 and their
-// products run on the FMA pipe (they rank the blocks); bf16 keys and P V run on mma.sync, with P as bf16 hi + lo, so the
-// probabilities keep 16 mantissa bits.  (tcgen05 tiles have 64 rows at least; a group has at most 16 heads.)
+// Launches overlap their ramp-up by programmatic dependent launch.
+//
+// The block choice is a discrete function of rounded sums: q and the compression's keys that round differently, or sums in
+// another order, let near-ties fall the other way (in 2 of 384 rows at 32000 cached tokens).  So all that the choice reads is
+// made as on the other paths: q and the new compression keys come from the caller, who forms them with the products that the tile kernels'
+// callers use; logits are one fma chain over the head dimension and the Eq. 8-10 sums run in the order of score_topn.cu.  The
+// chosen blocks are the same bit for bit.
+//
+// Keys of the compressed blocks stay fp32 and their products run on the FMA pipe (they rank the blocks); bf16 keys and P V run
+// on mma.sync, with P as bf16 hi + lo, so the probabilities keep 16 mantissa bits (the tile kernels: 8).  (tcgen05 tiles have 64
+// rows at least; a group has at most 16 heads.)
 #include <algorithm>
 
 #include "common.cuh"
 #include "fa_sm100.cuh"
+#include "phi.cuh"
 
 namespace nsa {
 namespace {
@@ -76,17 +85,17 @@ __device__ __forceinline__ uint4 ld_stream(const void* p) {
 // Row ranges ("segments") of stacked weight matrices, 16 rows a CTA; the four warps split d_model.  The weights stream from
 // HBM once: 16-byte loads, 64 consecutive k of 16 rows per warp and step.  The 32-k groups are multiplied in permuted order
 // (both operands alike), so that a thread's 16 bytes are two mma fragments.
-enum { kSegQ = 0, kSegK, kSegV, kSegGate };
+enum { kSegK = 0, kSegV, kSegGate, kSegCopy };      // kSegCopy: no product, k_new goes into its cache
 struct ProjSeg {
   const __nv_bfloat16 *w, *bias;
   __nv_bfloat16* dst;
   int tile0, D, kind;    // first tile of the segment, head dim (width for the gate), layout
 };
 struct ProjArgs {
-  ProjSeg seg[8];
-  int nseg, R, Tn, K, H, G, pos;
-  int64_t cap, sxb, sxt;
-  const __nv_bfloat16* x;
+  ProjSeg seg[7];
+  int nseg, R, Tn, K, G, pos;
+  int64_t cap, sxb, sxt, sk[4];
+  const __nv_bfloat16 *x, *k_new;
 };
 __global__ void __launch_bounds__(kProjThreads) decode_project_kernel(const __grid_constant__ ProjArgs p) {
   __shared__ float red[4][16][9];
@@ -97,6 +106,11 @@ __global__ void __launch_bounds__(kProjThreads) decode_project_kernel(const __gr
   while (si + 1 < p.nseg && (int)blockIdx.x >= p.seg[si + 1].tile0) ++si;
   const ProjSeg& sg = p.seg[si];
   const int row0 = ((int)blockIdx.x - sg.tile0) * 16;
+  const int n = threadIdx.x >> 4, r = threadIdx.x & 15, row = row0 + r, b = n / p.Tn, t = n % p.Tn, hd = row / sg.D, e = row % sg.D;
+  if (sg.kind == kSegCopy) {
+    if (n < p.R) sg.dst[(((int64_t)b * p.G + hd) * sg.D + e) * p.cap + p.pos + t] = p.k_new[b * p.sk[0] + hd * p.sk[1] + e * p.sk[2] + t * p.sk[3]];
+    return;
+  }
   const __nv_bfloat16* wa = sg.w + (int64_t)(row0 + g) * p.K + qd * 8;
   const __nv_bfloat16* wb = wa + (int64_t)8 * p.K;
   const bool have = g < p.R;
@@ -129,93 +143,13 @@ __global__ void __launch_bounds__(kProjThreads) decode_project_kernel(const __gr
   red[warp][g][qd * 2] = c[0];     red[warp][g][qd * 2 + 1] = c[1];
   red[warp][g + 8][qd * 2] = c[2]; red[warp][g + 8][qd * 2 + 1] = c[3];
   __syncthreads();
-  const int n = threadIdx.x >> 4, r = threadIdx.x & 15, row = row0 + r;
   if (n >= p.R) return;
   const float y = (red[0][r][n] + red[1][r][n]) + (red[2][r][n] + red[3][r][n]);
   __nv_bfloat16 o = __float2bfloat16_rn(y);
   if (sg.bias) o = __float2bfloat16_rn(__bfloat162float(o) + __bfloat162float(sg.bias[row]));
-  const int b = n / p.Tn, t = n % p.Tn, hd = row / sg.D, e = row % sg.D;
-  if (sg.kind == kSegQ) sg.dst[(((int64_t)b * p.H + hd) * p.Tn + t) * sg.D + e] = o;
-  else if (sg.kind == kSegK) sg.dst[(((int64_t)b * p.G + hd) * sg.D + e) * p.cap + p.pos + t] = o;
+  if (sg.kind == kSegK) sg.dst[(((int64_t)b * p.G + hd) * sg.D + e) * p.cap + p.pos + t] = o;
   else if (sg.kind == kSegV) sg.dst[(((int64_t)b * p.G + hd) * p.cap + p.pos + t) * sg.D + e] = o;
   else sg.dst[(int64_t)n * sg.D + row] = __bfloat162float(o) > 0.f ? o : __float2bfloat16_rn(0.f);
-}
-
-// ------------------------------------------------------------------------------------------------ block compression
-// hbar[u] = mean_j relu(b1[u] + W1[u] . [k_{id+j} || pos_j]) of one new block: 64 hidden units a CTA, four threads a unit
-// with 8 offsets each; the 32 inputs sit in shared memory as fp32, offsets contiguous.
-struct PhiArgs {
-  const __nv_bfloat16 *k, *v, *pos, *w1, *b1, *w2, *b2;
-  float *hbar, *k_cmp;
-  __nv_bfloat16 *k_lp, *v_cmp;
-  int32_t* block_ends;
-  int64_t cap, nbp;
-  int dk, dv, U, l, d, blk0;
-};
-__global__ void __launch_bounds__(256) decode_phi_hidden_kernel(const __grid_constant__ PhiArgs p) {
-  extern __shared__ __align__(16) float z[];     // [dk + l][32]
-  pdl_wait();
-  pdl_launch();
-  const int bg = blockIdx.z, blk = p.blk0 + blockIdx.y, W = p.dk + p.l;
-  const __nv_bfloat16* k = p.k + (int64_t)bg * p.dk * p.cap + (int64_t)blk * p.d;
-  for (int i = threadIdx.x; i < W * 32; i += 256) {
-    const int cidx = i >> 5, j = i & 31;
-    z[i] = j >= p.l ? 0.f : __bfloat162float(cidx < p.dk ? k[(int64_t)cidx * p.cap + j] : p.pos[j * p.l + cidx - p.dk]);
-  }
-  __syncthreads();
-  const int u = blockIdx.x * 64 + (threadIdx.x >> 2), jg = threadIdx.x & 3;
-  float sum = 0.f;
-  if (u < p.U) {
-    float acc[8];
-    const float b = p.b1 ? __bfloat162float(p.b1[u]) : 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = b;
-    const __nv_bfloat16* w = p.w1 + (int64_t)u * W;
-    for (int c0 = 0; c0 < W; c0 += 8) {
-      const uint4 wv = *reinterpret_cast<const uint4*>(w + c0);
-      const __nv_bfloat162* w2 = reinterpret_cast<const __nv_bfloat162*>(&wv);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float wf = (e & 1) ? __high2float(w2[e >> 1]) : __low2float(w2[e >> 1]);
-        const float4 z0 = *reinterpret_cast<const float4*>(z + (c0 + e) * 32 + jg * 8);
-        const float4 z1 = *reinterpret_cast<const float4*>(z + (c0 + e) * 32 + jg * 8 + 4);
-        acc[0] = fmaf(wf, z0.x, acc[0]); acc[1] = fmaf(wf, z0.y, acc[1]); acc[2] = fmaf(wf, z0.z, acc[2]); acc[3] = fmaf(wf, z0.w, acc[3]);
-        acc[4] = fmaf(wf, z1.x, acc[4]); acc[5] = fmaf(wf, z1.y, acc[5]); acc[6] = fmaf(wf, z1.z, acc[6]); acc[7] = fmaf(wf, z1.w, acc[7]);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (jg * 8 + i < p.l) sum += fmaxf(acc[i], 0.f);
-  }
-  sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-  sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-  if (jg == 0 && u < p.U) p.hbar[((int64_t)bg * gridDim.y + blockIdx.y) * p.U + u] = sum / (float)p.l;
-}
-__global__ void __launch_bounds__(256) decode_phi_out_kernel(const __grid_constant__ PhiArgs p) {
-  pdl_wait();
-  pdl_launch();
-  const int bg = blockIdx.z, blk = p.blk0 + blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const float* hb = p.hbar + ((int64_t)bg * gridDim.y + blockIdx.y) * p.U;
-  for (int c = blockIdx.x * 8 + warp; c < p.dk; c += gridDim.x * 8) {
-    float s = 0.f;
-    for (int u = lane; u < p.U; u += 32) s = fmaf(__bfloat162float(p.w2[(int64_t)c * p.U + u]), hb[u], s);
-    s = warp_sum(s);
-    if (lane == 0) {
-      if (p.b2) s += __bfloat162float(p.b2[c]);
-      const int64_t o = ((int64_t)bg * p.dk + c) * p.nbp + blk;
-      p.k_cmp[o] = s;
-      p.k_lp[o] = __float2bfloat16_rn(s);
-    }
-  }
-  if (blockIdx.x == 0) {
-    for (int c = threadIdx.x; c < p.dv; c += 256) {
-      float s = 0.f;
-#pragma unroll 8
-      for (int j = 0; j < p.l; ++j) s += __bfloat162float(p.v[((int64_t)bg * p.cap + (int64_t)blk * p.d + j) * p.dv + c]);
-      p.v_cmp[((int64_t)bg * p.nbp + blk) * p.dv + c] = __float2bfloat16_rn(s / (float)p.l);
-    }
-    if (bg == 0 && threadIdx.x == 0) p.block_ends[blk] = blk * p.d + p.l - 1;
-  }
 }
 
 // ------------------------------------------------------------------------------------------------ attention chunks
@@ -240,12 +174,12 @@ struct DecArgs {
   float* gates;              // optional [B,H,Tn,3]
 };
 
-template <int DK, int DV>
+template <int DK, int DV, bool WITH_CMP>
 struct DecSmem {
   static constexpr int kQ = 16 * (DK + 8) * 2;       // bf16 queries (rows 16 bytes off a bank period)
-  static constexpr int kK = DK * 72 * 2;             // bf16 key tile [DK][64]; compressed: fp32 queries [DK][16] + partial sums
-  static constexpr int kC = DK * 16 * 4 + 4 * 16 * 64 * 4;
-  static constexpr int kKC = kK > kC ? kK : kC;
+  static constexpr int kK = DK * 72 * 2;             // bf16 key tile [DK][64]
+  static constexpr int kC = DK * 16 * 4 + DK * 64 * 4;   // compressed: fp32 queries [DK][16], fp32 key tile [DK][64]
+  static constexpr int kKC = WITH_CMP ? kC : kK;
   static constexpr int kV = 64 * (DV + 8) * 2;
   static constexpr int kS = 16 * 66 * 4;
   static constexpr int kP = 2 * 16 * 72 * 2;
@@ -253,11 +187,12 @@ struct DecSmem {
 };
 
 // One chunk of 64 keys [key0, key0 + 64) for the heads of a group: S, its softmax over the chunk, P V.  Keys klo <= key < khi
-// count.  CMP: fp32 keys [DK][ld], whose logits are also kept for the block choice.
-template <int DK, int DV, bool CMP>
+// count.  CMP: fp32 keys [DK][ld], whose logits are also kept for the block choice: a thread owns a key and four heads and
+// walks the head dimension in one chain, the sums of score_logits_kernel.
+template <int DK, int DV, bool CMP, bool WITH_CMP>
 __device__ __forceinline__ void attend_chunk(const DecArgs& p, uint8_t* sm, int row, int chunk, const void* kbase, const __nv_bfloat16* vbase,
                                              int64_t ld, int key0, int klo, int khi, int b, int h0, int tn) {
-  using SM = DecSmem<DK, DV>;
+  using SM = DecSmem<DK, DV, WITH_CMP>;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   __nv_bfloat16* sQ = (__nv_bfloat16*)(sm + SM::oQ);
   __nv_bfloat16* sK = (__nv_bfloat16*)(sm + SM::oK);
@@ -275,6 +210,13 @@ __device__ __forceinline__ void attend_chunk(const DecArgs& p, uint8_t* sm, int 
       cp16(sQ + r * (DK + 8) + cc * 8, qb + (r < p.hpg ? r * p.sqh : 0) + cc * 8, r < p.hpg);
     }
     cp_commit();
+  } else {
+    float* sKf = (float*)(sm + SM::oK) + DK * 16;
+    for (int i = tid; i < DK * 16; i += kDecThreads) {
+      const int r = i >> 4, cc = i & 15;
+      cp16(sKf + r * 64 + cc * 4, (const float*)kbase + (int64_t)r * ld + key0 + cc * 4, true);
+    }
+    cp_commit();
   }
   // (rows outside the visible range arrive as zeros: stale values behind the newest token must not meet P = 0)
   for (int i = tid; i < 64 * (DV / 8); i += kDecThreads) {
@@ -285,46 +227,30 @@ __device__ __forceinline__ void attend_chunk(const DecArgs& p, uint8_t* sm, int 
   cp_commit();
   if (CMP) {
     float* qf = (float*)(sm + SM::oK);          // [DK][16]
-    float* part = qf + DK * 16;                 // [4][16][64]
+    const float* sKf = qf + DK * 16;            // [DK][64]
     for (int i = tid; i < DK * 16; i += kDecThreads) {
       const int r = i / DK, dd = i % DK;
       qf[dd * 16 + r] = r < p.hpg ? __bfloat162float(qb[r * p.sqh + dd]) : 0.f;
     }
+    cp_wait<1>();
     __syncthreads();
-    const int key = tid & 63, quarter = tid >> 6;
-    const bool in = key0 + key < khi;
-    const float* kp = (const float*)kbase + (int64_t)quarter * (DK / 4) * ld + key0 + key;
-    float acc[16];
-#pragma unroll
-    for (int u = 0; u < 16; ++u) acc[u] = 0.f;
-#pragma unroll
-    for (int d0 = 0; d0 < DK / 4; d0 += 16) {
-      float kv[16];
-#pragma unroll
-      for (int e = 0; e < 16; ++e) kv[e] = in ? kp[(int64_t)(d0 + e) * ld] : 0.f;
-#pragma unroll
-      for (int e = 0; e < 16; ++e) {
-        const float4* q4 = reinterpret_cast<const float4*>(qf + (quarter * (DK / 4) + d0 + e) * 16);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float4 qv = q4[u];
-          acc[4 * u] = fmaf(qv.x, kv[e], acc[4 * u]);         acc[4 * u + 1] = fmaf(qv.y, kv[e], acc[4 * u + 1]);
-          acc[4 * u + 2] = fmaf(qv.z, kv[e], acc[4 * u + 2]); acc[4 * u + 3] = fmaf(qv.w, kv[e], acc[4 * u + 3]);
-        }
-      }
+    const int kk = tid & 63, h4 = (tid >> 6) * 4;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 16
+    for (int dd = 0; dd < DK; ++dd) {
+      const float kv = sKf[dd * 64 + kk];
+      const float4 qv = *reinterpret_cast<const float4*>(qf + dd * 16 + h4);
+      acc[0] = fmaf(qv.x, kv, acc[0]); acc[1] = fmaf(qv.y, kv, acc[1]);
+      acc[2] = fmaf(qv.z, kv, acc[2]); acc[3] = fmaf(qv.w, kv, acc[3]);
     }
-#pragma unroll
-    for (int u = 0; u < 16; ++u) part[(quarter * 16 + u) * 64 + key] = acc[u];
-    __syncthreads();
     float* lg = p.slog + (int64_t)row * 16 * (p.nc * 64) + chunk * 64;
-    for (int i = tid; i < p.hpg * 64; i += kDecThreads) {
-      const int u = i >> 6, kk = i & 63;
-      const float s = (part[u * 64 + kk] + part[(16 + u) * 64 + kk]) + (part[(32 + u) * 64 + kk] + part[(48 + u) * 64 + kk]);
-      const float x = key0 + kk < khi ? s * p.scale : -CUDART_INF_F;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int u = h4 + e;
+      const float x = key0 + kk < khi && u < p.hpg ? acc[e] * p.scale : -CUDART_INF_F;
       sS[u * 66 + kk] = x;
-      lg[(int64_t)u * (p.nc * 64) + kk] = x;
+      if (u < p.hpg) lg[(int64_t)u * (p.nc * 64) + kk] = x;
     }
-    for (int i = p.hpg * 64 + tid; i < 16 * 64; i += kDecThreads) sS[(i >> 6) * 66 + (i & 63)] = -CUDART_INF_F;
   } else {
     cp_wait<1>();
     __syncthreads();
@@ -440,12 +366,12 @@ __global__ void __launch_bounds__(kDecThreads) decode_dense_kernel(const __grid_
   if (chunk < p.nc) {
     // block i is visible when it ends at or before t
     const int vis = t >= p.l - 1 ? min(p.nb, (t - p.l + 1) / p.d + 1) : 0;
-    attend_chunk<DK, DV, true>(p, dsm, row, chunk, p.k_cmp + (int64_t)bg * DK * p.nbp, p.v_cmp + (int64_t)bg * p.nbp * DV, p.nbp,
+    attend_chunk<DK, DV, true, true>(p, dsm, row, chunk, p.k_cmp + (int64_t)bg * DK * p.nbp, p.v_cmp + (int64_t)bg * p.nbp * DV, p.nbp,
                                chunk * 64, 0, vis, b, h0, tn);
   } else {
     const int klo = max(0, t - p.window + 1), key0 = (klo / 64 + chunk - p.nc) * 64;
     if (key0 > t) { empty_chunk(p, row, chunk); return; }
-    attend_chunk<DK, DV, false>(p, dsm, row, chunk, p.k_win + (int64_t)bg * DK * p.cap, p.v_win + (int64_t)bg * p.cap * DV, p.cap, key0,
+    attend_chunk<DK, DV, false, true>(p, dsm, row, chunk, p.k_win + (int64_t)bg * DK * p.cap, p.v_win + (int64_t)bg * p.cap * DV, p.cap, key0,
                                 klo, t + 1, b, h0, tn);
   }
 }
@@ -458,7 +384,7 @@ __global__ void __launch_bounds__(kDecThreads) decode_selected_kernel(const __gr
   const int row = blockIdx.y, slot = blockIdx.x, bg = row / p.Tn, tn = row % p.Tn, b = bg / p.G, h0 = (bg % p.G) * p.hpg;
   const int t = p.pos + tn, id = p.idx[(int64_t)row * p.n + slot];    // (ids of a row are distinct)
   if (id < 0 || (int64_t)id * 64 > t) { empty_chunk(p, row, p.nc + p.nw + slot); return; }
-  attend_chunk<DK, DV, false>(p, dsm, row, p.nc + p.nw + slot, p.k_slc + (int64_t)bg * DK * p.cap, p.v_slc + (int64_t)bg * p.cap * DV,
+  attend_chunk<DK, DV, false, false>(p, dsm, row, p.nc + p.nw + slot, p.k_slc + (int64_t)bg * DK * p.cap, p.v_slc + (int64_t)bg * p.cap * DV,
                               p.cap, id * 64, 0, t + 1, b, h0, tn);
 }
 
@@ -490,12 +416,15 @@ __device__ __forceinline__ void warp_top(unsigned long long* keys, int first, in
   __syncwarp();
 }
 constexpr int kTopWarps = 16;
-// One CTA per row: softmax statistics of the heads from the chunks', Eq. 9 sums per selection block summed over the heads in
-// order, then the top n: each warp of its share, one warp of the survivors.
+constexpr size_t kTopSmemMax = 200 * 1024;
+// One CTA per row: softmax statistics of the heads, Eq. 9 sums per selection block summed over the heads in order, then the top
+// n: each warp of its share, one warp of the survivors.  All sums run in the order of score_topn_kernel: a head's denominator as
+// that kernel's 256 threads form it (block i belongs to thread i % 256; a warp's sum, then the eight warps'), p = e * (1 / sum)
+// rounded, and a block's terms one after the other from zero.
 __global__ void __launch_bounds__(kTopWarps * 32) decode_topn_kernel(const __grid_constant__ DecArgs p, int n_sel, int n_eff) {
   extern __shared__ __align__(16) unsigned long long keys[];   // [n_eff], then [kTopWarps * n]
   unsigned long long* cand = keys + n_eff;
-  __shared__ float hm[16], hinv[16];
+  __shared__ float hm[16], hinv[16], red[16][8];
   __shared__ unsigned long long top[kDecMaxN];
   pdl_wait();
   pdl_launch();
@@ -505,35 +434,49 @@ __global__ void __launch_bounds__(kTopWarps * 32) decode_topn_kernel(const __gri
     float m = -CUDART_INF_F;
     for (int c = lane; c < p.nc; c += 32) m = fmaxf(m, st[c * 16].x);
     m = warp_max(m);
-    float s = 0.f;
-    for (int c = lane; c < p.nc; c += 32) {
-      const float2 v = st[c * 16];
-      if (v.y != 0.f) s += v.y * expf(v.x - m);
-    }
-    s = warp_sum(s);
-    if (lane == 0) { hm[warp] = m; hinv[warp] = s != 0.f ? 1.f / s : 0.f; }
+    if (lane == 0) hm[warp] = m;
   }
   __syncthreads();
   const int ncol = p.nc * 64;
   const float* lg = p.slog + (int64_t)row * 16 * ncol;
+  for (int i = warp; i < p.hpg * 8; i += kTopWarps) {
+    const int h = i >> 3, w8 = i & 7;
+    const float m = hm[h];
+    float s = 0.f;
+    if (m != -CUDART_INF_F)
+#pragma unroll 8
+      for (int c = w8 * 32 + lane; c < ncol; c += 256) s += expf(lg[(int64_t)h * ncol + c] - m);   // (hidden blocks add zero)
+    s = warp_sum(s);
+    if (lane == 0) red[h][w8] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x < p.hpg) {
+    float s = red[threadIdx.x][0];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) s += red[threadIdx.x][w];
+    hinv[threadIdx.x] = 1.f / s;
+  }
+  __syncthreads();
   for (int j = threadIdx.x; j < n_eff; j += kTopWarps * 32) {
     float agg = 0.f;
     for (int h = 0; h < p.hpg; ++h) {
       const float m = hm[h], inv = hinv[h];
+      const bool none = m == -CUDART_INF_F;    // nothing visible: block 0 alone (nsa/kernels.py:2316-2343)
+      const float* lh = lg + (int64_t)h * ncol;
+      auto prob = [&](int c) { return none ? (c == 0 ? 1.f : 0.f) : c < ncol ? __fmul_rn(expf(lh[c] - m), inv) : 0.f; };
       float sel = 0.f;
-      if (m == -CUDART_INF_F) {            // nothing visible: block 0 alone (nsa/kernels.py:2316-2343)
-        for (int mm = 0; mm < p.s_; ++mm)
-          for (int nn = 0; nn < p.a_; ++nn) sel += p.s_ * j + mm + nn == 0 ? 1.f : 0.f;
-      } else {
-        const float* lh = lg + (int64_t)h * ncol;
-        for (int i = 0; i < p.s_ + p.a_ - 1; ++i) {
-          const int c = p.s_ * j + i;
-          // block c is counted once per (m, n) with m + n = i, m < s, n < a
-          const int times = min(min(i + 1, p.s_ + p.a_ - 1 - i), min(p.s_, p.a_));
-          if (c < ncol) sel = fmaf((float)times, expf(lh[c] - m) * inv, sel);
+      if (p.a_ == 2) {                         // (a block's term is the next sum's first one)
+        float cur = prob(p.s_ * j);
+        for (int mm = 0; mm < p.s_; ++mm) {
+          const float next = prob(p.s_ * j + mm + 1);
+          sel = __fadd_rn(__fadd_rn(sel, cur), next);
+          cur = next;
         }
+      } else {
+        for (int mm = 0; mm < p.s_; ++mm)
+          for (int nn = 0; nn < p.a_; ++nn) sel = __fadd_rn(sel, prob(p.s_ * j + mm + nn));
       }
-      agg += sel;
+      agg = __fadd_rn(agg, sel);
     }
     if (!(agg >= 0.f)) agg = 0.f;          // (not a number)
     keys[j] = ((unsigned long long)__float_as_uint(agg) << 32) | (unsigned)~j;
@@ -632,7 +575,7 @@ bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 struct DecLayout {
   int rows, nc, nw, P, n_sel, n_eff;
-  size_t o_q, o_gh, o_logits, o_hbar, o_part, o_st, o_slog, o_idx, total;
+  size_t o_gh, o_logits, o_phi, o_part, o_st, o_slog, o_idx, total;
 };
 DecLayout dec_layout(const nsa_decode_desc& d) {
   DecLayout L;
@@ -646,10 +589,9 @@ DecLayout dec_layout(const nsa_decode_desc& d) {
   size_t o = 0;
   auto take = [&](size_t b) { const size_t r = o; o += al256(b); return r; };
   const size_t R = (size_t)d.B * d.Tn;
-  L.o_q = take(R * d.H * d.dk * 2);
   L.o_gh = take(R * d.d_gate * 2);
   L.o_logits = take(R * 3 * d.H * 4);
-  L.o_hbar = take((size_t)d.B * d.G * std::max(d.nb_new, 0) * d.U * 4);
+  L.o_phi = take(d.project && d.nb_new > 0 ? compress_blocks_workspace_bytes(d, NSA_BF16) : 0);
   L.o_part = take((size_t)L.rows * L.P * 16 * d.dv * 4);
   L.o_st = take((size_t)L.rows * L.P * 16 * sizeof(float2));
   L.o_slog = take((size_t)L.rows * 16 * L.nc * 64 * 4);
@@ -663,23 +605,23 @@ size_t topn_smem(const nsa_decode_desc& d, const DecLayout& L) {
 
 template <int DK, int DV>
 int launch_attend(const DecArgs& a, const nsa_decode_desc& d, const DecLayout& L, cudaStream_t st) {
-  constexpr int kBytes = DecSmem<DK, DV>::kBytes;
-  cudaFuncSetAttribute(decode_dense_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
-  cudaFuncSetAttribute(decode_selected_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+  constexpr int kDense = DecSmem<DK, DV, true>::kBytes, kSelected = DecSmem<DK, DV, false>::kBytes;
+  // (the attributes are the kernels' own, shared by all threads: bounds that do not depend on the call)
+  cudaFuncSetAttribute(decode_dense_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDense);
+  cudaFuncSetAttribute(decode_selected_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSelected);
+  cudaFuncSetAttribute(decode_topn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTopSmemMax);
   {
     KernelTimer kt("decode_dense", st);
     const int gate_ctas = a.gh ? (3 * d.H + 7) / 8 : 0;
-    if (int rc = launch_pdl("decode_dense", decode_dense_kernel<DK, DV>, dim3(L.rows * (L.nc + L.nw) + gate_ctas), kDecThreads, kBytes, st, a)) return rc;
+    if (int rc = launch_pdl("decode_dense", decode_dense_kernel<DK, DV>, dim3(L.rows * (L.nc + L.nw) + gate_ctas), kDecThreads, kDense, st, a)) return rc;
   }
   {
     KernelTimer kt("decode_topn", st);
-    const size_t sm = topn_smem(d, L);
-    if (sm > 40 * 1024) cudaFuncSetAttribute(decode_topn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (int rc = launch_pdl("decode_topn", decode_topn_kernel, dim3(L.rows), kTopWarps * 32, sm, st, a, L.n_sel, L.n_eff)) return rc;
+    if (int rc = launch_pdl("decode_topn", decode_topn_kernel, dim3(L.rows), kTopWarps * 32, topn_smem(d, L), st, a, L.n_sel, L.n_eff)) return rc;
   }
   {
     KernelTimer kt("decode_selected", st);
-    if (int rc = launch_pdl("decode_selected", decode_selected_kernel<DK, DV>, dim3(d.n, L.rows), kDecThreads, kBytes, st, a)) return rc;
+    if (int rc = launch_pdl("decode_selected", decode_selected_kernel<DK, DV>, dim3(d.n, L.rows), kDecThreads, kSelected, st, a)) return rc;
   }
   KernelTimer kt("decode_combine", st);
   return launch_pdl("decode_combine", decode_combine_kernel<DV>, dim3(L.rows, a.hpg), 4 * DV, (size_t)L.P * 4, st, a);
@@ -700,11 +642,10 @@ extern "C" NSA_API int nsa_decode_supported(const nsa_decode_desc* dp) {
   if (d.nb <= 0 || d.nb > d.nbp || d.nbp % 64 != 0 || d.cap % 64 != 0 || d.pos < 0 || (int64_t)d.pos + d.Tn > d.cap) return 0;
   if (d.project) {
     if (d.B * d.Tn > kDecTokens || d.d_model <= 0 || d.d_model % 64 != 0 || d.d_gate <= 0 || d.d_gate % 16 != 0) return 0;
-    if (d.nb_new < 0 || d.nb_new > d.nb || (d.nb_new > 0 && (d.U <= 0 || d.l > 32 || (d.dk + d.l) % 8 != 0))) return 0;
-    if (d.nb_new > 65535) return 0;
+    if (d.nb_new < 0 || d.nb_new > d.nb || (d.nb_new > 0 && d.U <= 0)) return 0;
   }
   const DecLayout L = dec_layout(d);
-  return topn_smem(d, L) <= 200 * 1024 && (size_t)L.P * 4 <= 32 * 1024;
+  return topn_smem(d, L) <= kTopSmemMax && (size_t)L.P * 4 <= 32 * 1024;
 }
 
 extern "C" NSA_API size_t nsa_decode_workspace_bytes(const nsa_decode_desc* d) {
@@ -726,53 +667,45 @@ extern "C" NSA_API int nsa_decode_fwd(const nsa_decode_desc* dp, void* workspace
   cudaStream_t st = (cudaStream_t)stream;
   char* w = (char*)workspace;
   DecArgs a = {};
+  NSA_REQUIRE(d.q && al16(d.q), "decode_fwd: null or misaligned q");
+  NSA_REQUIRE(d.sq[0] % 8 == 0 && d.sq[1] % 8 == 0 && d.sq[2] % 8 == 0, "decode_fwd: q rows must start on 16-byte boundaries");
+  a.q = (const __nv_bfloat16*)d.q;
+  a.sqb = d.sq[0]; a.sqh = d.sq[1]; a.sqt = d.sq[2];
   if (d.project) {
-    NSA_REQUIRE(d.x && al16(d.x) && d.gate_w1 && d.gate_w2 && al16(d.gate_w1) && al16(d.gate_w2) && d.k_src && d.v_src,
+    NSA_REQUIRE(d.x && al16(d.x) && d.gate_w1 && d.gate_w2 && al16(d.gate_w1) && al16(d.gate_w2) && d.k_src && d.v_src && d.k_new,
                 "decode_fwd: projection inputs missing or not 16-byte aligned");
     NSA_REQUIRE(d.sx[0] % 8 == 0 && d.sx[1] % 8 == 0, "decode_fwd: x rows must start on 16-byte boundaries");
+    NSA_REQUIRE(d.nb_new == 0 || (d.pos_embed && d.phi_w1 && d.phi_w2 && d.k_cmp_lp && d.block_ends), "decode_fwd: phi parameters missing");
     ProjArgs p = {};
-    p.R = d.B * d.Tn; p.Tn = d.Tn; p.K = d.d_model; p.H = d.H; p.G = d.G; p.pos = d.pos; p.cap = d.cap;
+    p.R = d.B * d.Tn; p.Tn = d.Tn; p.K = d.d_model; p.G = d.G; p.pos = d.pos; p.cap = d.cap;
     p.x = (const __nv_bfloat16*)d.x;
     p.sxb = d.sx[0]; p.sxt = d.sx[1];
-    void* dst[7] = {w + L.o_q, d.k_slc, d.v_slc, d.k_src, d.v_src, d.k_win, d.v_win};
+    p.k_new = (const __nv_bfloat16*)d.k_new;
+    for (int i = 0; i < 4; ++i) p.sk[i] = d.sk[i];
     int tile = 0;
-    for (int i = 0; i < 7; ++i) {
+    auto segment = [&](const void* wt, const void* bias, void* dst, int rows, int D, int kind) {
+      p.seg[p.nseg++] = {(const __nv_bfloat16*)wt, (const __nv_bfloat16*)bias, (__nv_bfloat16*)dst, tile, D, kind};
+      tile += rows / 16;
+    };
+    void* dst[5] = {d.k_slc, d.v_slc, d.v_src, d.k_win, d.v_win};
+    for (int i = 0; i < 5; ++i) {
       NSA_REQUIRE(d.w[i] && al16(d.w[i]), "decode_fwd: projection weight missing or not 16-byte aligned");
-      const bool key = i == 0 || (i & 1);
-      ProjSeg& s = p.seg[i];
-      s.w = (const __nv_bfloat16*)d.w[i]; s.bias = (const __nv_bfloat16*)d.bias[i]; s.dst = (__nv_bfloat16*)dst[i];
-      s.D = key ? d.dk : d.dv; s.kind = i == 0 ? kSegQ : key ? kSegK : kSegV; s.tile0 = tile;
-      tile += (i == 0 ? d.H : d.G) * s.D / 16;
+      const bool key = i == 0 || i == 3;
+      const int D = key ? d.dk : d.dv;
+      segment(d.w[i], d.bias[i], dst[i], d.G * D, D, key ? kSegK : kSegV);
     }
-    ProjSeg& s = p.seg[7];
-    s.w = (const __nv_bfloat16*)d.gate_w1; s.bias = (const __nv_bfloat16*)d.gate_b1; s.dst = (__nv_bfloat16*)(w + L.o_gh);
-    s.D = d.d_gate; s.kind = kSegGate; s.tile0 = tile;
-    tile += d.d_gate / 16;
-    p.nseg = 8;
+    segment(d.gate_w1, d.gate_b1, w + L.o_gh, d.d_gate, d.d_gate, kSegGate);
+    segment(nullptr, nullptr, d.k_src, d.G * d.dk, d.dk, kSegCopy);
     {
       KernelTimer kt("decode_project", st);
       if (int rc = launch_pdl("decode_project", decode_project_kernel, dim3(tile), kProjThreads, 0, st, p)) return rc;
     }
-    if (d.nb_new > 0) {
-      NSA_REQUIRE(d.pos_embed && d.phi_w1 && d.phi_w2 && d.k_cmp_lp && d.block_ends && al16(d.phi_w1), "decode_fwd: phi parameters missing");
-      KernelTimer kt("decode_phi", st);
-      PhiArgs f = {};
-      f.k = (const __nv_bfloat16*)d.k_src; f.v = (const __nv_bfloat16*)d.v_src; f.pos = (const __nv_bfloat16*)d.pos_embed;
-      f.w1 = (const __nv_bfloat16*)d.phi_w1; f.b1 = (const __nv_bfloat16*)d.phi_b1; f.w2 = (const __nv_bfloat16*)d.phi_w2; f.b2 = (const __nv_bfloat16*)d.phi_b2;
-      f.hbar = (float*)(w + L.o_hbar); f.k_cmp = (float*)d.k_cmp; f.k_lp = (__nv_bfloat16*)d.k_cmp_lp; f.v_cmp = (__nv_bfloat16*)d.v_cmp;
-      f.block_ends = d.block_ends; f.cap = d.cap; f.nbp = d.nbp; f.dk = d.dk; f.dv = d.dv; f.U = d.U; f.l = d.l; f.d = d.d; f.blk0 = d.nb - d.nb_new;
-      if (int rc = launch_pdl("decode_phi", decode_phi_hidden_kernel, dim3((d.U + 63) / 64, d.nb_new, d.B * d.G), 256, (size_t)(d.dk + d.l) * 32 * 4, st, f)) return rc;
-      if (int rc = launch_pdl("decode_phi", decode_phi_out_kernel, dim3(6, d.nb_new, d.B * d.G), 256, 0, st, f)) return rc;
-    }
-    a.q = (const __nv_bfloat16*)(w + L.o_q);
-    a.sqb = (int64_t)d.H * d.Tn * d.dk; a.sqh = (int64_t)d.Tn * d.dk; a.sqt = d.dk;
+    if (d.nb_new > 0)
+      if (int rc = compress_blocks(d, d.k_src, d.v_src, NSA_BF16, NSA_BF16, w + L.o_phi, st)) return rc;
     a.gh = (const __nv_bfloat16*)(w + L.o_gh); a.gw2 = (const __nv_bfloat16*)d.gate_w2; a.gb2 = (const __nv_bfloat16*)d.gate_b2; a.D2 = d.d_gate;
     a.logits = (float*)(w + L.o_logits);
   } else {
-    NSA_REQUIRE(d.q && al16(d.q) && d.gate_logits, "decode_fwd: null or misaligned q / gate logits");
-    NSA_REQUIRE(d.sq[0] % 8 == 0 && d.sq[1] % 8 == 0 && d.sq[2] % 8 == 0, "decode_fwd: q rows must start on 16-byte boundaries");
-    a.q = (const __nv_bfloat16*)d.q;
-    a.sqb = d.sq[0]; a.sqh = d.sq[1]; a.sqt = d.sq[2];
+    NSA_REQUIRE(d.gate_logits, "decode_fwd: null gate logits");
     a.logits = const_cast<float*>(d.gate_logits);
   }
   a.k_slc = (const __nv_bfloat16*)d.k_slc; a.v_slc = (const __nv_bfloat16*)d.v_slc; a.k_win = (const __nv_bfloat16*)d.k_win;

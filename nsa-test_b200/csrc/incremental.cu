@@ -133,6 +133,36 @@ ChunkLayout chunk_layout(const nsa_decode_desc& d) {
 bool al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 }  // namespace
+
+size_t compress_blocks_workspace_bytes(const nsa_decode_desc& d, int dtype) { return append_layout(d, dtype).total; }
+
+int compress_blocks(const nsa_decode_desc& d, const void* k, const void* v, int dtype, int param_dtype, void* workspace, cudaStream_t st) {
+  const AppendLayout L = append_layout(d, dtype);
+  char* w = (char*)workspace;
+  const void* in[5] = {d.pos_embed, d.phi_w1, d.phi_b1, d.phi_w2, d.phi_b2};
+  const float* par[5];
+  for (int i = 0; i < 5; ++i) par[i] = (const float*)in[i];
+  if (param_dtype == NSA_BF16) {
+    CastArgs c = {};
+    const int n[5] = {d.l * d.l, d.U * (d.dk + d.l), d.U, d.dk * d.U, d.dk};
+    for (int i = 0; i < 5; ++i) {
+      c.in[i] = (const __nv_bfloat16*)in[i];
+      c.out[i] = (float*)(w + L.o_par[i]);
+      c.n[i] = n[i];
+      par[i] = in[i] ? c.out[i] : nullptr;
+    }
+    cast_params_kernel<<<148, 256, 0, st>>>(c);
+  }
+  const size_t es = dtype == NSA_BF16 ? 2 : 4;
+  const int b0 = d.nb - d.nb_new;
+  append_block_ends_kernel<<<(d.nb_new + 255) / 256, 256, 0, st>>>(d.block_ends, b0, d.nb_new, d.l, d.d);
+  const char *ks = (const char*)k + (size_t)L.lo * es, *vs = (const char*)v + (size_t)L.lo * d.dv * es;
+  const int64_t vst[4] = {(int64_t)d.G * d.cap * d.dv, (int64_t)d.cap * d.dv, d.dv, 1};
+  return cmp_phi_fwd_strided(ks, d.cap, (int64_t)d.dk * d.cap, vs, vst, par[0], par[1], par[2], par[3], par[4], (float*)d.k_cmp + b0,
+                             d.k_cmp_lp ? (char*)d.k_cmp_lp + b0 * es : nullptr, (char*)d.v_cmp + (size_t)b0 * d.dv * es, d.B, d.G, L.T, L.T, d.dk,
+                             d.dv, d.l, d.d, d.U, d.nbp, false, dtype, w + L.o_saved, L.saved, w + L.o_ws, L.ws, st);
+}
+
 }  // namespace nsa
 
 using namespace nsa;
@@ -176,30 +206,7 @@ extern "C" NSA_API int nsa_cache_append(const nsa_decode_desc* dp, const void* c
   }
   if (int rc = check_launch("cache_append")) return rc;
   if (d.nb_new == 0) return NSA_OK;
-  char* w = (char*)workspace;
-  const void* in[5] = {d.pos_embed, d.phi_w1, d.phi_b1, d.phi_w2, d.phi_b2};
-  const float* par[5];
-  for (int i = 0; i < 5; ++i) par[i] = (const float*)in[i];
-  if (param_dtype == NSA_BF16) {
-    CastArgs c = {};
-    const int n[5] = {d.l * d.l, d.U * (d.dk + d.l), d.U, d.dk * d.U, d.dk};
-    for (int i = 0; i < 5; ++i) {
-      c.in[i] = (const __nv_bfloat16*)in[i];
-      c.out[i] = (float*)(w + L.o_par[i]);
-      c.n[i] = n[i];
-      par[i] = in[i] ? c.out[i] : nullptr;
-    }
-    cast_params_kernel<<<148, 256, 0, st>>>(c);
-  }
-  const size_t es = dtype == NSA_BF16 ? 2 : 4;
-  const int b0 = d.nb - d.nb_new;
-  append_block_ends_kernel<<<(d.nb_new + 255) / 256, 256, 0, st>>>(d.block_ends, b0, d.nb_new, d.l, d.d);
-  const char* ks = (const char*)(n_tensors == 2 ? d.k_slc : d.k_src) + (size_t)L.lo * es;
-  const char* vs = (const char*)(n_tensors == 2 ? d.v_slc : d.v_src) + (size_t)L.lo * d.dv * es;
-  const int64_t vst[4] = {(int64_t)d.G * d.cap * d.dv, (int64_t)d.cap * d.dv, d.dv, 1};
-  return cmp_phi_fwd_strided(ks, d.cap, (int64_t)d.dk * d.cap, vs, vst, par[0], par[1], par[2], par[3], par[4], (float*)d.k_cmp + b0,
-                             d.k_cmp_lp ? (char*)d.k_cmp_lp + b0 * es : nullptr, (char*)d.v_cmp + (size_t)b0 * d.dv * es, d.B, d.G, L.T, L.T, d.dk,
-                             d.dv, d.l, d.d, d.U, d.nbp, false, dtype, w + L.o_saved, L.saved, w + L.o_ws, L.ws, st);
+  return compress_blocks(d, n_tensors == 2 ? d.k_slc : d.k_src, n_tensors == 2 ? d.v_slc : d.v_src, dtype, param_dtype, workspace, st);
 }
 
 extern "C" NSA_API int nsa_incremental_supported(const nsa_decode_desc* dp) {

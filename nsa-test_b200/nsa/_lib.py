@@ -43,9 +43,9 @@ class DecodeDesc(ctypes.Structure):
                 + [(n_, c_void_p) for n_ in ("q", "gate_logits", "k_slc", "v_slc", "k_src", "v_src", "k_win", "v_win", "k_cmp",
                                              "k_cmp_lp", "v_cmp", "block_ends", "out", "indices", "gates", "o_cmp", "o_slc",
                                              "o_win", "x")]
-                + [("sx", c_int64 * 2), ("w", c_void_p * 7), ("bias", c_void_p * 7)]
+                + [("sx", c_int64 * 2), ("w", c_void_p * 5), ("bias", c_void_p * 5)]
                 + [(n_, c_void_p) for n_ in ("gate_w1", "gate_b1", "gate_w2", "gate_b2", "pos_embed", "phi_w1", "phi_b1",
-                                             "phi_w2", "phi_b2")])
+                                             "phi_w2", "phi_b2", "k_new")] + [("sk", c_int64 * 4)])
 
 
 # pieces of the layer's context buffer, in the order of enum nsa_layer_ctx_piece

@@ -200,11 +200,11 @@ def _decode_module(module, x: torch.Tensor, cache: NSACache):
     d = _cache_desc(cache, B, Tn, cache.length, nb, module.scale)
     if d is None:
         return None
-    lins = (module.q_proj, module.k_select, module.v_select, module.k_compress, module.v_compress, module.k_sliding, module.v_sliding)
+    lins = (module.k_select, module.v_select, module.v_compress, module.k_sliding, module.v_sliding)
     g0, g2 = module.gate_mlp[0], module.gate_mlp[2]
     pe, pw1, pb1, pw2, pb2 = module._phi_params()
     D2, U = g0.weight.shape[0], pw1.shape[0]
-    rows = (H * dk, G * dk, G * dv, G * dk, G * dv, G * dk, G * dv)
+    rows = (G * dk, G * dv, G * dv, G * dk, G * dv)
     params = [(lin.weight, r * dm) for lin, r in zip(lins, rows)] + [(lin.bias, r) for lin, r in zip(lins, rows)]
     params += [(g0.weight, D2 * dm), (g0.bias, D2), (g2.weight, 3 * H * D2), (g2.bias, 3 * H), (pe, c.l * c.l), (pw1, U * (dk + c.l)),
                (pb1, U), (pw2, dk * U), (pb2, dk)]
@@ -216,15 +216,22 @@ def _decode_module(module, x: torch.Tensor, cache: NSACache):
         if type(t) not in _PLAIN or t.dtype != torch.bfloat16 or t.numel() != n or t.device != dev or not t.is_contiguous():
             return None
         ptrs.append(t.data_ptr())
-    if any(p_ is None or p_ % 16 for p_ in ptrs[:7] + [ptrs[14], ptrs[16], ptrs[19]]) or ptrs[18] is None or ptrs[21] is None:
+    (d.gate_w1, d.gate_b1, d.gate_w2, d.gate_b2, d.pos_embed, d.phi_w1, d.phi_b1, d.phi_w2, d.phi_b2) = ptrs[10:]
+    if any(p_ is None or p_ % 16 for p_ in ptrs[:5] + [d.gate_w1, d.gate_w2]) or not (d.pos_embed and d.phi_w1 and d.phi_w2):
         return None
     d.project, d.nb_new, d.d_model, d.d_gate, d.U = 1, nb - cache.n_blocks, dm, D2, U
     if not _lib.lib.nsa_decode_supported(d):
         return None
+    # what the block choice depends on comes out of the products of the general path: rounded otherwise, near-ties would fall
+    # the other way
+    q, k_new = _project_heads(x, module.q_proj, H, dk), _project_heads(x, module.k_compress, G, dk, transposed=True)
+    if any(t.dtype != torch.bfloat16 or t.device != dev for t in (q, k_new)):
+        return None
+    q = q.contiguous()
     out = torch.empty(B, Tn, H * dv, device=dev, dtype=x.dtype)
+    d.q, d.sq, d.k_new, d.sk = q.data_ptr(), q.stride()[:3], k_new.data_ptr(), k_new.stride()
     d.x, d.sx, d.out = x.data_ptr(), x.stride()[:2], out.data_ptr()
-    d.w, d.bias = tuple(ptrs[:7]), tuple(ptrs[7:14])
-    (d.gate_w1, d.gate_b1, d.gate_w2, d.gate_b2, d.pos_embed, d.phi_w1, d.phi_b1, d.phi_w2, d.phi_b2) = ptrs[14:]
+    d.w, d.bias = tuple(ptrs[:5]), tuple(ptrs[5:10])
     ops.decode_fwd(d, dev)
     cache.length, cache.n_blocks = p1, nb
     return out
