@@ -238,6 +238,7 @@ class _BranchesAndMix(torch.autograd.Function):
          gates) = ctx.saved_tensors
         lo, hi, pad, kshape, vshape = ctx.win
         o_win = o_wp[:, :, pad:] if pad else o_wp
+        dout = torch.zeros_like(o_cmp) if dout is None else dout      # (a later node may hand back no gradient)
         d_cmp, d_slc, d_win, dlogits, delta = ops.gate_mix_bwd(gates, o_cmp, o_slc, o_win, dout, ctx.gate_mode,
                                                                want_delta=True)
         dq_c, dkc, dvc = ops.cmp_attn_bwd(q, k_cmp, v_cmp, block_ends, o_cmp, d_cmp, Lc, Mc, ctx.scale, ctx.blocks,
@@ -295,6 +296,8 @@ class _LayerC(torch.autograd.Function):
         q, k_slc, v_slc, k_cmp, k_win, v_win, pos, w1, w2, saved = ctx.saved_tensors
         desc = ctx.desc
         tm = bool(desc.out_token_major)
+        if dout is None:              # a later node handed back no gradient for the output
+            dout = ops._mixed_out(desc, q).zero_()
         # the upstream gradient in the layout the forward wrote: read as it lies when it has it, copied otherwise
         if tm:
             if not dout.permute(0, 2, 1, 3).is_contiguous():
@@ -411,6 +414,7 @@ class _GateMix(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout, _dgates):
         gates, o_cmp, o_slc, o_win = ctx.saved_tensors
+        dout = torch.zeros_like(o_cmp) if dout is None else dout      # (a later node may hand back no gradient)
         d0, d1, d2, dlogits = ops.gate_mix_bwd(gates, o_cmp, o_slc, o_win, dout, ctx.gate_mode)
         return dlogits.to(ctx.ldtype), d0, d1, d2, None
 

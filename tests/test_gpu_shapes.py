@@ -466,3 +466,22 @@ def test_mma_kernels_keep_32_bit_probabilities(dk, dv, H, G, T, w, n):
     torch.cuda.synchronize()
     for a, b in ((o[:, :, :T - 5], o2[:, :, :T - 5]), (dq[:, :, :T - 5], dq2[:, :, :T - 5]), (dkey[:, :, 8:], dkey2[:, :, 8:]), (dval[:, :, 8:], dval2[:, :, 8:])):
         assert torch.isfinite(b).all() and max_abs(a.float(), b.float()) <= 2 ** -7 * max(1.0, a.float().abs().max().item())
+
+
+@pytest.mark.parametrize("c_layer", [True, False])
+@pytest.mark.parametrize("token_major", [True, False])
+def test_layer_without_an_upstream_gradient(monkeypatch, c_layer, token_major):
+    """A later node that hands back no gradient for the layer's output: zero gradients, as for a gradient of zeros."""
+    import nsa
+    from nsa import kernels as K
+    from tests.test_host import DropGradient
+    monkeypatch.setattr(K, "_USE_C_LAYER", c_layer)
+    inp = O.make_inputs(1, 4, 2, 128, 64, 64, 64, 32, seed=1, dtype=torch.bfloat16)
+    cfg = nsa.NSAConfig(d_model=64, head_dim_qk=64, head_dim_v=64, n_heads=4, n_kv_groups=2, w=64)
+    q, k, v = (inp[x].to(DEV, torch.bfloat16).requires_grad_(True) for x in ("q", "k", "v"))
+    phi = tuple(getattr(inp["phi"], n_).to(DEV).requires_grad_(True) for n_ in ("pos_embed", "w1", "b1", "w2", "b2"))
+    logits = torch.zeros(1, 128, 12, device=DEV, requires_grad=True)
+    out = K.nsa_layer(q, k, v, logits, phi, cfg, token_major_out=token_major)
+    ins = (q, k, v, logits, *phi)
+    for g, t in zip(torch.autograd.grad(DropGradient.apply(out).sum(), ins), ins):
+        assert g.shape == t.shape and not g.any()

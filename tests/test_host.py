@@ -133,3 +133,26 @@ def test_projections_match_the_per_linear_products(monkeypatch):
     for p, q in zip((*a, *torch.autograd.grad(a, [x, *ws], gs)), (*b, *torch.autograd.grad(b, [x, *ws], gs))):
         assert p.shape == q.shape and (p - q).abs().max().item() < 1e-12
     assert all(t.is_contiguous() for t in a)
+
+
+class DropGradient(torch.autograd.Function):
+    """A node that hands back no gradient for its input."""
+
+    @staticmethod
+    def forward(ctx, x):
+        return x.clone()
+
+    @staticmethod
+    def backward(ctx, _g):
+        return None
+
+
+def test_gate_mix_without_an_upstream_gradient(monkeypatch):
+    """An undefined gradient of the mixed output counts as zeros."""
+    from nsa import kernels as K, ops
+    monkeypatch.setattr(ops, "gate_mix_fwd", lambda lg, a, b, c, mode: (a + b + c, lg))
+    monkeypatch.setattr(ops, "gate_mix_bwd", lambda g, a, b, c, d, mode: (d.contiguous(), d * 2, d * 3, g * d.sum()))
+    lg, a, b, c = (torch.randn(1, 2, 6, requires_grad=True), *(torch.randn(1, 2, 2, 4, requires_grad=True) for _ in range(3)))
+    out, _ = K._GateMix.apply(lg, a, b, c, "sigmoid")
+    grads = torch.autograd.grad((DropGradient.apply(out)).sum(), (lg, a, b, c))
+    assert all(g.shape == t.shape and not g.any() for g, t in zip(grads, (lg, a, b, c)))
