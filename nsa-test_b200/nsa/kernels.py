@@ -575,7 +575,8 @@ class _Projections(torch.autograd.Function):
             if transposed:
                 gt = g.reshape(B, heads * dim, T)
                 if ctx.needs_input_grad[2 + i]:
-                    dw = torch.mm(gt[0], x2) if B == 1 else torch.bmm(gt, x).sum(0)
+                    # (one product over all sequences: a product each, added up in the weights' type, would round B times)
+                    dw = torch.mm(gt.transpose(0, 1).reshape(heads * dim, B * T), x2)
                 if ctx.needs_input_grad[0]:
                     gt = gt.transpose(1, 2)
                     dx = torch.matmul(gt, w) if dx is None else dx.baddbmm_(gt, w.expand(B, -1, -1))

@@ -156,3 +156,20 @@ def test_gate_mix_without_an_upstream_gradient(monkeypatch):
     out, _ = K._GateMix.apply(lg, a, b, c, "sigmoid")
     grads = torch.autograd.grad((DropGradient.apply(out)).sum(), (lg, a, b, c))
     assert all(g.shape == t.shape and not g.any() for g, t in zip(grads, (lg, a, b, c)))
+
+
+def test_projection_weight_gradients_round_once(monkeypatch):
+    """bf16 weights shared by several sequences: the gradient is one 32-bit sum over all of them, as through the linears' own
+    products, so its error against 64 bits is one rounding, 2^-9 relative at most (and 2^-9 / sqrt(3) in the 2-norm)."""
+    from nsa import kernels as K, ops
+    monkeypatch.setattr(ops, "token_major", lambda x: x.transpose(1, 2).contiguous())
+    torch.manual_seed(1)
+    B, T, layouts = 4, 64, ((4, 8, False), (2, 8, True), (2, 4, False))
+    x = torch.randn(B, T, 32).bfloat16().requires_grad_(True)
+    ws = [torch.randn(h * d, 32).bfloat16().requires_grad_(True) for h, d, _ in layouts]
+    outs = K._Projections.apply(x, layouts, *ws)
+    gs = [torch.randn_like(t) for t in outs]
+    for (h, d, transposed), g, dw in zip(layouts, gs, torch.autograd.grad(outs, ws, gs)):
+        rows = g.transpose(2, 3) if transposed else g                  # [B,h,T,d]
+        want = torch.einsum("bhtd,btm->hdm", rows.double(), x.double()).reshape(h * d, 32)
+        assert ((dw.double() - want).norm() / want.norm()).item() < 2 ** -9
