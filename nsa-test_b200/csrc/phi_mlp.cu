@@ -138,8 +138,9 @@ __global__ void rows_to_f32_kernel(const T* __restrict__ in, float* __restrict__
 // Column sums out[c] = sum over rows of in[row, c] in a fixed order: chunks of rows are summed by 8 row lanes per column
 // (stage 1, partial sums to scratch), the chunks then one after the other (stage 2).  A chunk has up to 1024 rows, fewer as
 // long as the grid is short of four CTAs per SM: 1024 rows of a 1280-wide matrix were 40 CTAs and 15 us.
+int64_t colsum_want(int W) { return (4 * 148 + (W + 31) / 32 - 1) / ((W + 31) / 32); }      // chunks
 int colsum_chunk(int64_t rows, int W) {
-  const int64_t want = (4 * 148 + (W + 31) / 32 - 1) / ((W + 31) / 32);      // chunks
+  const int64_t want = colsum_want(W);
   return (int)std::min<int64_t>(1024, std::max<int64_t>(32, (rows + want - 1) / want));
 }
 template <typename T>
@@ -219,7 +220,12 @@ __global__ void table_grads_kernel(const float* __restrict__ dc, const float* __
 unsigned blocks_for(int64_t n) { return (unsigned)((n + 255) / 256); }
 
 int colsum_chunks(int64_t rows, int W) { return (int)((rows + colsum_chunk(rows, W) - 1) / colsum_chunk(rows, W)); }
-size_t colsum_scratch_bytes(int64_t rows, int W) { return al256((size_t)colsum_chunks(rows, W) * W * sizeof(float)); }
+// Enough for any row count up to `rows`: fewer rows can make more chunks (their length is rounded up), never more than asked
+// for, than 32-row chunks there are, or, with chunks of 1024 rows, than those.
+size_t colsum_scratch_bytes(int64_t rows, int W) {
+  const int64_t most = std::max(std::min(colsum_want(W), (rows + 31) / 32), (rows + 1023) / 1024);
+  return al256((size_t)most * W * sizeof(float));
+}
 template <typename T>
 void colsum(const T* in, int64_t rows, int W, float* out, float* scratch, cudaStream_t st) {
   const int chunks = colsum_chunks(rows, W);

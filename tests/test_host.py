@@ -173,3 +173,27 @@ def test_projection_weight_gradients_round_once(monkeypatch):
         rows = g.transpose(2, 3) if transposed else g                  # [B,h,T,d]
         want = torch.einsum("bhtd,btm->hdm", rows.double(), x.double()).reshape(h * d, 32)
         assert ((dw.double() - want).norm() / want.norm()).item() < 2 ** -9
+
+
+@pytest.mark.parametrize("BG,dk,dv", [(4, 192, 128), (8, 192, 128), (2, 128, 128), (4, 128, 128), (16, 64, 64)])
+def test_compression_backward_scratch_covers_its_column_sums(BG, dk, dv):
+    """The layer forms the products of ragged sequences over rows padded to 8, which may hold one block per plane more than the
+    sequence; the bytes reserved for those rows have to hold the column sums' partial rows over the blocks that there are."""
+    from nsa._lib import BF16, lib
+    al = lambda n: -(-n // 256) * 256
+    U, l, d = 2 * dk, 32, 16
+
+    def chunks(rows, W):                  # rows of W values in chunks of 32 to 1024, as many as four thread blocks per SM need
+        per_row = -(-W // 32)
+        want = -(-4 * 148 // per_row)
+        return -(-rows // min(1024, max(32, -(-rows // want))))
+
+    for T in [*range(2049, 9000, 7), *range(13080, 13088), *range(9001, 65536, 53)]:
+        rows = -(-T // 8) * 8
+        nb, nb_rows = (T - l) // d + 1, (rows - l) // d + 1
+        nbp = 1 << (nb - 1).bit_length()
+        nseg = -(-rows // 16)
+        parts = -(-nseg // max(4, -(-nseg * BG // 296)))
+        others = [BG * nb_rows * dk * 4, BG * nb_rows * U * 4, BG * nbp * dv * 4, BG * rows * U * 2, parts * BG * l * U * 4, l * U * 4, U * dk * 2]
+        reserved = lib.nsa_cmp_phi_workspace_bytes(1, BG, rows, dk, dv, l, d, U, nbp, BF16, 1) - 256 - sum(map(al, others))
+        assert reserved >= chunks(BG * nb, dk) * dk * 4, (T, reserved)
