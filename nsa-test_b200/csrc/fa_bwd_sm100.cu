@@ -424,7 +424,6 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
 #pragma unroll
       for (int c = 0; c < DK / 64; ++c) {
-        if (t >= p.Tq) break;
 #pragma unroll
         for (int e = 0; e < 32; e += 8) {
           uint4 pkt;
@@ -434,7 +433,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           __nv_bfloat162 a3 = __floats2bfloat162_rn(__uint_as_float(ov[c][e + 6]) * p.scale, __uint_as_float(ov[c][e + 7]) * p.scale);
           pkt.x = *reinterpret_cast<uint32_t*>(&a0); pkt.y = *reinterpret_cast<uint32_t*>(&a1);
           pkt.z = *reinterpret_cast<uint32_t*>(&a2); pkt.w = *reinterpret_cast<uint32_t*>(&a3);
-          *reinterpret_cast<uint4*>(dst + c * 32 + e) = pkt;
+          if (t < p.Tq) *reinterpret_cast<uint4*>(dst + c * 32 + e) = pkt;
         }
       }
     }
@@ -631,7 +630,6 @@ fa_bwd_dq_ds_kernel(const __grid_constant__ CUtensorMap tmDs, const __grid_const
 #pragma unroll
           for (int e = 0; e < 32; ++e) ov[e] = 0;
         }
-        if (t >= p.Tq) continue;
 #pragma unroll
         for (int e = 0; e < 32; e += 8) {
           uint4 pkt;
@@ -641,7 +639,8 @@ fa_bwd_dq_ds_kernel(const __grid_constant__ CUtensorMap tmDs, const __grid_const
           __nv_bfloat162 a3 = __floats2bfloat162_rn(__uint_as_float(ov[e + 6]) * p.scale, __uint_as_float(ov[e + 7]) * p.scale);
           pkt.x = *reinterpret_cast<uint32_t*>(&a0); pkt.y = *reinterpret_cast<uint32_t*>(&a1);
           pkt.z = *reinterpret_cast<uint32_t*>(&a2); pkt.w = *reinterpret_cast<uint32_t*>(&a3);
-          *reinterpret_cast<uint4*>(dst + c * 32 + e) = pkt;
+          // (a predicate, not a jump: the next column's tcgen05.ld wants the whole warp)
+          if (t < p.Tq) *reinterpret_cast<uint4*>(dst + c * 32 + e) = pkt;
         }
       }
       if (ntiles > 0) ++ic;
@@ -976,21 +975,24 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
                                                                 __uint_as_float(ov[e + 2]) * mul, __uint_as_float(ov[e + 3]) * mul);
             continue;
           }
-          if (key >= p.Tk) continue;
+          // (predicates, not a jump past the column: the next one's tcgen05.ld wants the whole warp)
+          const bool live = key < p.Tk;
           if (out_part) {
             float* dst = out_part + ((int64_t)hc * p.B * p.G * p.Tk + krow) * width + c * 32;
 #pragma unroll
             for (int e = 0; e < 32; e += 4)
-              *reinterpret_cast<float4*>(dst + e) = make_float4(__uint_as_float(ov[e]) * mul, __uint_as_float(ov[e + 1]) * mul,
-                                                                __uint_as_float(ov[e + 2]) * mul, __uint_as_float(ov[e + 3]) * mul);
+              if (live)
+                *reinterpret_cast<float4*>(dst + e) = make_float4(__uint_as_float(ov[e]) * mul, __uint_as_float(ov[e + 1]) * mul,
+                                                                  __uint_as_float(ov[e + 2]) * mul, __uint_as_float(ov[e + 3]) * mul);
           } else if (n_it > 0) {
             __nv_bfloat16* dst = out_bf + krow * width + c * 32;
 #pragma unroll
             for (int e = 0; e < 32; e += 2) {
-              __nv_bfloat162 cur = *reinterpret_cast<__nv_bfloat162*>(dst + e);
+              __nv_bfloat162 cur = __floats2bfloat162_rn(0.f, 0.f);
+              if (live) cur = *reinterpret_cast<__nv_bfloat162*>(dst + e);
               const float2 f = __bfloat1622float2(cur);
               cur = __floats2bfloat162_rn(f.x + __uint_as_float(ov[e]) * mul, f.y + __uint_as_float(ov[e + 1]) * mul);
-              *reinterpret_cast<__nv_bfloat162*>(dst + e) = cur;
+              if (live) *reinterpret_cast<__nv_bfloat162*>(dst + e) = cur;
             }
           }
         }
