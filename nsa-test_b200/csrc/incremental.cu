@@ -107,7 +107,8 @@ struct ChunkLayout {
   int Tk, ld;
   size_t o_hi, o_lo, o_lse, o_L, o_M, o_cmp, o_slc, o_win, o_gates, o_idx, o_stage, stage, total;
 };
-ChunkLayout chunk_layout(const nsa_decode_desc& d) {
+// `sums`: with the scratch for the block choice from the forward's own sums; without it the scoring kernel makes the choice
+ChunkLayout chunk_layout(const nsa_decode_desc& d, bool sums) {
   ChunkLayout L;
   const size_t BG = (size_t)d.B * d.G, R = (size_t)d.B * d.H * d.Tn;
   L.Tk = d.pos + d.Tn;
@@ -124,7 +125,8 @@ ChunkLayout chunk_layout(const nsa_decode_desc& d) {
   L.o_win = take(R * d.dv * 2);
   L.o_gates = take(R * 3 * 4);
   L.o_idx = take(BG * d.Tn * d.n * 4);
-  L.stage = std::max(nsa_cmp_attn_topn_workspace_bytes(d.B, d.H, d.G, d.Tn, d.nbp, d.dk, d.dv, d.l, d.d, d.l_prime, d.n, d.nb, NSA_FLAG_ANY_LENGTH),
+  L.stage = std::max(sums ? nsa_cmp_attn_topn_workspace_bytes(d.B, d.H, d.G, d.Tn, d.nbp, d.dk, d.dv, d.l, d.d, d.l_prime, d.n, d.nb, NSA_FLAG_ANY_LENGTH)
+                          : nsa_score_topn_workspace_bytes(d.B, d.H, d.G, d.Tn, d.dk, d.nbp, d.l, d.d, d.l_prime, d.n, NSA_BF16, NSA_FLAG_ANY_LENGTH),
                      nsa_slc_fwd_workspace_bytes(d.B, d.H, d.G, d.Tn, L.Tk, d.dk, d.dv, d.n, d.l_prime, NSA_BF16, NSA_FLAG_ANY_LENGTH));
   L.o_stage = take(L.stage);
   L.total = o;
@@ -220,7 +222,11 @@ extern "C" NSA_API int nsa_incremental_supported(const nsa_decode_desc* dp) {
 }
 
 extern "C" NSA_API size_t nsa_incremental_workspace_bytes(const nsa_decode_desc* d) {
-  return nsa_incremental_supported(d) ? chunk_layout(*d).total : 256;
+  return nsa_incremental_supported(d) ? chunk_layout(*d, true).total : 256;
+}
+
+extern "C" NSA_API size_t nsa_incremental_workspace_min_bytes(const nsa_decode_desc* d) {
+  return nsa_incremental_supported(d) ? chunk_layout(*d, false).total : 256;
 }
 
 extern "C" NSA_API int nsa_incremental_fwd(const nsa_decode_desc* dp, void* workspace, size_t workspace_bytes, void* stream) {
@@ -236,7 +242,8 @@ extern "C" NSA_API int nsa_incremental_fwd(const nsa_decode_desc* dp, void* work
   if (timeout_flagged())
     return fail(NSA_ERR_LAUNCH, "incremental_fwd: a tensor-core kernel gave up on a barrier wait earlier (device time-out); results since "
                 "then are invalid.  nsa_device_timeouts(1) reports and clears the condition");
-  const ChunkLayout L = chunk_layout(d);
+  ChunkLayout L = chunk_layout(d, true);
+  if (workspace_bytes < L.total) L = chunk_layout(d, false);
   if (!workspace || workspace_bytes < L.total) return fail(NSA_ERR_WORKSPACE, "incremental_fwd needs %zu workspace bytes, got %zu", L.total, workspace_bytes);
   cudaStream_t st = (cudaStream_t)stream;
   char* w = (char*)workspace;

@@ -150,9 +150,10 @@ struct Scratch {
   }
 };
 
-size_t stage_scratch_fwd(const nsa_layer_desc& d, const Sizes& s) {
+// `sums`: with the scratch for the block choice from the forward's own sums; without it the scoring kernel makes the choice
+size_t stage_scratch_fwd(const nsa_layer_desc& d, const Sizes& s, bool sums) {
   size_t m = nsa_score_topn_workspace_bytes(d.B, d.H, d.G, d.T, d.dk, s.nbp, d.l, d.d, d.l_prime, d.n, d.dtype, s.flags);
-  if (s.exact) m = std::max(m, nsa_cmp_attn_topn_workspace_bytes(d.B, d.H, d.G, d.T, s.nbp, d.dk, d.dv, d.l, d.d, d.l_prime, d.n, s.nb, s.flags));
+  if (s.exact && sums) m = std::max(m, nsa_cmp_attn_topn_workspace_bytes(d.B, d.H, d.G, d.T, s.nbp, d.dk, d.dv, d.l, d.d, d.l_prime, d.n, s.nb, s.flags));
   m = std::max(m, nsa_slc_fwd_workspace_bytes(d.B, d.H, d.G, d.T, d.T, d.dk, d.dv, d.n, d.l_prime, d.dtype, s.flags));
   if (s.nb > 0) m = std::max(m, nsa_cmp_phi_workspace_bytes(d.B, d.G, s.phi_rows, d.dk, d.dv, d.l, d.d, d.U, s.nbp, d.dtype, 0));
   return al256(m);
@@ -187,7 +188,13 @@ extern "C" NSA_API size_t nsa_layer_ctx_bytes(const nsa_layer_desc* d, size_t* o
 extern "C" NSA_API size_t nsa_layer_workspace_bytes(const nsa_layer_desc* d, int backward) {
   if (check_desc("layer_workspace_bytes", d)) return 0;
   const Sizes s = sizes_of(*d);
-  return backward ? fixed_scratch_bwd(*d, s) + stage_scratch_bwd(*d, s) + 256 : stage_scratch_fwd(*d, s) + 3 * s.pad_bytes + 256;
+  return backward ? fixed_scratch_bwd(*d, s) + stage_scratch_bwd(*d, s) + 256 : stage_scratch_fwd(*d, s, true) + 3 * s.pad_bytes + 256;
+}
+
+extern "C" NSA_API size_t nsa_layer_fwd_workspace_min_bytes(const nsa_layer_desc* d) {
+  if (check_desc("layer_fwd_workspace_min_bytes", d)) return 0;
+  const Sizes s = sizes_of(*d);
+  return stage_scratch_fwd(*d, s, false) + 3 * s.pad_bytes + 256;
 }
 
 extern "C" NSA_API int nsa_layer_fwd(const nsa_layer_desc* dp, const void* q, const void* k_slc, const void* v_slc, const void* k_cmp_src,
@@ -203,7 +210,7 @@ extern "C" NSA_API int nsa_layer_fwd(const nsa_layer_desc* dp, const void* q, co
   size_t off[NSA_CTX_PIECES + 1];
   ctx_layout(d, off);
   if (ctx_bytes < off[NSA_CTX_PIECES]) return fail(NSA_ERR_WORKSPACE, "layer_fwd needs a context of %zu bytes, got %zu", off[NSA_CTX_PIECES], ctx_bytes);
-  const size_t need = nsa_layer_workspace_bytes(dp, 0);
+  const size_t need = nsa_layer_fwd_workspace_min_bytes(dp);
   if (!workspace || workspace_bytes < need) return fail(NSA_ERR_WORKSPACE, "layer_fwd needs %zu workspace bytes, got %zu", need, workspace_bytes);
   cudaStream_t st = (cudaStream_t)stream;
   char* c = (char*)ctx;

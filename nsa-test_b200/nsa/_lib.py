@@ -86,6 +86,7 @@ PROTOTYPES = {
     "nsa_gate_mlp_bwd": (c_int, [_P] * 10 + [c_int64, c_int, c_int, c_int, c_int, _P, c_size_t, _P]),
     "nsa_layer_ctx_bytes": (c_size_t, [_DESCP, POINTER(c_size_t)]),
     "nsa_layer_workspace_bytes": (c_size_t, [_DESCP, c_int]),
+    "nsa_layer_fwd_workspace_min_bytes": (c_size_t, [_DESCP]),
     "nsa_layer_fwd": (c_int, [_DESCP] + [_P] * 16 + [c_size_t, _P, c_size_t, _P]),
     "nsa_layer_bwd": (c_int, [_DESCP] + [_P] * 10 + [c_size_t] + [_P] * 14 + [_P, c_size_t, _P]),
     "nsa_decode_supported": (c_int, [_DECP]),
@@ -95,6 +96,7 @@ PROTOTYPES = {
     "nsa_cache_append": (c_int, [_DECP, POINTER(_P), _I64P, c_int, c_int, c_int, _P, c_size_t, _P]),
     "nsa_incremental_supported": (c_int, [_DECP]),
     "nsa_incremental_workspace_bytes": (c_size_t, [_DECP]),
+    "nsa_incremental_workspace_min_bytes": (c_size_t, [_DECP]),
     "nsa_incremental_fwd": (c_int, [_DECP, _P, c_size_t, _P]),
     "nsa_phi_pool_fwd": (c_int, [_P, _P, _P, _I64P, _P, _P] + [c_int] * 10 + [_P]),
     "nsa_phi_pool_bwd": (c_int, [_P] * 7 + [c_int] * 9 + [_P]),

@@ -145,6 +145,15 @@ def cmp_attn_fwd(q, k_cmp, v_cmp, block_ends, scale: float, blocks=None, q_pos0:
     return (o, L, M) if k_lo is None else (o, L, M, lse2)
 
 
+def _scratch(dev, nbytes: int, least):
+    """A workspace of ``nbytes``, or of the ``least()`` the call takes where memory does not hold that."""
+    try:
+        return torch.empty(nbytes, device=dev, dtype=torch.uint8), nbytes
+    except torch.OutOfMemoryError:
+        nbytes = least()
+        return torch.empty(nbytes, device=dev, dtype=torch.uint8), nbytes
+
+
 def cmp_attn_topn_fwd(q, k_hi, k_lo, k_cmp, v_cmp, block_ends, l: int, d: int, l_prime: int, n: int, n_fixed: int, nb: int, scale: float,
                       q_pos0: int = 0, any_length: bool = False):
     """The exact-key form of ``cmp_attn_fwd`` with the Eq. 8-11 block choice -> (o, L, M, lse2, indices); k_cmp the fp32 keys."""
@@ -157,12 +166,8 @@ def cmp_attn_topn_fwd(q, k_hi, k_lo, k_cmp, v_cmp, block_ends, l: int, d: int, l
     lse2 = torch.empty(B, H, T, device=dev, dtype=torch.float32)
     idx = torch.empty(B, G, T, n, device=dev, dtype=torch.int32)
     flags = _flags(False, any_length=any_length)
-    nbytes = lib.nsa_cmp_attn_topn_workspace_bytes(B, H, G, T, NB, dk, dv, int(l), int(d), int(l_prime), int(n), int(nb), flags)
-    try:
-        ws = torch.empty(nbytes, device=dev, dtype=torch.uint8)
-    except torch.OutOfMemoryError:      # the same choice from the scoring kernel's own, smaller scratch
-        nbytes = lib.nsa_score_topn_workspace_bytes(B, H, G, T, dk, NB, int(l), int(d), int(l_prime), int(n), dtype_code(q), flags)
-        ws = torch.empty(nbytes, device=dev, dtype=torch.uint8)
+    ws, nbytes = _scratch(dev, lib.nsa_cmp_attn_topn_workspace_bytes(B, H, G, T, NB, dk, dv, int(l), int(d), int(l_prime), int(n), int(nb), flags),
+                          lambda: lib.nsa_score_topn_workspace_bytes(B, H, G, T, dk, NB, int(l), int(d), int(l_prime), int(n), dtype_code(q), flags))
     with torch.cuda.device(dev):
         check(lib.nsa_cmp_attn_topn_fwd(ptr(q), ptr(k_hi), ptr(k_lo), ptr(k_cmp), ptr(v_cmp), ptr(be), ptr(o), ptr(L), ptr(M), ptr(lse2), ptr(idx),
                                         i64(_fwd_strides(q, k_hi, v_cmp, o, L, M)), B, H, G, T, NB, NB, dk, dv, int(l), int(d), int(l_prime), int(n),
@@ -207,8 +212,7 @@ def decode_fwd(desc, dev) -> None:
 
 def incremental_fwd(desc, dev) -> None:
     """nsa_incremental_fwd likewise."""
-    nbytes = lib.nsa_incremental_workspace_bytes(desc)
-    ws = torch.empty(nbytes, device=dev, dtype=torch.uint8)
+    ws, nbytes = _scratch(dev, lib.nsa_incremental_workspace_bytes(desc), lambda: lib.nsa_incremental_workspace_min_bytes(desc))
     with torch.cuda.device(dev):
         check(lib.nsa_incremental_fwd(desc, ptr(ws), nbytes, stream_ptr(dev)), "nsa_incremental_fwd")
 
@@ -598,9 +602,8 @@ def layer_fwd(desc, q, kv_slc, kv_cmp, kv_win, gate_logits, phi, indices=None):
     if ctx_bytes == 0:
         raise _lib.NSAKernelError(f"nsa_layer_ctx_bytes: {lib.nsa_last_error().decode()}")
     ctx = torch.empty(ctx_bytes, device=dev, dtype=torch.uint8)
-    nbytes = lib.nsa_layer_workspace_bytes(ctypes.byref(desc), 0)
-    ws = torch.empty(nbytes, device=dev, dtype=torch.uint8)
     out = _mixed_out(desc, q)
+    ws, nbytes = _scratch(dev, lib.nsa_layer_workspace_bytes(ctypes.byref(desc), 0), lambda: lib.nsa_layer_fwd_workspace_min_bytes(ctypes.byref(desc)))
     pos, w1, b1, w2, b2 = phi
     with torch.cuda.device(dev):
         check(lib.nsa_layer_fwd(ctypes.byref(desc), ptr(q), ptr(kv_slc[0]), ptr(kv_slc[1]), ptr(kv_cmp[0]), ptr(kv_cmp[1]), ptr(kv_win[0]),

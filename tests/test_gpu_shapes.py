@@ -485,3 +485,44 @@ def test_layer_without_an_upstream_gradient(monkeypatch, c_layer, token_major):
     ins = (q, k, v, logits, *phi)
     for g, t in zip(torch.autograd.grad(DropGradient.apply(out).sum(), ins), ins):
         assert g.shape == t.shape and not g.any()
+
+
+@pytest.mark.parametrize("pos", [0, 300])
+def test_block_choice_in_the_smaller_scratch(monkeypatch, pos):
+    """Where memory does not hold the scratch of the faster block choice, the layer and a chunk against a cache run in the smaller
+    one, and choose the same blocks (the compressed branch's sums run alike: outputs bit for bit)."""
+    import nsa
+    from nsa import incremental as I, ops
+    from nsa.kernels import nsa_layer
+    H, G, T = 16, 8, 7201
+    cfg = nsa.NSAConfig(d_model=64, head_dim_qk=64, head_dim_v=64, n_heads=H, n_kv_groups=G, w=128)
+    inp = O.make_inputs(1, H, G, pos + T, 64, 64, 64, 32, seed=T, block_offset_std=0.5, dtype=torch.bfloat16)
+    q, k, v = (inp[x].to(DEV, torch.bfloat16) for x in ("q", "k", "v"))
+    phi = tuple(getattr(inp["phi"], n_).to(DEV) for n_ in ("pos_embed", "w1", "b1", "w2", "b2"))
+    logits = torch.zeros(1, pos + T, 3 * H, device=DEV)
+    if pos:
+        cache = I.NSACache(cfg, 1, pos + T, DEV, shared_kv=True)
+        cache.append(phi, k, v)
+        run = lambda: I.nsa_layer_incremental(q[:, :, pos:].contiguous(), logits[:, pos:], cache, return_info=True)
+    else:
+        run = lambda: nsa_layer(q, k, v, logits, phi, cfg, return_info=True)
+    with torch.no_grad():
+        a, info_a = run()
+        real, sizes = ops._scratch, []
+
+        def no_room(dev, nbytes, least):
+            sizes.append((nbytes, least()))
+            return real(dev, least(), None)
+        monkeypatch.setattr(ops, "_scratch", no_room)
+        b, info_b = run()
+    torch.cuda.synchronize()
+    _no_timeouts()
+    assert sizes and all(more > less for more, less in sizes)
+    assert torch.equal(info_a["o_cmp"], info_b["o_cmp"]) and torch.equal(info_a["indices"].sort(-1).values, info_b["indices"].sort(-1).values)
+    assert max_abs(a.float(), b.float()) < 2e-2
+
+
+def test_scratch_falls_back_where_memory_runs_out():
+    from nsa import ops
+    ws, n_ = ops._scratch(torch.device(DEV), 1 << 46, lambda: 1000)
+    assert n_ == ws.numel() == 1000
