@@ -555,6 +555,9 @@ __global__ void __launch_bounds__(256) pack_rows_kernel(const uint4* __restrict_
 // ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
+// Bounds of a launch's dynamic shared memory.  The kernels' attribute is set to them and not to a call's own size: it is shared by
+// all host threads.  (A tile kernel's static word comes on top: 256 bytes are left for it.)
+constexpr size_t kTileSmemMax = 227 * 1024 - 256, kRowsSmemMax = 200 * 1024;
 bool score_sm100_supported(int H, int G, int T, int dk, int nbp, int l, int d, int lprime, int n) {
   if (!(dk == 192 || dk == 128 || dk == 64) || G <= 0 || H % G != 0) return false;
   const int hpg = H / G;
@@ -562,7 +565,7 @@ bool score_sm100_supported(int H, int G, int T, int dk, int nbp, int l, int d, i
   const int s_ = lprime / d;
   const size_t smem = 4 * (size_t)128 * dk * 2 + 2 * (size_t)hpg * 512 + 256 + 1024;
   const size_t rows_smem = 4 * (size_t)(nbp / (s_ > 0 ? s_ : 1)) * sizeof(float);
-  return smem <= 227 * 1024 && rows_smem <= 200 * 1024 && T > 0 && nbp > 0 && 128 % s_ == 0 && n >= 1 &&
+  return smem <= kTileSmemMax && rows_smem <= kRowsSmemMax && T > 0 && nbp > 0 && 128 % s_ == 0 && n >= 1 &&
          n <= kScoreMaxN;
 }
 
@@ -589,9 +592,9 @@ static int launch_score_t(const CUtensorMap& tq, const CUtensorMap& thi, const C
   const int state_off = tiles, state_bytes = 2 * hpg * 128 * 4;
   const int bar_off = state_off + state_bytes;
   const int dyn = bar_off + 256 + 1024;
-  if (dyn > 227 * 1024) return fail(NSA_ERR_UNSUPPORTED, "score_topn: %d bytes of shared memory needed", dyn);
+  if (dyn > (int)kTileSmemMax) return fail(NSA_ERR_UNSUPPORTED, "score_topn: %d bytes of shared memory needed", dyn);
   auto kern = score_topn_tc_kernel<DK, LISTED>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmemMax) != cudaSuccess)
     return fail(NSA_ERR_LAUNCH, "score_topn: cannot reserve shared memory");
   KernelTimer kt("score_topn_tc", st);
   kern<<<dim3((p.T + 127) / 128, p.B * p.G), 384, dyn, st>>>(tq, thi, tlo, p, hpg, state_off, bar_off);
@@ -613,7 +616,7 @@ static int launch_topn_rows(const float* sel, int32_t* out, int B, int G, int T,
     NSA_ROWS_CASE(32);
   } else {
     const size_t sm = 4 * (size_t)n_sel * sizeof(float);
-    if (cudaFuncSetAttribute(topn_rows_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
+    if (cudaFuncSetAttribute(topn_rows_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmemMax) != cudaSuccess)
       return fail(NSA_ERR_LAUNCH, "score_topn: cannot reserve shared memory for the row selection");
     topn_rows_kernel<0><<<grid, 128, sm, st>>>(sel, out, rows, T, n_sel, 128 / s_, l, d, nb, lprime, n, n_fixed, q0);
   }

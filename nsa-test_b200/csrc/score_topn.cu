@@ -15,6 +15,7 @@ namespace nsa {
 
 constexpr int kThreads = 256;
 constexpr int kMaxN = 64;
+constexpr size_t kSmemMax = 200 * 1024;   // what a launch may ask for, and what the kernels' attribute is set to (it is shared by all host threads)
 
 __device__ __forceinline__ float block_max(float x, float* red) {
   x = warp_max(x);
@@ -275,7 +276,7 @@ extern "C" NSA_API int nsa_score_topn(const void* q, const int64_t* qs, const fl
   auto smem_for = [&](int hb) { return ((size_t)hpg * dk + (size_t)hb * (nbp + a_ + s_) + n_sel + 16 + kMaxN) * sizeof(float); };
   const int hb = (hpg % 4 == 0 && smem_for(4) <= 160 * 1024) ? 4 : (hpg % 2 == 0 && smem_for(2) <= 160 * 1024) ? 2 : 1;
   const size_t sm = smem_for(hb);
-  if (sm > 200 * 1024) return fail(NSA_ERR_UNSUPPORTED, "score_topn: %zu bytes of shared memory needed", sm);
+  if (sm > kSmemMax) return fail(NSA_ERR_UNSUPPORTED, "score_topn: %zu bytes of shared memory needed", sm);
   if (dtype != NSA_F32 && dtype != NSA_BF16) return fail(NSA_ERR_ARG, "score_topn: unsupported dtype %d", dtype);
   cudaStream_t st = (cudaStream_t)stream;
   const int q0 = q_pos0;
@@ -307,7 +308,7 @@ extern "C" NSA_API int nsa_score_topn(const void* q, const int64_t* qs, const fl
   dim3 grid(T, B * G);
 #define NSA_SCORE_LAUNCH(TYPE, HB_)                                                                                    \
   do {                                                                                                                 \
-    cudaFuncSetAttribute(score_topn_kernel<TYPE, HB_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);          \
+    cudaFuncSetAttribute(score_topn_kernel<TYPE, HB_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);    \
     score_topn_kernel<TYPE, HB_><<<grid, kThreads, sm, st>>>((const TYPE*)q, qs[0], qs[1], qs[2], qs[3], k_cmp,        \
                                                              block_ends, indices_out, H, G, T, dk, nbp, a_, s_, n_sel, \
                                                              l_prime, n, n_fixed, scale, q0, logits);                  \
@@ -327,8 +328,8 @@ extern "C" NSA_API int nsa_topn_from_scores(const float* scores, int32_t* indice
   NSA_REQUIRE(G > 0 && H % G == 0 && l_prime > 0 && n > 0 && n <= kMaxN && n_sel > 0, "topn_from_scores: bad sizes");
   if (B * G == 0 || T == 0) return NSA_OK;
   const size_t sm = ((size_t)n_sel + 16 + kMaxN) * sizeof(float);
-  if (sm > 200 * 1024) return fail(NSA_ERR_UNSUPPORTED, "topn_from_scores: n_sel too large");
-  cudaFuncSetAttribute(topn_from_scores_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (sm > kSmemMax) return fail(NSA_ERR_UNSUPPORTED, "topn_from_scores: n_sel too large");
+  cudaFuncSetAttribute(topn_from_scores_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
   topn_from_scores_kernel<<<dim3(T, B * G), kThreads, sm, (cudaStream_t)stream>>>(scores, indices_out, H, G, T, n_sel,
                                                                                  l_prime, n, n_fixed);
   return check_launch("topn_from_scores");

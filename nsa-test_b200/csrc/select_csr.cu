@@ -13,6 +13,9 @@
 namespace nsa {
 
 constexpr int kChunk = 128;      // queries per histogram chunk
+// Bounds of the two kernels' dynamic shared memory: the attribute that admits a launch belongs to the kernel and is shared by all
+// host threads, so it is set to the bound, never to the size of one call, which another thread's launch may exceed.
+constexpr size_t kCountSmemMax = 160 * 1024, kFillSmemMax = 200 * 1024;
 constexpr int kFillWarps = 8;    // warps ordering the entries of a chunk (one when the counters of eight do not fit)
 
 struct CsrArgs {
@@ -172,7 +175,7 @@ int build_slc_csr(const int* indices, const int64_t* sidx, int B, int G, int Tq,
     return fail(NSA_ERR_WORKSPACE, "selection backward needs %zu workspace bytes, got %zu", total, workspace_bytes);
   if (nslots > 32) return fail(NSA_ERR_UNSUPPORTED, "selection supports at most 32 slots per query here");
   if (Tq >= (1 << 24)) return fail(NSA_ERR_UNSUPPORTED, "selection inverse index supports fewer than 2^24 queries");
-  if ((size_t)a.nblk * sizeof(int) > 160 * 1024) return fail(NSA_ERR_UNSUPPORTED, "too many key blocks (%d)", a.nblk);
+  if ((size_t)a.nblk * sizeof(int) > kCountSmemMax) return fail(NSA_ERR_UNSUPPORTED, "too many key blocks (%d)", a.nblk);
   a.indices = indices;
   for (int i = 0; i < 4; ++i) a.sidx[i] = sidx[i];
   a.B = B; a.G = G; a.Tq = Tq; a.Tkv = Tkv; a.nslots = nslots; a.lprime = lprime; a.causal = causal; a.q0 = q0;
@@ -183,10 +186,10 @@ int build_slc_csr(const int* indices, const int64_t* sidx, int B, int G, int Tq,
   a.slots_pad = 1;
   while (a.slots_pad < nslots) a.slots_pad *= 2;
   const size_t sm = (size_t)a.nblk * sizeof(int);
-  const int W = (size_t)a.nblk * (sizeof(int) + kFillWarps) <= 200 * 1024 ? kFillWarps : 1;
+  const int W = (size_t)a.nblk * (sizeof(int) + kFillWarps) <= kFillSmemMax ? kFillWarps : 1;
   const size_t sm_fill = (size_t)a.nblk * (sizeof(int) + W);
-  if (sm > 48 * 1024) cudaFuncSetAttribute(csr_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  if (sm_fill > 48 * 1024) cudaFuncSetAttribute(csr_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_fill);
+  if (sm > 48 * 1024) cudaFuncSetAttribute(csr_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCountSmemMax);
+  if (sm_fill > 48 * 1024) cudaFuncSetAttribute(csr_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFillSmemMax);
   KernelTimer kt("slc_inverse_index", st);
   dim3 grid(a.nchunks, B * G);
   csr_count<<<grid, 256, sm, st>>>(a);

@@ -43,6 +43,7 @@ static int slc_nparts(int B, int G, int Tq, int nslots) {
 __device__ __forceinline__ int slc_range(const int* off, int nblk, int nparts, int qpc) {
   return ((off[nblk] + nparts - 1) / nparts + qpc - 1) / qpc * qpc;
 }
+constexpr size_t kMergeSmemMax = 100 * 1024;   // a query's partials in the merge kernels; also their attribute, which all host threads share
 constexpr float kLn2f = 0.6931471805599453f;
 constexpr float kLog2ef = 1.4426950408889634f;
 
@@ -1242,9 +1243,9 @@ static int launch_slc_fwd_t(const CUtensorMap& tk, const CUtensorMap& tv, const 
   const int64_t rows = (int64_t)p.B * p.H * p.Tq;
   const size_t qbytes = (size_t)p.nslots * p.hpg * DV * 2;  // one query's partials
   KernelTimer kt(mix.out ? "slc_combine_fwd_mix" : "slc_combine_fwd", st);
-  if (p.hpg <= 32 && qbytes <= 100 * 1024 && (int64_t)p.B * p.G * p.Tq < (1ll << 31)) {
+  if (p.hpg <= 32 && qbytes <= kMergeSmemMax && (int64_t)p.B * p.G * p.Tq < (1ll << 31)) {
     auto kc = slc_combine_fwd_bulk_kernel<DV>;
-    if (cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qbytes) != cudaSuccess)
+    if (cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMergeSmemMax) != cudaSuccess)
       return fail(NSA_ERR_LAUNCH, "slc_combine_fwd: cannot reserve shared memory");
     kc<<<(unsigned)((int64_t)p.B * p.G * p.Tq), p.hpg * 32, qbytes, st>>>(p.o_part, p.st_part, indices, sidx[0], sidx[1], sidx[2], sidx[3],
                                                                       out, L, M, p.B, p.H, p.G, p.Tq, p.Tk, p.nslots, 64, p.q0, p.timeouts, mix);
@@ -1338,9 +1339,9 @@ static int launch_slc_bwd_t(const CUtensorMap& tk, const CUtensorMap& tv, const 
   {
     KernelTimer kt("slc_combine_dq", st);
     const size_t qbytes = (size_t)p.nslots * p.hpg * DK * 2;  // one query's partials
-    if (p.hpg <= 32 && qbytes <= 100 * 1024 && (int64_t)p.B * p.G * p.Tq < (1ll << 31)) {
+    if (p.hpg <= 32 && qbytes <= kMergeSmemMax && (int64_t)p.B * p.G * p.Tq < (1ll << 31)) {
       auto kc = slc_combine_dq_bulk_kernel<DK>;
-      if (cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qbytes) != cudaSuccess)
+      if (cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMergeSmemMax) != cudaSuccess)
         return fail(NSA_ERR_LAUNCH, "slc_combine_dq: cannot reserve shared memory");
       kc<<<(unsigned)((int64_t)p.B * p.G * p.Tq), p.hpg * 32, qbytes, st>>>(p.dq_part, indices, sidx[0], sidx[1], sidx[2], sidx[3], dq, p.B,
                                                                         p.H, p.G, p.Tq, p.Tk, p.nslots, 64, p.scale, p.q0, p.timeouts,

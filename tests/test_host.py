@@ -197,3 +197,19 @@ def test_compression_backward_scratch_covers_its_column_sums(BG, dk, dv):
         others = [BG * nb_rows * dk * 4, BG * nb_rows * U * 4, BG * nbp * dv * 4, BG * rows * U * 2, parts * BG * l * U * 4, l * U * 4, U * dk * 2]
         reserved = lib.nsa_cmp_phi_workspace_bytes(1, BG, rows, dk, dv, l, d, U, nbp, BF16, 1) - 256 - sum(map(al, others))
         assert reserved >= chunks(BG * nb, dk) * dk * 4, (T, reserved)
+
+
+def test_shared_memory_attributes_do_not_depend_on_the_call():
+    """A kernel's dynamic shared memory attribute is shared by all host threads: set to one call's size, another thread's larger
+    launch would be refused.  Every place sets a constant (k..., SM::..., or a size made of template arguments alone)."""
+    import glob
+    import os
+    import re
+    import nsa
+    src = os.path.join(os.path.dirname(nsa.__file__), "..", "csrc", "*.cu")
+    sizes = [(os.path.basename(f), m) for f in glob.glob(src)
+             for m in re.findall(r"cudaFuncAttributeMaxDynamicSharedMemorySize,\s*([^;]*?)\)\s*(?:;|!=|==)", open(f).read())]
+    assert len(sizes) > 10
+    by_template = {("attn_generic.cu", "(int)sm"), ("attn_generic.cu", "(int)sm_dkv"), ("attn_mma.cu", "sm")}
+    for f, size in sizes:
+        assert re.fullmatch(r"(\(int\))?(k[A-Z]\w*|\w+(<[^>]*>)?::k\w+)", size) or (f, size) in by_template, (f, size)
