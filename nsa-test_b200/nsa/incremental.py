@@ -84,8 +84,10 @@ class NSACache:
         return p0
 
     def _append_in_place(self, phi_params, tensors, p0: int, Tn: int, nb: int) -> bool:
-        """The append as one library call; False where a tensor is not of the cache's type, shape and device."""
+        """The append as one library call; False where a tensor is not of the cache's type, shape and CUDA device."""
         c, dev = self.config, self.k_slc.device
+        if dev.type != "cuda":
+            return False
         B = self.k_slc.shape[0]
         for i, t in enumerate(tensors):
             want = (B, c.n_kv_groups, c.head_dim_qk, Tn) if i % 2 == 0 else (B, c.n_kv_groups, Tn, c.head_dim_v)

@@ -213,3 +213,14 @@ def test_shared_memory_attributes_do_not_depend_on_the_call():
     by_template = {("attn_generic.cu", "(int)sm"), ("attn_generic.cu", "(int)sm_dkv"), ("attn_mma.cu", "sm")}
     for f, size in sizes:
         assert re.fullmatch(r"(\(int\))?(k[A-Z]\w*|\w+(<[^>]*>)?::k\w+)", size) or (f, size) in by_template, (f, size)
+
+
+def test_append_to_a_cache_in_host_memory():
+    """Tokens before the first compressed block are only copied, wherever the cache lies."""
+    from nsa import NSAConfig
+    from nsa.incremental import NSACache
+    cache = NSACache(NSAConfig(d_model=64, head_dim_qk=16, head_dim_v=8, n_heads=4, n_kv_groups=2), 1, 64, "cpu", shared_kv=True)
+    phi = tuple(torch.zeros(*n_) for n_ in ((32, 32), (32, 48), (32,), (16, 32), (16,)))
+    k, v = torch.randn(1, 2, 16, 20).bfloat16(), torch.randn(1, 2, 20, 8).bfloat16()
+    assert cache.append(phi, k, v) == 0 and (cache.length, cache.n_blocks) == (20, 0)
+    assert torch.equal(cache.k_slc[..., :20], k) and torch.equal(cache.v_slc[:, :, :20], v)
