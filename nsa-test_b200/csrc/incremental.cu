@@ -67,7 +67,7 @@ __global__ void cast_params_kernel(const __grid_constant__ CastArgs a) {
 
 struct AppendLayout {
   int T, lo;                // tokens the new blocks cover, the first of them
-  size_t o_par[5], o_saved, saved, o_ws, ws, total;
+  size_t o_par[5], o_saved, saved, o_ws, ws, o_kc, total;
 };
 AppendLayout append_layout(const nsa_decode_desc& d, int dtype) {
   AppendLayout L = {};
@@ -82,6 +82,9 @@ AppendLayout append_layout(const nsa_decode_desc& d, int dtype) {
     L.o_saved = take(L.saved);
     L.ws = nsa_cmp_phi_workspace_bytes(d.B, d.G, L.T, d.dk, d.dv, d.l, d.d, d.U, d.nbp, dtype, 0);
     L.o_ws = take(L.ws);
+    int nbq = 1;
+    while (nbq < d.nb_new) nbq *= 2;
+    L.o_kc = take((size_t)d.B * d.G * d.dk * nbq * 4);
   }
   L.total = std::max<size_t>(o, 256);
   return L;
@@ -162,7 +165,7 @@ int compress_blocks(const nsa_decode_desc& d, const void* k, const void* v, int 
   const int64_t vst[4] = {(int64_t)d.G * d.cap * d.dv, (int64_t)d.cap * d.dv, d.dv, 1};
   return cmp_phi_fwd_strided(ks, d.cap, (int64_t)d.dk * d.cap, vs, vst, par[0], par[1], par[2], par[3], par[4], (float*)d.k_cmp + b0,
                              d.k_cmp_lp ? (char*)d.k_cmp_lp + b0 * es : nullptr, (char*)d.v_cmp + (size_t)b0 * d.dv * es, d.B, d.G, L.T, L.T, d.dk,
-                             d.dv, d.l, d.d, d.U, d.nbp, false, dtype, w + L.o_saved, L.saved, w + L.o_ws, L.ws, st);
+                             d.dv, d.l, d.d, d.U, d.nbp, (float*)(w + L.o_kc), dtype, w + L.o_saved, L.saved, w + L.o_ws, L.ws, st);
 }
 
 }  // namespace nsa

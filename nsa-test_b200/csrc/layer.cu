@@ -233,7 +233,7 @@ extern "C" NSA_API int nsa_layer_fwd(const nsa_layer_desc* dp, const void* q, co
     const int64_t vs[4] = {(int64_t)d.G * d.T * d.dv, (int64_t)d.T * d.dv, d.dv, 1};
     if (int rc = cmp_phi_fwd_strided(k_phi, s.phi_rows, (int64_t)d.dk * s.phi_rows, v_cmp_src, vs, pos_embed, w1, b1, w2, b2, k_cmp,
                                      exact ? nullptr : piece(NSA_CTX_K_CMP_LP), piece(NSA_CTX_V_CMP), d.B, d.G, d.T, s.phi_rows, d.dk, d.dv, d.l, d.d, d.U, s.nbp,
-                                     true, d.dtype, piece(NSA_CTX_PHI_SAVED), off[NSA_CTX_PHI_SAVED + 1] - off[NSA_CTX_PHI_SAVED], workspace,
+                                     nullptr, d.dtype, piece(NSA_CTX_PHI_SAVED), off[NSA_CTX_PHI_SAVED + 1] - off[NSA_CTX_PHI_SAVED], workspace,
                                      workspace_bytes, st))
       return rc;
   } else {

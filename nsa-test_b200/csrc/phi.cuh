@@ -9,9 +9,10 @@ namespace nsa {
 
 // Scratch and saved sizes as for nsa_cmp_phi_fwd with `arows` tokens, the rows of W1 K that are formed per plane: T, or where
 // phi_pool_bwd_fused_ok more, the keys' rows being zero there (T no multiple of 8 lets the products choose a slower kernel).  v_cmp planes and k_cmp rows are nbp apart.
+// kc: scratch of BG * dk * (next power of two of the blocks) floats, or null (see phi_mlp.cu).
 int cmp_phi_fwd_strided(const void* k, int64_t k_ld, int64_t k_plane, const void* v, const int64_t* vs, const float* pos_embed,
                         const float* w1, const float* b1, const float* w2, const float* b2, float* k_cmp, void* k_cmp_lp, void* v_cmp,
-                        int B, int G, int T, int arows, int dk, int dv, int l, int d, int U, int nbp, bool pad, int dtype, void* saved,
+                        int B, int G, int T, int arows, int dk, int dv, int l, int d, int U, int nbp, float* kc, int dtype, void* saved,
                         size_t saved_bytes, void* workspace, size_t workspace_bytes, cudaStream_t st);
 int cmp_phi_bwd_ld(const void* k, int64_t k_ld, const float* pos_embed, const float* w1, const float* w2, const void* dk_cmp,
                    const void* dv_cmp, const void* saved, size_t saved_bytes, void* dk_out, void* dv_out, float* dpos, float* dw1, float* db1,

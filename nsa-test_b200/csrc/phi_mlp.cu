@@ -111,16 +111,16 @@ __global__ void c_table_kernel(const float* __restrict__ pos, const float* __res
   for (int m = 0; m < l; ++m) acc = fmaf(pos[j * l + m], w1[(int64_t)u * (dk + l) + dk + m], acc);
   c[i] = acc;
 }
-// k_cmp[bg, c, i] += b2[c] for the real blocks, zeros in the columns nb..cols behind them (rows are nbp apart); an optional
-// copy in the I/O type is written alongside
+// k_cmp[bg, c, i] = in[bg, c, i] + b2[c] for the real blocks, zeros in the columns nb..cols behind them (rows in_ld and nbp apart;
+// in may be k_cmp); an optional copy in the I/O type is written alongside
 template <typename T>
-__global__ void kcmp_finish_kernel(float* __restrict__ k_cmp, const float* __restrict__ b2, T* __restrict__ lp, int dk, int nb, int cols,
-                                   int nbp, int64_t total) {
+__global__ void kcmp_finish_kernel(const float* in, int in_ld, float* k_cmp, const float* __restrict__ b2, T* __restrict__ lp, int dk, int nb,
+                                   int cols, int nbp, int64_t total) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const int blk = i % cols, c = (i / cols) % dk;
   const int64_t at = i / cols * nbp + blk;
-  float x = k_cmp[at];
+  float x = in[i / cols * in_ld + blk];
   if (blk < nb && b2) x += b2[c];
   if (blk >= nb) x = 0.f;
   k_cmp[at] = x;
@@ -282,11 +282,14 @@ extern "C" NSA_API size_t nsa_cmp_phi_workspace_bytes(int B, int G, int T, int d
 }
 
 // Forward on keys whose rows lie k_ld elements apart (planes k_plane) and values with strides vs; the nb blocks go to the first
-// columns of rows nbp apart and to rows of planes nbp apart.  `pad`: the rest of those rows and planes is cleared.
+// columns of rows nbp apart and to rows of planes nbp apart.  Without `kc` the rest of those rows and planes is cleared.  With it
+// (scratch [BG, dk, nbq], nbq the next power of two of nb) the rest stays, and the second product is formed there: written
+// into rows another distance apart, the library's product of a single block adds in another order.
 int nsa::cmp_phi_fwd_strided(const void* k, int64_t k_ld, int64_t k_plane, const void* v, const int64_t* vs, const float* pos_embed,
                              const float* w1, const float* b1, const float* w2, const float* b2, float* k_cmp, void* k_cmp_lp, void* v_cmp,
-                             int B, int G, int T, int arows, int dk, int dv, int l, int d, int U, int nbp, bool pad, int dtype, void* saved,
+                             int B, int G, int T, int arows, int dk, int dv, int l, int d, int U, int nbp, float* kc, int dtype, void* saved,
                              size_t saved_bytes, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+  const bool pad = !kc;
   const int nb = (T - l) / d + 1, BG = B * G;
   const SavedLayout sl = saved_layout(B, G, arows, l, d, U);
   if (saved_bytes < sl.total) return fail(NSA_ERR_WORKSPACE, "cmp_phi_fwd needs %zu bytes for the backward's inputs, got %zu", sl.total, saved_bytes);
@@ -327,15 +330,18 @@ int nsa::cmp_phi_fwd_strided(const void* k, int64_t k_ld, int64_t k_plane, const
     if (pad && nbp > nb)
       cudaMemset2DAsync((char*)v_cmp + (size_t)nb * dv * es, (size_t)nbp * dv * es, 0, (size_t)(nbp - nb) * dv * es, BG, st);
     // k_cmp[bg] (dk x nbp, row-major) = (hbar[bg] W2^T)^T; column-major: C(nb x dk, ld nbp) = op_T(hbar (U x nb)) W2 (U x dk)
-    if (int rc = gemm(h, CUBLAS_OP_T, CUBLAS_OP_N, nb, dk, U, hbar, CUDA_R_32F, U, (long long)nb * U, w2, CUDA_R_32F, U, 0, 0.f, k_cmp,
-                      CUDA_R_32F, nbp, (long long)dk * nbp, BG, "cmp_phi_fwd (hbar W2^T)"))
+    float* to = kc ? kc : k_cmp;
+    int ldc = kc ? 1 : nbp;
+    while (kc && ldc < nb) ldc *= 2;
+    if (int rc = gemm(h, CUBLAS_OP_T, CUBLAS_OP_N, nb, dk, U, hbar, CUDA_R_32F, U, (long long)nb * U, w2, CUDA_R_32F, U, 0, 0.f, to,
+                      CUDA_R_32F, ldc, (long long)dk * ldc, BG, "cmp_phi_fwd (hbar W2^T)"))
       return rc;
     const int cols = pad ? nbp : nb;
     const int64_t total = (int64_t)BG * dk * cols;
     if (dtype == NSA_BF16)
-      kcmp_finish_kernel<__nv_bfloat16><<<blocks_for(total), 256, 0, st>>>(k_cmp, b2, (__nv_bfloat16*)k_cmp_lp, dk, nb, cols, nbp, total);
+      kcmp_finish_kernel<__nv_bfloat16><<<blocks_for(total), 256, 0, st>>>(to, ldc, k_cmp, b2, (__nv_bfloat16*)k_cmp_lp, dk, nb, cols, nbp, total);
     else
-      kcmp_finish_kernel<float><<<blocks_for(total), 256, 0, st>>>(k_cmp, b2, (float*)k_cmp_lp, dk, nb, cols, nbp, total);
+      kcmp_finish_kernel<float><<<blocks_for(total), 256, 0, st>>>(to, ldc, k_cmp, b2, (float*)k_cmp_lp, dk, nb, cols, nbp, total);
   }
   return check_launch("cmp_phi_fwd");
 }
@@ -352,7 +358,7 @@ extern "C" NSA_API int nsa_cmp_phi_fwd(const void* k, const void* v, const float
   NSA_REQUIRE(nbp >= nb, "cmp_phi_fwd: nbp = %d holds fewer than the %d blocks of the sequence", nbp, nb);
   const int64_t vs[4] = {(int64_t)G * T * dv, (int64_t)T * dv, dv, 1};
   return cmp_phi_fwd_strided(k, T, (int64_t)dk * T, v, vs, pos_embed, w1, b1, w2, b2, k_cmp, k_cmp_lp, v_cmp, B, G, T, T, dk, dv, l, d, U,
-                             nbp, true, dtype, saved, saved_bytes, workspace, workspace_bytes, (cudaStream_t)stream);
+                             nbp, nullptr, dtype, saved, saved_bytes, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 extern "C" NSA_API int nsa_cmp_phi_bwd(const void* k, const float* pos_embed, const float* w1, const float* w2, const void* dk_cmp,

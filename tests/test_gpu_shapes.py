@@ -109,7 +109,7 @@ def _peaked_module(cfg, seed):
     ((16, 1, 192, 128), 1, 31, (1, 1, 8), 512, "sigmoid", False, 32),        # the first block completes with the first token
     ((32, 2, 128, 128), 8, 1999, (1, 1), 130, "sigmoid", True, 32),
     ((8, 4, 64, 64), 2, 6000, (1, 4, 3), 64, "sigmoid", False, 32),          # two heads per group; more candidates than one pass
-    ((12, 2, 64, 64), 1, 700, (4, 1), 200, "sigmoid", False, 64),            # six heads per group; a block overlaps three others
+    ((8, 2, 64, 64), 1, 700, (4, 1), 200, "sigmoid", False, 64),             # a block overlaps three others on either side
 ])
 def test_decode_kernels_match_the_tile_kernels(monkeypatch, heads, B, cached, news, w, gate, bias, l):
     """A handful of tokens through the decode kernels against the same call through the tile kernels: the chosen blocks and what
@@ -137,6 +137,8 @@ def test_decode_kernels_match_the_tile_kernels(monkeypatch, heads, B, cached, ne
     real, score = I.ops.decode_fwd, I.ops.score_topn
 
     def with_ids(d, dev):
+        if d.indices:
+            return real(d, dev)
         ids.append(torch.empty(d.B, d.G, d.Tn, d.n, device=dev, dtype=torch.int32))
         d.indices = ids[-1].data_ptr()
         real(d, dev)
@@ -495,7 +497,7 @@ def test_block_choice_in_the_smaller_scratch(monkeypatch, pos):
     from nsa import incremental as I, ops
     from nsa.kernels import nsa_layer
     H, G, T = 16, 8, 7201
-    cfg = nsa.NSAConfig(d_model=64, head_dim_qk=64, head_dim_v=64, n_heads=H, n_kv_groups=G, w=128)
+    cfg = nsa.NSAConfig(d_model=64, head_dim_qk=64, head_dim_v=64, n_heads=H, n_kv_groups=G, w=128, n=4)      # (few slots: the choice's scratch is the largest)
     inp = O.make_inputs(1, H, G, pos + T, 64, 64, 64, 32, seed=T, block_offset_std=0.5, dtype=torch.bfloat16)
     q, k, v = (inp[x].to(DEV, torch.bfloat16) for x in ("q", "k", "v"))
     phi = tuple(getattr(inp["phi"], n_).to(DEV) for n_ in ("pos_embed", "w1", "b1", "w2", "b2"))
