@@ -75,6 +75,27 @@ def test_keys_and_values_read_as_slices_of_a_longer_buffer(Tk, lo):
     assert max_abs(o.float(), ref) < 2e-2
 
 
+@pytest.mark.parametrize("dk,dv,G,B", [(192, 128, 4, 1), (192, 128, 4, 8), (128, 128, 2, 2), (64, 64, 2, 1)])
+def test_appended_blocks_are_those_of_the_copies(dk, dv, G, B, monkeypatch):
+    """One block at a time and many: the compressed keys rank blocks, so they are the same bit for bit on either route."""
+    import nsa
+    from nsa import incremental as I
+    cfg = nsa.NSAConfig(d_model=64, head_dim_qk=dk, head_dim_v=dv, n_heads=G * 4, n_kv_groups=G)
+    gen = torch.Generator(device=DEV).manual_seed(B)
+    rn = lambda *s_: torch.randn(*s_, generator=gen, device=DEV).bfloat16()
+    phi = (rn(32, 32), rn(2 * dk, dk + 32), rn(2 * dk), rn(dk, 2 * dk), rn(dk))
+    a, b = (I.NSACache(cfg, B, 1200, DEV, shared_kv=True) for _ in range(2))
+    for Tn in (32, 16, 1, 15, 17, 31, 48, 1, 700, 16):
+        k, v = rn(B, G, dk, Tn), rn(B, G, Tn, dv)
+        a.append(phi, k, v)
+        with monkeypatch.context() as mp:
+            mp.setattr(I.NSACache, "_append_in_place", lambda *x: False)
+            b.append(phi, k, v)
+    assert a.n_blocks == b.n_blocks == (877 - 32) // 16 + 1
+    for name in ("k_cmp", "k_cmp_lp", "v_cmp"):
+        assert torch.equal(getattr(a, name), getattr(b, name)), name
+
+
 def _rows_close(got, want, tol, what):
     """Relative 2-norm of the difference, row by row."""
     got, want = got.double().cpu(), want.double().cpu()
