@@ -2,9 +2,11 @@
 // not take by default (lengths that are no whole tiles, few compressed blocks, slices of longer buffers).
 //
 // Those calls used to run on the stride-generic FMA kernels, which hold P and dS in fp32 (a bf16 step of 1000 tokens took 27 ms
-// there, 207 ms before they were tiled; 3.8 ms here).  Products of bf16 inputs are exact on the tensor cores; P and dS enter their second
-// product as a bf16 pair hi + lo whose sum carries 16 mantissa bits, so nothing is held in 16 bits and the bf16 results round
-// alike.  (tcgen05 would need a second P tile in TMEM, which the backward kernels have no columns for.)  64 x 64 tiles, four
+// there, 207 ms before they were tiled; 3.95 ms here).  Products of bf16 inputs are exact on the tensor cores; P and dS enter their
+// second product as three bf16 terms whose sum is the fp32 value, so nothing is held in 16 bits and the bf16 results round alike:
+// from 301 to 1920 tokens the outputs' error against 64 bits is that of the FMA kernels to 2e-7 of itself, the gradients' to 1e-3
+// either way.  (Two terms, 16 bits, took 3.84 ms, their outputs 8e-7 more.  tcgen05 would need the further P tiles in TMEM, which
+// the backward kernels have no columns for.)  64 x 64 tiles, four
 // warps of 16 rows (forward, dQ) or 16 keys (dK/dV: S^T, so that P^T and dS^T are A operands where they lie in registers); two
 // CTAs per SM overlap one's loads with the other's products.  Bound by the mma.sync pipe and its ldmatrix traffic.
 //
@@ -45,20 +47,22 @@ __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint3
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// two values -> bf16 pair hi and the pair of what rounding left, lo
-__device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t& lo) {
+// the leading bf16 pair of two values, which keep what rounding left
+__device__ __forceinline__ uint32_t take2(float& x, float& y) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
   const float2 f = __bfloat1622float2(h);
-  const __nv_bfloat162 l = __floats2bfloat162_rn(x - f.x, y - f.y);
-  hi = *reinterpret_cast<const uint32_t*>(&h);
-  lo = *reinterpret_cast<const uint32_t*>(&l);
+  x -= f.x;
+  y -= f.y;
+  return *reinterpret_cast<const uint32_t*>(&h);
 }
-// C fragments of two neighbouring 8-column tiles -> A fragment of the 16-wide k step they span
-__device__ __forceinline__ void split_frag(const float (&c0)[4], const float (&c1)[4], uint32_t (&hi)[4], uint32_t (&lo)[4]) {
-  split2(c0[0], c0[1], hi[0], lo[0]);
-  split2(c0[2], c0[3], hi[1], lo[1]);
-  split2(c1[0], c1[1], hi[2], lo[2]);
-  split2(c1[2], c1[3], hi[3], lo[3]);
+// C fragments of two neighbouring 8-column tiles -> A fragments of the 16-wide k step they span: three terms of 8 bits, the
+// whole value (fp32 has 24; the differences are exact)
+__device__ __forceinline__ void split_frag(const float (&c0)[4], const float (&c1)[4], uint32_t (&t)[3][4]) {
+  float x[8] = {c0[0], c0[1], c0[2], c0[3], c1[0], c1[1], c1[2], c1[3]};
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) t[j][i] = take2(x[2 * i], x[2 * i + 1]);
 }
 
 // lane offsets (elements) of the four ldmatrix address patterns; see the fragment layouts of mma.m16n8k16
@@ -142,17 +146,18 @@ __device__ __forceinline__ void second_product(float (&acc)[2 * N2][4], const fl
   if (!guard) {
 #pragma unroll
     for (int kk = 0; kk < KK; ++kk) {
-      uint32_t hi[4], lo[4];
-      split_frag(w[2 * kk], w[2 * kk + 1], hi, lo);
+      uint32_t t[3][4];
+      split_frag(w[2 * kk], w[2 * kk + 1], t);
 #pragma unroll
       for (int nn = 0; nn < N2; ++nn) {
         uint32_t bf[4];
         if (trans) ldsm4t(bf, smem_addr(mat + (k0 + kk * 16) * ld + nn * 16 + pat_a(lane, ld)));      // mat [k][n]
         else ldsm4(bf, smem_addr(mat + nn * 16 * ld + k0 + kk * 16 + pat_at(lane, ld)));               // mat [n][k]
-        mma(acc[2 * nn], hi, bf[0], bf[1]);
-        mma(acc[2 * nn], lo, bf[0], bf[1]);
-        mma(acc[2 * nn + 1], hi, bf[2], bf[3]);
-        mma(acc[2 * nn + 1], lo, bf[2], bf[3]);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          mma(acc[2 * nn], t[j], bf[0], bf[1]);
+          mma(acc[2 * nn + 1], t[j], bf[2], bf[3]);
+        }
       }
     }
     return;
