@@ -121,7 +121,10 @@ __global__ void gate_mix_fwd_bf16x4_kernel(const float* __restrict__ logits, con
 // A block owns 16 heads x kMixRows consecutive tokens, half a warp a head: its loads go out together, and the 12 bytes a row has of
 // dlogits [B,T,3H] make whole sectors.  Memory bound: 64 heads x 65536 x 128 went from 1.64 ms, walking the tokens of one head, to
 // 1.36 ms (5.5 TB/s); two tokens in flight without this order gained nothing (1.72 ms).
+// Head counts that are no multiple of 16 are walked in (token pair, head) order, so that every half-warp has a row: 4 heads x 65536 x
+// 128 take 80 us (178 with the other half-warps idle, 97 a head's tokens at a time), 8 x 32768 82 (109, 98), 20 x 16384 100 (126, 119).
 constexpr int kMixRows = 2;
+__host__ __device__ inline int mix_heads(int H) { return H % 16 == 0 ? 16 : H; }      // heads that a run of blocks walks
 __global__ void __launch_bounds__(256) gate_mix_bwd_bf16x4_kernel(const float* __restrict__ gates, const __nv_bfloat16* __restrict__ oc,
                                            const __nv_bfloat16* __restrict__ os, const __nv_bfloat16* __restrict__ ow,
                                            const __nv_bfloat16* __restrict__ dout, __nv_bfloat16* __restrict__ doc,
@@ -129,14 +132,14 @@ __global__ void __launch_bounds__(256) gate_mix_bwd_bf16x4_kernel(const float* _
                                            int B, int H, int T_, int dv, int mode, float* __restrict__ delta, int dout_tm) {
   const int lane = threadIdx.x & 31, hl = lane & 15;
   const int64_t rows = (int64_t)B * H * T_;
-  const int nhb = (H + 15) / 16, ntb = (T_ + kMixRows - 1) / kMixRows, g16 = blockIdx.x / ntb, b = g16 / nhb;
-  const int h = (g16 - b * nhb) * 16 + (threadIdx.x >> 4), t0 = (blockIdx.x - g16 * ntb) * kMixRows;
+  const int hb = mix_heads(H), nhb = H / hb, ntb = (T_ + kMixRows - 1) / kMixRows, per = (ntb * hb + 15) / 16, grp = blockIdx.x / per, b = grp / nhb;
+  const int i = (blockIdx.x - grp * per) * 16 + (threadIdx.x >> 4), tb = i / hb, h = (grp - b * nhb) * hb + i - tb * hb, t0 = tb * kMixRows;
   int64_t row[kMixRows], dbase[kMixRows];
   bool live[kMixRows];
   float g[kMixRows][3], d[kMixRows][3];
 #pragma unroll
   for (int k = 0; k < kMixRows; ++k) {
-    live[k] = h < H && t0 + k < T_;      // (both halves stay for the shuffles)
+    live[k] = t0 + k < T_;      // (both halves stay for the shuffles)
     const int hh = live[k] ? h : 0, t = live[k] ? t0 + k : 0;
     row[k] = ((int64_t)b * H + hh) * T_ + t;
     dbase[k] = mixed_row(row[k], b, hh, t, H, T_, dout_tm) * dv;
@@ -236,7 +239,7 @@ extern "C" NSA_API int nsa_gate_mix_bwd_delta(const float* gates, const void* o_
                                                       (const float*)dout, (float*)do_cmp, (float*)do_slc, (float*)do_win,
                                                       dlogits, B, H, T, dv, gate_mode, delta, dout_tm);
   else if (dtype == NSA_BF16 && dv % 128 == 0)
-    gate_mix_bwd_bf16x4_kernel<<<(unsigned)((int64_t)B * ((H + 15) / 16) * ((T + kMixRows - 1) / kMixRows)), 256, 0, st>>>(gates, (const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)o_slc,
+    gate_mix_bwd_bf16x4_kernel<<<(unsigned)((int64_t)B * (H / mix_heads(H)) * (((T + kMixRows - 1) / kMixRows * mix_heads(H) + 15) / 16)), 256, 0, st>>>(gates, (const __nv_bfloat16*)o_cmp, (const __nv_bfloat16*)o_slc,
                                                      (const __nv_bfloat16*)o_win, (const __nv_bfloat16*)dout, (__nv_bfloat16*)do_cmp,
                                                      (__nv_bfloat16*)do_slc, (__nv_bfloat16*)do_win, dlogits, B, H, T, dv, gate_mode, delta, dout_tm);
   else if (dtype == NSA_BF16)

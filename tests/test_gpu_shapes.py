@@ -416,7 +416,7 @@ def test_block_scores_from_the_forward_match_the_scoring_kernel(dk, dv, H, G, T,
         assert torch.equal(got.sort(-1).values, want.sort(-1).values)
 
 
-@pytest.mark.parametrize("rows,dv", [((1, 2, 33), 128), ((2, 3, 21), 64), ((1, 1, 1), 128)])
+@pytest.mark.parametrize("rows,dv", [((1, 2, 33), 128), ((2, 3, 21), 64), ((1, 1, 1), 128), ((2, 20, 7), 128), ((1, 32, 5), 256)])
 def test_row_kernels_at_any_row_count(rows, dv):
     """Rows that do not fill a warp's share: gate/mix backward with its row sums, against the formulas."""
     from nsa import ops
