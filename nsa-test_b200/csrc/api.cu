@@ -120,6 +120,18 @@ static bool mma_bwd_ok(const AttnArgs& a, const int64_t* s, int mode, int flags,
   return true;
 }
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+// backward of such a call; its row sums dO.O go to `scratch` where that has room
+static size_t row_sum_bytes(int64_t rows) { return 2 * (((size_t)rows * sizeof(float) + 255) & ~size_t(255)); }
+static int launch_mma_bwd(AttnArgs a, int mode, void* scratch, size_t bytes, cudaStream_t st) {
+  const int64_t rows = (int64_t)a.B * a.H * a.Tq;
+  if (scratch && bytes >= row_sum_bytes(rows) && rows > 0) {
+    float* D = (float*)scratch;
+    launch_bwd_prep(a.o_in, a.dout, a.Lc, a.Mc, nullptr, D, (float*)((char*)scratch + row_sum_bytes(rows) / 2), rows, a.dv, st);
+    if (int rc = check_launch("attn_bwd_mma row sums")) return rc;
+    a.row_sums = D;
+  }
+  return launch_attn_mma(a, mode, true, st);
+}
 
 // canonical contiguous gradients: dq like q, dk [B,G,Tk,dk], dv [B,G,Tk,dv]
 static bool tensor_core_bwd_ok(const int64_t* s, int flags, int dtype, int B, int H, int G, int Tq, int Tk, int dk, int dv,
@@ -260,8 +272,7 @@ extern "C" NSA_API int nsa_sliding_bwd(const void* q, const void* k, const void*
   a.q = q; a.k = k; a.v = v; a.o_in = out; a.dout = dout; a.Lc = L; a.Mc = M; a.dq = dq; a.dk_out = dkey; a.dv_out = dval;
   fill_bwd_strides(a, strides);
   a.B = B; a.H = H; a.G = G; a.Tq = T; a.Tk = T; a.dk = dk; a.dv = dv; a.window = window; a.scale = scale; a.causal = 1;
-  a.row_delta = row_delta;
-  if (mma_bwd_ok(a, strides, kWin, flags, dtype)) return launch_attn_mma(a, kWin, true, (cudaStream_t)stream);
+  if (mma_bwd_ok(a, strides, kWin, flags, dtype)) return launch_mma_bwd(a, kWin, workspace, workspace_bytes, (cudaStream_t)stream);
   return launch_attn_generic(a, kWin, dtype, true, (cudaStream_t)stream);
 }
 
@@ -359,8 +370,7 @@ extern "C" NSA_API int nsa_cmp_attn_bwd(const void* q, const void* k_cmp, const 
   a.dq = dq; a.dk_out = dk_cmp; a.dv_out = dv_cmp;
   fill_bwd_strides(a, strides);
   a.B = B; a.H = H; a.G = G; a.Tq = T; a.Tk = NB; a.dk = dk; a.dv = dv; a.scale = scale; a.causal = 1;
-  a.row_delta = row_delta;
-  if (mma_bwd_ok(a, strides, kCmp, flags, dtype)) return launch_attn_mma(a, kCmp, true, (cudaStream_t)stream);
+  if (mma_bwd_ok(a, strides, kCmp, flags, dtype)) return launch_mma_bwd(a, kCmp, workspace, workspace_bytes, (cudaStream_t)stream);
   return launch_attn_generic(a, kCmp, dtype, true, (cudaStream_t)stream);
 }
 
@@ -433,7 +443,8 @@ extern "C" NSA_API size_t nsa_slc_bwd_workspace_bytes(int B, int H, int G, int T
   if (B <= 0 || G <= 0 || Tq <= 0 || Tkv <= 0 || n_slots <= 0 || l_prime <= 0) return 256;
   if (slc_sized_tc(flags, Tkv) && dtype == NSA_BF16 && slc_sm100_supported(H, G, Tq, Tkv, dk, dv, n_slots, l_prime))
     return slc_bwd_sm100_workspace_bytes(B, H, G, Tq, Tkv, dk, dv, n_slots, l_prime);
-  return slc_csr_workspace_bytes(B, G, Tq, Tkv, n_slots, l_prime);
+  const size_t csr = slc_csr_workspace_bytes(B, G, Tq, Tkv, n_slots, l_prime);
+  return want_tc(flags) && dtype == NSA_BF16 && attn_mma_supported(dk, dv, kSlc, l_prime) ? csr + row_sum_bytes((int64_t)B * H * Tq) : csr;
 }
 
 extern "C" NSA_API int nsa_slc_bwd(const void* q, const void* k, const void* v, const int32_t* indices, const void* out,
@@ -470,8 +481,10 @@ extern "C" NSA_API int nsa_slc_bwd(const void* q, const void* k, const void* v, 
   if (int rc = build_slc_csr(indices, a.sidx, B, G, Tq, Tkv, n_slots, l_prime, 1, 0, workspace, workspace_bytes,
                              &a.csr_off, &a.csr_t, st))
     return rc;
-  a.row_delta = row_delta;
-  if (int rc = mma_bwd_ok(a, strides, kSlc, flags, dtype) ? launch_attn_mma(a, kSlc, true, st) : launch_attn_generic(a, kSlc, dtype, true, st)) return rc;
+  const size_t csr = slc_csr_workspace_bytes(B, G, Tq, Tkv, n_slots, l_prime);      // (a multiple of 256; build_slc_csr asked for it)
+  if (int rc = mma_bwd_ok(a, strides, kSlc, flags, dtype) ? launch_mma_bwd(a, kSlc, (char*)workspace + csr, workspace_bytes - csr, st)
+                                                          : launch_attn_generic(a, kSlc, dtype, true, st))
+    return rc;
   if (add0 || add1) {
     const int64_t n = (int64_t)B * H * Tq * dk;
     const unsigned blocks = (unsigned)((n + 255) / 256);

@@ -15,7 +15,7 @@ struct AttnArgs {
   // backward
   const void *o_in, *dout;
   const float *Lc, *Mc;
-  const float* row_delta;  // row sums dO.O [B,H,Tq] when the caller has them (mma family only), else null
+  const float* row_sums;   // attn_mma.cu: dO.O [B,H,Tq] of these very tensors, or null (formed where they are needed)
   void *dq, *dk_out, *dv_out;
   // masks
   const int* block_ends;  // kCmp: [Tk]

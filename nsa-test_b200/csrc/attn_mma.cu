@@ -2,10 +2,10 @@
 // not take by default (lengths that are no whole tiles, few compressed blocks, slices of longer buffers).
 //
 // Those calls used to run on the stride-generic FMA kernels, which hold P and dS in fp32 (a bf16 step of 1000 tokens took 27 ms
-// there, 207 ms before they were tiled; 3.95 ms here).  Products of bf16 inputs are exact on the tensor cores; P and dS enter their
+// there, 207 ms before they were tiled; 3.98 ms here).  Products of bf16 inputs are exact on the tensor cores; P and dS enter their
 // second product as three bf16 terms whose sum is the fp32 value, so nothing is held in 16 bits and the bf16 results round alike:
 // from 301 to 1920 tokens the outputs' error against 64 bits is that of the FMA kernels to 2e-7 of itself, the gradients' to 1e-3
-// either way.  (Two terms, 16 bits, took 3.84 ms, their outputs 8e-7 more.  tcgen05 would need the further P tiles in TMEM, which
+// either way.  (Two terms, 16 bits, take 0.1 ms less, their outputs are 8e-7 further off.  tcgen05 would need the further P tiles in TMEM, which
 // the backward kernels have no columns for.)  64 x 64 tiles, four
 // warps of 16 rows (forward, dQ) or 16 keys (dK/dV: S^T, so that P^T and dS^T are A operands where they lie in registers); two
 // CTAs per SM overlap one's loads with the other's products.  Bound by the mma.sync pipe and its ldmatrix traffic.
@@ -116,12 +116,15 @@ __device__ __forceinline__ void load_kv(const MmaSmem<DK, DV>& s, const AttnArgs
 __device__ __forceinline__ void load_rows(__nv_bfloat16* dst, const __nv_bfloat16* base, int64_t row, int D, int r) {   // one row by one warp
   for (int c = (threadIdx.x & 31) * 8; c < D; c += 256) cp16(dst + r * (D + 8) + c, row < 0 ? base : base + row * D + c, row >= 0);
 }
-// row statistics of the backward: log-sum-exp (+inf: no such row, or it saw nothing) and dO.O, by one warp
+// Row statistics of the backward: log-sum-exp (+inf: no such row, or it saw nothing) and dO.O, by one warp.  dO.O is of the bf16 dO
+// that dP is formed from: taken from a caller who has it of dO before that rounding, dS = P (dP - dO.O) no longer adds up to zero
+// over a row, and the compression weights' gradients, sums in which that cancels, were off by up to twice as much.  A pass of its
+// own forms it where the scratch has room (a key tile's rows are read by up to 16 tiles: 5.46 ms a step of 1000 tokens without).
 template <int DK, int DV>
 __device__ __forceinline__ void load_stats(const MmaSmem<DK, DV>& s, const AttnArgs& a, int r, int t, int64_t row) {
   const int lane = threadIdx.x & 31;
   float d = 0.f;
-  if (t >= 0 && !a.row_delta) {
+  if (t >= 0 && !a.row_sums) {
     const __nv_bfloat16 *o = (const __nv_bfloat16*)a.o_in + row * DV, *g = (const __nv_bfloat16*)a.dout + row * DV;
     for (int c = lane * 2; c < DV; c += 64) {
       const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(o + c)), y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(g + c));
@@ -132,7 +135,7 @@ __device__ __forceinline__ void load_stats(const MmaSmem<DK, DV>& s, const AttnA
   if (lane == 0) {
     float lse = t >= 0 ? a.Mc[row] + a.Lc[row] : CUDART_INF_F;
     s.lse[r] = isfinite(lse) ? lse : CUDART_INF_F;
-    s.del[r] = t >= 0 && a.row_delta ? a.row_delta[row] : d;
+    s.del[r] = t >= 0 && a.row_sums ? a.row_sums[row] : d;
     s.t[r] = t;
   }
 }

@@ -73,6 +73,10 @@ int fa_bwd_sm100(const void* q, const void* k, const void* v, const void* o, con
                  int mode, int window, int cmp_l, int cmp_d, int cmp_nb, float scale, const float* row_delta,
                  const KvLayout& kv, void* workspace, size_t workspace_bytes, cudaStream_t st);
 
+// row sums dO.O (D; or copied from `delta`) and log-sum-exp in log2 units (+inf: the row saw nothing) of contiguous bf16 rows, dv = 64 or 128
+void launch_bwd_prep(const void* o, const void* dout, const float* L, const float* M, const float* delta, float* D, float* lse2,
+                     int64_t rows, int dv, cudaStream_t st);
+
 // bf16 row-major [rows, cols] matrix -> tensor map with box [box_rows, 64 columns], 128-byte swizzle
 // (rows `ld` elements apart; 0: contiguous)
 int make_tmap_bf16_2d(::CUtensorMap_st* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint64_t ld = 0);

@@ -1297,10 +1297,6 @@ int slc_fwd_sm100(const void* q, const void* k, const void* v, const int* indice
   return fail(NSA_ERR_UNSUPPORTED, "slc_fwd_sm100: unsupported head dims");
 }
 
-// prep kernel shared with the dense backward (defined in fa_bwd_sm100.cu)
-void launch_bwd_prep(const void* o, const void* dout, const float* L, const float* M, const float* delta, float* D, float* lse2,
-                     int64_t rows, int dv, cudaStream_t st);
-
 static void slc_bwd_layout(int B, int H, int G, int Tq, int Tk, int dk, int dv, int nslots, int lprime, size_t* o_stat,
                            size_t* o_dq, size_t* o_dk, size_t* o_dv, size_t* o_qt, size_t* o_dot, size_t* total) {
   const size_t rows = (size_t)B * H * Tq;

@@ -549,3 +549,26 @@ def test_scratch_falls_back_where_memory_runs_out():
     from nsa import ops
     ws, n_ = ops._scratch(torch.device(DEV), 1 << 46, lambda: 1000)
     assert n_ == ws.numel() == 1000
+
+
+@pytest.mark.parametrize("dk,dv,H,G,T", [(64, 64, 4, 2, 100), (192, 128, 16, 1, 637)])
+def test_compressed_gradients_of_ragged_calls_add_up_to_zero(dk, dv, H, G, T):
+    """A constant added to every compressed key leaves the softmax alone, so dK_cmp adds up to zero over the blocks but for the
+    rounding of its entries, the output's in dO.O and dO's.  Given the gate backward's row sums, which are of the gradient before its rounding,
+    a call must not be further off than one that forms them itself (as the FMA kernels do)."""
+    from nsa import ops
+    q, k, v, dout = (t.to(DEV) for t in _inputs(1, H, G, T, dk, dv, seed=T))
+    nb = (T - 32) // 16 + 1
+    kc, vc = k[..., :nb].contiguous(), v[:, :, :nb].contiguous()
+    pad = (0, -nb % 8)
+    kc, vc = torch.nn.functional.pad(kc, pad), torch.nn.functional.pad(vc, (0, 0, *pad))
+    ends = torch.full((kc.shape[-1],), 999999, device=DEV, dtype=torch.int32)
+    ends[:nb] = torch.arange(nb, device=DEV, dtype=torch.int32) * 16 + 31
+    o, L, M = ops.cmp_attn_fwd(q, kc, vc, ends, dk ** -0.5)
+    gates = torch.rand(1, H, T, 3, device=DEV)
+    d_cmp, _, _, _, delta = ops.gate_mix_bwd(gates, o, o, o, dout, "sigmoid", want_delta=True)
+    off = []
+    for kw in (dict(row_delta=delta[0]), dict(generic=True)):
+        _, dkc, _ = ops.cmp_attn_bwd(q, kc, vc, ends, o, d_cmp, L, M, dk ** -0.5, **kw)
+        off.append(dkc.float().sum(2).norm().item())
+    assert off[0] <= 1.15 * off[1], off
