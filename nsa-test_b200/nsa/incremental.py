@@ -8,8 +8,16 @@ corresponding rows of the full-sequence forward.  Forward only, no autograd.
 ``NSACache`` keeps, per layer, the three key/value streams of the module (selection, sliding window and the
 source of the compression), zero-padded to a fixed capacity, and the compressed keys/values, which grow by
 one block every ``d`` tokens once ``l`` tokens are there.  ``nsa_layer_incremental`` runs the scoring/top-n,
-the three branches and the gate mix for the new rows with a query position offset; the kernels work on
-128-row query tiles, so the new rows are padded to a tile with rows that are computed and dropped.
+the three branches and the gate mix for the new rows with a query position offset, for bf16 calls in one library
+call:
+
+* up to 64 (sequence, group, token) rows on the decode kernels (``nsa_decode_fwd``; ``module_forward_incremental``
+  hands it the hidden states of up to eight tokens, whose projections and cache update then run in the same call);
+* more rows on the layer's own tile kernels, which read the caches where they lie (``nsa_incremental_fwd``).
+
+Everything else (other types, head dims or block sizes) is composed here from the branch entry points, on new rows
+padded to a 128-row tile and key slices copied out of the cache.  Both one-call forms choose the blocks that this
+composition chooses for the same rows, bit for bit: the choice is made from the same products and sums in the same order.
 """
 from __future__ import annotations
 
@@ -224,14 +232,17 @@ def _decode_module(module, x: torch.Tensor, cache: NSACache):
     d.project, d.nb_new, d.d_model, d.d_gate, d.U = 1, nb - cache.n_blocks, dm, D2, U
     if not _lib.lib.nsa_decode_supported(d):
         return None
-    # what the block choice depends on comes out of the products of the general path: rounded otherwise, near-ties would fall
-    # the other way
-    q, k_new = _project_heads(x, module.q_proj, H, dk), _project_heads(x, module.k_compress, G, dk, transposed=True)
-    if any(t.dtype != torch.bfloat16 or t.device != dev for t in (q, k_new)):
+    # What the block choice depends on comes out of the library's products, as on the general path: rounded otherwise, near-ties
+    # would fall the other way.  (One product for q of all sequences: for up to eight tokens it has the bits of one batched over the
+    # heads per sequence, at every one of 1176 shapes tried, and reads the weights once; eight of those took 115 us a token.)
+    q = torch.nn.functional.linear(x, module.q_proj.weight).view(B, Tn, H, dk)
+    if module.q_proj.bias is not None:
+        q = q + module.q_proj.bias.view(H, dk)
+    k_new = _project_heads(x, module.k_compress, G, dk, transposed=True)
+    if any(type(t) not in _PLAIN or t.dtype != torch.bfloat16 or t.device != dev for t in (q, k_new)):
         return None
-    q = q.contiguous()
     out = torch.empty(B, Tn, H * dv, device=dev, dtype=x.dtype)
-    d.q, d.sq, d.k_new, d.sk = q.data_ptr(), q.stride()[:3], k_new.data_ptr(), k_new.stride()
+    d.q, d.sq, d.k_new, d.sk = q.data_ptr(), (q.stride(0), q.stride(2), q.stride(1)), k_new.data_ptr(), k_new.stride()
     d.x, d.sx, d.out = x.data_ptr(), x.stride()[:2], out.data_ptr()
     d.w, d.bias = tuple(ptrs[:5]), tuple(ptrs[5:10])
     ops.decode_fwd(d, dev)

@@ -207,6 +207,20 @@ def test_decode_kernels_match_the_tile_kernels(monkeypatch, heads, B, cached, ne
     _rows_close(out, mix, 2 ** -8, "out")
 
 
+@pytest.mark.parametrize("dm,H,dk", [(2560, 64, 192), (2048, 32, 128), (512, 8, 64), (8192, 8, 64), (64, 48, 128)])
+def test_queries_of_a_few_tokens_from_one_product(dm, H, dk):
+    """The decode path forms q of all sequences with one product, the general path with one batched over the heads per sequence:
+    the block choice wants the same bits of both."""
+    from nsa.kernels import _project_heads
+    lin = torch.nn.Linear(dm, H * dk, bias=False, device=DEV, dtype=torch.bfloat16)
+    gen = torch.Generator(device=DEV).manual_seed(dm)
+    with torch.no_grad():
+        for B, Tn in ((1, 1), (1, 3), (1, 8), (2, 1), (5, 1), (8, 1), (3, 2), (2, 4)):
+            x = torch.randn(B, Tn + 2, dm, generator=gen, device=DEV).bfloat16()[:, 1:1 + Tn]
+            one = torch.nn.functional.linear(x, lin.weight).view(B, Tn, H, dk).transpose(1, 2)
+            assert torch.equal(one, _project_heads(x, lin, H, dk)), (B, Tn)
+
+
 @pytest.mark.parametrize("B,G,hpg,dk,dv,cached", [(8, 4, 16, 192, 128, 32000), (1, 4, 16, 192, 128, 2100), (2, 2, 16, 128, 128, 60000), (4, 2, 4, 64, 64, 9001)])
 def test_decoded_rows_choose_the_tile_paths_blocks(monkeypatch, B, G, hpg, dk, dv, cached):
     """Long caches, where the n-th and the next block of some rows agree to 1e-7: ids bit for bit, over queries enough to meet such
