@@ -45,12 +45,16 @@ enum {
   NSA_ERR_UNSUPPORTED = -4 /* shape outside what the requested kernel family covers */
 };
 
-/* `flags` argument of the attention and scoring entry points (testing / cross-checks): by default a call runs the
- * tensor-core (tcgen05) kernels when it qualifies (bf16, canonical contiguous layouts, supported head dims, T a
- * multiple of 128) and the stride-generic kernels otherwise; NSA_FLAG_GENERIC forces the stride-generic kernels. */
-/* NSA_FLAG_ANY_LENGTH lets the tensor-core kernels, which round probabilities and dS to bf16 for their second products, take
- * lengths that are no whole tiles and keys / values that are slices of longer buffers; without it such calls run on
- * kernels that hold both in 32 bits.  The whole layer sets it for bf16 sequences of 2048 tokens and more. */
+/* `flags` argument of the attention and scoring entry points.  By default a call runs on one of three kernel families:
+ *   tcgen05   bf16, canonical layouts, head dims (192,128), (128,128) or (64,64), an even number of heads per group, whole tensors
+ *             whose lengths are whole tiles (128; 64 for the selection's keys).  P and dS are rounded to bf16 for their second products.
+ *   mma.sync  the attention calls of the same types, layouts and head dims at any other length, and on slices of longer buffers
+ *             (rows of keys a multiple of 8 elements apart): P and dS enter their second products as three bf16 terms, all 24
+ *             bits.
+ *   generic   everything else: any strides, fp32 or bf16, head dims up to 256; 32-bit FMAs throughout.
+ * NSA_FLAG_GENERIC forces the generic family (cross-checks).  NSA_FLAG_ANY_LENGTH lets the tcgen05 family take the mma.sync
+ * family's calls; the whole layer sets it for bf16 sequences of 2048 tokens and more, the cache path always.
+ * NSA_FLAG_RECOMPUTE (workspace sizes only): see nsa_attn_bwd_workspace_bytes. */
 enum { NSA_FLAG_GENERIC = 1, NSA_FLAG_RECOMPUTE = 2, NSA_FLAG_ANY_LENGTH = 4 };
 
 /* `q_pos0` argument (query-sharded long-context runs and incremental decoding; the reference has no counterpart, its
@@ -60,7 +64,7 @@ enum { NSA_FLAG_GENERIC = 1, NSA_FLAG_RECOMPUTE = 2, NSA_FLAG_ANY_LENGTH = 4 };
  *
  * `row_delta` argument of the backward entry points: the row sums dO . O [B,H,T] (fp32, contiguous) when the caller
  * has them already (nsa_gate_mix_bwd_delta writes them), else NULL and the call computes them (the reference computes
- * them inside its backward kernels, nsa/kernels.py:1004-1010).  Used by the tensor-core paths.
+ * them inside its backward kernels, nsa/kernels.py:1004-1010).  Used by the tcgen05 family; the others form them from dout.
  *
  * `dq_add0/dq_add1` of nsa_slc_bwd: dQ of the other two branches (same dtype and contiguous [B,H,T,dk] layout as dq,
  * either may be NULL); the call then writes dq = dq_selection + dq_add0 + dq_add1, summed in fp32 and rounded once (the
@@ -149,15 +153,22 @@ NSA_API int nsa_sliding_bwd_noalloc(const void* q, const void* k, const void* v,
  * block_ends[i] == i*blocks_d + blocks_l - 1 for i < blocks_n and that later blocks are never
  * visible, which lets the tensor-core kernels skip tiles; blocks_d == 0 makes no assumption.
  * Replaces _nsa_compression_fwd_kernel / _bwd_kernel (nsa/kernels.py:1533-1687, 1690-1917). */
-/* Exact-key form (k_cmp_lo and lse2_out both non-NULL; bf16 tensor-core path only, nsa_cmp_attn_exact_supported tells
+/* Exact-key form of nsa_cmp_attn_fwd (k_cmp_lo and lse2_out both non-NULL; bf16 tensor-core path only, nsa_cmp_attn_exact_supported tells
  * for a shape, and the call needs the block layout hint, canonical layouts and L, M): k_cmp is the bf16 rounding of the
  * fp32 compressed keys and k_cmp_lo [B,G,dk,NB] the bf16 rounding of the remainder (nsa_split_keys_hi_lo makes both);
  * the logits are q (k_cmp + k_cmp_lo), i.e. those of the fp32 keys to 16 mantissa bits, and lse2_out [B,H,T] fp32
  * receives their log-sum-exp in log2 units (+inf for rows that see no block).  That is the normaliser of Eq. 8, so
  * nsa_score_topn given it as cmp_lse2 skips its own first sweep over the compressed keys. */
+NSA_API int nsa_cmp_attn_exact_supported(int B, int H, int G, int T, int NB, int dk, int dv, int dtype);
+NSA_API int nsa_split_keys_hi_lo(const float* x, void* hi, void* lo, int64_t n, void* stream);
+NSA_API int nsa_cmp_attn_fwd(const void* q, const void* k_cmp, const void* v_cmp, const int32_t* block_ends,
+                     void* out, float* L, float* M, const int64_t* strides22, int B, int H, int G,
+                     int T, int NB, int dk, int dv, float scale, int dtype, int blocks_l, int blocks_d,
+                     int blocks_n, int q_pos0, int flags, const void* k_cmp_lo, float* lse2_out, void* stream);
 /* The exact-key form of the compressed attention and the Eq. 8-11 block choice in one call (k_cmp: the fp32 keys whose halves
  * k_hi, k_lo [B,G,dk,ld] are; arguments otherwise as for nsa_cmp_attn_fwd and nsa_score_topn): where the scratch it asks for
- * holds them, the forward leaves the sums of its probabilities and the choice only adds those up. */
+ * holds them, the forward leaves the sums of its probabilities and the choice only adds those up.  A workspace of
+ * nsa_score_topn_workspace_bytes is enough too: the scoring kernel then makes the same choice. */
 NSA_API size_t nsa_cmp_attn_topn_workspace_bytes(int B, int H, int G, int T, int NB, int dk, int dv, int l, int d, int l_prime,
                                                  int n, int n_real_blocks, int flags);
 NSA_API int nsa_cmp_attn_topn_fwd(const void* q, const void* k_hi, const void* k_lo, const float* k_cmp, const void* v_cmp,
@@ -165,12 +176,6 @@ NSA_API int nsa_cmp_attn_topn_fwd(const void* q, const void* k_hi, const void* k
                                   int32_t* indices_out, const int64_t* strides, int B, int H, int G, int T, int NB, int nbp,
                                   int dk, int dv, int l, int d, int l_prime, int n, int n_fixed, int n_real_blocks,
                                   float scale, int q_pos0, int flags, void* workspace, size_t workspace_bytes, void* stream);
-NSA_API int nsa_cmp_attn_exact_supported(int B, int H, int G, int T, int NB, int dk, int dv, int dtype);
-NSA_API int nsa_split_keys_hi_lo(const float* x, void* hi, void* lo, int64_t n, void* stream);
-NSA_API int nsa_cmp_attn_fwd(const void* q, const void* k_cmp, const void* v_cmp, const int32_t* block_ends,
-                     void* out, float* L, float* M, const int64_t* strides22, int B, int H, int G,
-                     int T, int NB, int dk, int dv, float scale, int dtype, int blocks_l, int blocks_d,
-                     int blocks_n, int q_pos0, int flags, const void* k_cmp_lo, float* lse2_out, void* stream);
 NSA_API int nsa_cmp_attn_bwd(const void* q, const void* k_cmp, const void* v_cmp, const int32_t* block_ends,
                      const void* out, const void* dout, const float* L, const float* M, void* dq,
                      void* dk_cmp, void* dv_cmp, const int64_t* strides34, int B, int H, int G, int T,

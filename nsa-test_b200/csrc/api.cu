@@ -100,7 +100,8 @@ static bool canonical_fwd(const int64_t* s, int B, int H, int G, int Tq, int Tk,
   if (s[6] != 1 || kv->k_ld < Tk || kv->k_ld % 8 != 0 || (G > 1 && s[5] != dk * kv->k_ld) || (B > 1 && s[4] != G * dk * kv->k_ld)) return false;
   return s[11] == 1 && s[10] == dv && kv->v_plane >= (int64_t)Tk * dv && kv->v_plane % 8 == 0 && (B == 1 || s[8] == G * kv->v_plane);
 }
-// Without NSA_FLAG_ANY_LENGTH: whole tiles of whole tensors only, everything else keeps fp32 probabilities (generic kernels).
+// Without NSA_FLAG_ANY_LENGTH: whole tiles of whole tensors only, everything else keeps fp32 probabilities (attn_mma.cu where its
+// layouts and head dims allow, the generic kernels otherwise).
 static bool length_ok(int flags, int Tq, int q_tile, int Tk, int k_tile, int dv, const KvLayout& kv) {
   return (flags & NSA_FLAG_ANY_LENGTH) || (Tq % q_tile == 0 && Tk % k_tile == 0 && kv.k_ld == Tk && kv.v_plane == (int64_t)Tk * dv);
 }

@@ -2,11 +2,11 @@
 // not take by default (lengths that are no whole tiles, few compressed blocks, slices of longer buffers).
 //
 // Those calls used to run on the stride-generic FMA kernels, which hold P and dS in fp32 (a bf16 step of 1000 tokens took 27 ms
-// there, 207 ms before they were tiled; 3.98 ms here).  Products of bf16 inputs are exact on the tensor cores; P and dS enter their
-// second product as three bf16 terms whose sum is the fp32 value, so nothing is held in 16 bits and the bf16 results round alike:
-// from 301 to 1920 tokens the outputs' error against 64 bits is that of the FMA kernels to 2e-7 of itself, the gradients' to 1e-3
-// either way.  (Two terms, 16 bits, take 0.1 ms less, their outputs are 8e-7 further off.  tcgen05 would need the further P tiles in TMEM, which
-// the backward kernels have no columns for.)  64 x 64 tiles, four
+// there, 207 ms before they were tiled; 3.98 ms here).  Products of bf16 inputs are exact on the tensor cores; P and dS enter
+// their second product as three bf16 terms whose sum is the fp32 value, so nothing is held in 16 bits and the bf16 results
+// round alike: from 301 to 1920 tokens the outputs' error against 64 bits is that of the FMA kernels to 2e-7 of itself, the
+// gradients' to 1e-3 either way.  (Two terms, 16 bits, take 0.1 ms less, their outputs are 8e-7 further off.  tcgen05 would need
+// the further P tiles in TMEM, which the backward kernels have no columns for.)  64 x 64 tiles, four
 // warps of 16 rows (forward, dQ) or 16 keys (dK/dV: S^T, so that P^T and dS^T are A operands where they lie in registers); two
 // CTAs per SM overlap one's loads with the other's products.  Bound by the mma.sync pipe and its ldmatrix traffic.
 //

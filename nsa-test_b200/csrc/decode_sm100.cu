@@ -2,10 +2,10 @@
 // block choice, the three attention branches and the gate mix, for up to 64 (sequence, group, token) rows.
 //
 // The tile kernels pad such a call to 128 query rows and need an inverse index, padded copies and one launch per piece:
-// 45 launches and 760 us per token at B=1, 2K cached; 80 launches and 1400 us at B=8, 32K.  What the work
-// cannot do without is reading the weights once (131 MB for the 64-head configuration, 20 us) and the visible keys and values
-// once, so here the keys of a row are cut into 64-key chunks, one CTA each, that serve all heads of the group, and everything
-// between two grid-wide dependencies is one launch:
+// 45 launches and 760 us per token at B=1, 2K cached; 80 launches and 1400 us at B=8, 32K (137 and 167 us here).
+// What the work cannot do without is reading the weights once (131 MB for the 64-head configuration, 20 us) and the visible
+// keys and values once, so here the keys of a row are cut into 64-key chunks, one CTA each, that serve all heads of the group,
+// and everything between two grid-wide dependencies is one launch:
 //   1 project     weights x tokens on mma.sync (8 tokens are one n tile; the weights stream through once), written straight
 //                 into the caches; the gate MLP's hidden layer is one more row range
 //   2 phi         only when the tokens complete compression blocks: the block compression of every other path
@@ -17,9 +17,9 @@
 //
 // The block choice is a discrete function of rounded sums: q and the compression's keys that round differently, or sums in
 // another order, let near-ties fall the other way (in 2 of 384 rows at 32000 cached tokens).  So all that the choice reads is
-// made as on the other paths: q and the new compression keys come from the caller, who forms them with the products that the tile kernels'
-// callers use; logits are one fma chain over the head dimension and the Eq. 8-10 sums run in the order of score_topn.cu.  The
-// chosen blocks are the same bit for bit.
+// made as on the other paths: q and the new compression keys come from the caller, who forms them with the products that the
+// tile kernels' callers use; logits are one fma chain over the head dimension and the Eq. 8-10 sums run in the order of
+// score_topn.cu.  The chosen blocks are the same bit for bit.
 //
 // Keys of the compressed blocks stay fp32 and their products run on the FMA pipe (they rank the blocks); bf16 keys and P V run
 // on mma.sync, with P as bf16 hi + lo, so the probabilities keep 16 mantissa bits (the tile kernels: 8).  (tcgen05 tiles have 64
