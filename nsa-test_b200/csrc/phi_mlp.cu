@@ -418,6 +418,8 @@ int nsa::cmp_phi_bwd_ld(const void* k, int64_t k_ld, const float* pos_embed, con
   }
   if (int rc = check_launch("cmp_phi_bwd")) return rc;
   const bool fused = phi_pool_bwd_fused_ok(l, d);
+  // (the scratch is laid out by arows: T padded to 8, which makes no further 16-token segment)
+  NSA_REQUIRE(!fused || phi_pool_bwd_parts(BG, T) == wl.parts, "cmp_phi_bwd: %d rows for a sequence of %d", arows, T);
   int rc_pool;
   if (!fused) rc_pool = nsa_phi_pool_bwd(a, c, dhbar, dvc, da, dcpart, dvt, B, G, T, U, dv, l, d, nb, nbp, st);
   else if (dtype == NSA_BF16)

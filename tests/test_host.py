@@ -193,6 +193,7 @@ def test_compression_backward_scratch_covers_its_column_sums(BG, dk, dv):
         nb, nb_rows = (T - l) // d + 1, (rows - l) // d + 1
         nbp = 1 << (nb - 1).bit_length()
         nseg = -(-rows // 16)
+        assert nseg == -(-T // 16)        # the pooling kernel walks the segments of T, the scratch holds those of the padded rows
         parts = -(-nseg // max(4, -(-nseg * BG // 296)))
         others = [BG * nb_rows * dk * 4, BG * nb_rows * U * 4, BG * nbp * dv * 4, BG * rows * U * 2, parts * BG * l * U * 4, l * U * 4, U * dk * 2]
         reserved = lib.nsa_cmp_phi_workspace_bytes(1, BG, rows, dk, dv, l, d, U, nbp, BF16, 1) - 256 - sum(map(al, others))
